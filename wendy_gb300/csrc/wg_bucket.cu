@@ -61,16 +61,16 @@ constexpr int BIGBINS = 4096;
 constexpr int CHUNK = CAP / 2;
 constexpr int kMaxChunks = kBucketCapBig / CHUNK + 1;
 // Two 16-bit bin counters (later offsets) per 32-bit word: bin b lives in the
-// half (b & 1) of word b / 2.  Words are padded with one per 32 so that a
-// thread scanning 16 consecutive words and its 31 neighbours hit 32
-// different banks.
+// half (b & 1) of word b / 2.  The scan takes each thread's consecutive words
+// with 16-byte loads, so the words need no padding against bank conflicts
+// (a quarter warp's loads of 32-byte pieces conflict twice, not eight times).
 constexpr int NWORD = NBIN / 2;
-constexpr int NBIN_PAD = NWORD + NWORD / 32 + 1;
-__device__ __forceinline__ int binp(int w) { return w + (w >> 5); }
 // Offset (or count) of bin b in the packed words.
 __device__ __forceinline__ uint32_t bin_get(const uint32_t* bins, int b) {
-  return (bins[binp(b >> 1)] >> ((b & 1) << 4)) & 0xffffu;
+  return (bins[b >> 1] >> ((b & 1) << 4)) & 0xffffu;
 }
+// Cells of the routing table over a splitter window (see route_table).
+constexpr int LUTN = 256;
 
 struct LsdSmem {
   uint32_t q[2][CAP];
@@ -100,7 +100,7 @@ struct TaskMeta {
   uint64_t pm_lo, pm_hi;  // their fixed-point mass
 };
 
-struct StepSmem {
+struct __align__(16) StepSmem {
   double x[CAP];
   double v[CAP];
   double m[CAP];
@@ -108,10 +108,9 @@ struct StepSmem {
   uint16_t perm[CAP];  // sorted position -> slot
   union {
     struct {
-      uint32_t bins[NBIN_PAD];
-      uint64_t skey[CAP];  // key and index of each position in bin order
-      int32_t sidx[CAP];
-      uint32_t nlong;      // bins too full for one thread's insertion sort
+      uint32_t bins[NWORD + 4];         // (+ the offset past the last bin)
+      uint16_t shared_bin[WARPS][32 * MAXI];  // per warp: bins its sheets found occupied once
+      uint32_t nlong;                   // bins too full for their owner to order
     } srt;
     LsdSmem lsd;
     struct {
@@ -129,6 +128,8 @@ struct StepSmem {
   uint32_t dcount[2 * RWIN + 2];  // sheets bound for each window entry (+ outside the window)
   uint32_t dstart[2 * RWIN + 3];  // their exclusive prefix: segments of the grouped order
   uint32_t dbase[2 * RWIN + 2];   // first slot of each window bucket taken by this bucket
+  uint8_t lut[LUTN + 4];          // routing table over the window (route_table)
+  float lut_x0, lut_scale;
   unsigned next_ticket;              // the next task's ticket and entry, read ahead
   BucketTask next_tk;
   u128 warp_mass[WARPS];
@@ -278,121 +279,207 @@ __device__ __forceinline__ void lsd_sort(StepSmem& S, int n, uint64_t kmin, uint
   __syncthreads();
 }
 
-// Sort the n <= CAP sheets of the bucket by (key, idx) into S.perm, with
-// 2^qb bins (9 <= qb <= 13).  The bin words are zero on entry (cleared while
-// the bucket loads).
-__device__ __forceinline__ void bucket_sort(StepSmem& S, int n, int ipt, uint64_t kmin,
-                                            uint64_t kmax, int qb) {
-  const int tid = threadIdx.x;
-  const uint64_t span = kmax - kmin;
-  const int nbin = 1 << qb;
-  const int wpt = nbin / (2 * BT);  // bin words per thread in the scan (1..16)
-  // Bin of a key: (key - kmin) * scale / 2^64, which is non-decreasing in the
-  // key and spreads the bucket's key range over all nbin bins (a shift would
-  // leave up to half of them empty).  The scale is a single-precision
-  // reciprocal shrunk by 2^-20, so the largest key still lands below nbin;
-  // a range narrower than nbin keys maps one key per bin.
-  const bool narrow = span < (uint64_t)nbin;
-  uint64_t scale = 0;
-  if (!narrow) {
-    const float f = (float)nbin / ((float)span + 1.0f) * 18446744073709551616.0f *
-                    (1.0f - 9.5367431640625e-07f);
-    scale = (uint64_t)f;
+// The smallest and largest key of a warp: the upper halves first, then the
+// lower halves among the lanes that share the extreme upper half (four
+// warp-reduce instructions instead of five rounds of 64-bit shuffles).
+__device__ __forceinline__ uint64_t warp_min_u64(uint64_t k) {
+  const uint32_t hi = (uint32_t)(k >> 32);
+  const uint32_t h = __reduce_min_sync(0xffffffffu, hi);
+  const uint32_t l = __reduce_min_sync(0xffffffffu, hi == h ? (uint32_t)k : 0xffffffffu);
+  return ((uint64_t)h << 32) | l;
+}
+__device__ __forceinline__ uint64_t warp_max_u64(uint64_t k) {
+  const uint32_t hi = (uint32_t)(k >> 32);
+  const uint32_t h = __reduce_max_sync(0xffffffffu, hi);
+  const uint32_t l = __reduce_max_sync(0xffffffffu, hi == h ? (uint32_t)k : 0u);
+  return ((uint64_t)h << 32) | l;
+}
+
+// (key, idx) of the sheet in slot a precedes that of slot b.
+__device__ __forceinline__ bool slot_less(const StepSmem& S, uint64_t ka, int a, uint64_t kb,
+                                          int b) {
+  if (ka != kb) return ka < kb;
+  return S.idx[a] < S.idx[b];
+}
+
+// Puts the places [lo, hi) of one bin in (key, idx) order (one thread).  Up
+// to four sheets -- nearly every shared bin -- are ranked by comparing all
+// pairs, their loads in flight together; more by insertion.
+__device__ __forceinline__ void order_bin(StepSmem& S, uint32_t lo, uint32_t hi) {
+  const uint32_t c = hi - lo;
+  if (c <= 4) {
+    int p[4];
+    uint64_t k[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) p[a] = S.perm[lo + ((uint32_t)a < c ? (uint32_t)a : 0u)];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) k[a] = key_of(S.x[p[a]]);
+    uint32_t r[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = a + 1; b < 4; ++b)
+        if ((uint32_t)b < c) {
+          const bool ba = slot_less(S, k[b], p[b], k[a], p[a]);
+          r[a] += ba ? 1u : 0u;
+          r[b] += ba ? 0u : 1u;
+        }
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+      if ((uint32_t)a < c) S.perm[lo + r[a]] = (uint16_t)p[a];
+    return;
   }
+  for (uint32_t a = lo + 1; a < hi; ++a) {
+    const uint16_t pa = S.perm[a];
+    const uint64_t ka = key_of(S.x[pa]);
+    uint32_t b = a;
+    while (b > lo) {
+      const uint16_t pb = S.perm[b - 1];
+      if (!slot_less(S, ka, pa, key_of(S.x[pb]), pb)) break;
+      S.perm[b] = pb;
+      --b;
+    }
+    S.perm[b] = pa;
+  }
+}
+
+// Sort the n <= CAP sheets of the bucket by (key, idx) into S.perm, with
+// 2^qb bins (11 <= qb <= 13).  The bin words are zero on entry (cleared while
+// the bucket loads).  pre != 0: the opening half drift of a call, applied to
+// the positions on the way.
+// Returns false, having changed nothing, if some thread did not see the
+// sheets arrive.
+__device__ __forceinline__ bool bucket_sort(StepSmem& S, int n, int ipt, int qb, bool arrived,
+                                            double pre) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nbin = 1 << qb;
   uint32_t* bins = S.u.srt.bins;
-  uint64_t* skey = S.u.srt.skey;
-  int32_t* sidx = S.u.srt.sidx;
-  if (tid == 0) S.u.srt.nlong = 0;  // read after the barriers below
-  uint16_t qv[MAXI], rk[MAXI];
+  // ---- keys (held in registers until they are counted) and their range
+  uint64_t key[MAXI];
+  uint64_t kmin = ~0ull, kmax = 0;
 #pragma unroll
   for (int i = 0; i < MAXI; ++i) {
     const int j = tid + i * BT;
-    if (i < ipt && j < n) {
-      const uint64_t dk = key_of(S.x[j]) - kmin;
-      qv[i] = (uint16_t)(narrow ? dk : __umul64hi(dk, scale));
-      const int sh = (qv[i] & 1) << 4;
-      rk[i] = (uint16_t)(atomicAdd(&bins[binp(qv[i] >> 1)], 1u << sh) >> sh);
+    key[i] = 0;
+    if (arrived && i < ipt && j < n) {
+      double x = S.x[j];
+      if (pre != 0.0) {
+        x = fma(pre, S.v[j], x);
+        S.x[j] = x;
+      }
+      key[i] = key_of(x);
+      kmin = key[i] < kmin ? key[i] : kmin;
+      kmax = key[i] > kmax ? key[i] : kmax;
     }
   }
-  __syncthreads();
-  // exclusive scan of the bins: thread t owns words [wpt t, wpt t + wpt)
-  constexpr int WMAX = NWORD / BT;
-  uint32_t c[WMAX];
-  uint32_t run = 0, mx = 0;
-#pragma unroll
-  for (int k = 0; k < WMAX; ++k) {
-    c[k] = k < wpt ? bins[binp(tid * wpt + k)] : 0u;
-    const uint32_t lo = c[k] & 0xffffu, hi = c[k] >> 16;
-    mx = lo > mx ? lo : mx;
-    mx = hi > mx ? hi : mx;
-    run += lo + hi;
+  kmin = warp_min_u64(kmin);
+  kmax = warp_max_u64(kmax);
+  if (lane == 0) {
+    S.red_min[warp] = kmin;
+    S.red_max[warp] = kmax;
   }
-  const int too_full = __syncthreads_or(mx > (uint32_t)MAXBIN);
-  if (too_full) {
+  if (tid == 0) S.u.srt.nlong = 0;  // read after the barriers below
+  if (__syncthreads_or(!arrived)) return false;
+  kmin = warp_min_u64(S.red_min[lane & (WARPS - 1)]);
+  kmax = warp_max_u64(S.red_max[lane & (WARPS - 1)]);
+  // Bin of a key: the top 32 bits of its offset in the range, times scale /
+  // 2^32, which is non-decreasing in the key and spreads the bucket's key
+  // range over all nbin bins (a shift alone would leave up to half of them
+  // empty).  The scale is a single-precision quotient shrunk by 2^-20, so
+  // the largest key still lands below nbin; a range narrower than nbin keys
+  // maps one key per bin.
+  const uint64_t span = kmax - kmin;
+  const int ksh = (span >> 32) ? 32 - __clz((int)(uint32_t)(span >> 32)) : 0;
+  const uint32_t span32 = (uint32_t)(span >> ksh);
+  const bool narrow = span32 < (uint32_t)nbin;
+  const uint32_t scale =
+      narrow ? 0u
+             : (uint32_t)((float)nbin / ((float)span32 + 1.0f) * 4294967296.0f *
+                          (1.0f - 9.5367431640625e-07f));
+  uint16_t qv[MAXI], rk[MAXI];
+  uint32_t nshared = 0;  // this warp's entries of shared_bin
+  bool full = false;
+#pragma unroll
+  for (int i = 0; i < MAXI; ++i) {
+    if (i < ipt) {
+      const int j = tid + i * BT;
+      rk[i] = 0;
+      qv[i] = 0;
+      if (j < n) {
+        const uint32_t d = (uint32_t)((key[i] - kmin) >> ksh);
+        const uint32_t q = narrow ? d : __umulhi(d, scale);
+        const int sh = (int)(q & 1u) << 4;
+        qv[i] = (uint16_t)q;
+        rk[i] = (uint16_t)(atomicAdd(&bins[q >> 1], 1u << sh) >> sh);
+        full |= rk[i] >= MAXBIN;
+      }
+      // The order inside a bin comes from atomics.  A bin holds two or more
+      // sheets exactly when one of them took rank 1 in it: the bins found
+      // that way are listed per warp (a fifth as many as sheets), so that
+      // ordering them below takes each lane about one bin.
+      const unsigned sm = __ballot_sync(0xffffffffu, rk[i] == 1);
+      if (rk[i] == 1)
+        S.u.srt.shared_bin[warp][nshared + __popc(sm & lanemask_lt())] = qv[i];
+      nshared += __popc(sm);
+    }
+  }
+  if (__syncthreads_or(full)) {
     lsd_sort(S, n, kmin, kmax);
-    return;
+    return true;
+  }
+  // exclusive scan of the bins: thread t owns w4 groups of four words
+  const int w4 = nbin / (8 * BT);  // 1, 2 or 4
+  uint4* const b4 = reinterpret_cast<uint4*>(bins) + tid * w4;
+  uint32_t run = 0;
+  for (int k = 0; k < w4; ++k) {
+    const uint4 c = b4[k];
+    const uint32_t s = c.x + c.y + c.z + c.w;
+    run += (s & 0xffffu) + (s >> 16);
   }
   uint32_t total;
   uint32_t off = block_excl_scan(S, run, total);
-#pragma unroll
-  for (int k = 0; k < WMAX; ++k) {
-    const uint32_t lo = c[k] & 0xffffu, hi = c[k] >> 16;
-    if (k < wpt) bins[binp(tid * wpt + k)] = off | ((off + lo) << 16);
-    off += lo + hi;
+  for (int k = 0; k < w4; ++k) {
+    uint4 c = b4[k];
+    // a word (lo, hi) becomes (off, off + lo)
+    uint32_t t = c.x;
+    c.x = off * 0x10001u + (t << 16);
+    off += (t & 0xffffu) + (t >> 16);
+    t = c.y;
+    c.y = off * 0x10001u + (t << 16);
+    off += (t & 0xffffu) + (t >> 16);
+    t = c.z;
+    c.z = off * 0x10001u + (t << 16);
+    off += (t & 0xffffu) + (t >> 16);
+    t = c.w;
+    c.w = off * 0x10001u + (t << 16);
+    off += (t & 0xffffu) + (t >> 16);
+    b4[k] = c;
   }
-  if (tid == 0) bins[binp(nbin >> 1)] = (uint32_t)n;  // offset of bin nbin
+  if (tid == 0) bins[nbin >> 1] = (uint32_t)n;  // offset of bin nbin
   __syncthreads();
 #pragma unroll
   for (int i = 0; i < MAXI; ++i) {
     const int j = tid + i * BT;
-    if (i < ipt && j < n) {
-      const uint32_t pos = bin_get(bins, qv[i]) + rk[i];
-      S.perm[pos] = (uint16_t)j;
-      skey[pos] = key_of(S.x[j]);
-      sidx[pos] = S.idx[j];
-    }
+    if (i < ipt && j < n) S.perm[bin_get(bins, qv[i]) + rk[i]] = (uint16_t)j;
   }
   __syncthreads();
-  // The order inside a bin came from atomics.  A bin holds two or more
-  // sheets exactly when one of them took rank 1 in it: that sheet puts the
-  // bin's few places in (key, idx) order, an insertion sort of their keys,
-  // indices and slots in shared memory; every other sheet has nothing to do.
-  // Bins of more than kOwnerSort sheets (rare) are counted and then ordered by
-  // the whole block, each of their sheets counting the bin-mates that precede
-  // it (owners never touch those bins).
+  // the shared bins, each ordered by one lane of the warp that listed it; bins
+  // of more than kOwnerSort sheets (rare) are counted and then ordered by the
+  // whole block (owners never touch those bins)
   constexpr uint32_t kOwnerSort = 8;
-#pragma unroll
-  for (int i = 0; i < MAXI; ++i) {
-    const int j = tid + i * BT;
-    if (i < ipt && j < n && rk[i] == 1) {
-      const uint32_t lo = bin_get(bins, qv[i]), hi = bin_get(bins, qv[i] + 1);
-      if (hi - lo <= kOwnerSort) {
-        for (uint32_t a = lo + 1; a < hi; ++a) {
-          const uint64_t ka = skey[a];
-          const int32_t ia = sidx[a];
-          const uint16_t pa = S.perm[a];
-          uint32_t b = a;
-          while (b > lo && pair_less(ka, ia, skey[b - 1], sidx[b - 1])) {
-            skey[b] = skey[b - 1];
-            sidx[b] = sidx[b - 1];
-            S.perm[b] = S.perm[b - 1];
-            --b;
-          }
-          skey[b] = ka;
-          sidx[b] = ia;
-          S.perm[b] = pa;
-        }
-      } else {
-        atomicAdd(&S.u.srt.nlong, 1u);
-      }
-    }
+  for (uint32_t e = (uint32_t)lane; e < nshared; e += 32) {
+    const int q = S.u.srt.shared_bin[warp][e];
+    const uint32_t lo = bin_get(bins, q), hi = bin_get(bins, q + 1);
+    if (hi - lo <= kOwnerSort)
+      order_bin(S, lo, hi);
+    else
+      atomicAdd(&S.u.srt.nlong, 1u);
   }
   __syncthreads();
-  if (S.u.srt.nlong == 0) return;
+  if (S.u.srt.nlong == 0) return true;
   // the full bins: each of their sheets counts the sheets of its bin that
-  // precede it, then takes that place (keys and indices read-only here)
+  // precede it, then takes that place (slots read-only here)
   uint32_t place[MAXI];
-  uint16_t slot[MAXI];
 #pragma unroll
   for (int i = 0; i < MAXI; ++i) {
     place[i] = 0xffffffffu;
@@ -400,20 +487,22 @@ __device__ __forceinline__ void bucket_sort(StepSmem& S, int n, int ipt, uint64_
     if (i < ipt && j < n) {
       const uint32_t lo = bin_get(bins, qv[i]), hi = bin_get(bins, qv[i] + 1);
       if (hi - lo > kOwnerSort) {
-        const uint64_t kj = skey[lo + rk[i]];
-        const int32_t ij = sidx[lo + rk[i]];
+        const uint64_t kj = key_of(S.x[j]);
         uint32_t r = 0;
-        for (uint32_t b = lo; b < hi; ++b) r += pair_less(skey[b], sidx[b], kj, ij) ? 1u : 0u;
+        for (uint32_t b = lo; b < hi; ++b) {
+          const int sb = S.perm[b];
+          r += slot_less(S, key_of(S.x[sb]), sb, kj, j) ? 1u : 0u;
+        }
         place[i] = lo + r;
-        slot[i] = (uint16_t)j;
       }
     }
   }
   __syncthreads();
 #pragma unroll
   for (int i = 0; i < MAXI; ++i)
-    if (place[i] != 0xffffffffu) S.perm[place[i]] = slot[i];
+    if (place[i] != 0xffffffffu) S.perm[place[i]] = (uint16_t)(tid + i * BT);
   __syncthreads();
+  return true;
 }
 
 // Bucket of the next layout covering (k, i): the largest j with Q_j <= (k, i).
@@ -624,66 +713,108 @@ __device__ __forceinline__ void claim_task(const StepLaunch& L, int sub, unsigne
   prepare_task(L, sub, ep, lane, t, tk, S, wbuf);
 }
 
+// Inverse of key_of (of the canonical key: +0 for the zeros), in single
+// precision; the ends of the key range saturate.
+__device__ __forceinline__ float float_of_key(uint64_t k) {
+  const uint64_t b = (k >> 63) ? (k & 0x7FFFFFFFFFFFFFFFull) : ~k;
+  return (float)__longlong_as_double((long long)b);
+}
+
+// Cell of a position in the routing table.  Every step (rounding to single
+// precision, subtraction, product with a non-negative scale, truncation,
+// clamping) is non-decreasing, so a splitter in a lower cell than a position
+// lies below it, whatever the rounding.
+__device__ __forceinline__ int lut_cell(float x, float x0, float scale) {
+  return (int)fminf(fmaxf((x - x0) * scale, 0.f), (float)(LUTN - 1));
+}
+
+// Routing table over the splitter window [lo, hi] of the next layout (wlen =
+// hi - lo buckets): lut[c] is the largest window entry whose splitter lies in
+// a cell below c, so the entry of a position in cell c is one of lut[c] ..
+// lut[c + 1] -- one or two candidates where the window's splitters are spread
+// over the cells, against the six or seven rounds of a search of the window.
+// Cells are cut in position, not in key, space (keys are logarithmic about
+// zero).  Threads 0 .. wlen - 1; a barrier must follow before its use.
+__device__ __forceinline__ void route_table(StepSmem& S, const uint64_t* wk, int lo, int hi,
+                                            int64_t nb) {
+  const int j = threadIdx.x, wlen = hi - lo;
+  if (j >= wlen) return;
+  // the first and last finite splitters of the window
+  const int j0 = lo == 0 ? 1 : 0, j1 = hi == (int)nb ? wlen - 1 : wlen;
+  float x0 = 0.f, scale = 0.f;
+  if (j1 > j0) {
+    x0 = float_of_key(wk[j0]);
+    const float w = float_of_key(wk[j1]) - x0;
+    if (w > 1e-30f && w < 1e30f) scale = (float)LUTN / w;
+  }
+  const int c0 = j == 0 ? -1 : lut_cell(float_of_key(wk[j]), x0, scale);
+  const int c1 = j == wlen - 1 ? LUTN : lut_cell(float_of_key(wk[j + 1]), x0, scale);
+  for (int c = c0 + 1; c <= c1; ++c) S.lut[c] = (uint8_t)j;
+  if (j == 0) {
+    S.lut_x0 = x0;
+    S.lut_scale = scale;
+  }
+}
+
+// Counting-sort bits of a simulation as the kernel uses them: at least four
+// bin words per thread.
+__device__ __forceinline__ int step_sort_bits(const SimDev& D) {
+  return D.sort_bits < 11 ? 11 : D.sort_bits;
+}
+__device__ __forceinline__ void clear_bins(StepSmem& S, int qb) {
+  uint4* const b4 = reinterpret_cast<uint4*>(S.u.srt.bins);
+  const int nw = 1 << (qb - 3);
+  for (int j = threadIdx.x; j < nw; j += BT) b4[j] = make_uint4(0u, 0u, 0u, 0u);
+}
+
 // Sort, scan, force, kick, drift, route and write out the n <= CAP sheets of
 // a bucket (or of one chunk of a big bucket) that sit in shared memory, with
-// their key range [kmin, kmax]; S.prefix_mass / S.prefix_cnt hold the
-// exclusive (mass, count) prefix of the first of them and the splitter window
-// of the next layout is in S.wkey[S.cur_wbuf].  PREP: warp 0 prepares the
-// next task (S.next_ticket, ntk) during the grouping, as the main kernel's
-// pipeline does; otherwise (chunks of a big bucket) the prefix base is
-// advanced past these sheets at the end.
+// their bins cleared; S.prefix_mass / S.prefix_cnt hold the exclusive (mass,
+// count) prefix of the first of them, the splitter window of the next layout
+// is in S.wkey[S.cur_wbuf] and its routing table in S.lut.  arrived: this
+// thread saw the sheets' copies complete; returns false, having done nothing,
+// if some thread did not.  pre: the opening half drift still to be applied.
+// PREP: warp 0 prepares the next task (ticket nt of thread 0) during the
+// grouping, as the main kernel's pipeline does; otherwise (chunks of a big
+// bucket) the prefix base is advanced past these sheets at the end.
 template <bool LAST, bool EXPR, bool PREP>
-__device__ __forceinline__ void process_bucket(const StepLaunch& L, StepSmem& S, const SimDev& D,
+__device__ __forceinline__ bool process_bucket(const StepLaunch& L, StepSmem& S, const SimDev& D,
                                                const int64_t b, const int lay, const int n,
-                                               const int sub, const unsigned ep, uint64_t kmin,
-                                               uint64_t kmax, const BucketTask ntk) {
+                                               const int sub, const unsigned ep,
+                                               const bool arrived, const double pre,
+                                               const unsigned nt) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ipt = (n + BT - 1) / BT;
   const int E = D.E;
+  // ---- sort the bucket
+  if (!bucket_sort(S, n, ipt, step_sort_bits(D), arrived, pre)) return false;
+  BucketTask ntk{0, 0};
+  if (PREP && tid == 0 && nt < (unsigned)L.ntasks) ntk = L.tasks[nt];
   const uint64_t* const wk = S.wkey[S.cur_wbuf];
   const int32_t* const wi = S.widx[S.cur_wbuf];
-  // ---- sort the bucket
-  if (n > 1) {
-    bucket_sort(S, n, ipt, kmin, kmax, D.sort_bits);
-  } else {
-    if (tid == 0) S.perm[0] = 0;
-    __syncthreads();
-  }
 
   // ---- exact prefix of the masses in sorted order: thread tid holds the
   // sorted positions [tid * ipt, tid * ipt + ipt)
-  if (PREP && tid == 0) S.next_tk = ntk;
   const int j0 = tid * ipt;
   const int nmine = (j0 < n) ? ((n - j0) < ipt ? (n - j0) : ipt) : 0;
   u128 tot = 0;
+#pragma unroll 2
   for (int i = 0; i < nmine; ++i) {
     const u128 M = mass_to_fixed(S.m[S.perm[j0 + i]], E);
     S.u.pos.mfix[j0 + i] = M;
     tot += M;
   }
   const u128 incl = warp_inclusive_scan_u128(tot, lane);
-  uint32_t cin = (uint32_t)nmine;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, cin, o);
-    if (lane >= o) cin += y;
-  }
-  if (lane == 31) {
-    S.warp_mass[warp] = incl;
-    S.warp_cnt[warp] = cin;
+  if (lane == 31) S.warp_mass[warp] = incl;
+  if (PREP && tid == 0) {
+    S.next_ticket = nt;
+    S.next_tk = ntk;
   }
   __syncthreads();
   u128 C = S.prefix_mass;
-  uint32_t rank0 = S.prefix_cnt;
-#pragma unroll
-  for (int w = 0; w < WARPS; ++w) {
-    if (w < warp) {
-      C += S.warp_mass[w];
-      rank0 += S.warp_cnt[w];
-    }
-  }
+  for (int w = 0; w < warp; ++w) C += S.warp_mass[w];
   C += incl - tot;
-  rank0 += cin - (uint32_t)nmine;
+  const uint32_t rank0 = S.prefix_cnt + (uint32_t)j0;
 
   // ---- splitters of the layout after next: keys at global ranks j*T
   uint64_t* qnk = D.qk[1 - ((D.qsel0 + sub) & 1)];
@@ -715,7 +846,6 @@ __device__ __forceinline__ void process_bucket(const StepLaunch& L, StepSmem& S,
   const double dt = L.profile ? 0.0 : D.dt;
   const double dt_drift = LAST ? dt / 2. : dt;
   const double dest_dt = (LAST && !L.profile) ? dt / 2. : 0.0;
-  const i128 T = (i128)((((u128)D.T_hi) << 64) | D.T_lo);
   unsigned long long maxv = 0;
   StateTable* const ptab = D.ptab;  // predicted splitters this sub-step
 
@@ -724,15 +854,19 @@ __device__ __forceinline__ void process_bucket(const StepLaunch& L, StepSmem& S,
   uint32_t qnext = (rank0 + target - 1) / target;
   qnext = qnext ? qnext : 1u;
   const uint32_t rnext = qnext * target;
-  // two sheets at a time, interleaved, so that their shared-memory and
-  // FP64 latencies overlap; the window searches run in lock-step
   const int wlen = S.win_hi - S.win_lo;
-  int top = 1;
-  while ((top << 1) < wlen) top <<= 1;
+  const uint64_t wk_lo = wk[0], wk_hi = wk[wlen];
+  const float lut_x0 = S.lut_x0, lut_scale = S.lut_scale;
+  // the acceleration of the sheet at position j is A_j = T - 2 C_j - M_j with
+  // C_j the mass before it; from one sheet to the next A falls by M_j + M_j+1
+  i128 A = (i128)(((((u128)D.T_hi) << 64) | D.T_lo) - 2 * C);
+  // two sheets at a time, interleaved, so that their shared-memory and
+  // FP64 latencies overlap
   for (int i0 = 0; i0 < nmine; i0 += 2) {
     const bool ok1 = i0 + 1 < nmine;
     int sl[2];
     uint64_t kd[2];
+    float xf[2];
     int32_t idv[2];
     bool live[2] = {true, ok1};
 #pragma unroll
@@ -744,6 +878,7 @@ __device__ __forceinline__ void process_bucket(const StepLaunch& L, StepSmem& S,
     for (int u = 0; u < 2; ++u) {
       if (!live[u]) {
         kd[u] = 0;
+        xf[u] = 0.f;
         continue;
       }
       const int sidx = sl[u];
@@ -762,9 +897,9 @@ __device__ __forceinline__ void process_bucket(const StepLaunch& L, StepSmem& S,
         }
       }
       const u128 M = S.u.pos.mfix[j0 + i0 + u];
-      const i128 A = T - 2 * (i128)C - (i128)M;
-      C += M;
+      A -= (i128)M;
       double acc = fixed_to_double(A, E);
+      A -= (i128)M;
       if (has_omega) acc = fma(-omega2, x, acc);
       if constexpr (EXPR) {
         if (ext.kind == EXT_EXPR)
@@ -803,30 +938,40 @@ __device__ __forceinline__ void process_bucket(const StepLaunch& L, StepSmem& S,
           xi_out[r] = rec;
         }
       }
-      kd[u] = key_of(LAST && dest_dt != 0.0 ? fma(dest_dt, vn, xn) : xn);
+      const double xd = LAST && dest_dt != 0.0 ? fma(dest_dt, vn, xn) : xn;
+      kd[u] = key_of(xd);
+      xf[u] = (float)xd;
     }
-    // routing: binary lifting over the window, both sheets in lock-step
-    int l[2] = {0, 0};
-    bool inw[2];
+    // routing: the window entry among the table's candidates
+    int l[2], h[2];
 #pragma unroll
-    for (int u = 0; u < 2; ++u)
-      inw[u] = live[u] && win_ge(wk, wi, 0, kd[u], idv[u]) && !win_ge(wk, wi, wlen, kd[u], idv[u]);
-    // the largest l with key Q_l <= key, on keys alone; then splitters with
-    // an equal key and a larger index step back (pair order)
-    for (int step = top; step >= 1; step >>= 1) {
-#pragma unroll
-      for (int u = 0; u < 2; ++u)
-        if (l[u] + step < wlen && wk[l[u] + step] <= kd[u]) l[u] += step;
+    for (int u = 0; u < 2; ++u) {
+      const int c = lut_cell(xf[u], lut_x0, lut_scale);
+      l[u] = S.lut[c];
+      h[u] = S.lut[c + 1];
     }
-#pragma unroll
-    for (int u = 0; u < 2; ++u)
-      while (l[u] > 0 && wk[l[u]] == kd[u] && wi[l[u]] > idv[u]) --l[u];
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       if (!live[u]) continue;
-      // destination: window entry l, or wlen for a bucket outside the
-      // window (found again, by a global search, where it is needed)
-      const int w = inw[u] ? l[u] : wlen;
+      // strictly inside the window's keys; anything else (its ends included)
+      // is found by the search over all splitters where it is needed
+      const bool inw = kd[u] > wk_lo && kd[u] < wk_hi;
+      int w = wlen;
+      if (inw) {
+        // the largest entry with key Q <= key; then splitters with an equal
+        // key and a larger index step back (pair order)
+        int a = l[u], z = h[u];
+        while (a < z) {
+          const int mid = (a + z + 1) >> 1;
+          if (wk[mid] <= kd[u])
+            a = mid;
+          else
+            z = mid - 1;
+        }
+        while (a > 0 && wk[a] == kd[u] && wi[a] > idv[u]) --a;
+        w = a;
+      }
+      // destination: window entry w, or wlen for a bucket outside the window
       const int pq = j0 + i0 + u;
       S.u.pos.dw[pq] = (uint8_t)w;
       S.u.pos.drk[pq] = (uint16_t)atomicAdd(&S.dcount[w], 1u);
@@ -841,6 +986,8 @@ __device__ __forceinline__ void process_bucket(const StepLaunch& L, StepSmem& S,
     for (int o = 16; o >= 1; o >>= 1) vsum += __shfl_xor_sync(0xffffffffu, vsum, o);
     if (lane == 0) S.vsum[warp] = vsum;
   }
+  maxv = warp_max_u64(maxv);
+  if (lane == 0 && maxv) atomicMax(&S.maxv, maxv);
   __syncthreads();
   if (ptab && tid < (int)min(S.nsamp, 4u)) {
     // the sample's position moved on by two drifts at the bucket's mean
@@ -979,12 +1126,6 @@ __device__ __forceinline__ void process_bucket(const StepLaunch& L, StepSmem& S,
       }
     }
   }
-#pragma unroll
-  for (int d = 16; d >= 1; d >>= 1) {
-    const unsigned long long o = __shfl_xor_sync(0xffffffffu, maxv, d);
-    maxv = o > maxv ? o : maxv;
-  }
-  if (lane == 0 && maxv) atomicMax(&S.maxv, maxv);
   if (overflow) atomicCAS(D.ocount + 1, 0u, (unsigned)(sub + 1));
   __syncthreads();
   if (tid == 0 && S.maxv) atomicMax(&D.flags[sub + 1].max_v, S.maxv);
@@ -997,6 +1138,7 @@ __device__ __forceinline__ void process_bucket(const StepLaunch& L, StepSmem& S,
     S.prefix_mass += tot_all;
     S.prefix_cnt += (uint32_t)n;
   }
+  return true;
 }
 
 // Appends a big bucket's task to the list k_bucket_big works through (one
@@ -1092,40 +1234,15 @@ __global__ void __launch_bounds__(BT, 2) k_bucket_step(const StepLaunch L) {
       S.amp = tm.amp;
       S.inv_h = tm.inv_h;
     }
-    {
-      // counting-sort bins, cleared while the copies are in flight
-      for (int j = tid; j < NBIN_PAD; j += BT) S.u.srt.bins[j] = 0u;
-    }
+    // while the copies are in flight: the counting-sort bins are cleared and
+    // the routing table is made
+    clear_bins(S, step_sort_bits(D));
+    route_table(S, S.wkey[tm.wbuf], tm.wlo, tm.whi, D.nb);
     // the copies' completion: a thread that did not see it within the bounded
-    // wait leaves the data alone, and the barrier after the key range below
-    // (which every thread reaches) decides for the whole CTA
+    // wait leaves the data alone, and the first barrier of the sort (which
+    // every thread reaches) decides for the whole CTA
     const bool arrived = n4 > 0 ? mbar_wait(&S.mbar, parity) : true;
-    uint64_t kmin = ~0ull, kmax = 0;
-    if (arrived) {
-#pragma unroll 4
-      for (int j = tid; j < n; j += BT) {
-        double x = S.x[j];
-        if (pre != 0.0) {
-          x = fma(pre, S.v[j], x);
-          S.x[j] = x;
-        }
-        const uint64_t k = key_of(x);
-        kmin = k < kmin ? k : kmin;
-        kmax = k > kmax ? k : kmax;
-      }
-    }
-#pragma unroll
-    for (int d = 16; d >= 1; d >>= 1) {
-      const uint64_t o1 = __shfl_xor_sync(0xffffffffu, kmin, d);
-      const uint64_t o2 = __shfl_xor_sync(0xffffffffu, kmax, d);
-      kmin = o1 < kmin ? o1 : kmin;
-      kmax = o2 > kmax ? o2 : kmax;
-    }
-    if (lane == 0) {
-      S.red_min[warp] = kmin;
-      S.red_max[warp] = kmax;
-    }
-    if (__syncthreads_or(!arrived)) {
+    if (!process_bucket<LAST, EXPR, true>(L, S, D, b, lay, n, sub, ep, arrived, pre, nt)) {
       // the bucket's copies did not complete within the bounded wait: its
       // contents are unknown, so this CTA writes nothing more.  It gives the
       // copies a second bounded wait and stops; the host sees the error word
@@ -1135,19 +1252,6 @@ __global__ void __launch_bounds__(BT, 2) k_bucket_step(const StepLaunch L) {
       break;
     }
     if (n4 > 0) parity ^= 1u;
-    BucketTask ntk{0, 0};
-    if (tid == 0) {
-      S.next_ticket = nt;
-      if (nt < (unsigned)L.ntasks) ntk = L.tasks[nt];
-    }
-    kmin = ~0ull;
-    kmax = 0;
-#pragma unroll
-    for (int w = 0; w < WARPS; ++w) {
-      kmin = S.red_min[w] < kmin ? S.red_min[w] : kmin;
-      kmax = S.red_max[w] > kmax ? S.red_max[w] : kmax;
-    }
-    process_bucket<LAST, EXPR, true>(L, S, D, b, lay, n, sub, ep, kmin, kmax, ntk);
   }
 }
 
@@ -1244,6 +1348,8 @@ __global__ void __launch_bounds__(BT, 2) k_bucket_big(const StepLaunch L) {
       S.splittable = 1u;
       for (int c = 0; c <= kMaxChunks; ++c) S.chunk_lo[c] = BIGBINS;
     }
+    __syncthreads();
+    route_table(S, S.wkey[0], bt.wlo, bt.whi, D.nb);
     // ---- the bucket's key range and the histogram of its keys
     uint64_t kmin = ~0ull, kmax = 0;
     for (int j = tid; j < n; j += BT) {
@@ -1309,14 +1415,13 @@ __global__ void __launch_bounds__(BT, 2) k_bucket_big(const StepLaunch L) {
     // ---- the chunks in key order
     for (int ch = 0; ch < nchunks; ++ch) {
       const int blo = S.chunk_lo[ch], bhi = S.chunk_lo[ch + 1];
-      for (int j = tid; j < NBIN_PAD; j += BT) S.u.srt.bins[j] = 0u;
+      clear_bins(S, step_sort_bits(D));
       for (int j = tid; j <= S.win_hi - S.win_lo; j += BT) S.dcount[j] = 0;
       if (tid == 0) {
         S.load_cnt = 0;
         S.nsamp = 0;  // splitter samples of this chunk
       }
       __syncthreads();
-      uint64_t cmin = ~0ull, cmax = 0;
       for (int j = tid; j < n; j += BT) {
         const double x = big_pos(gx, gv, j, pre);
         const uint64_t k = key_of(x);
@@ -1328,20 +1433,17 @@ __global__ void __launch_bounds__(BT, 2) k_bucket_big(const StepLaunch L) {
             S.v[slot] = gv[j];
             S.m[slot] = gm[j];
             S.idx[slot] = gi[j];
-            cmin = k < cmin ? k : cmin;
-            cmax = k > cmax ? k : cmax;
           }
         }
       }
-      block_range(S, cmin, cmax);
+      __syncthreads();
       const int nc = (int)S.load_cnt;
       if (nc > CAP) {  // cannot happen with the chunk rule; never write past the arrays
         if (tid == 0) atomicOr(L.err, DEV_ERR_BAD_STATE);
         break;
       }
       if (nc == 0) continue;
-      process_bucket<LAST, EXPR, false>(L, S, D, bt.bucket, bt.lay, nc, sub, ep, cmin, cmax,
-                                        BucketTask{0, 0});
+      process_bucket<LAST, EXPR, false>(L, S, D, bt.bucket, bt.lay, nc, sub, ep, true, 0.0, 0u);
     }
   }
 }

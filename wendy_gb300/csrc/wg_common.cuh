@@ -50,7 +50,7 @@ __device__ __forceinline__ uint64_t key_of(double x) {
 // The acceleration totmass - 2 C_i - m_i (wendy/wendy.c:375-383) is formed
 // exactly in the integers and rounded to double once.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ u128 mass_to_fixed(double m, int E) {
+static __device__ __noinline__ u128 mass_to_fixed_slow(double m, int E) {
   uint64_t b = (uint64_t)__double_as_longlong(m);
   int ex = (int)((b >> 52) & 0x7FF);
   uint64_t mant = b & 0xFFFFFFFFFFFFFull;
@@ -67,12 +67,40 @@ __device__ __forceinline__ u128 mass_to_fixed(double m, int E) {
   return (u128)((mant + (1ull << (r - 1))) >> r);
 }
 
-// Signed 128-bit integer A times 2^-E, rounded to nearest even.  The normal
-// range is handled with integer operations only (FP64 issue slots are the
-// scarce resource on this part): the top 64 bits of |A| are normalised with
-// one count-leading-zeros, the mantissa is their top 53 bits and the rest
-// (plus a sticky bit for everything below) decides the rounding.  Values
-// below 2^64 units or outside the normal exponent range take ldexp.
+__device__ __forceinline__ u128 u128_of(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3) {
+  return ((u128)(((uint64_t)w3 << 32) | w2) << 64) | (((uint64_t)w1 << 32) | w0);
+}
+
+// The shift of a 53-bit mantissa to its place, in 32-bit words: shifted
+// inside its three words by funnel shifts, then set down at the word its
+// place begins in (a general 128-bit shift costs about twice as much).  A
+// mass of at least 2^-73 of the total needs no rounding and is never above
+// bit 124 (s <= 72); anything else takes the general conversion.
+__device__ __forceinline__ u128 mass_to_fixed(double m, int E) {
+  const uint32_t mh = (uint32_t)__double2hiint(m), ml = (uint32_t)__double2loint(m);
+  const int ex = (int)((mh >> 20) & 0x7FFu);
+  const int s = ex - 1075 + E;
+  if (ex == 0 || (unsigned)s > 72u) return mass_to_fixed_slow(m, E);
+  const uint32_t hi = (mh & 0xFFFFFu) | 0x100000u;
+  const int bs = s & 31;
+  const uint32_t a0 = ml << bs;
+  const uint32_t a1 = __funnelshift_l(ml, hi, bs);
+  const uint32_t a2 = __funnelshift_l(hi, 0u, bs);
+  const bool at1 = s >= 32, at2 = s >= 64;
+  const uint32_t w0 = at1 ? 0u : a0;
+  const uint32_t w1 = at2 ? 0u : at1 ? a0 : a1;
+  const uint32_t w2 = at2 ? a0 : at1 ? a1 : a2;
+  const uint32_t w3 = at2 ? a1 : at1 ? a2 : 0u;
+  return u128_of(w0, w1, w2, w3);
+}
+
+// Signed 128-bit integer A times 2^-E, rounded to nearest even.  The usual
+// range (|A| of at least 2^96 units, a normal result) is handled with 32-bit
+// integer operations only (FP64 issue slots are the scarce resource on this
+// part): |A| is normalised with one count-leading-zeros and four funnel
+// shifts, the mantissa is its top 53 bits, and the bits below (plus a sticky
+// bit) decide the rounding, whose carry may run into the exponent.  Smaller
+// |A| and results outside the normal range take ldexp.
 static __device__ __noinline__ double fixed_to_double_slow(i128 A, int E) {
   const bool neg = A < 0;
   const u128 u = neg ? (u128)(-A) : (u128)A;
@@ -104,27 +132,26 @@ static __device__ __noinline__ double fixed_to_double_slow(i128 A, int E) {
 }
 
 __device__ __forceinline__ double fixed_to_double(i128 A, int E) {
-  const bool neg = A < 0;
-  const u128 u = neg ? (u128)(-A) : (u128)A;
-  const uint64_t hi = (uint64_t)(u >> 64), lo = (uint64_t)u;
-  if (hi == 0) return fixed_to_double_slow(A, E);
-  const int lz = __clzll((long long)hi);
-  const uint64_t t = lz ? (hi << lz) | (lo >> (64 - lz)) : hi;  // top 64 bits
-  const uint64_t rest = lo << lz;                                  // bits below t
-  uint64_t mant = t >> 11;
-  const uint64_t r = t & 0x7FFull;
-  int bexp = 127 - lz - E + 1023;
-  if (r > 0x400ull || (r == 0x400ull && (rest != 0 || (mant & 1ull)))) {
-    ++mant;
-    if (mant == (1ull << 53)) {
-      mant >>= 1;
-      ++bexp;
-    }
-  }
-  if (bexp <= 0 || bexp >= 2047) return fixed_to_double_slow(A, E);
-  const uint64_t bits = ((uint64_t)bexp << 52) | (mant & 0xFFFFFFFFFFFFFull) |
-                        (neg ? 0x8000000000000000ull : 0ull);
-  return __longlong_as_double((long long)bits);
+  const uint32_t sign = (uint32_t)((uint64_t)((u128)A >> 64) >> 32) & 0x80000000u;
+  const u128 u = sign ? (u128)(-A) : (u128)A;
+  const uint64_t uh = (uint64_t)(u >> 64), ul = (uint64_t)u;
+  const uint32_t w3 = (uint32_t)(uh >> 32), w2 = (uint32_t)uh;
+  const uint32_t w1 = (uint32_t)(ul >> 32), w0 = (uint32_t)ul;
+  const int lz = __clz((int)w3);
+  const int bexp = 127 + 1023 - lz - E;  // biased exponent of the leading bit
+  if (w3 == 0u || (unsigned)(bexp - 1) > 2044u) return fixed_to_double_slow(A, E);
+  const uint32_t t3 = __funnelshift_l(w2, w3, lz);
+  const uint32_t t2 = __funnelshift_l(w1, w2, lz);
+  const uint32_t t1 = __funnelshift_l(w0, w1, lz);
+  const uint32_t t0 = w0 << lz;
+  const uint32_t lo = __funnelshift_r(t2, t3, 11);
+  // the leading bit (bit 20 of t3 >> 11) adds one to the exponent field
+  const uint32_t hi = ((uint32_t)(bexp - 1) << 20) + (t3 >> 11);
+  // the eleven bits below the mantissa at the top of a word, everything under
+  // them as a sticky bit: round up above half, and at half if odd
+  const uint32_t r = (t2 << 21) | ((t1 | t0) ? 1u : 0u);
+  const uint64_t bits = (((uint64_t)hi << 32) | lo) + ((r + (lo & 1u)) > 0x80000000u ? 1u : 0u);
+  return __longlong_as_double((long long)(bits | ((uint64_t)sign << 32)));
 }
 
 // ---------------------------------------------------------------------------
