@@ -331,6 +331,27 @@ void free_sim(wg_sim* s) {
   delete s;
 }
 
+// Sheets per bucket of a single simulation: the tuned target, unless its
+// buckets would leave resident CTAs of the sub-step kernel idle.  A launch
+// takes its buckets in rounds of `grid`; up to kBalanceRounds rounds the
+// buckets are sized to fill the last round too, since a round lasts about as
+// long however few of its CTAs have a bucket, and a bucket's time falls with
+// its sheets until its fixed part dominates (kMinTarget).  Measured per
+// sub-step, sech^2 disk, with targets of 1536 / 768 / 384 / 256 sheets: 39.4 /
+// 29.8 / 19.4 / 19.2 us at 1e4 sheets, 40.0 / 31.9 / 24.2 / 26.0 at 1e5, 43.3 /
+// 36.7 (one round) / 40.4 (two) / 50.7 at 3e5; at 1e6, 1280 (two rounds) 70.1 against
+// 1536 (two rounds, the second half empty) 77.5 and 1024 (three) 81.4.
+constexpr int kBalanceRounds = 4;
+constexpr int kMinTarget = 384;
+int balanced_target(int64_t n, int target, int grid) {
+  const int64_t rounds = (n + (int64_t)grid * target - 1) / ((int64_t)grid * target);
+  if (rounds > kBalanceRounds) return target;
+  int64_t t = (n + rounds * grid - 1) / (rounds * grid);
+  t = (t + 31) / 32 * 32;
+  if (t < kMinTarget) t = kMinTarget;
+  return t < target ? (int)t : target;
+}
+
 // Allocate a simulation for n sheets with the given physics; sheet data is
 // uploaded by the caller.
 int make_sim(int64_t n, double totmass, double omega2, const ExtSpec& ext, wg_sim** out,
@@ -403,6 +424,13 @@ int make_sim(int64_t n, double totmass, double omega2, const ExtSpec& ext, wg_si
   // bucket layout: two layouts of nb buckets x capacity, counts, splitters,
   // look-back records, the overflow list
   s->tune = tuning_for(n);
+  {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    s->grid_bucket = bucket_step_grid(sms, s->tune.ctas_per_sm);
+  }
+  s->tune.target = balanced_target(n, s->tune.target, s->grid_bucket);
   s->nb = (n + s->tune.target - 1) / s->tune.target;
   const int64_t nb = s->nb;
   // layouts with room for big buckets where asked for and where the memory
@@ -418,7 +446,9 @@ int make_sim(int64_t n, double totmass, double omega2, const ExtSpec& ext, wg_si
            al(8 * 4 * (size_t)(kEnergyBlocks + 1)) +
            (capg > kBucketCap ? al(sizeof(BigTask) * (size_t)nb) : 0);
   };
-  s->capg = big_buckets ? kBucketCapBig : kBucketCap;
+  // (a bucket of up to kBucketCap / 4 sheets has room for four times its
+  // target already: such layouts need no big buckets)
+  s->capg = big_buckets && 4 * s->tune.target > kBucketCap ? kBucketCapBig : kBucketCap;
   bucket_bytes(s->capg);
   e = cudaMalloc(&s->bk, bk_b);
   if (e != cudaSuccess && s->capg > kBucketCap) {
@@ -518,12 +548,6 @@ int make_sim(int64_t n, double totmass, double omega2, const ExtSpec& ext, wg_si
                       s->stream) != cudaSuccess) {
     set_error("memset failed");
     return fail(WG_ERR_CUDA);
-  }
-  {
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    s->grid_bucket = s->tune.ctas_per_sm * sms;
   }
   rc = alloc_call_arrays(s, 64);
   if (rc != WG_OK) return fail(rc);

@@ -51,7 +51,10 @@ constexpr int CAP = kBucketCap;     // 2048
 constexpr int MAXI = CAP / BT;      // 8 sheets per thread at most
 constexpr int WARPS = BT / 32;
 constexpr int RWIN = kSplitterWindow;
-constexpr int NBIN = 1 << kSortBitsMax;  // bins the shared memory is sized for
+constexpr int QB_MIN = 11, QB_MAX = 12;  // counting-sort bits the kernel uses
+constexpr int NBIN = 1 << QB_MAX;        // bins the shared memory is sized for
+constexpr int SHLIST = 64;               // shared bins a warp can list
+constexpr int CTAS = 3;                  // resident CTAs per SM
 constexpr int MAXBIN = 48;          // a fuller bin sends the bucket to the radix sort
 // Big buckets are cut into chunks of at most CAP sheets along 4096 key bins:
 // a chunk starts at every bin whose exclusive count passes a multiple of
@@ -71,11 +74,12 @@ __device__ __forceinline__ uint32_t bin_get(const uint32_t* bins, int b) {
 }
 // Cells of the routing table over a splitter window (see route_table).
 constexpr int LUTN = 256;
+// Sheets a thread takes at once through the force loop.
+constexpr int FU = 1;
 
 struct LsdSmem {
-  uint32_t q[2][CAP];
-  uint16_t p[2][CAP];
-  uint32_t hist[WARPS][256];
+  uint16_t p[CAP];           // the other slot permutation (S.perm is the first)
+  uint16_t hist[WARPS][256];
 };
 
 // What the processing of one task needs, prepared by warp 0 one task ahead
@@ -83,7 +87,7 @@ struct LsdSmem {
 // load waits only for its bulk copies and not for a chain of dependent global
 // reads, and its mass prefix is known before it starts.
 struct TaskMeta {
-  const double* x;
+  const double* x;  // the bucket's sheets
   const double* v;
   const double* m;
   const int32_t* idx;
@@ -108,18 +112,15 @@ struct __align__(16) StepSmem {
   uint16_t perm[CAP];  // sorted position -> slot
   union {
     struct {
-      uint32_t bins[NWORD + 4];         // (+ the offset past the last bin)
-      uint16_t shared_bin[WARPS][32 * MAXI];  // per warp: bins its sheets found occupied once
-      uint32_t nlong;                   // bins too full for their owner to order
+      uint32_t bins[NWORD + 4];              // (+ the offset past the last bin)
+      uint16_t shared_bin[WARPS][SHLIST];    // per warp: bins its sheets found occupied once
+      uint32_t nlong;                        // bins too full for their owner to order
     } srt;
     LsdSmem lsd;
-    struct {
-      u128 mfix[CAP];      // fixed-point mass of each sorted position
-      uint16_t drk[CAP];   // rank of each sorted position among the sheets of its destination
-      uint16_t order[CAP]; // sorted positions grouped by destination
-      uint8_t dw[CAP];     // destination of each sorted position: window entry, or the
-                           // window length for a bucket outside the window
-    } pos;
+    // destination (window entry << 16 | rank among its sheets) of each sorted
+    // position, then (window entry << 16 | slot) grouped by destination; the
+    // entry is the window length for a bucket outside the window
+    uint32_t dest[CAP];
   } u;
   // splitter windows of the next layout, double-buffered: the one of the
   // next task is read while the current task runs
@@ -129,11 +130,11 @@ struct __align__(16) StepSmem {
   uint32_t dstart[2 * RWIN + 3];  // their exclusive prefix: segments of the grouped order
   uint32_t dbase[2 * RWIN + 2];   // first slot of each window bucket taken by this bucket
   uint8_t lut[LUTN + 4];          // routing table over the window (route_table)
+  uint32_t cell_cnt[LUTN / 4];    // splitters of the window in each of its cells (bytes)
   float lut_x0, lut_scale;
   unsigned next_ticket;              // the next task's ticket and entry, read ahead
   BucketTask next_tk;
   u128 warp_mass[WARPS];
-  uint32_t warp_cnt[WARPS];
   uint32_t scan_tmp[WARPS];
   u128 prefix_mass;
   uint32_t prefix_cnt;
@@ -156,8 +157,15 @@ struct __align__(16) StepSmem {
   unsigned splittable;
 };
 
-// Two CTAs per SM: 228 KiB of shared memory per SM, 1 KiB reserved per CTA.
-static_assert(2 * (sizeof(StepSmem) + 1024) <= 228 * 1024, "StepSmem too large for 2 CTAs/SM");
+// CTAS CTAs per SM: 228 KiB of shared memory per SM, 1 KiB reserved per CTA.
+// Three (24 warps at 80 registers) rather than two with more of the work kept
+// in shared memory (fixed-point masses, 64-bit sort keys): the kernel is
+// bound by latency and issue, and the third CTA hides more of it than the
+// recomputed conversions cost.
+static_assert(CTAS * (sizeof(StepSmem) + 1024) <= 228 * 1024, "StepSmem too large");
+static_assert(LUTN == BT, "one routing-table cell per thread");
+// k_bucket_big keeps its histogram where its chunks' positions go later
+static_assert(sizeof(double) * CAP >= 4 * BIGBINS, "big-bucket histogram");
 
 __device__ __forceinline__ bool pair_less(uint64_t k1, int32_t i1, uint64_t k2, int32_t i2) {
   return k1 < k2 || (k1 == k2 && i1 < i2);
@@ -187,14 +195,9 @@ __device__ __forceinline__ uint32_t block_excl_scan(StepSmem& S, uint32_t v, uin
   return pre + incl - v;
 }
 
-// Barrier of warps 1 .. WARPS-1 only (named barrier 1): warp 0 meanwhile
-// prepares the next task.
-__device__ __forceinline__ void bar_sync_workers() {
-  asm volatile("bar.sync 1, %0;" ::"n"(BT - 32) : "memory");
-}
-
-// Multi-pass fallback: stable LSD radix sort of 32-bit order-preserving
-// offsets, 8 bits per pass over the bits that differ, then exact tie order.
+// Multi-pass fallback: stable LSD radix sort of the slots by 32-bit
+// order-preserving offsets (recomputed from the positions), 8 bits per pass
+// over the bits that differ, then exact tie order.
 __device__ __forceinline__ void lsd_sort(StepSmem& S, int n, uint64_t kmin, uint64_t kmax) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint64_t span = kmax - kmin;
@@ -202,33 +205,37 @@ __device__ __forceinline__ void lsd_sort(StepSmem& S, int n, uint64_t kmin, uint
   const int shift = bits > 32 ? bits - 32 : 0;
   const int passes = (bits - shift + 7) / 8;
   LsdSmem& L = S.u.lsd;
+  auto offset = [&](int slot) { return (uint32_t)((key_of(S.x[slot]) - kmin) >> shift); };
   __syncthreads();  // the union was just used as counting-sort bins
-  for (int j = tid; j < n; j += BT) {
-    L.q[0][j] = (uint32_t)((key_of(S.x[j]) - kmin) >> shift);
-    L.p[0][j] = (uint16_t)j;
-  }
-  int cur = 0;
+  // an even number of permutation moves ends in S.perm
+  uint16_t* src = (passes & 1) ? L.p : S.perm;
+  uint16_t* dst = (passes & 1) ? S.perm : L.p;
+  for (int j = tid; j < n; j += BT) src[j] = (uint16_t)j;
   __syncthreads();
   for (int pass = 0; pass < passes; ++pass) {
     const int ds = 8 * pass;
     for (int i = lane; i < 256; i += 32) L.hist[warp][i] = 0;
     __syncwarp();
-    uint32_t rank[MAXI];
-    unsigned dig[MAXI];
+    uint16_t rank[MAXI], slot[MAXI];
+    uint8_t dig[MAXI];
 #pragma unroll
     for (int i = 0; i < MAXI; ++i) {
       const int j = warp * (32 * MAXI) + i * 32 + lane;
       const bool ok = j < n;
-      const unsigned d = ok ? ((L.q[cur][j] >> ds) & 255u) : (256u + lane);
-      dig[i] = d;
+      unsigned d = 256u + lane;
+      if (ok) {
+        slot[i] = src[j];
+        d = (offset(slot[i]) >> ds) & 255u;
+      }
+      dig[i] = (uint8_t)d;
       const unsigned peers = __match_any_sync(0xffffffffu, d);
       uint32_t old = 0;
       if (ok) {
         old = L.hist[warp][d];
-        rank[i] = old + __popc(peers & lanemask_lt());
+        rank[i] = (uint16_t)(old + __popc(peers & lanemask_lt()));
       }
       __syncwarp();
-      if (ok && lane == __ffs(peers) - 1) L.hist[warp][d] = old + __popc(peers);
+      if (ok && lane == __ffs(peers) - 1) L.hist[warp][d] = (uint16_t)(old + __popc(peers));
       __syncwarp();
     }
     __syncthreads();
@@ -236,34 +243,30 @@ __device__ __forceinline__ void lsd_sort(StepSmem& S, int n, uint64_t kmin, uint
 #pragma unroll
     for (int w = 0; w < WARPS; ++w) {
       const uint32_t c = L.hist[w][tid];
-      L.hist[w][tid] = run;
+      L.hist[w][tid] = (uint16_t)run;
       run += c;
     }
     uint32_t total;
     const uint32_t base = block_excl_scan(S, run, total);
 #pragma unroll
-    for (int w = 0; w < WARPS; ++w) L.hist[w][tid] += base;
+    for (int w = 0; w < WARPS; ++w) L.hist[w][tid] += (uint16_t)base;
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < MAXI; ++i) {
       const int j = warp * (32 * MAXI) + i * 32 + lane;
-      if (j < n) {
-        const uint32_t dst = L.hist[warp][dig[i]] + rank[i];
-        L.q[1 - cur][dst] = L.q[cur][j];
-        L.p[1 - cur][dst] = L.p[cur][j];
-      }
+      if (j < n) dst[L.hist[warp][dig[i]] + rank[i]] = slot[i];
     }
     __syncthreads();
-    cur = 1 - cur;
+    uint16_t* const t = src;
+    src = dst;
+    dst = t;
   }
-  for (int j = tid; j < n; j += BT) S.perm[j] = L.p[cur][j];
-  __syncthreads();
   // equal offsets: order by the full (key, idx)
   for (int j = tid; j + 1 < n; j += BT) {
-    const uint32_t qj = L.q[cur][j];
-    if (qj != L.q[cur][j + 1] || (j > 0 && L.q[cur][j - 1] == qj)) continue;
+    const uint32_t qj = offset(S.perm[j]);
+    if (qj != offset(S.perm[j + 1]) || (j > 0 && offset(S.perm[j - 1]) == qj)) continue;
     int e = j + 1;
-    while (e + 1 < n && L.q[cur][e + 1] == qj) ++e;
+    while (e + 1 < n && offset(S.perm[e + 1]) == qj) ++e;
     for (int a = j + 1; a <= e; ++a) {
       const uint16_t s = S.perm[a];
       const uint64_t ks = key_of(S.x[s]);
@@ -277,6 +280,11 @@ __device__ __forceinline__ void lsd_sort(StepSmem& S, int n, uint64_t kmin, uint
     }
   }
   __syncthreads();
+}
+
+// Inverse of key_of (of the canonical key: +0 for the zeros).
+__device__ __forceinline__ double pos_of_key(uint64_t k) {
+  return __longlong_as_double((long long)((k >> 63) ? (k & 0x7FFFFFFFFFFFFFFFull) : ~k));
 }
 
 // The smallest and largest key of a warp: the upper halves first, then the
@@ -293,6 +301,49 @@ __device__ __forceinline__ uint64_t warp_max_u64(uint64_t k) {
   const uint32_t h = __reduce_max_sync(0xffffffffu, hi);
   const uint32_t l = __reduce_max_sync(0xffffffffu, hi == h ? (uint32_t)k : 0u);
   return ((uint64_t)h << 32) | l;
+}
+
+// Cell of a position in the routing table.  Every step (rounding to single
+// precision, subtraction, product with a non-negative scale, truncation,
+// clamping) is non-decreasing, so a splitter in a lower cell than a position
+// lies below it, whatever the rounding.
+__device__ __forceinline__ int lut_cell(float x, float x0, float scale) {
+  return (int)fminf(fmaxf((x - x0) * scale, 0.f), (float)(LUTN - 1));
+}
+
+// Routing table over the splitter window [lo, hi] of the next layout (wlen =
+// hi - lo buckets): lut[c] is the largest window entry whose splitter lies in
+// a cell below c, so the entry of a position in cell c is one of lut[c] ..
+// lut[c + 1] -- one or two candidates where the window's splitters are spread
+// over the cells, against the six or seven rounds of a search of the window.
+// Cells are cut in position, not in key, space (keys are logarithmic about
+// zero).  Here the cell of this thread's splitter (threads 1 .. wlen - 1;
+// -1 for the others); the sort counts the splitters per cell and sums the
+// counts along with its own bins.
+__device__ __forceinline__ int route_cell(StepSmem& S, const uint64_t* wk, int lo, int hi,
+                                          int64_t nb) {
+  const int j = threadIdx.x, wlen = hi - lo;
+  if (j < LUTN / 4) S.cell_cnt[j] = 0u;
+  if (j >= wlen) return -1;
+  // the first and last finite splitters of the window
+  const int j0 = lo == 0 ? 1 : 0, j1 = hi == (int)nb ? wlen - 1 : wlen;
+  float x0 = 0.f, scale = 0.f;
+  if (j1 > j0) {
+    x0 = (float)pos_of_key(wk[j0]);
+    const float w = (float)pos_of_key(wk[j1]) - x0;
+    if (w > 1e-30f && w < 1e30f) scale = (float)LUTN / w;
+  }
+  if (j == 0) {
+    S.lut_x0 = x0;
+    S.lut_scale = scale;
+    return -1;
+  }
+  return lut_cell((float)pos_of_key(wk[j]), x0, scale);
+}
+
+// The splitters in this thread's cell (at most 128 in all: a byte holds them).
+__device__ __forceinline__ uint32_t cell_count(const StepSmem& S) {
+  return reinterpret_cast<const uint8_t*>(S.cell_cnt)[threadIdx.x];
 }
 
 // (key, idx) of the sheet in slot a precedes that of slot b.
@@ -344,13 +395,13 @@ __device__ __forceinline__ void order_bin(StepSmem& S, uint32_t lo, uint32_t hi)
 }
 
 // Sort the n <= CAP sheets of the bucket by (key, idx) into S.perm, with
-// 2^qb bins (11 <= qb <= 13).  The bin words are zero on entry (cleared while
+// 2^qb bins (QB_MIN <= qb <= QB_MAX).  The bin words are zero on entry (cleared while
 // the bucket loads).  pre != 0: the opening half drift of a call, applied to
 // the positions on the way.
 // Returns false, having changed nothing, if some thread did not see the
 // sheets arrive.
 __device__ __forceinline__ bool bucket_sort(StepSmem& S, int n, int ipt, int qb, bool arrived,
-                                            double pre) {
+                                            double pre, int rcell) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nbin = 1 << qb;
   uint32_t* bins = S.u.srt.bins;
@@ -380,6 +431,7 @@ __device__ __forceinline__ bool bucket_sort(StepSmem& S, int n, int ipt, int qb,
   }
   if (tid == 0) S.u.srt.nlong = 0;  // read after the barriers below
   if (__syncthreads_or(!arrived)) return false;
+  if (rcell >= 0) atomicAdd(&S.cell_cnt[rcell >> 2], 1u << (8 * (rcell & 3)));
   kmin = warp_min_u64(S.red_min[lane & (WARPS - 1)]);
   kmax = warp_max_u64(S.red_max[lane & (WARPS - 1)]);
   // Bin of a key: the top 32 bits of its offset in the range, times scale /
@@ -389,46 +441,68 @@ __device__ __forceinline__ bool bucket_sort(StepSmem& S, int n, int ipt, int qb,
   // the largest key still lands below nbin; a range narrower than nbin keys
   // maps one key per bin.
   const uint64_t span = kmax - kmin;
-  const int ksh = (span >> 32) ? 32 - __clz((int)(uint32_t)(span >> 32)) : 0;
+  int ksh = (span >> 32) ? 32 - __clz((int)(uint32_t)(span >> 32)) : 0;
   const uint32_t span32 = (uint32_t)(span >> ksh);
-  const bool narrow = span32 < (uint32_t)nbin;
+  bool narrow = span32 < (uint32_t)nbin;
   const uint32_t scale =
       narrow ? 0u
              : (uint32_t)((float)nbin / ((float)span32 + 1.0f) * 4294967296.0f *
                           (1.0f - 9.5367431640625e-07f));
-  uint16_t qv[MAXI], rk[MAXI];
+  // Keys are logarithmic in the position: a range of more than two binades --
+  // a bucket about x = 0, in the far tail, or a whole small simulation -- would
+  // crowd most sheets into a few of its bins.  Such a bucket is cut linearly
+  // in position instead (difference, conversion, product and truncation are
+  // each non-decreasing); elsewhere the integer map is the cheaper one.
+  if (span > (2ull << 52)) {
+    const double xmin = pos_of_key(kmin);
+    const float w = (float)(pos_of_key(kmax) - xmin);
+    const float wscale = w > 1e-30f && w < 1e30f ? (float)nbin / w : 0.f;
+#pragma unroll
+    for (int i = 0; i < MAXI; ++i) {
+      const int j = tid + i * BT;
+      if (i < ipt && j < n)
+        key[i] = kmin + (uint32_t)fminf((float)(S.x[j] - xmin) * wscale, (float)(nbin - 1));
+    }
+    ksh = 0;
+    narrow = true;
+  }
+  uint32_t qr[MAXI];     // bin << 16 | rank in it
   uint32_t nshared = 0;  // this warp's entries of shared_bin
   bool full = false;
 #pragma unroll
   for (int i = 0; i < MAXI; ++i) {
     if (i < ipt) {
       const int j = tid + i * BT;
-      rk[i] = 0;
-      qv[i] = 0;
+      uint32_t rk = 0;
+      qr[i] = 0;
       if (j < n) {
         const uint32_t d = (uint32_t)((key[i] - kmin) >> ksh);
         const uint32_t q = narrow ? d : __umulhi(d, scale);
         const int sh = (int)(q & 1u) << 4;
-        qv[i] = (uint16_t)q;
-        rk[i] = (uint16_t)(atomicAdd(&bins[q >> 1], 1u << sh) >> sh);
-        full |= rk[i] >= MAXBIN;
+        rk = (atomicAdd(&bins[q >> 1], 1u << sh) >> sh) & 0xffffu;
+        qr[i] = (q << 16) | rk;
+        full |= rk >= MAXBIN;
       }
       // The order inside a bin comes from atomics.  A bin holds two or more
       // sheets exactly when one of them took rank 1 in it: the bins found
       // that way are listed per warp (a fifth as many as sheets), so that
       // ordering them below takes each lane about one bin.
-      const unsigned sm = __ballot_sync(0xffffffffu, rk[i] == 1);
-      if (rk[i] == 1)
-        S.u.srt.shared_bin[warp][nshared + __popc(sm & lanemask_lt())] = qv[i];
+      const unsigned sm = __ballot_sync(0xffffffffu, rk == 1);
+      const uint32_t at = nshared + __popc(sm & lanemask_lt());
+      if (rk == 1 && at < SHLIST) S.u.srt.shared_bin[warp][at] = (uint16_t)(qr[i] >> 16);
       nshared += __popc(sm);
     }
   }
+  full |= nshared > SHLIST;  // more than the list holds: crowded keys
   if (__syncthreads_or(full)) {
+    uint32_t total;
+    S.lut[tid] = (uint8_t)block_excl_scan(S, cell_count(S), total);
+    if (tid == 0) S.lut[LUTN] = (uint8_t)total;
     lsd_sort(S, n, kmin, kmax);
     return true;
   }
   // exclusive scan of the bins: thread t owns w4 groups of four words
-  const int w4 = nbin / (8 * BT);  // 1, 2 or 4
+  const int w4 = nbin / (8 * BT);  // 1 or 2
   uint4* const b4 = reinterpret_cast<uint4*>(bins) + tid * w4;
   uint32_t run = 0;
   for (int k = 0; k < w4; ++k) {
@@ -436,8 +510,12 @@ __device__ __forceinline__ bool bucket_sort(StepSmem& S, int n, int ipt, int qb,
     const uint32_t s = c.x + c.y + c.z + c.w;
     run += (s & 0xffffu) + (s >> 16);
   }
+  // (the routing table's counts ride in the upper half: at most 128 splitters)
   uint32_t total;
-  uint32_t off = block_excl_scan(S, run, total);
+  const uint32_t both = block_excl_scan(S, run | (cell_count(S) << 16), total);
+  S.lut[tid] = (uint8_t)(both >> 16);
+  if (tid == 0) S.lut[LUTN] = (uint8_t)(total >> 16);
+  uint32_t off = both & 0xffffu;
   for (int k = 0; k < w4; ++k) {
     uint4 c = b4[k];
     // a word (lo, hi) becomes (off, off + lo)
@@ -460,7 +538,7 @@ __device__ __forceinline__ bool bucket_sort(StepSmem& S, int n, int ipt, int qb,
 #pragma unroll
   for (int i = 0; i < MAXI; ++i) {
     const int j = tid + i * BT;
-    if (i < ipt && j < n) S.perm[bin_get(bins, qv[i]) + rk[i]] = (uint16_t)j;
+    if (i < ipt && j < n) S.perm[bin_get(bins, (int)(qr[i] >> 16)) + (qr[i] & 0xffffu)] = (uint16_t)j;
   }
   __syncthreads();
   // the shared bins, each ordered by one lane of the warp that listed it; bins
@@ -485,7 +563,8 @@ __device__ __forceinline__ bool bucket_sort(StepSmem& S, int n, int ipt, int qb,
     place[i] = 0xffffffffu;
     const int j = tid + i * BT;
     if (i < ipt && j < n) {
-      const uint32_t lo = bin_get(bins, qv[i]), hi = bin_get(bins, qv[i] + 1);
+      const int q = (int)(qr[i] >> 16);
+      const uint32_t lo = bin_get(bins, q), hi = bin_get(bins, q + 1);
       if (hi - lo > kOwnerSort) {
         const uint64_t kj = key_of(S.x[j]);
         uint32_t r = 0;
@@ -689,10 +768,10 @@ __device__ __forceinline__ void prepare_task(const StepLaunch& L, int sub, unsig
     out.whi = whi;
     out.bucket = b;
     out.lay = lay;
-    out.x = D.bx[lay];
-    out.v = D.bv[lay];
-    out.m = D.bm[lay];
-    out.idx = D.bi[lay];
+    out.x = D.bx[lay] + b * capg;
+    out.v = D.bv[lay] + b * capg;
+    out.m = D.bm[lay] + b * capg;
+    out.idx = D.bi[lay] + b * capg;
     out.n = n;
     out.amp = amp;
     out.inv_h = inv_h;
@@ -713,53 +792,10 @@ __device__ __forceinline__ void claim_task(const StepLaunch& L, int sub, unsigne
   prepare_task(L, sub, ep, lane, t, tk, S, wbuf);
 }
 
-// Inverse of key_of (of the canonical key: +0 for the zeros), in single
-// precision; the ends of the key range saturate.
-__device__ __forceinline__ float float_of_key(uint64_t k) {
-  const uint64_t b = (k >> 63) ? (k & 0x7FFFFFFFFFFFFFFFull) : ~k;
-  return (float)__longlong_as_double((long long)b);
-}
-
-// Cell of a position in the routing table.  Every step (rounding to single
-// precision, subtraction, product with a non-negative scale, truncation,
-// clamping) is non-decreasing, so a splitter in a lower cell than a position
-// lies below it, whatever the rounding.
-__device__ __forceinline__ int lut_cell(float x, float x0, float scale) {
-  return (int)fminf(fmaxf((x - x0) * scale, 0.f), (float)(LUTN - 1));
-}
-
-// Routing table over the splitter window [lo, hi] of the next layout (wlen =
-// hi - lo buckets): lut[c] is the largest window entry whose splitter lies in
-// a cell below c, so the entry of a position in cell c is one of lut[c] ..
-// lut[c + 1] -- one or two candidates where the window's splitters are spread
-// over the cells, against the six or seven rounds of a search of the window.
-// Cells are cut in position, not in key, space (keys are logarithmic about
-// zero).  Threads 0 .. wlen - 1; a barrier must follow before its use.
-__device__ __forceinline__ void route_table(StepSmem& S, const uint64_t* wk, int lo, int hi,
-                                            int64_t nb) {
-  const int j = threadIdx.x, wlen = hi - lo;
-  if (j >= wlen) return;
-  // the first and last finite splitters of the window
-  const int j0 = lo == 0 ? 1 : 0, j1 = hi == (int)nb ? wlen - 1 : wlen;
-  float x0 = 0.f, scale = 0.f;
-  if (j1 > j0) {
-    x0 = float_of_key(wk[j0]);
-    const float w = float_of_key(wk[j1]) - x0;
-    if (w > 1e-30f && w < 1e30f) scale = (float)LUTN / w;
-  }
-  const int c0 = j == 0 ? -1 : lut_cell(float_of_key(wk[j]), x0, scale);
-  const int c1 = j == wlen - 1 ? LUTN : lut_cell(float_of_key(wk[j + 1]), x0, scale);
-  for (int c = c0 + 1; c <= c1; ++c) S.lut[c] = (uint8_t)j;
-  if (j == 0) {
-    S.lut_x0 = x0;
-    S.lut_scale = scale;
-  }
-}
-
 // Counting-sort bits of a simulation as the kernel uses them: at least four
-// bin words per thread.
+// bin words per thread, at most what the shared memory has room for.
 __device__ __forceinline__ int step_sort_bits(const SimDev& D) {
-  return D.sort_bits < 11 ? 11 : D.sort_bits;
+  return min(max(D.sort_bits, QB_MIN), QB_MAX);
 }
 __device__ __forceinline__ void clear_bins(StepSmem& S, int qb) {
   uint4* const b4 = reinterpret_cast<uint4*>(S.u.srt.bins);
@@ -773,7 +809,7 @@ __device__ __forceinline__ void clear_bins(StepSmem& S, int qb) {
 // count) prefix of the first of them, the splitter window of the next layout
 // is in S.wkey[S.cur_wbuf] and its routing table in S.lut.  arrived: this
 // thread saw the sheets' copies complete; returns false, having done nothing,
-// if some thread did not.  pre: the opening half drift still to be applied.
+// if some thread did not.  rcell: from route_cell.  pre: the opening half drift still to be applied.
 // PREP: warp 0 prepares the next task (ticket nt of thread 0) during the
 // grouping, as the main kernel's pipeline does; otherwise (chunks of a big
 // bucket) the prefix base is advanced past these sheets at the end.
@@ -782,12 +818,12 @@ __device__ __forceinline__ bool process_bucket(const StepLaunch& L, StepSmem& S,
                                                const int64_t b, const int lay, const int n,
                                                const int sub, const unsigned ep,
                                                const bool arrived, const double pre,
-                                               const unsigned nt) {
+                                               const int rcell, const unsigned nt) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int ipt = (n + BT - 1) / BT;
   const int E = D.E;
   // ---- sort the bucket
-  if (!bucket_sort(S, n, ipt, step_sort_bits(D), arrived, pre)) return false;
+  if (!bucket_sort(S, n, ipt, step_sort_bits(D), arrived, pre, rcell)) return false;
   BucketTask ntk{0, 0};
   if (PREP && tid == 0 && nt < (unsigned)L.ntasks) ntk = L.tasks[nt];
   const uint64_t* const wk = S.wkey[S.cur_wbuf];
@@ -800,12 +836,11 @@ __device__ __forceinline__ bool process_bucket(const StepLaunch& L, StepSmem& S,
   u128 tot = 0;
 #pragma unroll 2
   for (int i = 0; i < nmine; ++i) {
-    const u128 M = mass_to_fixed(S.m[S.perm[j0 + i]], E);
-    S.u.pos.mfix[j0 + i] = M;
-    tot += M;
+    tot += mass_to_fixed(S.m[S.perm[j0 + i]], E);
   }
   const u128 incl = warp_inclusive_scan_u128(tot, lane);
   if (lane == 31) S.warp_mass[warp] = incl;
+  // (the barrier below also ends the use of the bins)
   if (PREP && tid == 0) {
     S.next_ticket = nt;
     S.next_tk = ntk;
@@ -855,27 +890,25 @@ __device__ __forceinline__ bool process_bucket(const StepLaunch& L, StepSmem& S,
   qnext = qnext ? qnext : 1u;
   const uint32_t rnext = qnext * target;
   const int wlen = S.win_hi - S.win_lo;
-  const uint64_t wk_lo = wk[0], wk_hi = wk[wlen];
   const float lut_x0 = S.lut_x0, lut_scale = S.lut_scale;
   // the acceleration of the sheet at position j is A_j = T - 2 C_j - M_j with
   // C_j the mass before it; from one sheet to the next A falls by M_j + M_j+1
   i128 A = (i128)(((((u128)D.T_hi) << 64) | D.T_lo) - 2 * C);
-  // two sheets at a time, interleaved, so that their shared-memory and
-  // FP64 latencies overlap
-  for (int i0 = 0; i0 < nmine; i0 += 2) {
-    const bool ok1 = i0 + 1 < nmine;
-    int sl[2];
-    uint64_t kd[2];
-    float xf[2];
-    int32_t idv[2];
-    bool live[2] = {true, ok1};
+#pragma unroll 1
+  for (int i0 = 0; i0 < nmine; i0 += FU) {
+    int sl[FU];
+    uint64_t kd[FU];
+    float xf[FU];
+    int32_t idv[FU];
+    bool live[FU];
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
+    for (int u = 0; u < FU; ++u) {
+      live[u] = u == 0 || i0 + u < nmine;
       sl[u] = S.perm[j0 + (live[u] ? i0 + u : i0)];
       idv[u] = S.idx[sl[u]];
     }
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
+    for (int u = 0; u < FU; ++u) {
       if (!live[u]) {
         kd[u] = 0;
         xf[u] = 0.f;
@@ -896,7 +929,7 @@ __device__ __forceinline__ bool process_bucket(const StepLaunch& L, StepSmem& S,
           }
         }
       }
-      const u128 M = S.u.pos.mfix[j0 + i0 + u];
+      const u128 M = mass_to_fixed(S.m[sidx], E);
       A -= (i128)M;
       double acc = fixed_to_double(A, E);
       A -= (i128)M;
@@ -943,38 +976,35 @@ __device__ __forceinline__ bool process_bucket(const StepLaunch& L, StepSmem& S,
       xf[u] = (float)xd;
     }
     // routing: the window entry among the table's candidates
-    int l[2], h[2];
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int c = lut_cell(xf[u], lut_x0, lut_scale);
-      l[u] = S.lut[c];
-      h[u] = S.lut[c + 1];
-    }
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
+    for (int u = 0; u < FU; ++u) {
       if (!live[u]) continue;
-      // strictly inside the window's keys; anything else (its ends included)
-      // is found by the search over all splitters where it is needed
-      const bool inw = kd[u] > wk_lo && kd[u] < wk_hi;
-      int w = wlen;
-      if (inw) {
-        // the largest entry with key Q <= key; then splitters with an equal
-        // key and a larger index step back (pair order)
-        int a = l[u], z = h[u];
-        while (a < z) {
-          const int mid = (a + z + 1) >> 1;
-          if (wk[mid] <= kd[u])
-            a = mid;
-          else
-            z = mid - 1;
+      const int c = lut_cell(xf[u], lut_x0, lut_scale);
+      int a = S.lut[c], z = S.lut[c + 1];
+      // a position in an end cell may lie outside the window (or on its end):
+      // unless it is strictly inside, its bucket is found by the search over
+      // all splitters where it is needed.  The cells between lie inside.
+      bool inw = true;
+      if (c == 0 || c == LUTN - 1) inw = kd[u] > wk[0] && kd[u] < wk[wlen];
+      // the largest entry with key Q <= key (entry a of the table lies below
+      // the position's cell); then splitters with an equal key and a larger
+      // index step back (pair order)
+      bool eq = false;
+      while (a < z) {
+        const int mid = (a + z + 1) >> 1;
+        const uint64_t K = wk[mid];
+        if (K <= kd[u]) {
+          a = mid;
+          eq = K == kd[u];
+        } else {
+          z = mid - 1;
         }
-        while (a > 0 && wk[a] == kd[u] && wi[a] > idv[u]) --a;
-        w = a;
       }
-      // destination: window entry w, or wlen for a bucket outside the window
-      const int pq = j0 + i0 + u;
-      S.u.pos.dw[pq] = (uint8_t)w;
-      S.u.pos.drk[pq] = (uint16_t)atomicAdd(&S.dcount[w], 1u);
+      if (eq)
+        while (a > 0 && wk[a] == kd[u] && wi[a] > idv[u]) --a;
+      // destination: window entry a, or wlen for a bucket outside the window
+      const int w = inw ? a : wlen;
+      S.u.dest[j0 + i0 + u] = ((uint32_t)w << 16) | atomicAdd(&S.dcount[w], 1u);
     }
   }
   if (ptab) {
@@ -1004,125 +1034,128 @@ __device__ __forceinline__ bool process_bucket(const StepLaunch& L, StepSmem& S,
     c.x[q - 1] = fma(2.0 * dt, (double)(vs / (float)n), S.samp_x[tid]);
     c.idx[q - 1] = S.samp_idx[tid];
   }
-  // ---- the sheets grouped by destination bucket of the next layout.  Warp 0
-  // prepares the next task meanwhile; the other warps synchronise among
-  // themselves (named barrier 1) until the block-wide barrier below.
+  // ---- the sheets grouped by destination bucket of the next layout: every
+  // thread takes its positions' destinations into registers, one warp forms
+  // the segments, and the same array then holds the grouped order
   const int cw = (D.cs0 + sub + 1) % kAggSlots;
   unsigned* const cnt_out = D.bcnt[cw];
   unsigned long long* const mass_out = D.bmass[cw];
   const uint64_t* const qfar = D.qk[(D.qsel0 + sub) & 1];
   const int32_t* const ifar = D.qi[(D.qsel0 + sub) & 1];
-  uint32_t db = 0;
-  if (warp == 0) {
-    if constexpr (PREP) prepare_task(L, sub, ep, lane, S.next_ticket, S.next_tk, S, S.cur_wbuf ^ 1);
-  } else {
-    const int wt = tid - 32;  // 0 .. BT - 33
-    // slots: one atomic per window bucket, its round trip overlapping the
-    // grouping and the mass sums
-    if (wt < wlen) {
-      const uint32_t c = S.dcount[wt];
-      if (c) {
-        db = atomicAdd(&cnt_out[S.win_lo + wt], c);
-        atomicMax(&S.maxc, db + c);
-      }
-    }
-    if (warp == 1) {
-      // segments: exclusive prefix of the counts of the wlen + 1 entries
-      constexpr int E5 = (2 * RWIN + 2 + 31) / 32;
-      uint32_t cv[E5];
-      uint32_t sum = 0;
+  // slots: one atomic per window bucket, its round trip overlapping the
+  // grouping (warps 2 on; warp 1 forms the segments)
+  uint32_t db = 0, dcn = 0;
+  const int wt = tid - 64;
+  if (wt >= 0 && wt < wlen) {
+    dcn = S.dcount[wt];
+    if (dcn) db = atomicAdd(&cnt_out[S.win_lo + wt], dcn);
+  }
+  uint32_t mydest[MAXI];
 #pragma unroll
-      for (int k = 0; k < E5; ++k) {
-        const int j = lane * E5 + k;
-        cv[k] = j <= wlen ? S.dcount[j] : 0u;
-        sum += cv[k];
-      }
-      uint32_t incl = sum;
+  for (int i = 0; i < MAXI; ++i)
+    if (i < nmine) mydest[i] = S.u.dest[j0 + i];
+  if (warp == 1) {
+    // segments: exclusive prefix of the counts of the wlen + 1 entries
+    constexpr int E5 = (2 * RWIN + 2 + 31) / 32;
+    uint32_t cv[E5];
+    uint32_t sum = 0;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-      }
-      uint32_t ex = incl - sum;
+    for (int k = 0; k < E5; ++k) {
+      const int j = lane * E5 + k;
+      cv[k] = j <= wlen ? S.dcount[j] : 0u;
+      sum += cv[k];
+    }
+    uint32_t incl2 = sum;
 #pragma unroll
-      for (int k = 0; k < E5; ++k) {
-        const int j = lane * E5 + k;
-        if (j <= wlen) S.dstart[j] = ex;
-        ex += cv[k];
-      }
-      if (lane == 31) S.dstart[wlen + 1] = incl;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl2, o);
+      if (lane >= o) incl2 += y;
     }
-    bar_sync_workers();
-    for (int pq = wt; pq < n; pq += BT - 32)
-      S.u.pos.order[S.dstart[S.u.pos.dw[pq]] + S.u.pos.drk[pq]] = (uint16_t)pq;
-    bar_sync_workers();
-    // ---- masses of the next layout: a warp sums the fixed-point masses of
-    // a window bucket's segment and adds them to that bucket's accumulators
-    for (int w = warp - 1; w < wlen; w += WARPS - 1) {
-      const int q0 = (int)S.dstart[w], q1 = (int)S.dstart[w + 1];
-      if (q0 == q1) continue;
-      u128 P = 0;
-      for (int q = q0 + lane; q < q1; q += 32) P += S.u.pos.mfix[S.u.pos.order[q]];
-      P = warp_sum_u128(P);
-      if (lane < 4) {
-        const unsigned long long limb = (unsigned long long)(uint32_t)(P >> (32 * lane));
-        if (limb) atomicAdd(&mass_out[4 * (int64_t)(S.win_lo + w) + lane], limb);
-      }
-    }
-    // sheets bound outside the window: one by one
-    for (int q = (int)S.dstart[wlen] + wt; q < n; q += BT - 32) {
-      const int pq = S.u.pos.order[q];
-      const int sl = S.perm[pq];
-      const double xn = S.x[sl];
-      const uint64_t kf = key_of(LAST && dest_dt != 0.0 ? fma(dest_dt, S.v[sl], xn) : xn);
-      const int d = dest_bucket(wk, wi, S.win_lo, wlen, qfar, ifar, nbk, kf, S.idx[sl]);
-      const u128 M = S.u.pos.mfix[pq];
+    uint32_t ex = incl2 - sum;
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const unsigned long long limb = (unsigned long long)(uint32_t)(M >> (32 * k));
-        if (limb) atomicAdd(&mass_out[4 * (int64_t)d + k], limb);
-      }
+    for (int k = 0; k < E5; ++k) {
+      const int j = lane * E5 + k;
+      if (j <= wlen) S.dstart[j] = ex;
+      ex += cv[k];
     }
-    if (wt < wlen) S.dbase[wt] = db;
+    if (lane == 31) S.dstart[wlen + 1] = incl2;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < MAXI; ++i)
+    if (i < nmine) {
+      const uint32_t w = mydest[i] >> 16;
+      S.u.dest[S.dstart[w] + (mydest[i] & 0xffffu)] = (w << 16) | S.perm[j0 + i];
+    }
+  if (dcn) {
+    S.dbase[wt] = db;
+    atomicMax(&S.maxc, db + dcn);
   }
   __syncthreads();
   bool overflow = false;
-  {
+  if (PREP && warp == 0) {
+    // warp 0 prepares the next task while the others write out
+    prepare_task(L, sub, ep, lane, S.next_ticket, S.next_tk, S, S.cur_wbuf ^ 1);
+  } else {
+    const int nw = PREP ? BT - 32 : BT, t0 = PREP ? tid - 32 : tid;
     // write-out grouped by destination: consecutive positions of a segment
     // take consecutive slots, so a warp's stores coalesce
     double* const xout = D.bx[1 - lay];
     double* const vout = D.bv[1 - lay];
     double* const mout = D.bm[1 - lay];
     int32_t* const iout = D.bi[1 - lay];
-    for (int q = tid; q < n; q += BT) {
-      const int pq = S.u.pos.order[q];
-      const int w = S.u.pos.dw[pq];
-      const int sl = S.perm[pq];
+    const unsigned capg = (unsigned)D.capg;
+    for (int q = t0; q < n; q += nw) {
+      const uint32_t e = S.u.dest[q];
+      const int w = (int)(e >> 16), sl = (int)(e & 0xffffu);
+      const double xn = S.x[sl], vn = S.v[sl], mn = S.m[sl];
+      const int32_t in = S.idx[sl];
       int d;
       uint32_t slot;
       if (w < wlen) {
         d = S.win_lo + w;
         slot = S.dbase[w] + (uint32_t)q - S.dstart[w];
       } else {
-        const double xn = S.x[sl];
-        const uint64_t kf = key_of(LAST && dest_dt != 0.0 ? fma(dest_dt, S.v[sl], xn) : xn);
-        d = dest_bucket(wk, wi, S.win_lo, wlen, qfar, ifar, nbk, kf, S.idx[sl]);
+        // outside the window: its bucket is found among all splitters, its
+        // slot and mass are added one by one
+        const uint64_t kf = key_of(LAST && dest_dt != 0.0 ? fma(dest_dt, vn, xn) : xn);
+        d = dest_bucket(wk, wi, S.win_lo, wlen, qfar, ifar, nbk, kf, in);
         slot = atomicAdd(&cnt_out[d], 1u);
         atomicMax(&S.maxc, slot + 1u);
+        const u128 M = mass_to_fixed(mn, E);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const unsigned long long limb = (unsigned long long)(uint32_t)(M >> (32 * k));
+          if (limb) atomicAdd(&mass_out[4 * (int64_t)d + k], limb);
+        }
       }
-      if (slot < (uint32_t)D.capg) {
-        const int64_t o = (int64_t)d * D.capg + slot;
-        xout[o] = S.x[sl];
-        vout[o] = S.v[sl];
-        mout[o] = S.m[sl];
-        iout[o] = S.idx[sl];
+      if (slot < capg) {
+        const int64_t o = (int64_t)d * capg + slot;
+        xout[o] = xn;
+        vout[o] = vn;
+        mout[o] = mn;
+        iout[o] = in;
       } else {
         const uint32_t o = atomicAdd(D.ocount, 1u);
-        D.ox[o] = S.x[sl];
-        D.ov[o] = S.v[sl];
-        D.om[o] = S.m[sl];
-        D.oi[o] = S.idx[sl];
+        D.ox[o] = xn;
+        D.ov[o] = vn;
+        D.om[o] = mn;
+        D.oi[o] = in;
         overflow = true;
+      }
+    }
+    // ---- masses of the next layout: a warp sums the fixed-point masses of
+    // a window bucket's segment and adds them to that bucket's accumulators
+    for (int w = PREP ? warp - 1 : warp; w < wlen; w += PREP ? WARPS - 1 : WARPS) {
+      const int q0 = (int)S.dstart[w], q1 = (int)S.dstart[w + 1];
+      if (q0 == q1) continue;
+      u128 P = 0;
+      for (int q = q0 + lane; q < q1; q += 32)
+        P += mass_to_fixed(S.m[S.u.dest[q] & 0xffffu], E);
+      P = warp_sum_u128(P);
+      if (lane < 4) {
+        const unsigned long long limb = (unsigned long long)(uint32_t)(P >> (32 * lane));
+        if (limb) atomicAdd(&mass_out[4 * (int64_t)(S.win_lo + w) + lane], limb);
       }
     }
   }
@@ -1171,7 +1204,7 @@ static __device__ __noinline__ void list_big(const TaskMeta* tm, unsigned* big_c
 // EXPR: the launch has simulations with expression forces (the interpreter
 // is compiled only into this instantiation).
 template <bool LAST, bool EXPR>
-__global__ void __launch_bounds__(BT, 2) k_bucket_step(const StepLaunch L) {
+__global__ void __launch_bounds__(BT, CTAS) k_bucket_step(const StepLaunch L) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   StepSmem& S = *reinterpret_cast<StepSmem*>(smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1201,7 +1234,6 @@ __global__ void __launch_bounds__(BT, 2) k_bucket_step(const StepLaunch L) {
     const int64_t b = tm.bucket;
     const int lay = tm.lay;
     const int n = tm.n;
-    const int64_t base = b * D.capg;
     // ---- load: the bucket's four arrays arrive by bulk copy (sizes rounded
     // up to 4 sheets, which stays inside the bucket's capacity), then its
     // keys and key range are formed from shared memory
@@ -1209,10 +1241,10 @@ __global__ void __launch_bounds__(BT, 2) k_bucket_step(const StepLaunch L) {
     if (n4 > 0 && tid == 0) {
       fence_proxy_async_smem();  // earlier generic accesses to these buffers are done
       mbar_expect_tx(&S.mbar, (uint32_t)n4 * 28u);
-      bulk_g2s(S.x, tm.x + base, (uint32_t)n4 * 8u, &S.mbar);
-      bulk_g2s(S.v, tm.v + base, (uint32_t)n4 * 8u, &S.mbar);
-      bulk_g2s(S.m, tm.m + base, (uint32_t)n4 * 8u, &S.mbar);
-      bulk_g2s(S.idx, tm.idx + base, (uint32_t)n4 * 4u, &S.mbar);
+      bulk_g2s(S.x, tm.x, (uint32_t)n4 * 8u, &S.mbar);
+      bulk_g2s(S.v, tm.v, (uint32_t)n4 * 8u, &S.mbar);
+      bulk_g2s(S.m, tm.m, (uint32_t)n4 * 8u, &S.mbar);
+      bulk_g2s(S.idx, tm.idx, (uint32_t)n4 * 4u, &S.mbar);
     }
     // the next task's ticket and task-list entry are read ahead (thread 0)
     // and the task is prepared by warp 0 during the write-out
@@ -1235,14 +1267,15 @@ __global__ void __launch_bounds__(BT, 2) k_bucket_step(const StepLaunch L) {
       S.inv_h = tm.inv_h;
     }
     // while the copies are in flight: the counting-sort bins are cleared and
-    // the routing table is made
+    // the window's splitters take their cells of the routing table
     clear_bins(S, step_sort_bits(D));
-    route_table(S, S.wkey[tm.wbuf], tm.wlo, tm.whi, D.nb);
+    const int rcell = route_cell(S, S.wkey[tm.wbuf], tm.wlo, tm.whi, D.nb);
     // the copies' completion: a thread that did not see it within the bounded
     // wait leaves the data alone, and the first barrier of the sort (which
     // every thread reaches) decides for the whole CTA
     const bool arrived = n4 > 0 ? mbar_wait(&S.mbar, parity) : true;
-    if (!process_bucket<LAST, EXPR, true>(L, S, D, b, lay, n, sub, ep, arrived, pre, nt)) {
+    if (!process_bucket<LAST, EXPR, true>(L, S, D, b, lay, n, sub, ep, arrived, pre, rcell,
+                                          nt)) {
       // the bucket's copies did not complete within the bounded wait: its
       // contents are unknown, so this CTA writes nothing more.  It gives the
       // copies a second bounded wait and stops; the host sees the error word
@@ -1302,7 +1335,7 @@ __device__ __forceinline__ void block_range(StepSmem& S, uint64_t& kmin, uint64_
 // cut this way: the simulation is flagged (ocount[2]) and its host side
 // re-sorts the layout this sub-step read, which the sub-step leaves intact.
 template <bool LAST, bool EXPR>
-__global__ void __launch_bounds__(BT, 2) k_bucket_big(const StepLaunch L) {
+__global__ void __launch_bounds__(BT, CTAS) k_bucket_big(const StepLaunch L) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   StepSmem& S = *reinterpret_cast<StepSmem*>(smem_raw);
   const int tid = threadIdx.x;
@@ -1348,8 +1381,6 @@ __global__ void __launch_bounds__(BT, 2) k_bucket_big(const StepLaunch L) {
       S.splittable = 1u;
       for (int c = 0; c <= kMaxChunks; ++c) S.chunk_lo[c] = BIGBINS;
     }
-    __syncthreads();
-    route_table(S, S.wkey[0], bt.wlo, bt.whi, D.nb);
     // ---- the bucket's key range and the histogram of its keys
     uint64_t kmin = ~0ull, kmax = 0;
     for (int j = tid; j < n; j += BT) {
@@ -1357,7 +1388,8 @@ __global__ void __launch_bounds__(BT, 2) k_bucket_big(const StepLaunch L) {
       kmin = k < kmin ? k : kmin;
       kmax = k > kmax ? k : kmax;
     }
-    uint32_t* hist = S.u.srt.bins;  // BIGBINS 32-bit counters
+    // BIGBINS 32-bit counters where the chunks' positions go later
+    uint32_t* hist = reinterpret_cast<uint32_t*>(S.x);
     for (int j = tid; j < BIGBINS; j += BT) hist[j] = 0u;
     block_range(S, kmin, kmax);
     const uint64_t span = kmax - kmin;
@@ -1443,7 +1475,9 @@ __global__ void __launch_bounds__(BT, 2) k_bucket_big(const StepLaunch L) {
         break;
       }
       if (nc == 0) continue;
-      process_bucket<LAST, EXPR, false>(L, S, D, bt.bucket, bt.lay, nc, sub, ep, true, 0.0, 0u);
+      const int rcell = route_cell(S, S.wkey[0], bt.wlo, bt.whi, D.nb);
+      process_bucket<LAST, EXPR, false>(L, S, D, bt.bucket, bt.lay, nc, sub, ep, true, 0.0, rcell,
+                                        0u);
     }
   }
 }
@@ -1561,7 +1595,9 @@ __global__ void k_count_offsets(const unsigned* cnt, int64_t nb, int capg, unsig
 
 }  // namespace
 
-int bucket_step_grid(int sm_count) { return 2 * sm_count; }
+int bucket_step_grid(int sm_count, int ctas_per_sm) {
+  return sm_count * (ctas_per_sm < 2 ? 1 : CTAS);
+}
 
 namespace {
 std::mutex g_tune_mu;

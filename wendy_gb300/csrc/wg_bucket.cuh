@@ -28,7 +28,7 @@ struct BucketTuning {
   int target = 1536;      // sheets per bucket right after a re-sort (<= kMaxTarget)
   int window = 64;        // splitters searched in shared memory on each side
   int sort_bits = 12;     // counting-sort bins = 2^sort_bits (9..13)
-  int ctas_per_sm = 2;    // persistent CTAs per SM (1 or 2)
+  int ctas_per_sm = 2;    // persistent CTAs per SM: 1, or 2 for as many as fit
 };
 BucketTuning tuning_for(int64_t n);
 }  // namespace wg
@@ -211,7 +211,8 @@ void launch_split_out(const OutRec* rec, int64_t n, double* x_out, double* v_out
                       cudaStream_t s);
 // One-time kernel attribute set-up; call before any stream capture.
 void bucket_step_prepare();
-int bucket_step_grid(int sm_count);
+// CTAs of a launch: one per SM, or (ctas_per_sm = 2) as many as fit.
+int bucket_step_grid(int sm_count, int ctas_per_sm);
 // Compact sorted state -> layout 0 with `target` sheets per bucket; fills
 // aggregate slot 0 and clears the other two.
 void launch_bucketize(const StateTable* table, int64_t n, int target, int64_t nb, int capg, int E,

@@ -894,7 +894,7 @@ static int pool_step_begin(wg_pool* p, int count, const int* ids, const double* 
         nmax = a->n;
         cps = a->tune.ctas_per_sm;
       }
-    const int grid = cps * p->sms;
+    const int grid = bucket_step_grid(p->sms, cps);
     for (int i = 0; i < nleap; ++i) {
       StepLaunch L;
       L.sims = p->d_dev;
@@ -1170,7 +1170,7 @@ static int pool_step_end(wg_pool* p, double* time_elapsed) {
       L.big_count = nullptr;
       L.big_ticket = nullptr;
       L.big_cap = 0;
-      launch_bucket_step(L, cps * p->sms, p->stream);
+      launch_bucket_step(L, bucket_step_grid(p->sms, cps), p->stream);
       launch_member_splitters(p->d_dev, p->rlist, (int)m, i, p->stream);
       p->launches += 2;
     }
