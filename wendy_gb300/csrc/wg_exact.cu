@@ -13,9 +13,16 @@
 // the minimum of its 32 children and where it lies), so the next event is a
 // read of the root and an update rewrites three leaves and their paths, each
 // level one coalesced 32-wide load and a warp minimum.  The state lives in
-// shared memory when it fits (a few thousand sheets), in global memory
-// otherwise; the loop is a strict sequence of dependent steps, which is why
-// this stays a cross-check at small N rather than a fast path.
+// position order, in shared memory when it fits (a few thousand sheets), in
+// global memory otherwise.
+//
+// The loop is a strict sequence of crossings, each a chain of dependent FP64
+// operations, so what bounds it is that chain's latency.  The four sheets
+// around a crossing sit in four lanes: they are advanced at once, the five
+// divisions of the three new pair times are one division of five lanes (a
+// second group of four lanes takes the constant terms), the two square roots
+// one square root, and a minimum is two warp-reduce instructions.  Measured
+// at 1001 sheets of a sech^2 disk: EXACT_NUMBERS
 //
 // Arithmetic, operation order and the per-sheet clocks follow the
 // reference (this file is compiled without FMA contraction, as the
@@ -44,12 +51,14 @@ struct ExactState {
   double* a;
   double* m;
   double* t;      // each sheet's own clock within the output interval
-  int32_t* sindx; // sheet at each position
+  int32_t* id;    // the sheet at each position (the arrays above are in
+                  // position order while the event loop runs)
   double* tcoll;  // crossing time of the pair at positions (i, i + 1)
 };
 
 struct ExactArgs {
-  ExactState g;        // global memory copy of the state
+  ExactState g;        // the state in global memory, by sheet (id: the position order)
+  ExactState p;        // the same by position, where shared memory does not hold it
   int n;
   double omega;        // > 0: harmonic external potential
   double dt;
@@ -88,69 +97,75 @@ __device__ double solve_coll_harm(double c0, double c1, double c2, double omega)
 __device__ __forceinline__ uint64_t time_key(double t) {
   return isnan(t) ? ~0ull : key_of(t);
 }
-
-// The smallest (key, index) over the warp; ties to the lower index.
-__device__ __forceinline__ void warp_min(uint64_t& k, int& i) {
-#pragma unroll
-  for (int d = 16; d >= 1; d >>= 1) {
-    const uint64_t ok = __shfl_xor_sync(0xffffffffu, k, d);
-    const int oi = __shfl_xor_sync(0xffffffffu, i, d);
-    if (ok < k || (ok == k && oi < i)) {
-      k = ok;
-      i = oi;
-    }
-  }
+// The time of a key that is not NaN's (+0 for either zero).
+__device__ __forceinline__ double time_of_key(uint64_t k) {
+  return __longlong_as_double((long long)((k >> 63) ? (k & 0x7FFFFFFFFFFFFFFFull) : ~k));
 }
 
-// Recomputes the tree path above pair time `leaf` (all lanes).
-__device__ void tree_update(const ExactArgs& A, uint64_t* const* tkey, int32_t* const* tidx,
-                            const double* tcoll, int leaf, int lane) {
+// The smallest key over the warp and the lowest lane that holds it.
+__device__ __forceinline__ uint64_t warp_min_key(uint64_t k, int& where) {
+  const uint32_t hi = (uint32_t)(k >> 32), lo = (uint32_t)k;
+  const uint32_t h = __reduce_min_sync(0xffffffffu, hi);
+  const uint32_t l = __reduce_min_sync(0xffffffffu, hi == h ? lo : 0xffffffffu);
+  where = __ffs(__ballot_sync(0xffffffffu, hi == h && lo == l)) - 1;
+  return ((uint64_t)h << 32) | l;
+}
+
+// Recomputes the tree path above pair time `leaf` (all lanes); returns the
+// root's pair index and key.
+__device__ __forceinline__ int tree_update(const ExactArgs& A, uint64_t* const* tkey,
+                                           int32_t* const* tidx, const double* tcoll, int leaf,
+                                           int lane, uint64_t& root) {
   int g = leaf / kTreeFan;  // group at level 0
-  for (int lv = 0; lv < A.levels; ++lv) {
-    const int j = g * kTreeFan + lane;
-    uint64_t k = ~0ull;
-    int i = 0x7fffffff;
-    if (j < A.level_n[lv]) {
-      if (lv == 0) {
-        k = time_key(tcoll[j]);
-        i = j;
-      } else {
-        k = tkey[lv - 1][j];
-        i = tidx[lv - 1][j];
-      }
-    }
-    warp_min(k, i);
+  int j = g * kTreeFan + lane;
+  uint64_t k = j < A.level_n[0] ? time_key(tcoll[j]) : ~0ull;
+  int where;
+  uint64_t best = warp_min_key(k, where);
+  int idx = g * kTreeFan + where;
+  if (idx >= A.level_n[0]) idx = A.level_n[0] - 1;  // a group of NaN times only
+  for (int lv = 1;; ++lv) {
     if (lane == 0) {
-      tkey[lv][g] = k;
-      tidx[lv][g] = i;
+      tkey[lv - 1][g] = best;
+      tidx[lv - 1][g] = idx;
     }
-    __syncwarp();
+    if (lv == A.levels) break;
+    const int child = g;
     g /= kTreeFan;
+    j = g * kTreeFan + lane;
+    // the child just rewritten comes from registers
+    k = j == child ? best : j < A.level_n[lv] ? tkey[lv - 1][j] : ~0ull;
+    int i = j == child ? idx : j < A.level_n[lv] ? tidx[lv - 1][j] : 0;
+    best = warp_min_key(k, where);
+    idx = __shfl_sync(0xffffffffu, i, where);
   }
+  root = best;
+  return idx;
 }
 
-// Advance sheet s to time tn (reference operation order).
-__device__ __forceinline__ void advance(const ExactState& S, int s, double tn, double omega) {
-  const double tdt = tn - S.t[s];
+// Advance (x, v) from the sheet's own clock t to time tn (reference
+// operation order).
+__device__ __forceinline__ void advance(double& x, double& v, double a, double t, double tn,
+                                        double omega) {
+  const double tdt = tn - t;
   if (omega > 0) {
     const double sinot = sin(omega * tdt);
     const double cosot = sqrt(1. - sinot * sinot);
-    const double tmpd = S.x[s] - S.a[s];
-    S.x[s] = tmpd * cosot + S.v[s] / omega * sinot + S.a[s];
-    S.v[s] = -tmpd * omega * sinot + S.v[s] * cosot;
+    const double tmpd = x - a;
+    const double xo = tmpd * cosot + v / omega * sinot + a;
+    v = -tmpd * omega * sinot + v * cosot;
+    x = xo;
   } else {
-    const double dv = S.a[s] * tdt;
-    S.x[s] += dv * tdt / 2. + S.v[s] * tdt;
-    S.v[s] += dv;
+    const double dv = a * tdt;
+    x += dv * tdt / 2. + v * tdt;
+    v += dv;
   }
-  S.t[s] = tn;
 }
 
 __global__ void __launch_bounds__(32, 1) k_exact_step(const ExactArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x;
   const int n = A.n;
-  ExactState S = A.g;
+  ExactState S = A.p;
   // the tree's internal levels: in shared memory always (n / 31 entries)
   uint64_t* tkey[kMaxLevels];
   int32_t* tidx[kMaxLevels];
@@ -171,7 +186,7 @@ __global__ void __launch_bounds__(32, 1) k_exact_step(const ExactArgs A) {
       }
     p = smem + A.tree_bytes;
     if (A.use_smem) {
-      // stage the state in shared memory too: x v a m t tcoll, then sindx
+      // stage the state in shared memory too: x v a m t tcoll, then id
       double* d = reinterpret_cast<double*>(p);
       S.x = d;
       S.v = d + n;
@@ -179,13 +194,14 @@ __global__ void __launch_bounds__(32, 1) k_exact_step(const ExactArgs A) {
       S.m = d + 3 * n;
       S.t = d + 4 * n;
       S.tcoll = d + 5 * n;
-      S.sindx = reinterpret_cast<int32_t*>(d + 6 * n);
+      S.id = reinterpret_cast<int32_t*>(d + 6 * n);
       for (int i = lane; i < n; i += 32) {
-        S.x[i] = A.g.x[i];
-        S.v[i] = A.g.v[i];
-        S.a[i] = A.g.a[i];
-        S.m[i] = A.g.m[i];
-        S.sindx[i] = A.g.sindx[i];
+        const int s = A.g.id[i];
+        S.id[i] = s;
+        S.x[i] = A.g.x[s];
+        S.v[i] = A.g.v[s];
+        S.a[i] = A.g.a[s];
+        S.m[i] = A.g.m[s];
         if (i < n - 1) S.tcoll[i] = A.g.tcoll[i];
       }
     }
@@ -196,84 +212,110 @@ __global__ void __launch_bounds__(32, 1) k_exact_step(const ExactArgs A) {
   int cindx = *A.cindx;
   double next = *A.next_tcoll;
   long long cnt = 0;
+  // lanes 0 .. 3 (and 4 .. 7 again, for the second divisions) hold the
+  // sheets at positions ci - 1 .. ci + 2 of a crossing of ci and ci + 1
+  const int role = lane & 3;
+  const bool mid = role == 1 || role == 2, first = lane < 4;
   while (next < dt && cnt < A.maxcoll) {
     ++cnt;
-    if (lane == 0) {
-      const int ci = cindx;
-      int i1 = S.sindx[ci], i2 = S.sindx[ci + 1];
-      advance(S, i1, next, omega);
-      advance(S, i2, next, omega);
-      S.sindx[ci] = i2;
-      S.sindx[ci + 1] = i1;
-      const double dm = S.m[i2] - S.m[i1];
-      S.a[i1] -= dm;
-      S.a[i2] -= dm;
-      const double tmp = S.a[i1];
-      S.a[i1] = S.a[i2];
-      S.a[i2] = tmp;
-      // the pair that just crossed (i1 still names the sheet now at ci + 1)
-      double tn;
-      if (omega > 0) {
-        double q = (S.v[i1] - S.v[i2]) / (S.a[i2] - S.a[i1]) / omega;
+    const int ci = cindx;
+    const int pos = ci - 1 + role;
+    const bool have = pos >= 0 && pos < n;  // the outer two may not exist
+    const int at = have ? pos : ci;
+    double x = S.x[at], v = S.v[at], a = S.a[at], t = S.t[at];
+    const double m = S.m[at];
+    const int32_t id = S.id[at];
+    // to the time of the crossing.  Without a harmonic potential the outer
+    // two are only extrapolated, in the reference's order of additions
+    // ((x + a t^2 / 2) + v t, against x + (a t^2 / 2 + v t)), and keep their
+    // clocks
+    if (omega > 0) {
+      advance(x, v, a, t, next, omega);
+    } else {
+      const double tdt = next - t;
+      const double dv = a * tdt;
+      const double p = dv * tdt / 2., q = v * tdt;
+      x = (p + (mid ? q : x)) + (mid ? x : q);
+      v += dv;
+    }
+    // the two swap places and exchange accelerations by the mass difference
+    {
+      const double mo = __shfl_xor_sync(0xffffffffu, m, 3);
+      const double dm = role == 1 ? mo - m : m - mo;
+      const double ad = a - dm;
+      const double ao = __shfl_xor_sync(0xffffffffu, ad, 3);
+      if (mid) a = ao;
+    }
+    // partners of the new pairs: the left neighbour meets the sheet from
+    // ci + 1, the right one that from ci, and those two each other
+    const int partner = (lane & 4) | (role == 0 ? 2 : role == 3 ? 1 : role ^ 3);
+    const double xp = __shfl_sync(0xffffffffu, x, partner);
+    const double vp = __shfl_sync(0xffffffffu, v, partner);
+    const double ap = __shfl_sync(0xffffffffu, a, partner);
+    double tn;
+    if (omega > 0) {
+      if (mid) {
+        double q = (v - vp) / (ap - a) / omega;
         q *= q;
         q = (1. - q) / (1. + q);
         tn = acos(q) / omega;
       } else {
-        tn = 2. * (S.v[i1] - S.v[i2]) / (S.a[i2] - S.a[i1]);
+        tn = solve_coll_harm(x - xp, v - vp, a - ap, omega);
       }
-      S.tcoll[ci] = next + tn;
-      if (ci > 0) {
-        const int j1 = S.sindx[ci - 1], j2 = S.sindx[ci];
-        if (omega > 0) {
-          advance(S, j1, next, omega);
-          S.tcoll[ci - 1] = next + solve_coll_harm(S.x[j1] - S.x[j2], S.v[j1] - S.v[j2],
-                                                   S.a[j1] - S.a[j2], omega);
-        } else {
-          const double tdt = S.t[j1] - next;
-          S.tcoll[ci - 1] =
-              next + solve_coll_quad(S.x[j1] + S.a[j1] * tdt * tdt / 2. - S.v[j1] * tdt - S.x[j2],
-                                     S.v[j1] - S.a[j1] * tdt - S.v[j2],
-                                     0.5 * (S.a[j1] - S.a[j2]));
-        }
+    } else {
+      // the outer pairs' quadratic c2 t^2 + c1 t + c0 (wendy/wendy.c:33-38)
+      // and the inner pair's other root, one division per lane
+      const double c0 = x - xp, c1 = v - vp, c2 = 0.5 * (a - ap);
+      const double num = mid ? 2. * c1 : first ? -c1 : 4. * c0;
+      const double quo = num / (mid ? ap - a : c2);
+      const double qc = __shfl_xor_sync(0xffffffffu, quo, 4);
+      tn = mid ? quo : 0.5 * (quo + sqrt(quo * quo - qc));
+    }
+    if (first) {
+      if (mid) {
+        const int to = role == 1 ? ci + 1 : ci;
+        S.x[to] = x;
+        S.v[to] = v;
+        S.a[to] = a;
+        S.m[to] = m;
+        S.t[to] = next;
+        S.id[to] = id;
+      } else if (have && omega > 0) {
+        S.x[at] = x;
+        S.v[at] = v;
+        S.t[at] = next;
       }
-      if (ci < n - 2) {
-        const int j1 = S.sindx[ci + 2], j2 = S.sindx[ci + 1];
-        if (omega > 0) {
-          advance(S, j1, next, omega);
-          S.tcoll[ci + 1] = next + solve_coll_harm(S.x[j1] - S.x[j2], S.v[j1] - S.v[j2],
-                                                   S.a[j1] - S.a[j2], omega);
-        } else {
-          const double tdt = S.t[j1] - next;
-          S.tcoll[ci + 1] =
-              next + solve_coll_quad(S.x[j1] + S.a[j1] * tdt * tdt / 2. - S.v[j1] * tdt - S.x[j2],
-                                     S.v[j1] - S.a[j1] * tdt - S.v[j2],
-                                     0.5 * (S.a[j1] - S.a[j2]));
-        }
-      }
+      // role 0: pair ci - 1, role 1: pair ci, role 3: pair ci + 1
+      if (role != 2 && have) S.tcoll[role == 3 ? ci + 1 : ci - 1 + role] = next + tn;
     }
     __syncwarp();
-    // the three pair times that changed, and their paths up the tree
-    const int ci = cindx;
+    // the three pair times that changed, and their paths up the tree; the
+    // next crossing is the root
     const int lo = ci > 0 ? ci - 1 : ci, hi = ci < n - 2 ? ci + 1 : ci;
-    tree_update(A, tkey, tidx, S.tcoll, lo, lane);
-    if (hi / kTreeFan != lo / kTreeFan) tree_update(A, tkey, tidx, S.tcoll, hi, lane);
-    // the next crossing: the root
-    const int i = tidx[A.levels - 1][0];
-    const double v = S.tcoll[i];
-    cindx = i;
-    next = isnan(v) ? INFINITY : v;
+    uint64_t root;
+    cindx = tree_update(A, tkey, tidx, S.tcoll, lo, lane, root);
+    if (hi / kTreeFan != lo / kTreeFan) {
+      __syncwarp();
+      cindx = tree_update(A, tkey, tidx, S.tcoll, hi, lane, root);
+    }
+    next = root == ~0ull ? INFINITY : time_of_key(root);
+    __syncwarp();
   }
   // every sheet to the end of the interval, clocks and pending times shifted
-  for (int s = lane; s < n; s += 32) advance(S, s, dt, omega);
-  for (int i = lane; i < n - 1; i += 32) S.tcoll[i] -= dt;
-  __syncwarp();
-  if (A.use_smem) {
-    for (int i = lane; i < n; i += 32) {
-      A.g.x[i] = S.x[i];
-      A.g.v[i] = S.v[i];
-      A.g.a[i] = S.a[i];
-      A.g.sindx[i] = S.sindx[i];
-      if (i < n - 1) A.g.tcoll[i] = S.tcoll[i];
+  for (int i = lane; i < n; i += 32) {
+    double x = S.x[i], v = S.v[i];
+    advance(x, v, S.a[i], S.t[i], dt, omega);
+    if (A.use_smem) {
+      const int s = S.id[i];
+      A.g.id[i] = s;
+      A.g.x[s] = x;
+      A.g.v[s] = v;
+      A.g.a[s] = S.a[i];
+      if (i < n - 1) A.g.tcoll[i] = S.tcoll[i] - dt;
+    } else {
+      S.x[i] = x;
+      S.v[i] = v;
+      if (i < n - 1) S.tcoll[i] -= dt;
     }
   }
   // the tree holds absolute times of this interval: rebuilt by the host's
@@ -286,6 +328,30 @@ __global__ void __launch_bounds__(32, 1) k_exact_step(const ExactArgs A) {
   }
 }
 
+// The state by position from the state by sheet, and back (simulations
+// whose state does not fit in shared memory).
+__global__ void k_exact_gather(ExactArgs A) {
+  const int stride = gridDim.x * blockDim.x;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < A.n; i += stride) {
+    const int s = A.g.id[i];
+    A.p.id[i] = s;
+    A.p.x[i] = A.g.x[s];
+    A.p.v[i] = A.g.v[s];
+    A.p.a[i] = A.g.a[s];
+    A.p.m[i] = A.g.m[s];
+  }
+}
+__global__ void k_exact_scatter(ExactArgs A) {
+  const int stride = gridDim.x * blockDim.x;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < A.n; i += stride) {
+    const int s = A.p.id[i];
+    A.g.id[i] = s;
+    A.g.x[s] = A.p.x[i];
+    A.g.v[s] = A.p.v[i];
+    A.g.a[s] = A.p.a[i];
+  }
+}
+
 // Builds the tree over the current pair times (one warp per level-0 group,
 // then level by level).
 __global__ void k_exact_tree_level(ExactArgs A, int lv) {
@@ -295,7 +361,7 @@ __global__ void k_exact_tree_level(ExactArgs A, int lv) {
   if (g >= ng) return;
   const int j = g * kTreeFan + lane;
   uint64_t k = ~0ull;
-  int i = 0x7fffffff;
+  int i = A.level_n[0] - 1;
   if (j < A.level_n[lv]) {
     if (lv == 0) {
       k = time_key(A.g.tcoll[j]);
@@ -305,7 +371,9 @@ __global__ void k_exact_tree_level(ExactArgs A, int lv) {
       i = A.tree_idx[lv - 1][j];
     }
   }
-  warp_min(k, i);
+  int where;
+  k = warp_min_key(k, where);
+  i = __shfl_sync(0xffffffffu, i, where);
   if (lane == 0) {
     A.tree_key[lv][g] = k;
     A.tree_idx[lv][g] = i;
@@ -317,7 +385,7 @@ __global__ void k_exact_tree_level(ExactArgs A, int lv) {
 __global__ void k_exact_pairs(ExactState S, int n, double omega) {
   const int stride = gridDim.x * blockDim.x;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n - 1; i += stride) {
-    const int p = S.sindx[i], q = S.sindx[i + 1];
+    const int p = S.id[i], q = S.id[i + 1];
     S.tcoll[i] = omega > 0
                      ? solve_coll_harm(S.x[p] - S.x[q], S.v[p] - S.v[q], S.a[p] - S.a[q], omega)
                      : solve_coll_quad(S.x[p] - S.x[q], S.v[p] - S.v[q], (S.a[p] - S.a[q]) / 2.);
@@ -406,7 +474,19 @@ int wg_exact_create(int64_t n, const double* x, const double* v, const double* a
   size_t tree_b = 0;
   for (int lv = 0; lv < A.levels; ++lv)
     tree_b += al(8 * (size_t)A.level_n[lv + 1]) + al(4 * (size_t)A.level_n[lv + 1]);
-  const size_t total = 6 * nd + ni + tree_b + al(64);
+  const size_t smem_tree = [&] {
+    size_t b = 0;
+    for (int lv = 0; lv < A.levels; ++lv) b += 12 * (size_t)A.level_n[lv + 1];
+    return (b + 15) & ~(size_t)15;
+  }();
+  // the tree's internal levels always live in shared memory; the state too
+  // when it fits (6 doubles and an index per sheet)
+  const size_t smem = smem_tree + 52 * (size_t)n + 64;
+  int dev = 0, optin = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  A.use_smem = smem <= (size_t)optin;
+  const size_t total = 6 * nd + ni + tree_b + al(64) + (A.use_smem ? 0 : 4 * nd + ni);
   if (cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreate(&e->ev0) != cudaSuccess || cudaEventCreate(&e->ev1) != cudaSuccess ||
       cudaMallocHost(&e->h_ret, 64) != cudaSuccess) {
@@ -426,25 +506,25 @@ int wg_exact_create(int64_t n, const double* x, const double* v, const double* a
   A.g.m = reinterpret_cast<double*>(p); p += nd;
   A.g.t = reinterpret_cast<double*>(p); p += nd;
   A.g.tcoll = reinterpret_cast<double*>(p); p += nd;
-  A.g.sindx = reinterpret_cast<int32_t*>(p); p += ni;
-  A.tree_bytes = 0;
+  A.g.id = reinterpret_cast<int32_t*>(p); p += ni;
+  A.p = A.g;
+  if (!A.use_smem) {
+    // (the clocks and pair times belong to positions and have one copy)
+    A.p.x = reinterpret_cast<double*>(p); p += nd;
+    A.p.v = reinterpret_cast<double*>(p); p += nd;
+    A.p.a = reinterpret_cast<double*>(p); p += nd;
+    A.p.m = reinterpret_cast<double*>(p); p += nd;
+    A.p.id = reinterpret_cast<int32_t*>(p); p += ni;
+  }
   for (int lv = 0; lv < A.levels; ++lv) {
     A.tree_key[lv] = reinterpret_cast<uint64_t*>(p); p += al(8 * (size_t)A.level_n[lv + 1]);
     A.tree_idx[lv] = reinterpret_cast<int32_t*>(p); p += al(4 * (size_t)A.level_n[lv + 1]);
-    A.tree_bytes += 12 * (size_t)A.level_n[lv + 1];
   }
-  A.tree_bytes = (A.tree_bytes + 15) & ~(size_t)15;
+  A.tree_bytes = smem_tree;
   A.cindx = reinterpret_cast<int*>(p);
   A.err = A.cindx + 1;
   A.ncoll = reinterpret_cast<long long*>(A.cindx + 2);
   A.next_tcoll = reinterpret_cast<double*>(A.cindx + 4);
-  // the tree's internal levels always live in shared memory; the state too
-  // when it fits (6 doubles and an index per sheet)
-  const size_t smem = A.tree_bytes + 52 * (size_t)n + 64;
-  int dev = 0, optin = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  A.use_smem = smem <= (size_t)optin;
   e->smem = A.use_smem ? smem : A.tree_bytes;
   if (e->smem > (size_t)optin ||
       cudaFuncSetAttribute(k_exact_step, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -463,7 +543,7 @@ int wg_exact_create(int64_t n, const double* x, const double* v, const double* a
   up(A.g.v, v, 8 * n);
   up(A.g.a, a, 8 * n);
   up(A.g.m, m, 8 * n);
-  up(A.g.sindx, sindx, 4 * n);
+  up(A.g.id, sindx, 4 * n);
   if (ce == cudaSuccess) {
     k_exact_pairs<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(A.g, (int)n, A.omega);
     ce = cudaGetLastError();
@@ -502,8 +582,11 @@ int wg_exact_step(wg_exact* e, double dt, int64_t maxcoll, int64_t* ncoll,
     const int groups = (A.level_n[lv] + kTreeFan - 1) / kTreeFan;
     k_exact_tree_level<<<(unsigned)((groups + 7) / 8), 256, 0, s>>>(A, lv);
   }
+  const unsigned blocks = (unsigned)((e->n + 255) / 256);
   cudaEventRecord(e->ev0, s);
+  if (!A.use_smem) k_exact_gather<<<blocks, 256, 0, s>>>(A);
   k_exact_step<<<1, 32, e->smem, s>>>(A);
+  if (!A.use_smem) k_exact_scatter<<<blocks, 256, 0, s>>>(A);
   cudaEventRecord(e->ev1, s);
   cudaMemcpyAsync(e->h_ret, A.cindx, 24, cudaMemcpyDeviceToHost, s);
   const cudaError_t ce = cudaStreamSynchronize(s);
@@ -530,7 +613,7 @@ int wg_exact_download(wg_exact* e, double* x, double* v, double* a, int32_t* sin
   down(x, A.g.x, 8 * (size_t)e->n);
   down(v, A.g.v, 8 * (size_t)e->n);
   down(a, A.g.a, 8 * (size_t)e->n);
-  down(sindx, A.g.sindx, 4 * (size_t)e->n);
+  down(sindx, A.g.id, 4 * (size_t)e->n);
   if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
   if (ce != cudaSuccess) return fail(WG_ERR_CUDA, "exact solver: %s", cudaGetErrorString(ce));
   return WG_OK;
