@@ -8,21 +8,30 @@
 // exchange their accelerations by the mass difference, and recompute the
 // crossing times of the three neighbour pairs that changed.  The reference
 // keeps the pair times in an unbalanced binary search tree
-// (wendy/wendy.c:53-315, wendy/bst.c); here one warp owns the whole event
-// loop and keeps them in a 32-ary tournament tree (each internal node holds
-// the minimum of its 32 children and where it lies), so the next event is a
-// read of the root and an update rewrites three leaves and their paths, each
-// level one coalesced 32-wide load and a warp minimum.  The state lives in
-// position order, in shared memory when it fits (a few thousand sheets), in
-// global memory otherwise.
+// (wendy/wendy.c:53-315, wendy/bst.c); here they sit in a 32-ary tournament
+// tree (each internal node holds the minimum of its 32 children and where it
+// lies), each level of an update one coalesced 32-wide load and a warp
+// minimum.  The state lives in position order, in shared memory when it fits
+// (a few thousand sheets), in global memory otherwise.
 //
 // The loop is a strict sequence of crossings, each a chain of dependent FP64
-// operations, so what bounds it is that chain's latency.  The four sheets
-// around a crossing sit in four lanes: they are advanced at once, the five
-// divisions of the three new pair times are one division of five lanes (a
-// second group of four lanes takes the constant terms), the two square roots
-// one square root, and a minimum is two warp-reduce instructions.  Measured
-// at 1001 sheets of a sech^2 disk: EXACT_NUMBERS
+// operations, and an FP64 instruction takes a warp 64 cycles on this part,
+// dependent or not, however few of its lanes are active (a division about 600,
+// a square root 635).  So:
+//  * the four sheets around a crossing sit in four lanes, twice: one group of
+//    four follows the velocities while the other follows the positions, so
+//    that one instruction does an operation of each (an addition as 1 a + b, a
+//    product as a b - 0: the same roundings), and the five divisions of the
+//    three new pair times are one;
+//  * times are compared as integer keys;
+//  * a second warp keeps the tree: while the first one finds the three new
+//    pair times it inserts the three before them and finds the smallest pair
+//    time outside the pairs that are changing, so that the next crossing is
+//    the smallest of four numbers.
+// A crossing of 1001 sheets of a sech^2 disk takes 1.9 us (about 160 cycles of
+// loads, 1100 to the pair's coefficients, 800 for the division, 1000 for the
+// square root, 500 to the next crossing); one lane doing all of it, with the
+// tree updated in between, took 5.3 us.
 //
 // Arithmetic, operation order and the per-sheet clocks follow the
 // reference (this file is compiled without FMA contraction, as the
@@ -43,6 +52,7 @@ using namespace wg;
 namespace {
 
 constexpr int kTreeFan = 32;
+constexpr size_t kExactStatic = 128;  // bound on k_exact_step's static shared memory
 constexpr int kMaxLevels = 6;  // 32^6 pair times: more than any N this accepts
 
 struct ExactState {
@@ -73,6 +83,7 @@ struct ExactArgs {
   double* next_tcoll;  // in/out: its time
   long long* ncoll;    // out: crossings processed
   int* err;            // out: -2 when maxcoll was reached
+  int idx0_global;     // the lowest level's indices stay in global memory
   int use_smem;        // the state is staged in shared memory (after the tree)
   size_t tree_bytes;   // shared memory of the tree's internal levels (16-byte multiple)
 };
@@ -95,7 +106,8 @@ __device__ double solve_coll_harm(double c0, double c1, double c2, double omega)
 // Order key of a pair time: increasing in the time (integer compares, off
 // the FP64 pipe), NaN after everything.
 __device__ __forceinline__ uint64_t time_key(double t) {
-  return isnan(t) ? ~0ull : key_of(t);
+  const uint64_t b = (uint64_t)__double_as_longlong(t);
+  return (b << 1) > 0xffe0000000000000ull ? ~0ull : key_of(t);
 }
 // The time of a key that is not NaN's (+0 for either zero).
 __device__ __forceinline__ double time_of_key(uint64_t k) {
@@ -111,35 +123,89 @@ __device__ __forceinline__ uint64_t warp_min_key(uint64_t k, int& where) {
   return ((uint64_t)h << 32) | l;
 }
 
-// Recomputes the tree path above pair time `leaf` (all lanes); returns the
-// root's pair index and key.
-__device__ __forceinline__ int tree_update(const ExactArgs& A, uint64_t* const* tkey,
-                                           int32_t* const* tidx, const double* tcoll, int leaf,
-                                           int lane, uint64_t& root) {
-  int g = leaf / kTreeFan;  // group at level 0
-  int j = g * kTreeFan + lane;
-  uint64_t k = j < A.level_n[0] ? time_key(tcoll[j]) : ~0ull;
-  int where;
-  uint64_t best = warp_min_key(k, where);
-  int idx = g * kTreeFan + where;
-  if (idx >= A.level_n[0]) idx = A.level_n[0] - 1;  // a group of NaN times only
-  for (int lv = 1;; ++lv) {
-    if (lane == 0) {
-      tkey[lv - 1][g] = best;
-      tidx[lv - 1][g] = idx;
+// The smallest key among the children of node g of level lv (all lanes) and
+// the pair it belongs to; children ca and cb (-1: none) of the level below
+// are taken from (ka, ia) and (kb, ib), and at level 0 the pairs lo .. hi are
+// left out.
+__device__ __forceinline__ uint64_t node_min(const ExactArgs& A, uint64_t* const* tkey,
+                                             int32_t* const* tidx, const double* tcoll, int lv,
+                                             int g, int lane, int lo, int hi, int ca, uint64_t ka,
+                                             int ia, int cb, uint64_t kb, int ib, int& idx) {
+  const int j = g * kTreeFan + lane;
+  uint64_t k = ~0ull;
+  int i = j;
+  if (j < A.level_n[lv]) {
+    if (lv == 0) {
+      if (j < lo || j > hi) k = time_key(tcoll[j]);
+    } else {
+      k = tkey[lv - 1][j];
+      i = tidx[lv - 1][j];
     }
-    if (lv == A.levels) break;
-    const int child = g;
-    g /= kTreeFan;
-    j = g * kTreeFan + lane;
-    // the child just rewritten comes from registers
-    k = j == child ? best : j < A.level_n[lv] ? tkey[lv - 1][j] : ~0ull;
-    int i = j == child ? idx : j < A.level_n[lv] ? tidx[lv - 1][j] : 0;
-    best = warp_min_key(k, where);
-    idx = __shfl_sync(0xffffffffu, i, where);
   }
-  root = best;
-  return idx;
+  if (lv > 0 && j == ca) {
+    k = ka;
+    i = ia;
+  }
+  if (lv > 0 && j == cb) {
+    k = kb;
+    i = ib;
+  }
+  int where;
+  const uint64_t best = warp_min_key(k, where);
+  idx = __shfl_sync(0xffffffffu, i, where);
+  return best;
+}
+
+// Rewrites the tree's path above pair time `leaf` (all lanes of one warp).
+__device__ __forceinline__ void tree_update(const ExactArgs& A, uint64_t* const* tkey,
+                                            int32_t* const* tidx, const double* tcoll, int leaf,
+                                            int lane) {
+  int child = -1, idx = 0;
+  uint64_t best = 0;
+  int g = leaf / kTreeFan;
+  for (int lv = 0; lv < A.levels; ++lv) {
+    best = node_min(A, tkey, tidx, tcoll, lv, g, lane, 0, -1, child, best, idx, -1, 0, 0, idx);
+    if (lane == 0) {
+      tkey[lv][g] = best;
+      tidx[lv][g] = idx;
+    }
+    child = g;
+    g /= kTreeFan;
+  }
+  __syncwarp();
+}
+
+// The smallest pair time outside the pairs lo .. hi (at most three, in one
+// group of leaves or two adjacent ones) and its pair; the tree is left alone.
+__device__ __forceinline__ uint64_t tree_min_outside(const ExactArgs& A, uint64_t* const* tkey,
+                                                     int32_t* const* tidx, const double* tcoll,
+                                                     int lo, int hi, int lane, int& idx) {
+  int ca = -1, cb = -1, ia = 0, ib = 0;
+  uint64_t ka = 0, kb = 0;
+  int ga = lo / kTreeFan, gb = hi / kTreeFan;
+  for (int lv = 0; lv < A.levels; ++lv) {
+    int na, nb = 0;
+    const uint64_t qa = node_min(A, tkey, tidx, tcoll, lv, ga, lane, lo, hi, ca, ka, ia, cb, kb,
+                                 ib, na);
+    uint64_t qb = 0;
+    if (gb != ga)
+      qb = node_min(A, tkey, tidx, tcoll, lv, gb, lane, lo, hi, ca, ka, ia, cb, kb, ib, nb);
+    ca = ga;
+    ka = qa;
+    ia = na;
+    cb = gb != ga ? gb : -1;
+    kb = qb;
+    ib = nb;
+    ga /= kTreeFan;
+    gb /= kTreeFan;
+  }
+  idx = ia;
+  return ka;
+}
+
+// -x without an FP64 instruction.
+__device__ __forceinline__ double negated(double x) {
+  return __longlong_as_double(__double_as_longlong(x) ^ (long long)0x8000000000000000ull);
 }
 
 // Advance (x, v) from the sheet's own clock t to time tn (reference
@@ -161,9 +227,18 @@ __device__ __forceinline__ void advance(double& x, double& v, double a, double t
   }
 }
 
-__global__ void __launch_bounds__(32, 1) k_exact_step(const ExactArgs A) {
+template <bool HARM>
+__global__ void __launch_bounds__(64, 1) k_exact_step(const ExactArgs A) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const int lane = threadIdx.x;
+  // the new times of the pairs ci - 1, ci, ci + 1 and the smallest time
+  // elsewhere, written before and read after the barrier that ends a
+  // crossing; used alternately, so that neither is overwritten while the
+  // other warp still reads it
+  __shared__ double s_new[2][3];
+  __shared__ uint64_t s_newkey[2][3];
+  __shared__ uint64_t s_rest[2];
+  __shared__ int s_rest_idx[2];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n = A.n;
   ExactState S = A.p;
   // the tree's internal levels: in shared memory always (n / 31 entries)
@@ -175,14 +250,15 @@ __global__ void __launch_bounds__(32, 1) k_exact_step(const ExactArgs A) {
       tkey[lv] = reinterpret_cast<uint64_t*>(p);
       p += 8 * (size_t)A.level_n[lv + 1];
     }
-    for (int lv = 0; lv < A.levels; ++lv) {
+    for (int lv = A.levels - 1; lv >= 0; --lv) {
       tidx[lv] = reinterpret_cast<int32_t*>(p);
       p += 4 * (size_t)A.level_n[lv + 1];
     }
+    if (A.idx0_global) tidx[0] = A.tree_idx[0];
     for (int lv = 0; lv < A.levels; ++lv)
-      for (int j = lane; j < A.level_n[lv + 1]; j += 32) {
+      for (int j = tid; j < A.level_n[lv + 1]; j += 64) {
         tkey[lv][j] = A.tree_key[lv][j];
-        tidx[lv][j] = A.tree_idx[lv][j];
+        if (lv > 0 || !A.idx0_global) tidx[lv][j] = A.tree_idx[lv][j];
       }
     p = smem + A.tree_bytes;
     if (A.use_smem) {
@@ -195,7 +271,7 @@ __global__ void __launch_bounds__(32, 1) k_exact_step(const ExactArgs A) {
       S.t = d + 4 * n;
       S.tcoll = d + 5 * n;
       S.id = reinterpret_cast<int32_t*>(d + 6 * n);
-      for (int i = lane; i < n; i += 32) {
+      for (int i = tid; i < n; i += 64) {
         const int s = A.g.id[i];
         S.id[i] = s;
         S.x[i] = A.g.x[s];
@@ -206,103 +282,155 @@ __global__ void __launch_bounds__(32, 1) k_exact_step(const ExactArgs A) {
       }
     }
   }
-  for (int i = lane; i < n; i += 32) S.t[i] = 0.;
-  __syncwarp();
+  for (int i = tid; i < n; i += 64) S.t[i] = 0.;
+  __syncthreads();
   const double omega = A.omega, dt = A.dt;
   int cindx = *A.cindx;
   double next = *A.next_tcoll;
+  uint64_t knext = time_key(next);
+  const uint64_t kdt = key_of(dt);
   long long cnt = 0;
-  // lanes 0 .. 3 (and 4 .. 7 again, for the second divisions) hold the
-  // sheets at positions ci - 1 .. ci + 2 of a crossing of ci and ci + 1
+  // warp 0: lanes 0 .. 3, and again lanes 4 .. 7, hold the sheets at positions
+  // ci - 1 .. ci + 2 of a crossing of ci and ci + 1 (the other lanes do the
+  // same work and write nothing)
   const int role = lane & 3;
-  const bool mid = role == 1 || role == 2, first = lane < 4;
-  while (next < dt && cnt < A.maxcoll) {
+  const bool mid = role == 1 || role == 2;
+  const bool pos_chain = (lane & 4) != 0;  // follows positions (else velocities)
+  // partners in the new pairs: the left neighbour meets the sheet from
+  // ci + 1, the right one that from ci, and those two each other
+  const int partner = (lane & 28) | (role == 0 ? 2 : role == 3 ? 1 : role ^ 3);
+  const double num_scale = mid ? 2.0 : pos_chain ? 4.0 : -1.0;
+  const double den_scale = mid ? -1.0 : 0.5;
+  int prev = -1;  // pair of the crossing before (its new times await insertion)
+  while (knext < kdt && cnt < A.maxcoll) {
+    const int buf = (int)(cnt & 1);
     ++cnt;
     const int ci = cindx;
-    const int pos = ci - 1 + role;
-    const bool have = pos >= 0 && pos < n;  // the outer two may not exist
-    const int at = have ? pos : ci;
-    double x = S.x[at], v = S.v[at], a = S.a[at], t = S.t[at];
-    const double m = S.m[at];
-    const int32_t id = S.id[at];
-    // to the time of the crossing.  Without a harmonic potential the outer
-    // two are only extrapolated, in the reference's order of additions
-    // ((x + a t^2 / 2) + v t, against x + (a t^2 / 2 + v t)), and keep their
-    // clocks
-    if (omega > 0) {
-      advance(x, v, a, t, next, omega);
-    } else {
-      const double tdt = next - t;
-      const double dv = a * tdt;
-      const double p = dv * tdt / 2., q = v * tdt;
-      x = (p + (mid ? q : x)) + (mid ? x : q);
-      v += dv;
-    }
-    // the two swap places and exchange accelerations by the mass difference
-    {
-      const double mo = __shfl_xor_sync(0xffffffffu, m, 3);
-      const double dm = role == 1 ? mo - m : m - mo;
-      const double ad = a - dm;
-      const double ao = __shfl_xor_sync(0xffffffffu, ad, 3);
-      if (mid) a = ao;
-    }
-    // partners of the new pairs: the left neighbour meets the sheet from
-    // ci + 1, the right one that from ci, and those two each other
-    const int partner = (lane & 4) | (role == 0 ? 2 : role == 3 ? 1 : role ^ 3);
-    const double xp = __shfl_sync(0xffffffffu, x, partner);
-    const double vp = __shfl_sync(0xffffffffu, v, partner);
-    const double ap = __shfl_sync(0xffffffffu, a, partner);
-    double tn;
-    if (omega > 0) {
-      if (mid) {
-        double q = (v - vp) / (ap - a) / omega;
-        q *= q;
-        q = (1. - q) / (1. + q);
-        tn = acos(q) / omega;
+    if (warp == 0) {
+      const int pos = ci - 1 + role;
+      const bool have = pos >= 0 && pos < n;  // the outer two may not exist
+      const int at = have ? pos : ci;
+      const double t = S.t[at], v = S.v[at], m = S.m[at];
+      double x = S.x[at], a = S.a[at];
+      const int32_t id = S.id[at];
+      double tn, vn;
+      if constexpr (HARM) {
+        vn = v;
+        advance(x, vn, a, t, next, omega);
+        // the two swap places and exchange accelerations by the mass difference
+        const double mo = __shfl_xor_sync(0xffffffffu, m, 3);
+        const double dm = (role == 1 ? mo : m) - (role == 1 ? m : mo);
+        const double ad = a - dm;
+        const double ao = __shfl_xor_sync(0xffffffffu, ad, 3);
+        if (mid) a = ao;
+        const double xp = __shfl_sync(0xffffffffu, x, partner);
+        const double vp = __shfl_sync(0xffffffffu, vn, partner);
+        const double ap = __shfl_sync(0xffffffffu, a, partner);
+        if (mid) {
+          double q = (vn - vp) / (ap - a) / omega;
+          q *= q;
+          q = (1. - q) / (1. + q);
+          tn = acos(q) / omega;
+        } else {
+          tn = solve_coll_harm(x - xp, vn - vp, a - ap, omega);
+        }
       } else {
-        tn = solve_coll_harm(x - xp, v - vp, a - ap, omega);
+        // to the time of the crossing; the outer two are only extrapolated,
+        // in the reference's order of additions ((x + a t^2 / 2) + v t,
+        // against x + (a t^2 / 2 + v t)), and keep their state
+        const double tdt = next - t;
+        const double dv = a * tdt;
+        // velocities: v + dv          positions: dv tdt
+        const double r3 = __fma_rn(pos_chain ? dv : 1.0, pos_chain ? tdt : dv,
+                                   pos_chain ? -0.0 : v);
+        // velocities: mass difference   positions: v tdt
+        const double mo = __shfl_xor_sync(0xffffffffu, m, 3);
+        const double r4 = __fma_rn(pos_chain ? v : 1.0, pos_chain ? tdt : role == 1 ? mo : m,
+                                   pos_chain ? -0.0 : negated(role == 1 ? m : mo));
+        const double half = r3 * 0.5;
+        // velocities: a less that difference   positions: first addition
+        const double r5 = (pos_chain ? half : a) +
+                          (pos_chain ? (mid ? r4 : x) : negated(r4));
+        const double ao = __shfl_xor_sync(0xffffffffu, r5, 3);
+        if (mid) a = ao;
+        const double ap = __shfl_sync(0xffffffffu, a, partner);
+        // velocities: difference of accelerations   positions: second addition
+        const double r6 = (pos_chain ? r5 : a) + (pos_chain ? (mid ? x : r4) : negated(ap));
+        vn = r3;
+        x = r6;
+        const double y = pos_chain ? r6 : r3;
+        const double c = y - __shfl_sync(0xffffffffu, y, partner);
+        const double da = __shfl_sync(0xffffffffu, r6, lane & 27);
+        // the outer pairs' quadratic c2 t^2 + c1 t + c0 (wendy/wendy.c:33-38),
+        // -c1 / c2 in the velocity lanes and 4 c0 / c2 in the position lanes,
+        // and the inner pair's other root
+        const double quo = (c * num_scale) / (da * den_scale);
+        const double qc = __shfl_xor_sync(0xffffffffu, quo, 4);
+        const double disc = quo * quo - qc;
+        // (lanes without a root of their own take 1: negative numbers would
+        // send the whole warp through the slow path of the square root)
+        tn = mid ? quo : 0.5 * (quo + sqrt(mid || pos_chain ? 1.0 : disc));
+      }
+      if (lane < 8) {
+        const int to = mid ? (role == 1 ? ci + 1 : ci) : at;
+        const bool moves = mid || (HARM && have);
+        if (moves && pos_chain) S.x[to] = x;
+        if (moves && !pos_chain) {
+          S.v[to] = vn;
+          S.t[to] = next;
+        }
+        if (mid && !pos_chain) {
+          S.a[to] = a;
+          S.m[to] = m;
+          S.id[to] = id;
+        }
+        // role 0: pair ci - 1, role 1: pair ci, role 3: pair ci + 1
+        if (!pos_chain && role != 2) {
+          const double when = next + tn;
+          s_new[buf][role == 3 ? 2 : role] = when;
+          s_newkey[buf][role == 3 ? 2 : role] = have ? time_key(when) : ~0ull;
+        }
       }
     } else {
-      // the outer pairs' quadratic c2 t^2 + c1 t + c0 (wendy/wendy.c:33-38)
-      // and the inner pair's other root, one division per lane
-      const double c0 = x - xp, c1 = v - vp, c2 = 0.5 * (a - ap);
-      const double num = mid ? 2. * c1 : first ? -c1 : 4. * c0;
-      const double quo = num / (mid ? ap - a : c2);
-      const double qc = __shfl_xor_sync(0xffffffffu, quo, 4);
-      tn = mid ? quo : 0.5 * (quo + sqrt(quo * quo - qc));
-    }
-    if (first) {
-      if (mid) {
-        const int to = role == 1 ? ci + 1 : ci;
-        S.x[to] = x;
-        S.v[to] = v;
-        S.a[to] = a;
-        S.m[to] = m;
-        S.t[to] = next;
-        S.id[to] = id;
-      } else if (have && omega > 0) {
-        S.x[at] = x;
-        S.v[at] = v;
-        S.t[at] = next;
+      // the new times of the crossing before enter the tree, then the
+      // smallest time outside this crossing's pairs
+      if (prev >= 0) {
+        const int lo = prev > 0 ? prev - 1 : prev, hi = prev < n - 2 ? prev + 1 : prev;
+        if (lane < 3 && prev - 1 + lane >= lo && prev - 1 + lane <= hi)
+          S.tcoll[prev - 1 + lane] = s_new[buf ^ 1][lane];
+        __syncwarp();
+        tree_update(A, tkey, tidx, S.tcoll, lo, lane);
+        if (hi / kTreeFan != lo / kTreeFan) tree_update(A, tkey, tidx, S.tcoll, hi, lane);
       }
-      // role 0: pair ci - 1, role 1: pair ci, role 3: pair ci + 1
-      if (role != 2 && have) S.tcoll[role == 3 ? ci + 1 : ci - 1 + role] = next + tn;
+      int idx;
+      const uint64_t rest = tree_min_outside(A, tkey, tidx, S.tcoll, ci > 0 ? ci - 1 : ci,
+                                             ci < n - 2 ? ci + 1 : ci, lane, idx);
+      if (lane == 0) {
+        s_rest[buf] = rest;
+        s_rest_idx[buf] = idx;
+      }
     }
-    __syncwarp();
-    // the three pair times that changed, and their paths up the tree; the
-    // next crossing is the root
-    const int lo = ci > 0 ? ci - 1 : ci, hi = ci < n - 2 ? ci + 1 : ci;
-    uint64_t root;
-    cindx = tree_update(A, tkey, tidx, S.tcoll, lo, lane, root);
-    if (hi / kTreeFan != lo / kTreeFan) {
-      __syncwarp();
-      cindx = tree_update(A, tkey, tidx, S.tcoll, hi, lane, root);
+    __syncthreads();
+    // the next crossing: ties to the lower pair; NaN times (pairs that never
+    // meet) never come first
+    prev = ci;
+    knext = s_rest[buf];
+    cindx = s_rest_idx[buf];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      const uint64_t k = s_newkey[buf][r];
+      if (k < knext || (k == knext && k != ~0ull && ci - 1 + r < cindx)) {
+        knext = k;
+        cindx = ci - 1 + r;
+      }
     }
-    next = root == ~0ull ? INFINITY : time_of_key(root);
-    __syncwarp();
+    next = knext == ~0ull ? INFINITY : time_of_key(knext);
   }
+  if (warp == 1 && prev >= 0 && lane < 3 && prev - 1 + lane >= 0 && prev - 1 + lane < n - 1)
+    S.tcoll[prev - 1 + lane] = s_new[(int)(cnt & 1) ^ 1][lane];
+  __syncthreads();
   // every sheet to the end of the interval, clocks and pending times shifted
-  for (int i = lane; i < n; i += 32) {
+  for (int i = tid; i < n; i += 64) {
     double x = S.x[i], v = S.v[i];
     advance(x, v, S.a[i], S.t[i], dt, omega);
     if (A.use_smem) {
@@ -319,8 +447,8 @@ __global__ void __launch_bounds__(32, 1) k_exact_step(const ExactArgs A) {
     }
   }
   // the tree holds absolute times of this interval: rebuilt by the host's
-  // next call (k_exact_tree), like the reference rebuilds its BST per call
-  if (lane == 0) {
+  // next call (k_exact_tree_level), like the reference rebuilds its BST per call
+  if (tid == 0) {
     *A.cindx = cindx;
     *A.next_tcoll = next - dt;
     *A.ncoll = cnt;
@@ -485,7 +613,7 @@ int wg_exact_create(int64_t n, const double* x, const double* v, const double* a
   int dev = 0, optin = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  A.use_smem = smem <= (size_t)optin;
+  A.use_smem = smem + kExactStatic <= (size_t)optin;
   const size_t total = 6 * nd + ni + tree_b + al(64) + (A.use_smem ? 0 : 4 * nd + ni);
   if (cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreate(&e->ev0) != cudaSuccess || cudaEventCreate(&e->ev1) != cudaSuccess ||
@@ -526,8 +654,14 @@ int wg_exact_create(int64_t n, const double* x, const double* v, const double* a
   A.ncoll = reinterpret_cast<long long*>(A.cindx + 2);
   A.next_tcoll = reinterpret_cast<double*>(A.cindx + 4);
   e->smem = A.use_smem ? smem : A.tree_bytes;
-  if (e->smem > (size_t)optin ||
-      cudaFuncSetAttribute(k_exact_step, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  bool fits = e->smem <= (size_t)optin;
+  // the kernel's own shared variables come on top: within that of the limit,
+  // the lowest level's indices (the last part of the tree) stay outside
+  A.idx0_global = fits && e->smem + kExactStatic > (size_t)optin;
+  if (A.idx0_global) e->smem -= 4 * (size_t)A.level_n[1];
+  if (!fits ||
+      cudaFuncSetAttribute(A.omega > 0 ? k_exact_step<true> : k_exact_step<false>,
+                           cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)e->smem) != cudaSuccess) {
     cudaGetLastError();
     free_exact(e);
@@ -585,7 +719,10 @@ int wg_exact_step(wg_exact* e, double dt, int64_t maxcoll, int64_t* ncoll,
   const unsigned blocks = (unsigned)((e->n + 255) / 256);
   cudaEventRecord(e->ev0, s);
   if (!A.use_smem) k_exact_gather<<<blocks, 256, 0, s>>>(A);
-  k_exact_step<<<1, 32, e->smem, s>>>(A);
+  if (A.omega > 0)
+    k_exact_step<true><<<1, 64, e->smem, s>>>(A);
+  else
+    k_exact_step<false><<<1, 64, e->smem, s>>>(A);
   if (!A.use_smem) k_exact_scatter<<<blocks, 256, 0, s>>>(A);
   cudaEventRecord(e->ev1, s);
   cudaMemcpyAsync(e->h_ret, A.cindx, 24, cudaMemcpyDeviceToHost, s);
