@@ -14,6 +14,7 @@
 #include "wg_bucket.cuh"
 #include "wg_ext.cuh"
 #include "wg_internal.cuh"
+#include "wg_small.cuh"
 
 using namespace wg;
 
@@ -159,6 +160,7 @@ struct wg_sim {
   // a call enqueued by wg_step_begin and not yet completed by wg_step_end
   bool pend_active = false;
   bool pend_compact = false;     // ... and it runs on the compact path
+  bool pend_small = false;       // ... or in one launch (wg_small.cu)
   double pend_dt = 0;
   int pend_nleap = 0, pend_lay0 = 0, pend_cs0 = 0;
   double pend_pre = 0;           // the opening half drift its first sub-step applies
@@ -981,6 +983,47 @@ static int run_call_begin(wg_sim* s, double dt, int nleap, double* t0, bool reco
   int rc = alloc_call_arrays(s, nleap);
   if (rc) return rc;
   fill_times(s, dt, nleap, t0);
+  if (s->n <= kSmallSheets) {
+    // one launch for the whole call; the sheets stay in the compact sets
+    if (record_start) WG_CUDA(cudaEventRecord(s->ev0, s->stream));
+    if (s->mode == 1) {
+      WG_CUDA(cudaMemsetAsync(s->ocount, 0, 16, s->stream));
+      bucket_to_compact(s, s->lay, s->cslot);
+      s->mode = 0;
+    }
+    if (s->ext.kind == EXT_PULSE_TANH || s->ext.kind == EXT_EXPR)
+      WG_CUDA(cudaMemcpyAsync(s->t_seq, s->h_t, 8 * (size_t)nleap, cudaMemcpyHostToDevice,
+                              s->stream));
+    SmallArgs a;
+    a.table = s->table;
+    a.n = (int)s->n;
+    a.nleap = nleap;
+    a.dt = dt;
+    a.pre = dt / 2.;
+    a.T_lo = s->T_lo;
+    a.T_hi = s->T_hi;
+    a.E = s->E;
+    a.has_omega = s->omega2 >= 0;
+    a.omega2 = s->omega2;
+    a.ext = s->ext;
+    a.t_seq = s->t_seq;
+    a.x_out = s->x_out;
+    a.v_out = s->v_out;
+    a.a_out = s->call_a;
+    a.xi_out = s->call_xi;
+    a.flag = s->flags;
+    WG_CUDA(cudaMemsetAsync(s->flags, 0, sizeof(StepFlags), s->stream));
+    s->st.launches += launch_small_run(a, s->stream);
+    WG_CUDA(cudaGetLastError());
+    WG_CUDA(cudaMemcpyAsync(s->h_flags, s->flags, sizeof(StepFlags), cudaMemcpyDeviceToHost,
+                            s->stream));
+    WG_CUDA(cudaEventRecord(s->ev1, s->stream));
+    s->pend_active = true;
+    s->pend_small = true;
+    s->pend_dt = dt;
+    s->pend_nleap = nleap;
+    return WG_OK;
+  }
   if (s->compact_calls > 0) {
     // a recent overflow right after a re-sort: this call runs on the compact
     // path (full re-sort + fused force kernel per sub-step)
@@ -1067,6 +1110,24 @@ static int run_call_end(wg_sim* s, double* time_elapsed) {
   const double dt = s->pend_dt;
   const int nleap = s->pend_nleap;
   int rc = WG_OK;
+  if (s->pend_small) {
+    s->pend_small = false;
+    WG_CUDA(cudaEventSynchronize(s->ev1));
+    s->out_valid = true;
+    s->mode = 0;
+    s->pending_dt = dt;
+    s->st.substeps += nleap;
+    s->st.sorts_full += s->h_flags[0].unsorted;
+    s->st.sorts_window += nleap - (int64_t)s->h_flags[0].unsorted;
+    s->st.last_max_count = s->h_flags[0].max_cnt;
+    double vmax;
+    std::memcpy(&vmax, &s->h_flags[0].max_v, 8);
+    s->st.last_max_disp = vmax * std::fabs(dt / 2.);
+    float ms = 0;
+    cudaEventElapsedTime(&ms, s->ev0, s->ev1);
+    if (time_elapsed) *time_elapsed = ms * 1e-3;
+    return WG_OK;
+  }
   if (s->pend_compact) {
     s->pend_compact = false;
     WG_CUDA(cudaEventRecord(s->ev1, s->stream));
@@ -1325,8 +1386,17 @@ int wg_profile(wg_sim* s, int what, int reps, double* avg_seconds) {
     return WG_ERR_ARG;
   }
   if (what == WG_PROF_BUCKET && s->mode != 1) {
-    set_error("wg_profile(WG_PROF_BUCKET) needs the bucket layout: run wg_step first");
-    return WG_ERR_ARG;
+    if (s->n > kSmallSheets || s->st.substeps == 0) {
+      set_error("wg_profile(WG_PROF_BUCKET) needs the bucket layout: run wg_step first");
+      return WG_ERR_ARG;
+    }
+    // a small simulation's steps leave it compact: lay its sheets out here
+    launch_drift(s->table, s->n, 0.0, &s->flags[0], s->stream);  // (marks "unsorted")
+    radix_sort_state(s->table, s->n, &s->radix, &s->flags[0], s->err, s->stream);
+    launch_bucketize(s->table, s->n, s->tune.target, s->nb, s->capg, s->E, s->bx[0], s->bv[0],
+                     s->bm[0], s->bi[0], s->bcnt, s->bmass, s->qk[0], s->qi[0], s->stream);
+    s->lay = s->qsel = s->cslot = 0;
+    s->mode = 1;
   }
   // the force and sort kernels run on the compact sets, which hold other
   // data while the sheets live in buckets: hand the current state back to
@@ -1760,7 +1830,7 @@ int wg_nbody_approx_onestep(int n, wg_sheet* xi, double* x, double* v, const dou
     } else {
       drop_spec();
     }
-  } else if (candidate && s->mode == 1) {
+  } else if (candidate && (s->mode == 1 || n <= kSmallSheets)) {
     WG_CUDA(cudaEventSynchronize(s->ev_up));
     if (*h_diff == 0) {
       point_at(out);
@@ -1802,7 +1872,8 @@ int wg_nbody_approx_onestep(int n, wg_sheet* xi, double* x, double* v, const dou
   }
   // desorts above ran on the main stream: done before the downloads
   WG_CUDA(cudaStreamSynchronize(s->stream));
-  s->resume_ok = s->mode == 1;
+  // (small simulations end compact, in the state the next call opens from)
+  s->resume_ok = s->mode == 1 || n <= kSmallSheets;
   s->resume_totmass = totmass;
   // the next call's sub-steps, enqueued now on the main stream: they run
   // while this call's outputs download and the caller works on them
