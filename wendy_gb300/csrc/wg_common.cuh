@@ -294,6 +294,27 @@ struct ExtForce {
   const long long* ttab;  // EXT_PULSE_TANH: the device's tanh table (wg_tanh.cuh)
 };
 
+// a^b of an expression.  pow() is some hundred FP64 instructions; a power of 3
+// .. 8 is a few products, each with its rounding error carried along (so the
+// result is within half an ulp and a few 2^-53 of it, pow() is within one).
+// Results that are not comfortably normal (zeros, their signs, underflow,
+// overflow, infinities, NaN) are left to pow().
+__device__ __forceinline__ double expr_pow(double a, double b) {
+  const int k = __double2int_rn(b);
+  if ((unsigned)(k - 3) <= 5u && (double)k == b) {
+    double h = a, l = 0.0;
+    for (int i = 1; i < k; ++i) {
+      const double t = h * a;
+      l = fma(l, a, fma(h, a, -t));
+      h = t;
+    }
+    h += l;
+    const unsigned e = ((unsigned)__double2hiint(h) >> 20) & 0x7ffu;
+    if (e - 100u < 1900u) return h;
+  }
+  return pow(a, b);
+}
+
 // Runs ops [lo, hi) of an expression program on the registers r.
 static __device__ __noinline__ void expr_run(const ExprOp* __restrict__ prog, int lo, int hi,
                                              double* r, double x, double t) {
@@ -311,7 +332,7 @@ static __device__ __noinline__ void expr_run(const ExprOp* __restrict__ prog, in
       case XOP_MUL: y = va * vb; break;
       case XOP_DIV: y = va / vb; break;
       case XOP_NEG: y = -va; break;
-      case XOP_POW: y = pow(va, vb); break;
+      case XOP_POW: y = expr_pow(va, vb); break;
       case XOP_EXP: y = exp(va); break;
       case XOP_LOG: y = log(va); break;
       case XOP_SQRT: y = sqrt(va); break;
