@@ -780,9 +780,14 @@ void launch_substep(wg_sim* s, int i, int nleap, int profile) {
     // the samples this sub-step wrote, sorted, become the splitters it
     // would have published (those of the layout after next)
     const int q = 1 - ((s->dev.qsel0 + i) & 1);
-    radix_sort_state(s->ptab, s->nb - 1, &s->pradix, s->pflag, s->err, s->stream);
-    launch_samples_to_splitters(s->ptab, s->nb - 1, s->qk[q], s->qi[q], s->stream);
-    s->st.launches += kRadixLaunches + 1;
+    if (s->nb - 1 <= kRankSamples) {
+      launch_rank_samples(s->ptab, (int)(s->nb - 1), s->qk[q], s->qi[q], s->stream);
+      s->st.launches += 1;
+    } else {
+      radix_sort_state(s->ptab, s->nb - 1, &s->pradix, s->pflag, s->err, s->stream);
+      launch_samples_to_splitters(s->ptab, s->nb - 1, s->qk[q], s->qi[q], s->stream);
+      s->st.launches += kRadixLaunches + 1;
+    }
     if (!profile) s->st.substeps_predicted += 1;
   }
 }
@@ -794,6 +799,14 @@ void fill_times(wg_sim* s, double dt, int nleap, double* t0) {
     if (s->ext.kind != EXT_NONE) t += dt;  // wendy/wendy.c:403-404,409-410
   }
   if (t0) *t0 = t;
+}
+
+// Whether a call runs as one launch of one CTA (wg_small.cu).  An expression
+// force is FP64 work for every sheet, which one SM does at its own rate only:
+// it stops paying earlier (measured per sub-step at 1500 / 2048 sheets: 25.6 /
+// 34.0 us in one CTA against 29.4 in buckets).
+bool one_launch(const wg_sim* s) {
+  return s->n <= (s->ext.kind == EXT_EXPR ? kSmallExprSheets : kSmallSheets);
 }
 
 // Cache of one simulation for the stateless reference-shaped entry point.
@@ -983,7 +996,7 @@ static int run_call_begin(wg_sim* s, double dt, int nleap, double* t0, bool reco
   int rc = alloc_call_arrays(s, nleap);
   if (rc) return rc;
   fill_times(s, dt, nleap, t0);
-  if (s->n <= kSmallSheets) {
+  if (one_launch(s)) {
     // one launch for the whole call; the sheets stay in the compact sets
     if (record_start) WG_CUDA(cudaEventRecord(s->ev0, s->stream));
     if (s->mode == 1) {
@@ -1386,7 +1399,7 @@ int wg_profile(wg_sim* s, int what, int reps, double* avg_seconds) {
     return WG_ERR_ARG;
   }
   if (what == WG_PROF_BUCKET && s->mode != 1) {
-    if (s->n > kSmallSheets || s->st.substeps == 0) {
+    if (!one_launch(s) || s->st.substeps == 0) {
       set_error("wg_profile(WG_PROF_BUCKET) needs the bucket layout: run wg_step first");
       return WG_ERR_ARG;
     }
@@ -1830,7 +1843,7 @@ int wg_nbody_approx_onestep(int n, wg_sheet* xi, double* x, double* v, const dou
     } else {
       drop_spec();
     }
-  } else if (candidate && (s->mode == 1 || n <= kSmallSheets)) {
+  } else if (candidate && (s->mode == 1 || one_launch(s))) {
     WG_CUDA(cudaEventSynchronize(s->ev_up));
     if (*h_diff == 0) {
       point_at(out);
@@ -1873,7 +1886,7 @@ int wg_nbody_approx_onestep(int n, wg_sheet* xi, double* x, double* v, const dou
   // desorts above ran on the main stream: done before the downloads
   WG_CUDA(cudaStreamSynchronize(s->stream));
   // (small simulations end compact, in the state the next call opens from)
-  s->resume_ok = s->mode == 1 || n <= kSmallSheets;
+  s->resume_ok = s->mode == 1 || one_launch(s);
   s->resume_totmass = totmass;
   // the next call's sub-steps, enqueued now on the main stream: they run
   // while this call's outputs download and the caller works on them

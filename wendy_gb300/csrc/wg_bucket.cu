@@ -1749,6 +1749,47 @@ __global__ void k_samples_to_splitters(const StateTable* table, int64_t m, uint6
   }
 }
 
+// One warp per sample: its rank among all (key, index, place) triples is the
+// splitter it becomes.  A quadratic count, but one launch: for the few hundred
+// to few thousand buckets that predicted splitters are sorted for after every
+// sub-step, the radix sort's fourteen dependent launches took 110 us
+// whatever their size, this takes about 4 us at 650 samples (bound by the
+// latency of its loads) and 40 at the limit (by issue).
+constexpr int kRankThreads = 256;
+__global__ void __launch_bounds__(kRankThreads) k_rank_samples(const StateTable* table, int m,
+                                                               uint64_t* qk, int32_t* qi) {
+  const int lane = threadIdx.x & 31;
+  const int j = blockIdx.x * (kRankThreads / 32) + (threadIdx.x >> 5);
+  if (j >= m) return;
+  const StateRef c = table->cur;
+  const uint64_t kj = key_of(c.x[j]);
+  const int32_t ij = c.idx[j];
+  unsigned r = 0;
+#pragma unroll 4
+  for (int i = lane; i < m; i += 32) {
+    const uint64_t k = key_of(c.x[i]);
+    if (k <= kj) {
+      bool less = k < kj;
+      if (!less) {
+        const int32_t x = c.idx[i];
+        less = x < ij || (x == ij && i < j);
+      }
+      r += less ? 1u : 0u;
+    }
+  }
+  r = __reduce_add_sync(0xffffffffu, r);
+  if (lane == 0) {
+    qk[r + 1] = kj;
+    qi[r + 1] = ij;
+  }
+}
+
+void launch_rank_samples(const StateTable* table, int m, uint64_t* qk, int32_t* qi,
+                         cudaStream_t s) {
+  const int per = kRankThreads / 32;
+  k_rank_samples<<<(unsigned)((m + per - 1) / per), kRankThreads, 0, s>>>(table, m, qk, qi);
+}
+
 // Exclusive scan of each batch member's clamped bucket counts (one block per
 // member): offs[toff + b] = sheets of the member's buckets before b.
 __global__ void k_batch_offsets(const SimDev* devs, const BatchSeg* segs, unsigned* offs) {

@@ -206,6 +206,11 @@ void launch_batch_bucketize(const SimDev* devs, const BatchSeg* segs, const Buck
 // (predicted splitters): keys of their positions, and their indices.
 void launch_samples_to_splitters(const StateTable* table, int64_t m, uint64_t* qk, int32_t* qi,
                                  cudaStream_t s);
+// The same from unsorted samples, m of them at most kRankSamples: each sample's
+// splitter is its rank, counted against all the others.
+constexpr int kRankSamples = 8192;
+void launch_rank_samples(const StateTable* table, int m, uint64_t* qk, int32_t* qi,
+                         cudaStream_t s);
 // x_out, v_out (and a_out when not null) from the records of rec_out.
 void launch_split_out(const OutRec* rec, int64_t n, double* x_out, double* v_out, double* a_out,
                       cudaStream_t s);

@@ -13,7 +13,9 @@
 //
 // What bounds it is the latency of a sub-step's dependent FP64 operations (64
 // cycles each) and two barriers; launches, the routing between buckets and
-// their look-back are gone.  SMALL_NUMBERS
+// their look-back are gone.  Per sub-step, against the bucket kernel: 0.5 us
+// against 20 (64 sheets), 4.3 against 34.9 (1000 sheets, few crossings), 9.9
+// against 41.7 (1000 sheets, all moving by several places).
 //
 // Arithmetic as in k_bucket_step, operation by operation, so results do not
 // depend on which of the two ran.
