@@ -69,12 +69,10 @@ struct ForceArgs {
 struct RadixWork {
   uint64_t* keys[2];
   uint32_t* pos[2];
-  uint32_t* hist;       // 8 x 256 digit counts
   uint32_t* plan;       // per-pass: active, src, dst; final buffer; digit starts
-  uint32_t* status;     // 8 passes x tiles x 256 look-back words
-  uint32_t* counters;   // 8 tile tickets + tie flag
-  int64_t n_tiles;
-  size_t scratch_bytes; // bytes of status + counters (cleared before each sort)
+  uint32_t* hist;       // 8 x 256 digit counts ...
+  uint32_t* counters;   // ... tile tickets, tie flag ...
+  uint32_t* status;     // ... passes x tiles x 256 look-back words: cleared together
 };
 
 // Devices whose one-time kernel set-up (attributes, occupancy) is cached;
@@ -102,8 +100,13 @@ constexpr int kForceItems = 8;
 constexpr int kForceTile = kForceThreads * kForceItems;
 
 constexpr int kRadixThreads = 256;
-constexpr int kRadixItems = 16;
+// Keys per thread of a pass: tiles of 4096 keys where they fill the device;
+// smaller sorts take tiles of 1024, whose latency (a tile is ranked, staged and
+// written by one CTA) is a third of it.
+constexpr int kRadixItems = 16, kRadixItemsSmall = 4;
 constexpr int kRadixTile = kRadixThreads * kRadixItems;
+constexpr int kRadixTileSmall = kRadixThreads * kRadixItemsSmall;
+constexpr int64_t kRadixSmallSheets = 1 << 18;
 
 // --- launchers (wg_kernels.cu) ---
 void launch_force(const ForceArgs& a, int64_t n_tiles, cudaStream_t s);
@@ -138,14 +141,17 @@ void record_last_error(const char* msg);
 void host_pages_dirty(void* p, size_t bytes);
 
 // --- launchers (wg_radix.cu) ---
-constexpr int kRadixLaunches = 14;  // kernels radix_sort_state enqueues (hist, plan, 8 passes,
-                                    // gather, ties, long ties, flip)
+constexpr int kRadixLaunches = 9;  // kernels radix_sort_state enqueues (hist, five passes,
+                                   // gather, ties, long ties)
 size_t radix_bytes(int64_t n);
 void radix_bind(RadixWork* w, void* base, int64_t n);
 // Sort table->cur by (position key, original index) unless flags->unsorted
 // is zero; the sorted sheets end in table->cur (the sets are swapped on the
-// device).  err receives DEV_ERR_RADIX_TIMEOUT if a wait expired.
+// device).  err receives DEV_ERR_RADIX_TIMEOUT if a wait expired.  whole_keys:
+// sort by all eight bytes of the keys (for keys that differ in low bytes
+// only); otherwise by their leading bytes first, which is faster for
+// positions.
 void radix_sort_state(StateTable* table, int64_t n, RadixWork* w, const StepFlags* flag,
-                      unsigned* err, cudaStream_t s);
+                      unsigned* err, cudaStream_t s, bool whole_keys = false);
 
 }  // namespace wg

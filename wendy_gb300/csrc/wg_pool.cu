@@ -1097,7 +1097,7 @@ static int pool_step_end(wg_pool* p, double* time_elapsed) {
         while ((int64_t)1 << rank_bits < sheets) ++rank_bits;
         k_seg_prep_b<<<grid_1d(sheets), 256, 0, p->stream>>>(p->btA, p->bseg_out, nseg,
                                                              p->bB[0], sheets, rank_bits);
-        radix_sort_state(p->btB, sheets, &p->bradix, p->bflag, p->err, p->stream);
+        radix_sort_state(p->btB, sheets, &p->bradix, p->bflag, p->err, p->stream, true);
         p->launches += 1 + kRadixLaunches;
       }
       k_seg_final<<<grid_1d(sheets), 256, 0, p->stream>>>(p->btA, nseg > 1 ? p->btB : nullptr,

@@ -1,22 +1,36 @@
 // wg_radix.cu -- full on-device re-sort of the sheets: a least-significant-
-// digit radix sort of the 64-bit position keys with 8-bit digits, one pass
-// per digit, each pass a single read and write of (key, slot) pairs whose
-// tile offsets come from a decoupled look-back over per-tile digit counts
-// ("onesweep").  It replaces the serial argsort of the reference
+// digit radix sort of the leading bytes of the 64-bit position keys, 8 bits a
+// pass, each pass a single read and write of (key, slot) pairs whose tile
+// offsets come from a decoupled look-back over per-tile digit counts
+// ("onesweep"), and then the few sheets that share those bytes put in order
+// by their whole keys.  It replaces the serial argsort of the reference
 // (wendy/wendy.c:341-357) when the order cannot be repaired locally.
 //
-//   hist   one read of the positions: all eight digit histograms
-//   plan   exclusive digit offsets; passes whose digit is the same for every
-//          key are skipped (decided on the device)
-//   pass   8x, persistent: bulk-copy the tile into shared memory (the next
+// Positions of N sheets are told apart by about log2 N bits, not by 64: the
+// leading five bytes of a key (sign, exponent, 28 bits of the mantissa) leave
+// one pair in a hundred together at 1e6 sheets, four bytes one in thirty at
+// 65536.  A pass costs a launch and about 10 us at least, and what the
+// following passes need fits in 32 bits once the first one is done, so five
+// passes move 80 bytes per sheet where eight of 64-bit keys moved 190.
+// A sort of 20011 sheets with its force evaluation 205 -> 126 us, of 2^21 in a
+// diagnostics call 560 -> 350 us.
+//
+//   hist   one read of the positions: the digit histograms; its last block
+//          forms the exclusive digit offsets; passes whose digit is the same
+//          for every key are skipped (decided on the device)
+//   pass   persistent: bulk-copy the tile into shared memory (the next
 //          tile's copy overlaps this one's write-out), rank within the tile
 //          (bit-plane ballots + per-warp shared-memory counters, stable),
 //          publish the tile's digit counts, stage in digit order, look back
 //          for the tile's global digit offsets, write out
-//   gather permute x, v, m, idx into the other state set
-//   ties   equal keys are ordered by original index (rare; usually no-op):
-//          short runs in place, long runs by one CTA each
-//   flip   the other set becomes the current one
+//   gather permute x, v, m, idx into the other state set; notes whether any
+//          sheet precedes its predecessor in (key, index)
+//   ties   (only then) runs of equal leading bytes are ordered by key and
+//          original index: short runs in place, long runs by one CTA each,
+//          whose last block makes the other set the current one
+//
+// Keys that differ in their low bytes only (ranks packed into the bits of a
+// double) are sorted whole: first_byte = 0, eight passes of 64-bit keys.
 //
 // Every kernel first reads the sub-step's `unsorted` flag and returns at once
 // when the sheets are already in order, so the sequence can be captured in a
@@ -46,13 +60,22 @@ constexpr int kPlanFinal = 24;   // [1]
 constexpr int kPlanStarts = 32;  // [8 * 256]
 constexpr int kPlanWords = kPlanStarts + 8 * R;
 
+// counters (uint32 words, cleared before each sort)
+constexpr int kCntClaim = 0;   // [8] next tile of each pass
+constexpr int kCntTie = 8;     // some sheet out of (key, index) order after the gather
+constexpr int kCntRuns = 9;    // long runs listed
+constexpr int kCntHist = 10;   // histogram blocks done
+constexpr int kCntLong = 11;   // k_radix_long_ties blocks done
+constexpr int kCounters = 16;
+
 struct PassArgs {
   const StateTable* table;
   int64_t n;
-  int pass;
+  int pass;            // byte of the key
+  int first;           // the first pass's byte
   int64_t n_tiles;
-  uint64_t* keys0;
-  uint64_t* keys1;
+  void* keys0;         // u64 (whole keys) or u32 (their upper halves)
+  void* keys1;
   uint32_t* pos0;
   uint32_t* pos1;
   const uint32_t* plan;
@@ -62,55 +85,78 @@ struct PassArgs {
   unsigned* err;
 };
 
-__global__ void k_radix_hist(const StateTable* table, int64_t n, uint32_t* hist,
-                             const StepFlags* flag) {
+// Digit histograms of bytes first .. 7; the last block to finish turns them
+// into the plan.  The top byte (sign and seven exponent bits) takes a few
+// values only, so its counts are formed per warp, one atomic per value.
+constexpr int kHistThreads = 256;
+__global__ void __launch_bounds__(kHistThreads) k_radix_hist(
+    const StateTable* table, int64_t n, int first, uint32_t* hist, uint32_t* plan,
+    uint32_t* counters, const StepFlags* flag) {
   if (!flag->unsorted) return;
   __shared__ uint32_t sh[8 * R];
-  for (int i = threadIdx.x; i < 8 * R; i += blockDim.x) sh[i] = 0;
+  __shared__ int s_last;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = tid; i < 8 * R; i += kHistThreads) sh[i] = 0;
   __syncthreads();
   const double* x = table->cur.x;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
-    const uint64_t k = key_of(x[i]);
-#pragma unroll
-    for (int p = 0; p < 8; ++p) atomicAdd(&sh[p * R + ((k >> (8 * p)) & 255u)], 1u);
+  const int64_t stride = (int64_t)gridDim.x * kHistThreads;
+  for (int64_t i0 = (int64_t)blockIdx.x * kHistThreads + (tid & ~31); i0 < n; i0 += stride) {
+    const bool ok = i0 + lane < n;
+    const uint64_t k = ok ? key_of(x[i0 + lane]) : 0ull;
+    if (ok)
+      for (int p = first; p < 7; ++p) atomicAdd(&sh[p * R + ((k >> (8 * p)) & 255u)], 1u);
+    unsigned todo = __ballot_sync(0xffffffffu, ok);
+    const unsigned top = (unsigned)(k >> 56);
+    while (todo) {
+      const int leader = __ffs(todo) - 1;
+      const unsigned t = __shfl_sync(0xffffffffu, top, leader);
+      const unsigned same = __ballot_sync(0xffffffffu, ok && top == t);
+      if (lane == leader) atomicAdd(&sh[7 * R + t], (uint32_t)__popc(same));
+      todo &= ~same;
+    }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < 8 * R; i += blockDim.x)
+  for (int i = first * R + tid; i < 8 * R; i += kHistThreads)
     if (sh[i]) atomicAdd(&hist[i], sh[i]);
-}
-
-// One block of 256 threads.
-__global__ void k_radix_plan(int64_t n, const uint32_t* hist, uint32_t* plan,
-                             const StepFlags* flag) {
-  if (!flag->unsorted) return;
-  __shared__ uint32_t s_tmp[R / 32];
-  __shared__ int s_trivial[8];
-  const int d = threadIdx.x, lane = d & 31, warp = d >> 5;
-  for (int p = 0; p < 8; ++p) {
-    const uint32_t c = hist[p * R + d];
-    const int triv = __syncthreads_or(c == (uint32_t)n);
-    uint32_t incl = c;
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) s_last = atomicAdd(&counters[kCntHist], 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  // ---- the plan: warp w takes byte w, eight digits per lane
+  __threadfence();
+  if (warp >= first) {
+    uint32_t c[8], sum = 0;
+    bool triv = false;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      c[q] = __ldcg(&hist[warp * R + lane * 8 + q]);
+      sum += c[q];
+      triv |= c[q] == (uint32_t)n;
+    }
+    uint32_t incl = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
       if (lane >= o) incl += y;
     }
-    if (lane == 31) s_tmp[warp] = incl;
-    __syncthreads();
-    uint32_t wpre = 0;
-    for (int w = 0; w < warp; ++w) wpre += s_tmp[w];
-    plan[kPlanStarts + p * R + d] = wpre + incl - c;
-    if (d == 0) s_trivial[p] = triv;
-    __syncthreads();
+    uint32_t ex = incl - sum;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      plan[kPlanStarts + warp * R + lane * 8 + q] = ex;
+      ex += c[q];
+    }
+    const unsigned t = __ballot_sync(0xffffffffu, triv);
+    if (lane == 0) sh[warp] = t != 0u;
   }
-  if (d == 0) {
+  __syncthreads();
+  if (tid == 0) {
     int cur = 0;
-    plan[kPlanActive + 0] = 1;
-    plan[kPlanSrc + 0] = 0;
-    plan[kPlanDst + 0] = 0;
-    for (int p = 1; p < 8; ++p) {
-      const int act = !s_trivial[p];
+    plan[kPlanActive + first] = 1;
+    plan[kPlanSrc + first] = 0;
+    plan[kPlanDst + first] = 0;
+    for (int p = first + 1; p < 8; ++p) {
+      const int act = !sh[p];
       plan[kPlanActive + p] = act;
       plan[kPlanSrc + p] = cur;
       plan[kPlanDst + p] = act ? 1 - cur : cur;
@@ -119,12 +165,23 @@ __global__ void k_radix_plan(int64_t n, const uint32_t* hist, uint32_t* plan,
     plan[kPlanFinal] = cur;
   }
 }
+constexpr int kHistWarps = kHistThreads / 32;
+static_assert(kHistWarps == 8, "one warp per byte, one thread per digit");
 
-template <int THREADS, int ITEMS>
+template <bool WIDE>
+struct KeyWord {
+  typedef uint32_t type;  // the upper half of the key
+};
+template <>
+struct KeyWord<true> {
+  typedef uint64_t type;
+};
+
+template <int THREADS, int ITEMS, typename KEY>
 struct PassSmem {
   static constexpr int TILE = THREADS * ITEMS;
   static constexpr int WARPS = THREADS / 32;
-  uint64_t keys[2][TILE];  // tile k lands in keys[k & 1] (positions on pass 0) ...
+  KEY keys[2][TILE];       // tile k lands in keys[k & 1] (positions on the first pass) ...
   uint32_t vals[2][TILE];  // ... and is staged in digit order in the same buffer
   uint32_t whist[WARPS][R];
   uint32_t tile_excl[R];
@@ -144,9 +201,13 @@ struct PassSmem {
 // staging time to finish.  Claims are dynamic, so only running CTAs ever
 // hold a tile and the look-back always progresses: the smallest tile in work
 // has every predecessor finished.
-template <int THREADS, int ITEMS>
+template <int THREADS, int ITEMS, bool FIRST, bool WIDE>
 __global__ void __launch_bounds__(THREADS, 2) k_radix_pass(const PassArgs a) {
-  using Smem = PassSmem<THREADS, ITEMS>;
+  // what a tile is read and staged as (the first pass reads positions and
+  // needs the whole key for its digit), and what is written
+  using KEY = typename KeyWord<FIRST || WIDE>::type;
+  using OUT = typename KeyWord<WIDE>::type;
+  using Smem = PassSmem<THREADS, ITEMS, KEY>;
   constexpr int TILE = Smem::TILE;
   constexpr int WARPS = Smem::WARPS;
   static_assert(THREADS == R, "one thread per digit");
@@ -159,17 +220,17 @@ __global__ void __launch_bounds__(THREADS, 2) k_radix_pass(const PassArgs a) {
   const int pass = a.pass;
   if (!a.plan[kPlanActive + pass]) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int shift = 8 * pass;
+  const int shift = 8 * (FIRST || WIDE ? pass : pass - 4);
   const int srcb = (int)a.plan[kPlanSrc + pass], dstb = (int)a.plan[kPlanDst + pass];
-  const uint64_t* ksrc = srcb ? a.keys1 : a.keys0;
+  const OUT* ksrc = static_cast<const OUT*>(srcb ? a.keys1 : a.keys0);
   const uint32_t* psrc = srcb ? a.pos1 : a.pos0;
-  uint64_t* kdst = dstb ? a.keys1 : a.keys0;
+  OUT* kdst = static_cast<OUT*>(dstb ? a.keys1 : a.keys0);
   uint32_t* pdst = dstb ? a.pos1 : a.pos0;
   const double* x = a.table->cur.x;
-  const void* kfrom = pass == 0 ? (const void*)x : (const void*)ksrc;
-  const bool bulk_ok = ((uintptr_t)kfrom & 15u) == 0 && (pass == 0 || ((uintptr_t)psrc & 15u) == 0);
-  uint32_t* stat = a.status + ((int64_t)pass * a.n_tiles) * R;
-  unsigned* claim = a.counters + pass;
+  const void* kfrom = FIRST ? (const void*)x : (const void*)ksrc;
+  const bool bulk_ok = ((uintptr_t)kfrom & 15u) == 0 && (FIRST || ((uintptr_t)psrc & 15u) == 0);
+  uint32_t* stat = a.status + ((int64_t)(pass - a.first) * a.n_tiles) * R;
+  unsigned* claim = a.counters + kCntClaim + pass;
 
   // thread 0: start the copy of tile t into buffer b; partial tiles (and
   // unaligned sources) are read with plain loads, their phase completes at once
@@ -177,10 +238,11 @@ __global__ void __launch_bounds__(THREADS, 2) k_radix_pass(const PassArgs a) {
     if (t >= a.n_tiles) return;
     const int64_t base = t * TILE;
     if (bulk_ok && a.n - base >= TILE) {
-      const uint32_t kb = TILE * 8u, vb = pass ? TILE * 4u : 0u;
+      constexpr uint32_t kb = TILE * sizeof(KEY), vb = FIRST ? 0u : TILE * 4u;
       mbar_expect_tx(&S.mbar[b], kb + vb);
-      bulk_g2s(S.keys[b], static_cast<const char*>(kfrom) + base * 8, kb, &S.mbar[b]);
-      if (pass) bulk_g2s(S.vals[b], psrc + base, vb, &S.mbar[b]);
+      bulk_g2s(S.keys[b], static_cast<const char*>(kfrom) + base * (int64_t)sizeof(KEY), kb,
+               &S.mbar[b]);
+      if (!FIRST) bulk_g2s(S.vals[b], psrc + base, vb, &S.mbar[b]);
     } else {
       mbar_expect_tx(&S.mbar[b], 0u);
     }
@@ -215,7 +277,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_radix_pass(const PassArgs a) {
       S.bad = tile + 1;
       S.stop = 1;
     }
-    uint64_t key[ITEMS];
+    KEY key[ITEMS];
     uint32_t val[ITEMS];
     uint32_t rank[ITEMS];
 #pragma unroll
@@ -223,16 +285,12 @@ __global__ void __launch_bounds__(THREADS, 2) k_radix_pass(const PassArgs a) {
       const int local = warp * (32 * ITEMS) + i * 32 + lane;
       const int64_t e = base + local;
       if (local < tile_n) {
-        if (via_bulk) {
-          const uint64_t raw = S.keys[b][local];
-          key[i] = pass == 0 ? key_of(__longlong_as_double((long long)raw)) : raw;
-          val[i] = pass == 0 ? (uint32_t)e : S.vals[b][local];
-        } else if (pass == 0) {
-          key[i] = key_of(x[e]);
+        if constexpr (FIRST) {
+          key[i] = key_of(via_bulk ? __longlong_as_double((long long)S.keys[b][local]) : x[e]);
           val[i] = (uint32_t)e;
         } else {
-          key[i] = ksrc[e];
-          val[i] = psrc[e];
+          key[i] = via_bulk ? S.keys[b][local] : ksrc[e];
+          val[i] = via_bulk ? S.vals[b][local] : psrc[e];
         }
       } else {
         key[i] = 0;
@@ -383,10 +441,10 @@ __global__ void __launch_bounds__(THREADS, 2) k_radix_pass(const PassArgs a) {
     for (int jj = 0; jj < ITEMS; ++jj) {
       const int p = jj * THREADS + tid;
       if (p < tile_n && !skip) {
-        const uint64_t kk = S.keys[b][p];
+        const KEY kk = S.keys[b][p];
         const unsigned dd = (unsigned)((kk >> shift) & 255u);
         const int64_t o = (int64_t)S.gbase[dd] + p;
-        kdst[o] = kk;
+        kdst[o] = FIRST && !WIDE ? (OUT)((uint64_t)kk >> 32) : (OUT)kk;
         pdst[o] = S.vals[b][p];
       }
     }
@@ -398,114 +456,144 @@ __global__ void __launch_bounds__(THREADS, 2) k_radix_pass(const PassArgs a) {
 // loads in flight together (the reads are random when the input was).
 constexpr int kGatherThreads = 256, kGatherUnroll = 4;
 __global__ void __launch_bounds__(kGatherThreads) k_radix_gather(
-    StateTable* table, int64_t n, const uint64_t* keys0, const uint64_t* keys1,
-    const uint32_t* pos0, const uint32_t* pos1, const uint32_t* plan, uint32_t* counters,
-    const StepFlags* flag, const unsigned* err) {
+    StateTable* table, int64_t n, const uint32_t* pos0, const uint32_t* pos1,
+    const uint32_t* plan, uint32_t* counters, const StepFlags* flag, const unsigned* err) {
   constexpr int GU = kGatherUnroll;
   // nothing after a pass that gave up on a wait: its slots are incomplete
   if (!flag->unsorted || (*err & DEV_ERR_RADIX_TIMEOUT)) return;
   const int fb = (int)plan[kPlanFinal];
-  const uint64_t* __restrict__ keys = fb ? keys1 : keys0;
   const uint32_t* __restrict__ pos = fb ? pos1 : pos0;
   const StateRef cur = table->cur, oth = table->other;
+  const int lane = threadIdx.x & 31;
   const int64_t chunk = (int64_t)gridDim.x * kGatherThreads * GU;
   bool tie = false;
-  for (int64_t p0 = (int64_t)blockIdx.x * kGatherThreads * GU + threadIdx.x; p0 < n;
-       p0 += chunk) {
-    uint32_t q[GU];
+  for (int64_t b0 = (int64_t)blockIdx.x * kGatherThreads * GU; b0 < n; b0 += chunk) {
+    const int64_t p0 = b0 + threadIdx.x;
+    uint32_t q[GU], qn[GU];
 #pragma unroll
     for (int u = 0; u < GU; ++u) {
       const int64_t p = p0 + (int64_t)u * kGatherThreads;
       q[u] = p < n ? __ldcs(pos + p) : 0u;
+      qn[u] = lane == 31 && p + 1 < n ? __ldg(pos + p + 1) : 0u;
     }
-    double xs[GU], vs[GU], ms[GU];
-    int32_t is[GU];
+    double xs[GU], vs[GU], ms[GU], xn[GU];
+    int32_t is[GU], in[GU];
 #pragma unroll
     for (int u = 0; u < GU; ++u) {
       const int64_t p = p0 + (int64_t)u * kGatherThreads;
+      xs[u] = xn[u] = 0.0;
+      is[u] = in[u] = 0;
       if (p < n) {
         xs[u] = __ldg(cur.x + q[u]);
         vs[u] = __ldg(cur.v + q[u]);
         ms[u] = __ldg(cur.m + q[u]);
         is[u] = __ldg(cur.idx + q[u]);
       }
+      if (lane == 31 && p + 1 < n) {  // the first sheet of the next warp
+        xn[u] = __ldg(cur.x + qn[u]);
+        in[u] = __ldg(cur.idx + qn[u]);
+      }
     }
 #pragma unroll
     for (int u = 0; u < GU; ++u) {
       const int64_t p = p0 + (int64_t)u * kGatherThreads;
+      const double xd = __shfl_down_sync(0xffffffffu, xs[u], 1);
+      const int32_t id = __shfl_down_sync(0xffffffffu, is[u], 1);
       if (p < n) {
         oth.x[p] = xs[u];
         oth.v[p] = vs[u];
         oth.m[p] = ms[u];
         oth.idx[p] = is[u];
-        if (p + 1 < n && keys[p] == keys[p + 1]) tie = true;
+        if (p + 1 < n) {
+          const uint64_t k = key_of(xs[u]), kn = key_of(lane < 31 ? xd : xn[u]);
+          tie |= kn < k || (kn == k && (lane < 31 ? id : in[u]) < is[u]);
+        }
       }
     }
   }
-  if (__syncthreads_or(tie) && threadIdx.x == 0) atomicOr(&counters[8], 1u);
+  if (__syncthreads_or(tie) && threadIdx.x == 0) atomicOr(&counters[kCntTie], 1u);
 }
 
-// Equal keys: order each run by original index.  The thread at a run's
-// first sheet finds its end by binary search over the sorted keys; runs of up
-// to kShortRun sheets are insertion-sorted in place, longer ones are listed
-// (start in list_start, length in list_len, count in counters[9]) for
-// k_radix_long_ties, so no thread ever does work quadratic in a run.
+// Runs of equal leading bytes (key >> low_bits): each is ordered by key and
+// original index.  The thread at a run's first sheet finds its end by binary
+// search over the sorted leading bytes; runs of up to kShortRun sheets are
+// insertion-sorted in place, longer ones are listed (start in list_start,
+// length in list_len, count in counters[kCntRuns]) for k_radix_long_ties, so
+// no thread ever does work quadratic in a run.  Threads read the leading bytes
+// of sheets that the run's first thread may be moving: moves stay inside a
+// run, whose leading bytes are all the same, and both sides use relaxed
+// accesses.
 constexpr int64_t kShortRun = 32;
-__global__ void k_radix_ties(StateTable* table, int64_t n, const uint64_t* keys0,
-                             const uint64_t* keys1, const uint32_t* plan, uint32_t* counters,
+__global__ void k_radix_ties(StateTable* table, int64_t n, int low_bits, uint32_t* counters,
                              uint32_t* list_start, uint32_t* list_len, const StepFlags* flag,
                              const unsigned* err) {
-  if (!flag->unsorted || !counters[8] || (*err & DEV_ERR_RADIX_TIMEOUT)) return;
-  const int fb = (int)plan[kPlanFinal];
-  const uint64_t* keys = fb ? keys1 : keys0;
+  if (!flag->unsorted || !counters[kCntTie] || (*err & DEV_ERR_RADIX_TIMEOUT)) return;
   const StateRef oth = table->other;
+  auto lead = [&](int64_t p) { return key_of(ld_relaxed_f64(oth.x + p)) >> low_bits; };
+  const int lane = threadIdx.x & 31;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p + 1 < n; p += stride) {
-    const uint64_t kp = keys[p];
-    if (kp != keys[p + 1] || (p > 0 && keys[p - 1] == kp)) continue;
-    // last index e with keys[e] == kp: keys[p + 1] == kp, keys are sorted
+  for (int64_t w0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); w0 < n;
+       w0 += stride) {
+    const int64_t p = w0 + lane;
+    const uint64_t kp = p < n ? lead(p) : 0ull;
+    uint64_t kn = __shfl_down_sync(0xffffffffu, kp, 1);
+    uint64_t kb = __shfl_up_sync(0xffffffffu, kp, 1);
+    if (lane == 31 && p + 1 < n) kn = lead(p + 1);
+    if (lane == 0 && p > 0) kb = lead(p - 1);
+    if (p + 1 >= n || kp != kn || (p > 0 && kb == kp)) continue;
+    // last index e with the same leading bytes
     int64_t lo = p + 1, hi = n - 1;
+    if (hi > p + 1 && lead(p + 2) != kp) hi = p + 1;  // nearly every run is a pair
     while (lo < hi) {
       const int64_t mid = lo + (hi - lo + 1) / 2;
-      if (keys[mid] == kp) lo = mid; else hi = mid - 1;
+      if (lead(mid) == kp) lo = mid; else hi = mid - 1;
     }
     const int64_t e = lo;
     if (e - p + 1 > kShortRun) {
-      const unsigned slot = atomicAdd(&counters[9], 1u);
+      const unsigned slot = atomicAdd(&counters[kCntRuns], 1u);
       list_start[slot] = (uint32_t)p;
       list_len[slot] = (uint32_t)(e - p + 1);
       continue;
     }
     for (int64_t i = p + 1; i <= e; ++i) {
-      const double xi = oth.x[i], vi = oth.v[i], mi = oth.m[i];
+      const double xi = ld_relaxed_f64(oth.x + i), vi = oth.v[i], mi = oth.m[i];
+      const uint64_t ki = key_of(xi);
       const int32_t ii = oth.idx[i];
       int64_t j = i - 1;
-      while (j >= p && oth.idx[j] > ii) {
-        oth.x[j + 1] = oth.x[j];
+      while (j >= p) {
+        const double xj = ld_relaxed_f64(oth.x + j);
+        const uint64_t kj = key_of(xj);
+        if (kj < ki || (kj == ki && oth.idx[j] < ii)) break;
+        st_relaxed_f64(oth.x + j + 1, xj);
         oth.v[j + 1] = oth.v[j];
         oth.m[j + 1] = oth.m[j];
         oth.idx[j + 1] = oth.idx[j];
         --j;
       }
-      oth.x[j + 1] = xi;
-      oth.v[j + 1] = vi;
-      oth.m[j + 1] = mi;
-      oth.idx[j + 1] = ii;
+      if (j + 1 != i) {
+        st_relaxed_f64(oth.x + j + 1, xi);
+        oth.v[j + 1] = vi;
+        oth.m[j + 1] = mi;
+        oth.idx[j + 1] = ii;
+      }
     }
   }
 }
 
-// Long runs of equal keys, one CTA per run: a stable LSD radix sort (4-bit
-// digits, each thread a contiguous chunk) of (index, place in run) pairs in
-// the key buffers' slots of the run, then the run's sheets are permuted
-// through the current set (free until the flip) and copied back.  Runs
-// already in index order are left alone.  O(run length) work per digit.
+// Long runs of equal leading bytes, one CTA per run: a stable LSD radix sort
+// (4-bit digits, each thread a contiguous chunk) of (index, place in run)
+// pairs in the key buffers' slots of the run, by index and then by the low
+// bits of the key, then the run's sheets are permuted through the current set
+// (free until the flip) and copied back.  Runs already in order are left
+// alone.  O(run length) work per digit.  The last block to finish makes the
+// other set the current one.
 constexpr int kLongTieThreads = 256;
 __global__ void __launch_bounds__(kLongTieThreads) k_radix_long_ties(
-    StateTable* table, int64_t n, uint64_t* bufa, uint64_t* bufb, const uint32_t* counters,
-    const uint32_t* list_start, const uint32_t* list_len, const StepFlags* flag,
-    const unsigned* err) {
-  if (!flag->unsorted || !counters[9] || (*err & DEV_ERR_RADIX_TIMEOUT)) return;
+    StateTable* table, int64_t n, int low_bits, uint64_t* bufa, uint64_t* bufb,
+    uint32_t* counters, const uint32_t* list_start, const uint32_t* list_len,
+    const StepFlags* flag, const unsigned* err) {
+  // after an expired wait the current set stays as it was (unsorted, intact)
+  if (!flag->unsorted || (*err & DEV_ERR_RADIX_TIMEOUT)) return;
   constexpr int T = kLongTieThreads;
   __shared__ uint32_t cnt[16][T + 1];
   __shared__ uint32_t tot[16];
@@ -513,12 +601,15 @@ __global__ void __launch_bounds__(kLongTieThreads) k_radix_long_ties(
   const StateRef oth = table->other, cur = table->cur;
   int bits = 1;
   while (bits < 31 && ((int64_t)1 << bits) < n) ++bits;
-  const int npass = (bits + 3) / 4;
-  const unsigned nruns = counters[9];
+  const int ipass = (bits + 3) / 4, npass = ipass + (low_bits + 3) / 4;
+  const unsigned nruns = counters[kCntRuns];
   for (unsigned r = blockIdx.x; r < nruns; r += gridDim.x) {
     const int64_t s = list_start[r], L = list_len[r];
     bool unordered = false;
-    for (int64_t j = tid; j + 1 < L; j += T) unordered |= oth.idx[s + j] > oth.idx[s + j + 1];
+    for (int64_t j = tid; j + 1 < L; j += T) {
+      const uint64_t k = key_of(oth.x[s + j]), kn = key_of(oth.x[s + j + 1]);
+      unordered |= kn < k || (kn == k && oth.idx[s + j + 1] < oth.idx[s + j]);
+    }
     if (!__syncthreads_or(unordered)) continue;
     uint64_t* src = bufa + s;
     uint64_t* dst = bufb + s;
@@ -529,10 +620,13 @@ __global__ void __launch_bounds__(kLongTieThreads) k_radix_long_ties(
     const int64_t c_hi = c_lo + chunk < L ? c_lo + chunk : L;
     __syncthreads();
     for (int ps = 0; ps < npass; ++ps) {
-      const int shift = 32 + 4 * ps;
+      auto digit = [&](uint64_t w) {
+        return ps < ipass ? (unsigned)(w >> (32 + 4 * ps)) & 15u
+                          : (unsigned)(key_of(oth.x[s + (uint32_t)w]) >> (4 * (ps - ipass))) & 15u;
+      };
 #pragma unroll
       for (int d = 0; d < 16; ++d) cnt[d][tid] = 0;
-      for (int64_t j = c_lo; j < c_hi; ++j) ++cnt[(src[j] >> shift) & 15u][tid];
+      for (int64_t j = c_lo; j < c_hi; ++j) ++cnt[digit(src[j])][tid];
       __syncthreads();
       if (tid < 16) {  // digit-major exclusive offsets of each thread's chunk
         uint32_t run = 0;
@@ -552,7 +646,7 @@ __global__ void __launch_bounds__(kLongTieThreads) k_radix_long_ties(
       __syncthreads();
       for (int64_t j = c_lo; j < c_hi; ++j) {
         const uint64_t w = src[j];
-        dst[cnt[(w >> shift) & 15u][tid]++] = w;
+        dst[cnt[digit(w)][tid]++] = w;
       }
       __syncthreads();
       uint64_t* t2 = src;
@@ -575,36 +669,62 @@ __global__ void __launch_bounds__(kLongTieThreads) k_radix_long_ties(
     }
     __syncthreads();
   }
-}
-
-__global__ void k_radix_flip(StateTable* table, const StepFlags* flag, const unsigned* err) {
-  // after an expired wait the current set stays as it was (unsorted, intact)
-  if (!flag->unsorted || (*err & DEV_ERR_RADIX_TIMEOUT)) return;
-  const StateRef t = table->cur;
-  table->cur = table->other;
-  table->other = t;
+  __syncthreads();
+  if (tid == 0) {
+    __threadfence();
+    if (atomicAdd(&counters[kCntLong], 1u) == gridDim.x - 1) {
+      table->cur = oth;
+      table->other = cur;
+    }
+  }
 }
 
 size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 // Launch configuration of the radix passes on one device: its SM count and
-// the resident pass CTAs per SM, after raising the pass kernel's dynamic
-// shared-memory limit on that device.  Set up once per device (thread-safe).
+// the resident pass CTAs per SM, after raising the pass kernels' dynamic
+// shared-memory limits on that device.  Set up once per device (thread-safe).
 struct RadixDevCfg {
   int sms = 1;
-  int per_sm = 1;
+  int per_sm[2][4] = {};  // [small tiles][kind]
 };
 
+// The four kinds of pass: whole keys or their upper halves, first or not.
+constexpr int kKinds = 4;
+template <int ITEMS, bool FIRST, bool WIDE>
+constexpr size_t pass_smem() {
+  return sizeof(PassSmem<kRadixThreads, ITEMS, typename KeyWord<FIRST || WIDE>::type>);
+}
+template <int ITEMS, bool FIRST, bool WIDE>
+void pass_init(int& per_sm) {
+  constexpr size_t dyn = pass_smem<ITEMS, FIRST, WIDE>();
+  auto* k = k_radix_pass<kRadixThreads, ITEMS, FIRST, WIDE>;
+  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+  int c = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, k, kRadixThreads, dyn);
+  per_sm = c < 1 ? 1 : c;
+}
+template <int ITEMS, bool FIRST, bool WIDE>
+void pass_launch(const PassArgs& a, int per_sm, int sms, cudaStream_t s) {
+  int64_t pg = (int64_t)per_sm * sms;
+  if (pg > a.n_tiles) pg = a.n_tiles;
+  if (pg < 1) pg = 1;
+  k_radix_pass<kRadixThreads, ITEMS, FIRST, WIDE>
+      <<<(unsigned)pg, kRadixThreads, pass_smem<ITEMS, FIRST, WIDE>(), s>>>(a);
+}
+
 void radix_cfg_init(RadixDevCfg& c, int dev) {
-  constexpr size_t dyn = sizeof(PassSmem<kRadixThreads, kRadixItems>);
-  int sms = 0, per_sm = 0;
+  int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaFuncSetAttribute(k_radix_pass<kRadixThreads, kRadixItems>,
-                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-      &per_sm, k_radix_pass<kRadixThreads, kRadixItems>, kRadixThreads, dyn);
   c.sms = sms < 1 ? 1 : sms;
-  c.per_sm = per_sm < 1 ? 1 : per_sm;
+  pass_init<kRadixItems, true, false>(c.per_sm[0][0]);
+  pass_init<kRadixItems, false, false>(c.per_sm[0][1]);
+  pass_init<kRadixItems, true, true>(c.per_sm[0][2]);
+  pass_init<kRadixItems, false, true>(c.per_sm[0][3]);
+  pass_init<kRadixItemsSmall, true, false>(c.per_sm[1][0]);
+  pass_init<kRadixItemsSmall, false, false>(c.per_sm[1][1]);
+  pass_init<kRadixItemsSmall, true, true>(c.per_sm[1][2]);
+  pass_init<kRadixItemsSmall, false, true>(c.per_sm[1][3]);
 }
 
 RadixDevCfg radix_cfg() {
@@ -620,53 +740,59 @@ RadixDevCfg radix_cfg() {
   return cfg[dev];
 }
 
+int64_t tiles_of(int64_t n) {
+  const int64_t t = n <= kRadixSmallSheets ? kRadixTileSmall : kRadixTile;
+  return (n + t - 1) / t;
+}
+
 }  // namespace
 
 size_t radix_bytes(int64_t n) {
-  const int64_t tiles = (n + kRadixTile - 1) / kRadixTile;
+  // a workspace for n sheets also serves smaller sorts, whose tiles may be
+  // the small ones
+  const int64_t small = tiles_of(n < kRadixSmallSheets ? n : kRadixSmallSheets);
+  const int64_t tiles = tiles_of(n) > small ? tiles_of(n) : small;
   size_t b = 0;
   b += 2 * align256((size_t)n * 8);
   b += 2 * align256((size_t)n * 4);
-  b += align256(8 * R * 4);
   b += align256(kPlanWords * 4);
-  b += align256((size_t)8 * tiles * R * 4 + 16 * 4);
+  b += 8 * R * 4 + kCounters * 4;
+  b += align256((size_t)8 * tiles * R * 4);
   return b;
 }
 
 void radix_bind(RadixWork* w, void* base, int64_t n) {
   char* p = static_cast<char*>(base);
-  w->n_tiles = (n + kRadixTile - 1) / kRadixTile;
   w->keys[0] = reinterpret_cast<uint64_t*>(p); p += align256((size_t)n * 8);
   w->keys[1] = reinterpret_cast<uint64_t*>(p); p += align256((size_t)n * 8);
   w->pos[0] = reinterpret_cast<uint32_t*>(p); p += align256((size_t)n * 4);
   w->pos[1] = reinterpret_cast<uint32_t*>(p); p += align256((size_t)n * 4);
-  w->hist = reinterpret_cast<uint32_t*>(p); p += align256(8 * R * 4);
   w->plan = reinterpret_cast<uint32_t*>(p); p += align256(kPlanWords * 4);
-  w->status = reinterpret_cast<uint32_t*>(p);
-  w->counters = w->status + (size_t)8 * w->n_tiles * R;
-  w->scratch_bytes = (size_t)8 * w->n_tiles * R * 4 + 16 * 4;
+  w->hist = reinterpret_cast<uint32_t*>(p);
+  w->counters = w->hist + 8 * R;
+  w->status = w->counters + kCounters;
 }
 
 void radix_sort_state(StateTable* table, int64_t n, RadixWork* w, const StepFlags* flag,
-                      unsigned* err, cudaStream_t s) {
-  constexpr size_t dyn = sizeof(PassSmem<kRadixThreads, kRadixItems>);
-  static_assert(kRadixTile == PassSmem<kRadixThreads, kRadixItems>::TILE, "tile size");
+                      unsigned* err, cudaStream_t s, bool whole_keys) {
   const RadixDevCfg cfg = radix_cfg();
-  const int pass_grid_per_sm = cfg.per_sm, sms = cfg.sms;
+  const int sms = cfg.sms;
+  // bytes sorted by: five tell the positions of any number of sheets apart
+  // well enough, four those of up to 2^17 (see the top of this file)
+  const int first = whole_keys ? 0 : n <= (1 << 17) ? 4 : 3;
   // the workspace may be bound for more sheets than this sort has: tiles,
   // look-back words and launches follow n
-  const int64_t tiles = (n + kRadixTile - 1) / kRadixTile;
-  cudaMemsetAsync(w->hist, 0, 8 * R * 4, s);
-  cudaMemsetAsync(w->status, 0, (size_t)8 * tiles * R * 4, s);
-  cudaMemsetAsync(w->counters, 0, 16 * 4, s);
-  int hist_grid = (int)((n + 255) / 256);
-  if (hist_grid > 152 * 8) hist_grid = 152 * 8;
-  if (hist_grid < 1) hist_grid = 1;
-  k_radix_hist<<<hist_grid, 256, 0, s>>>(table, n, w->hist, flag);
-  k_radix_plan<<<1, R, 0, s>>>(n, w->hist, w->plan, flag);
+  const int64_t tiles = tiles_of(n);
+  cudaMemsetAsync(w->hist, 0, (8 * R + kCounters + (size_t)(8 - first) * tiles * R) * 4, s);
+  int64_t hist_grid = (n + 16 * kHistThreads - 1) / (16 * kHistThreads);
+  if (hist_grid < 8) hist_grid = n < 8 * kHistThreads ? (n + kHistThreads - 1) / kHistThreads : 8;
+  if (hist_grid > sms * 4) hist_grid = sms * 4;
+  k_radix_hist<<<(unsigned)hist_grid, kHistThreads, 0, s>>>(table, n, first, w->hist, w->plan,
+                                                            w->counters, flag);
   PassArgs a;
   a.table = table;
   a.n = n;
+  a.first = first;
   a.n_tiles = tiles;
   a.keys0 = w->keys[0];
   a.keys1 = w->keys[1];
@@ -677,31 +803,37 @@ void radix_sort_state(StateTable* table, int64_t n, RadixWork* w, const StepFlag
   a.counters = w->counters;
   a.flag = flag;
   a.err = err;
-  int64_t pg = (int64_t)pass_grid_per_sm * sms;
-  if (pg > tiles) pg = tiles;
-  if (pg < 1) pg = 1;
-  for (int p = 0; p < 8; ++p) {
+  const bool small = n <= kRadixSmallSheets;
+  const int* per_sm = cfg.per_sm[small ? 1 : 0];
+  for (int p = first; p < 8; ++p) {
     a.pass = p;
-    k_radix_pass<kRadixThreads, kRadixItems><<<(unsigned)pg, kRadixThreads, dyn, s>>>(a);
+    const int kind = (whole_keys ? 2 : 0) + (p == first ? 0 : 1);
+    if (small) {
+      if (kind == 0) pass_launch<kRadixItemsSmall, true, false>(a, per_sm[0], sms, s);
+      if (kind == 1) pass_launch<kRadixItemsSmall, false, false>(a, per_sm[1], sms, s);
+      if (kind == 2) pass_launch<kRadixItemsSmall, true, true>(a, per_sm[2], sms, s);
+      if (kind == 3) pass_launch<kRadixItemsSmall, false, true>(a, per_sm[3], sms, s);
+    } else {
+      if (kind == 0) pass_launch<kRadixItems, true, false>(a, per_sm[0], sms, s);
+      if (kind == 1) pass_launch<kRadixItems, false, false>(a, per_sm[1], sms, s);
+      if (kind == 2) pass_launch<kRadixItems, true, true>(a, per_sm[2], sms, s);
+      if (kind == 3) pass_launch<kRadixItems, false, true>(a, per_sm[3], sms, s);
+    }
   }
   int64_t gg = (n + kGatherThreads * kGatherUnroll - 1) / (kGatherThreads * kGatherUnroll);
   if (gg > (int64_t)sms * 8) gg = (int64_t)sms * 8;
   if (gg < 1) gg = 1;
-  k_radix_gather<<<(unsigned)gg, kGatherThreads, 0, s>>>(table, n, w->keys[0], w->keys[1],
-                                                          w->pos[0], w->pos[1], w->plan,
+  k_radix_gather<<<(unsigned)gg, kGatherThreads, 0, s>>>(table, n, w->pos[0], w->pos[1], w->plan,
                                                           w->counters, flag, err);
-  int g = (int)((n + 255) / 256);
-  if (g > 152 * 16) g = 152 * 16;
+  int64_t g = (n + 255) / 256;
+  if (g > (int64_t)sms * 16) g = (int64_t)sms * 16;
   if (g < 1) g = 1;
   // pos[] is free once gathered: it holds the list of long runs
-  k_radix_ties<<<g, 256, 0, s>>>(table, n, w->keys[0], w->keys[1], w->plan, w->counters,
-                                 w->pos[0], w->pos[1], flag, err);
-  // and, once the runs are listed, the key buffers are scratch for long ones
-  k_radix_long_ties<<<sms, kLongTieThreads, 0, s>>>(table, n, w->keys[0], w->keys[1],
-                                                    w->counters, w->pos[0], w->pos[1], flag,
-                                                    err);
-  k_radix_flip<<<1, 1, 0, s>>>(table, flag, err);
+  k_radix_ties<<<(unsigned)g, 256, 0, s>>>(table, n, 8 * first, w->counters, w->pos[0], w->pos[1],
+                                           flag, err);
+  // and the key buffers are scratch for long ones
+  k_radix_long_ties<<<sms, kLongTieThreads, 0, s>>>(table, n, 8 * first, w->keys[0], w->keys[1],
+                                                    w->counters, w->pos[0], w->pos[1], flag, err);
 }
 
 }  // namespace wg
-
