@@ -156,7 +156,8 @@ struct wg_sim {
   double* h_t = nullptr;         // pinned host mirrors
   unsigned* h_ep = nullptr;
   StepFlags* h_flags = nullptr;
-  unsigned* h_ab = nullptr;      // page-locked copy of the overflow count and abort word
+  unsigned* h_big = nullptr;
+  unsigned* h_ab = nullptr;      // page-locked: overflow words [0..3], error word [4], drop-in [8]
   // a call enqueued by wg_step_begin and not yet completed by wg_step_end
   bool pend_active = false;
   bool pend_compact = false;     // ... and it runs on the compact path
@@ -169,10 +170,11 @@ struct wg_sim {
   int64_t nb = 0;        // buckets: ceil(n / target)
   // Slots per bucket in the layouts: kBucketCapBig where the memory allows
   // (a bucket above kBucketCap sheets is then taken in chunks by
-  // k_bucket_big), else kBucketCap (a fuller bucket overflows).
+  // process_big), else kBucketCap (a fuller bucket overflows).
   int capg = kBucketCap;
-  BigTask* big_list = nullptr;  // [nb]: big buckets of the sub-step in flight
-  unsigned* big_counts = nullptr;  // [2 cap]: per sub-step, listed and taken
+  TaskMeta* big_list = nullptr;  // [nb]: big buckets of the sub-step in flight
+  int* big_next = nullptr;       // [nb]
+  unsigned* big_counts = nullptr;  // [cap]: big buckets taken in each sub-step
   double* bx[2] = {nullptr, nullptr};
   double* bv[2] = {nullptr, nullptr};
   double* bm[2] = {nullptr, nullptr};
@@ -278,10 +280,12 @@ int alloc_call_arrays(wg_sim* s, int nleap) {
   if (s->h_t) cudaFreeHost(s->h_t);
   if (s->h_ep) cudaFreeHost(s->h_ep);
   if (s->h_flags) cudaFreeHost(s->h_flags);
+  if (s->h_big) cudaFreeHost(s->h_big);
   s->small = nullptr;
   s->h_t = nullptr;
   s->h_ep = nullptr;
   s->h_flags = nullptr;
+  s->h_big = nullptr;
   const size_t b = al(sizeof(StateTable)) + al(64) + al(sizeof(StepFlags) * (cap + 1)) +
                    al(4 * (size_t)cap) + al(8 * (size_t)cap) + al(4 * (size_t)cap) +
                    al(8 * (size_t)cap);
@@ -293,12 +297,13 @@ int alloc_call_arrays(wg_sim* s, int nleap) {
   s->tickets = reinterpret_cast<unsigned*>(p); p += al(4 * (size_t)cap);
   s->t_seq = reinterpret_cast<double*>(p); p += al(8 * (size_t)cap);
   s->epochs = reinterpret_cast<unsigned*>(p); p += al(4 * (size_t)cap);
-  s->big_counts = reinterpret_cast<unsigned*>(p); p += al(8 * (size_t)cap);
+  s->big_counts = reinterpret_cast<unsigned*>(p); p += al(4 * (size_t)cap);
   WG_CUDA(cudaMemsetAsync(s->small, 0, b, s->stream));
   WG_CUDA(cudaMemcpyAsync(s->table, &t, sizeof(t), cudaMemcpyHostToDevice, s->stream));
   WG_CUDA(cudaMallocHost(&s->h_t, 8 * (size_t)cap));
   WG_CUDA(cudaMallocHost(&s->h_ep, 4 * (size_t)cap));
   WG_CUDA(cudaMallocHost(&s->h_flags, sizeof(StepFlags) * (cap + 1)));
+  WG_CUDA(cudaMallocHost(&s->h_big, 4 * (size_t)cap));
   if (!s->h_ab) WG_CUDA(cudaMallocHost(&s->h_ab, 64));
   WG_CUDA(cudaStreamSynchronize(s->stream));
   s->cap = cap;
@@ -316,6 +321,7 @@ void free_sim(wg_sim* s) {
   if (s->h_t) cudaFreeHost(s->h_t);
   if (s->h_ep) cudaFreeHost(s->h_ep);
   if (s->h_flags) cudaFreeHost(s->h_flags);
+  if (s->h_big) cudaFreeHost(s->h_big);
   if (s->h_ab) cudaFreeHost(s->h_ab);
   if (s->up_stream) cudaStreamSynchronize(s->up_stream);
   if (s->down_stream) cudaStreamSynchronize(s->down_stream);
@@ -446,7 +452,7 @@ int make_sim(int64_t n, double totmass, double omega2, const ExtSpec& ext, wg_si
            al(sizeof(BucketRec) * (size_t)nb) + 3 * nd + ni + al(64) + al(4 * (size_t)nb) +
            al(sizeof(SimDev)) + al(sizeof(BucketTask) * (size_t)nb) +
            al(8 * 4 * (size_t)(kEnergyBlocks + 1)) +
-           (capg > kBucketCap ? al(sizeof(BigTask) * (size_t)nb) : 0);
+           (capg > kBucketCap ? al(sizeof(TaskMeta) * (size_t)nb) + al(4 * (size_t)nb) : 0);
   };
   // (a bucket of up to kBucketCap / 4 sheets has room for four times its
   // target already: such layouts need no big buckets)
@@ -493,8 +499,8 @@ int make_sim(int64_t n, double totmass, double omega2, const ExtSpec& ext, wg_si
   s->d_tasks = reinterpret_cast<BucketTask*>(p); p += al(sizeof(BucketTask) * (size_t)nb);
   s->diag = reinterpret_cast<double*>(p); p += al(8 * 4 * (size_t)(kEnergyBlocks + 1));
   if (s->capg > kBucketCap) {
-    s->big_list = reinterpret_cast<BigTask*>(p);
-    p += al(sizeof(BigTask) * (size_t)nb);
+    s->big_list = reinterpret_cast<TaskMeta*>(p); p += al(sizeof(TaskMeta) * (size_t)nb);
+    s->big_next = reinterpret_cast<int*>(p); p += al(4 * (size_t)nb);
   }
   {
     std::vector<BucketTask> tasks((size_t)nb);
@@ -594,13 +600,23 @@ int validate_sheets(int64_t n, const double* x, const double* v, const double* m
   return WG_OK;
 }
 
-// Read the device error word and the per-sub-step flags of the last call.
-int finish_call(wg_sim* s, int nleap, bool count_sorts = true) {
-  unsigned err = 0;
-  WG_CUDA(cudaMemcpyAsync(&err, s->err, 4, cudaMemcpyDeviceToHost, s->stream));
+// Enqueue the copies of what the host looks at after a call: the overflow
+// words, the device error word, the per-sub-step flags and big-bucket counts.
+int copy_back(wg_sim* s, int nleap) {
+  WG_CUDA(cudaMemcpyAsync(s->h_ab, s->ocount, 16, cudaMemcpyDeviceToHost, s->stream));
+  WG_CUDA(cudaMemcpyAsync(s->h_ab + 4, s->err, 4, cudaMemcpyDeviceToHost, s->stream));
   WG_CUDA(cudaMemcpyAsync(s->h_flags, s->flags, sizeof(StepFlags) * (nleap + 1),
                           cudaMemcpyDeviceToHost, s->stream));
-  WG_CUDA(cudaStreamSynchronize(s->stream));
+  if (s->capg > kBucketCap && nleap > 0)
+    WG_CUDA(cudaMemcpyAsync(s->h_big, s->big_counts, 4 * (size_t)nleap, cudaMemcpyDeviceToHost,
+                            s->stream));
+  return WG_OK;
+}
+
+// Account for a call whose copy_back has arrived; fails if a kernel raised the
+// device error word.
+int finish_copied(wg_sim* s, int nleap, bool count_sorts) {
+  const unsigned err = s->h_ab[4];
   for (int i = 0; i < nleap && count_sorts; ++i) {
     if (s->h_flags[i].unsorted)
       s->st.sorts_full++;
@@ -618,15 +634,9 @@ int finish_call(wg_sim* s, int nleap, bool count_sorts = true) {
     s->pred_calls = kPredCalls;
   else if (s->pred_calls > 0 && mc > 0)
     --s->pred_calls;
-  if (s->big_list && nleap > 0) {
-    // big buckets listed per sub-step (of the launches that ran last for each)
-    std::vector<unsigned> bc(2 * (size_t)nleap);
-    if (cudaMemcpy(bc.data(), s->big_counts, 8 * (size_t)nleap, cudaMemcpyDeviceToHost) ==
-        cudaSuccess)
-      for (int i = 0; i < nleap; ++i) s->st.big_buckets += bc[2 * (size_t)i];
-    else
-      cudaGetLastError();
-  }
+  if (s->capg > kBucketCap)
+    // big buckets taken per sub-step (of the launches that ran last for each)
+    for (int i = 0; i < nleap; ++i) s->st.big_buckets += s->h_big[i];
   if (err) {
     set_error("device error word 0x%x (%s); the simulation's state is lost, destroy it", err,
               device_error_names(err).c_str());
@@ -635,6 +645,14 @@ int finish_call(wg_sim* s, int nleap, bool count_sorts = true) {
     return WG_ERR_DEVICE;
   }
   return WG_OK;
+}
+
+// Both, with a wait in between.
+int finish_call(wg_sim* s, int nleap, bool count_sorts = true) {
+  const int rc = copy_back(s, nleap);
+  if (rc) return rc;
+  WG_CUDA(cudaStreamSynchronize(s->stream));
+  return finish_copied(s, nleap, count_sorts);
 }
 
 static_assert(kMaxLeap == WG_MAX_LEAP, "sub-step limit of the C header");
@@ -764,18 +782,15 @@ StepLaunch step_launch(wg_sim* s, int i, int nleap, int profile) {
   L.profile = profile;
   L.any_expr = s->ext.kind == EXT_EXPR;
   L.big_list = s->big_list;
-  L.big_count = s->big_counts + 2 * i;
-  L.big_ticket = s->big_counts + 2 * i + 1;
-  L.big_cap = s->big_list ? (unsigned)s->nb : 0u;
+  L.big_next = s->big_next;
+  L.big_count = s->big_counts + i;
   return L;
 }
 
-// One sub-step on the bucket path: the fused kernel, then (simulations whose
-// buckets can outgrow shared memory) the big buckets it listed.
+// One sub-step on the bucket path.
 void launch_substep(wg_sim* s, int i, int nleap, int profile) {
   const StepLaunch L = step_launch(s, i, nleap, profile);
   launch_bucket_step(L, s->grid_bucket, s->stream);
-  if (s->big_list) launch_bucket_big(L, s->grid_bucket, s->stream);
   if (s->dev.ptab) {
     // the samples this sub-step wrote, sorted, become the splitters it
     // would have published (those of the layout after next)
@@ -1048,12 +1063,15 @@ static int run_call_begin(wg_sim* s, double dt, int nleap, double* t0, bool reco
     }
     rc = enqueue_step(s, dt, nleap, s->call_a != nullptr, dt / 2.);
     if (rc) return rc;
-    WG_CUDA(cudaMemsetAsync(s->big_counts, 0, 8 * (size_t)nleap, s->stream));
+    WG_CUDA(cudaMemsetAsync(s->big_counts, 0, 4 * (size_t)nleap, s->stream));
     s->st.substeps_compact += nleap;
     if (s->call_a) launch_scatter_accel(s->table, s->n, s->a_sorted, s->call_a, s->stream);
     if (s->call_xi)
       store_sheets(s->table, s->n, reinterpret_cast<wg_sheet*>(s->call_xi), s->stream);
     s->compact_calls--;
+    rc = copy_back(s, nleap);
+    if (rc) return rc;
+    WG_CUDA(cudaEventRecord(s->ev1, s->stream));
     s->pend_active = true;
     s->pend_compact = true;
     s->pend_dt = dt;
@@ -1067,7 +1085,7 @@ static int run_call_begin(wg_sim* s, double dt, int nleap, double* t0, bool reco
   WG_CUDA(cudaMemcpyAsync(s->epochs, s->h_ep, 4 * (size_t)nleap, cudaMemcpyHostToDevice, s->stream));
   WG_CUDA(cudaMemsetAsync(s->flags, 0, sizeof(StepFlags) * (nleap + 1), s->stream));
   WG_CUDA(cudaMemsetAsync(s->tickets, 0, 4 * (size_t)nleap, s->stream));
-  WG_CUDA(cudaMemsetAsync(s->big_counts, 0, 8 * (size_t)nleap, s->stream));
+  WG_CUDA(cudaMemsetAsync(s->big_counts, 0, 4 * (size_t)nleap, s->stream));
   // overflow count, abort word and redo word
   WG_CUDA(cudaMemsetAsync(s->ocount, 0, 16, s->stream));
   if (s->mode == 1 && dt != s->pending_dt) {
@@ -1101,9 +1119,9 @@ static int run_call_begin(wg_sim* s, double dt, int nleap, double* t0, bool reco
   s->cslot = (cs0 + nleap) % kAggSlots;
   s->st.launches += nleap + 1;
   WG_CUDA(cudaGetLastError());
-  WG_CUDA(cudaMemcpyAsync(s->h_ab, s->ocount, 16, cudaMemcpyDeviceToHost, s->stream));
-  WG_CUDA(cudaMemcpyAsync(s->h_flags, s->flags, sizeof(StepFlags) * (nleap + 1),
-                          cudaMemcpyDeviceToHost, s->stream));
+  rc = copy_back(s, nleap);
+  if (rc) return rc;
+  WG_CUDA(cudaEventRecord(s->ev1, s->stream));
   s->pend_active = true;
   s->pend_dt = dt;
   s->pend_nleap = nleap;
@@ -1143,8 +1161,8 @@ static int run_call_end(wg_sim* s, double* time_elapsed) {
   }
   if (s->pend_compact) {
     s->pend_compact = false;
-    WG_CUDA(cudaEventRecord(s->ev1, s->stream));
-    rc = finish_call(s, nleap, true);  // waits
+    WG_CUDA(cudaEventSynchronize(s->ev1));
+    rc = finish_copied(s, nleap, true);
     s->out_valid = false;  // the sheets are sorted, x_out is stale
     s->mode = 0;
     s->pending_dt = dt;
@@ -1157,7 +1175,7 @@ static int run_call_end(wg_sim* s, double* time_elapsed) {
     return rc;
   }
   int lay0 = s->pend_lay0, cs0 = s->pend_cs0, qs0 = (s->qsel - nleap) & 1;
-  WG_CUDA(cudaStreamSynchronize(s->stream));
+  WG_CUDA(cudaEventSynchronize(s->ev1));
   s->out_valid = true;
   s->mode = 1;
   s->pending_dt = dt;
@@ -1239,8 +1257,7 @@ static int run_call_end(wg_sim* s, double* time_elapsed) {
     WG_CUDA(cudaMemsetAsync(s->ocount, 0, 16, s->stream));
     // the skipped launches of these sub-steps consumed their tickets
     WG_CUDA(cudaMemsetAsync(s->tickets + from, 0, 4 * (size_t)(nleap - from), s->stream));
-    WG_CUDA(cudaMemsetAsync(s->big_counts + 2 * from, 0, 8 * (size_t)(nleap - from),
-                            s->stream));
+    WG_CUDA(cudaMemsetAsync(s->big_counts + from, 0, 4 * (size_t)(nleap - from), s->stream));
     for (int i = from; i < nleap; ++i) launch_substep(s, i, nleap, 0);
     launch_split_out(s->dev.rec_out, s->n, s->x_out, s->v_out, s->call_a, s->stream);
     s->lay = (lay0 + nleap) & 1;
@@ -1248,15 +1265,18 @@ static int run_call_end(wg_sim* s, double* time_elapsed) {
     s->cslot = (cs0 + nleap) % kAggSlots;
     s->st.launches += 4 + kRadixLaunches + (nleap - from);
     WG_CUDA(cudaGetLastError());
-    WG_CUDA(cudaMemcpyAsync(s->h_ab, s->ocount, 16, cudaMemcpyDeviceToHost, s->stream));
-    WG_CUDA(cudaMemcpyAsync(s->h_flags, s->flags, sizeof(StepFlags) * (nleap + 1),
-                            cudaMemcpyDeviceToHost, s->stream));
+    rc = copy_back(s, nleap);
+    if (rc) return rc;
     WG_CUDA(cudaStreamSynchronize(s->stream));
   }
   s->st.sorts_window += window_steps;
   if (clean && s->backoff > 1) s->backoff /= 2;
-  WG_CUDA(cudaEventRecord(s->ev1, s->stream));
-  rc = finish_call(s, nleap, false);
+  if (clean) {
+    rc = finish_copied(s, nleap, false);  // its copies came with the call
+  } else {
+    WG_CUDA(cudaEventRecord(s->ev1, s->stream));
+    rc = finish_call(s, nleap, false);
+  }
   float ms = 0;
   cudaEventElapsedTime(&ms, s->ev0, s->ev1);
   if (time_elapsed) *time_elapsed = ms * 1e-3;
@@ -1426,7 +1446,7 @@ int wg_profile(wg_sim* s, int what, int reps, double* avg_seconds) {
   WG_CUDA(cudaMemcpyAsync(s->t_seq, s->h_t, 8 * (size_t)reps, cudaMemcpyHostToDevice, s->stream));
   WG_CUDA(cudaMemcpyAsync(s->epochs, s->h_ep, 4 * (size_t)reps, cudaMemcpyHostToDevice, s->stream));
   WG_CUDA(cudaMemsetAsync(s->tickets, 0, 4 * (size_t)reps, s->stream));
-  WG_CUDA(cudaMemsetAsync(s->big_counts, 0, 8 * (size_t)reps, s->stream));
+  WG_CUDA(cudaMemsetAsync(s->big_counts, 0, 4 * (size_t)reps, s->stream));
   // flags[i].unsorted = 1 forces every sort to run in full
   for (int i = 0; i < reps; ++i) s->h_flags[i] = StepFlags{1u, 0u, 0ull};
   WG_CUDA(cudaMemcpyAsync(s->flags, s->h_flags, sizeof(StepFlags) * (size_t)reps,

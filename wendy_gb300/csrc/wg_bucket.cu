@@ -82,28 +82,6 @@ struct LsdSmem {
   uint16_t hist[WARPS][256];
 };
 
-// What the processing of one task needs, prepared by warp 0 one task ahead
-// (while the other warps write out the current bucket), so that a bucket's
-// load waits only for its bulk copies and not for a chain of dependent global
-// reads, and its mass prefix is known before it starts.
-struct TaskMeta {
-  const double* x;  // the bucket's sheets
-  const double* v;
-  const double* m;
-  const int32_t* idx;
-  int64_t bucket;
-  unsigned task;  // ticket; ntasks or more ends the launch
-  int sim;
-  int n;          // sheets in the bucket; -1: the simulation has aborted this call
-  int lay;        // layout read by this sub-step
-  uint32_t pcnt;  // sheets in the simulation's earlier buckets
-  int wlo, whi;   // splitter window [wlo, whi] of the next layout ...
-  int wbuf;       // ... in wkey[wbuf], widx[wbuf]
-  double amp;     // time factor of a pulsed external force at this sub-step
-  double inv_h;   // 1 / h of a pulsed external force
-  uint64_t pm_lo, pm_hi;  // their fixed-point mass
-};
-
 struct __align__(16) StepSmem {
   double x[CAP];
   double v[CAP];
@@ -150,7 +128,8 @@ struct __align__(16) StepSmem {
   int32_t samp_idx[4];
   uint32_t samp_q[4];
   uint64_t mbar;  // completion of the bucket's bulk copies
-  // a big bucket (k_bucket_big): its chunks as ranges of key bins
+  int big_head;   // first of the big buckets this CTA has claimed (-1: none)
+  // a big bucket (process_big): its chunks as ranges of key bins
   int chunk_lo[kMaxChunks + 1];
   int nchunks;
   unsigned load_cnt;  // sheets of the current chunk gathered so far
@@ -164,7 +143,7 @@ struct __align__(16) StepSmem {
 // recomputed conversions cost.
 static_assert(CTAS * (sizeof(StepSmem) + 1024) <= 228 * 1024, "StepSmem too large");
 static_assert(LUTN == BT, "one routing-table cell per thread");
-// k_bucket_big keeps its histogram where its chunks' positions go later
+// process_big keeps its histogram where its chunks' positions go later
 static_assert(sizeof(double) * CAP >= 4 * BIGBINS, "big-bucket histogram");
 
 __device__ __forceinline__ bool pair_less(uint64_t k1, int32_t i1, uint64_t k2, int32_t i2) {
@@ -1174,46 +1153,216 @@ __device__ __forceinline__ bool process_bucket(const StepLaunch& L, StepSmem& S,
   return true;
 }
 
-// Appends a big bucket's task to the list k_bucket_big works through (one
-// thread).  Kept out of line: inlined, its fields stayed live across the
-// bucket loop and pushed the kernel into register spills.
-static __device__ __noinline__ void list_big(const TaskMeta* tm, unsigned* big_count,
-                                             unsigned big_cap, BigTask* big_list,
-                                             unsigned* err) {
-  const unsigned slot = atomicAdd(big_count, 1u);
-  if (slot >= big_cap) {
-    atomicOr(err, DEV_ERR_BAD_STATE);
+// Bin of a key in [kmin, kmin + span] among BIGBINS (non-decreasing in the
+// key; the same multiplicative map as the in-bucket counting sort).
+__device__ __forceinline__ int big_bin(uint64_t k, uint64_t kmin, uint64_t span, uint64_t scale) {
+  const uint64_t dk = k - kmin;
+  return span < (uint64_t)BIGBINS ? (int)dk : (int)__umul64hi(dk, scale);
+}
+
+// Position (with the opening half drift of a call applied) of slot j.
+__device__ __forceinline__ double big_pos(const double* gx, const double* gv, int j, double pre) {
+  const double x = gx[j];
+  return pre != 0.0 ? fma(pre, gv[j], x) : x;
+}
+
+// Block-wide minimum and maximum of per-thread key ranges (all threads).
+__device__ __forceinline__ void block_range(StepSmem& S, uint64_t& kmin, uint64_t& kmax) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+#pragma unroll
+  for (int d = 16; d >= 1; d >>= 1) {
+    const uint64_t o1 = __shfl_xor_sync(0xffffffffu, kmin, d);
+    const uint64_t o2 = __shfl_xor_sync(0xffffffffu, kmax, d);
+    kmin = o1 < kmin ? o1 : kmin;
+    kmax = o2 > kmax ? o2 : kmax;
+  }
+  if (lane == 0) {
+    S.red_min[warp] = kmin;
+    S.red_max[warp] = kmax;
+  }
+  __syncthreads();
+  kmin = ~0ull;
+  kmax = 0;
+#pragma unroll
+  for (int w = 0; w < WARPS; ++w) {
+    kmin = S.red_min[w] < kmin ? S.red_min[w] : kmin;
+    kmax = S.red_max[w] > kmax ? S.red_max[w] : kmax;
+  }
+  __syncthreads();  // red_min / red_max are free again
+}
+
+// Puts a big bucket's task on this CTA's list (one thread; entries by bucket,
+// chained from S.big_head).  Kept out of line: inlined, its fields stayed live
+// across the bucket loop and pushed the kernel into register spills.
+static __device__ __noinline__ void list_big(StepSmem& S, TaskMeta* big_list, int* big_next,
+                                             unsigned* big_count) {
+  const int b = (int)S.next.bucket;
+  big_list[b] = S.next;
+  big_next[b] = S.big_head;
+  S.big_head = b;
+  atomicAdd(big_count, 1u);
+}
+
+// A big bucket (kBucketCap < n <= capg sheets): cut by key into chunks that
+// fit in shared memory -- a histogram of its keys over BIGBINS bins, chunks
+// along the bins -- each chunk gathered from the layout and processed like a
+// bucket, the chunks in key order with the mass and rank prefix carried from
+// one to the next.  A bucket whose keys crowd into one bin beyond CAP - CHUNK
+// cannot be cut this way: the simulation is flagged (ocount[2]) and its host
+// side re-sorts the layout this sub-step read, which the sub-step leaves
+// intact.  A CTA keeps the big buckets it has claimed for when it has no other
+// task left; a second launch per sub-step for buckets that are rarely there
+// cost 3.3 us and the gap before it, empty.
+template <bool LAST, bool EXPR>
+__device__ __forceinline__ void process_big(const StepLaunch& L, StepSmem& S, const TaskMeta& bt,
+                                            int sub, unsigned ep) {
+  const int tid = threadIdx.x;
+  const SimDev& D = L.sims[bt.sim];
+  const int n = bt.n;
+  const double* gx = bt.x;
+  const double* gv = bt.v;
+  const double* gm = bt.m;
+  const int32_t* gi = bt.idx;
+  const double pre = sub == 0 ? D.pre_dt : 0.0;
+  // the splitter window of the next layout around the bucket
+  {
+    const int qs = (D.qsel0 + sub) & 1;
+    for (int j = tid; j <= bt.whi - bt.wlo; j += BT) {
+      S.wkey[0][j] = D.qk[qs][bt.wlo + j];
+      S.widx[0][j] = D.qi[qs][bt.wlo + j];
+    }
+  }
+  if (tid == 0) {
+    S.win_lo = bt.wlo;
+    S.win_hi = bt.whi;
+    S.cur_wbuf = 0;
+    S.maxv = 0;
+    S.maxc = 0;
+    S.nsamp = 0;
+    S.prefix_mass = (((u128)bt.pm_hi) << 64) | bt.pm_lo;
+    S.prefix_cnt = bt.pcnt;
+    S.amp = bt.amp;
+    S.inv_h = bt.inv_h;
+    S.nchunks = 0;
+    S.splittable = 1u;
+    for (int c = 0; c <= kMaxChunks; ++c) S.chunk_lo[c] = BIGBINS;
+  }
+  // ---- the bucket's key range and the histogram of its keys
+  uint64_t kmin = ~0ull, kmax = 0;
+  for (int j = tid; j < n; j += BT) {
+    const uint64_t k = key_of(big_pos(gx, gv, j, pre));
+    kmin = k < kmin ? k : kmin;
+    kmax = k > kmax ? k : kmax;
+  }
+  // BIGBINS 32-bit counters where the chunks' positions go later
+  uint32_t* hist = reinterpret_cast<uint32_t*>(S.x);
+  for (int j = tid; j < BIGBINS; j += BT) hist[j] = 0u;
+  block_range(S, kmin, kmax);
+  const uint64_t span = kmax - kmin;
+  uint64_t scale = 0;
+  if (span >= (uint64_t)BIGBINS)
+    scale = (uint64_t)((float)BIGBINS / ((float)span + 1.0f) * 18446744073709551616.0f *
+                       (1.0f - 9.5367431640625e-07f));
+  for (int j = tid; j < n; j += BT) {
+    const int bin = big_bin(key_of(big_pos(gx, gv, j, pre)), kmin, span, scale);
+    atomicAdd(&hist[bin], 1u);
+  }
+  __syncthreads();
+  // ---- chunks: thread tid owns bins [16 tid, 16 tid + 16)
+  {
+    constexpr int BPT = BIGBINS / BT;
+    uint32_t c[BPT], sum = 0, mx = 0;
+#pragma unroll
+    for (int k = 0; k < BPT; ++k) {
+      c[k] = hist[tid * BPT + k];
+      sum += c[k];
+      mx = c[k] > mx ? c[k] : mx;
+    }
+    uint32_t tot;
+    uint32_t ex = block_excl_scan(S, sum, tot);
+    if (mx > (uint32_t)(CAP - CHUNK)) atomicAnd(&S.splittable, 0u);
+    // non-empty bin i belongs to chunk floor(ex_i / CHUNK), ex_i the
+    // sheets in earlier bins; a chunk starts at its first bin.  With no
+    // bin above CHUNK, consecutive non-empty bins differ by at most one
+    // chunk, and a chunk holds fewer than 2 CHUNK = CAP sheets.
+#pragma unroll
+    for (int k = 0; k < BPT; ++k) {
+      if (c[k]) {
+        const uint32_t chunk = ex / CHUNK;
+        if (chunk < (uint32_t)kMaxChunks) atomicMin(&S.chunk_lo[chunk], tid * BPT + k);
+        atomicMax(&S.nchunks, (int)chunk + 1);
+      }
+      ex += c[k];
+    }
+  }
+  __syncthreads();
+  const int nchunks = S.nchunks;
+  if (!S.splittable || nchunks > kMaxChunks) {
+    // keys crowded into one bin: the host re-sorts the layout read here
+    if (tid == 0) {
+      atomicCAS(D.ocount + 2, 0u, (unsigned)(sub + 1));
+      atomicCAS(D.ocount + 1, 0u, (unsigned)(sub + 1));
+    }
     return;
   }
-  BigTask bt;
-  bt.sim = tm->sim;
-  bt.bucket = (int)tm->bucket;
-  bt.n = tm->n;
-  bt.lay = tm->lay;
-  bt.wlo = tm->wlo;
-  bt.whi = tm->whi;
-  bt.pcnt = tm->pcnt;
-  bt.pm_lo = tm->pm_lo;
-  bt.pm_hi = tm->pm_hi;
-  bt.amp = tm->amp;
-  bt.inv_h = tm->inv_h;
-  big_list[slot] = bt;
+  if (tid == 0) {
+    S.chunk_lo[0] = 0;  // bins below the first non-empty one are empty
+    S.chunk_lo[nchunks] = BIGBINS;
+  }
+  __syncthreads();
+  // ---- the chunks in key order
+  for (int ch = 0; ch < nchunks; ++ch) {
+    const int blo = S.chunk_lo[ch], bhi = S.chunk_lo[ch + 1];
+    clear_bins(S, step_sort_bits(D));
+    for (int j = tid; j <= S.win_hi - S.win_lo; j += BT) S.dcount[j] = 0;
+    if (tid == 0) {
+      S.load_cnt = 0;
+      S.nsamp = 0;  // splitter samples of this chunk
+    }
+    __syncthreads();
+    for (int j = tid; j < n; j += BT) {
+      const double x = big_pos(gx, gv, j, pre);
+      const uint64_t k = key_of(x);
+      const int bin = big_bin(k, kmin, span, scale);
+      if (bin >= blo && bin < bhi) {
+        const unsigned slot = atomicAdd(&S.load_cnt, 1u);
+        if (slot < (unsigned)CAP) {
+          S.x[slot] = x;
+          S.v[slot] = gv[j];
+          S.m[slot] = gm[j];
+          S.idx[slot] = gi[j];
+        }
+      }
+    }
+    __syncthreads();
+    const int nc = (int)S.load_cnt;
+    if (nc > CAP) {  // cannot happen with the chunk rule; never write past the arrays
+      if (tid == 0) atomicOr(L.err, DEV_ERR_BAD_STATE);
+      break;
+    }
+    if (nc == 0) continue;
+    const int rcell = route_cell(S, S.wkey[0], bt.wlo, bt.whi, D.nb);
+    process_bucket<LAST, EXPR, false>(L, S, D, bt.bucket, bt.lay, nc, sub, ep, true, 0.0, rcell,
+                                      0u);
+  }
 }
 
 // The fused sub-step.  LAST: the call's last sub-step (half drift, outputs).
 // EXPR: the launch has simulations with expression forces (the interpreter
 // is compiled only into this instantiation).
 template <bool LAST, bool EXPR>
-__global__ void __launch_bounds__(BT, CTAS) k_bucket_step(const StepLaunch L) {
+__global__ void __launch_bounds__(BT, CTAS) k_bucket_step(const __grid_constant__ StepLaunch L) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   StepSmem& S = *reinterpret_cast<StepSmem*>(smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int sub = L.sub;
-  const unsigned ep = L.epochs[sub];
   if (tid == 0) {
+    S.big_head = -1;
     mbar_init(&S.mbar, 1);
     fence_proxy_async_smem();
   }
+  chain_begin();
+  const unsigned ep = L.epochs[sub];
   if (warp == 0) claim_task(L, sub, ep, lane, S, 0);
   unsigned parity = 0;
   for (;;) {
@@ -1223,9 +1372,8 @@ __global__ void __launch_bounds__(BT, CTAS) k_bucket_step(const StepLaunch L) {
     if (tm.n < 0 || tm.n > CAP) {
       // n < 0: the simulation has aborted this call.  n > CAP: more sheets
       // than shared memory holds (a simulation whose layout has room for
-      // them): listed for k_bucket_big, which runs next on the stream and
-      // takes the bucket in chunks; its prefix is known already.
-      if (tm.n > CAP && tid == 0) list_big(&S.next, L.big_count, L.big_cap, L.big_list, L.err);
+      // them), taken in chunks after the others
+      if (tm.n > CAP && tid == 0) list_big(S, L.big_list, L.big_next, L.big_count);
       __syncthreads();  // every thread has read S.next
       if (warp == 0) claim_task(L, sub, ep, lane, S, tm.wbuf);
       continue;
@@ -1282,203 +1430,16 @@ __global__ void __launch_bounds__(BT, CTAS) k_bucket_step(const StepLaunch L) {
       // (the call fails and the simulation is given up).
       if (tid == 0) atomicOr(L.err, DEV_ERR_COPY_TIMEOUT);
       mbar_wait(&S.mbar, parity);
-      break;
+      return;
     }
     if (n4 > 0) parity ^= 1u;
   }
-}
-
-// Bin of a key in [kmin, kmin + span] among BIGBINS (non-decreasing in the
-// key; the same multiplicative map as the in-bucket counting sort).
-__device__ __forceinline__ int big_bin(uint64_t k, uint64_t kmin, uint64_t span, uint64_t scale) {
-  const uint64_t dk = k - kmin;
-  return span < (uint64_t)BIGBINS ? (int)dk : (int)__umul64hi(dk, scale);
-}
-
-// Position (with the opening half drift of a call applied) of slot j.
-__device__ __forceinline__ double big_pos(const double* gx, const double* gv, int j, double pre) {
-  const double x = gx[j];
-  return pre != 0.0 ? fma(pre, gv[j], x) : x;
-}
-
-// Block-wide minimum and maximum of per-thread key ranges (all threads).
-__device__ __forceinline__ void block_range(StepSmem& S, uint64_t& kmin, uint64_t& kmax) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-#pragma unroll
-  for (int d = 16; d >= 1; d >>= 1) {
-    const uint64_t o1 = __shfl_xor_sync(0xffffffffu, kmin, d);
-    const uint64_t o2 = __shfl_xor_sync(0xffffffffu, kmax, d);
-    kmin = o1 < kmin ? o1 : kmin;
-    kmax = o2 > kmax ? o2 : kmax;
-  }
-  if (lane == 0) {
-    S.red_min[warp] = kmin;
-    S.red_max[warp] = kmax;
-  }
-  __syncthreads();
-  kmin = ~0ull;
-  kmax = 0;
-#pragma unroll
-  for (int w = 0; w < WARPS; ++w) {
-    kmin = S.red_min[w] < kmin ? S.red_min[w] : kmin;
-    kmax = S.red_max[w] > kmax ? S.red_max[w] : kmax;
-  }
-  __syncthreads();  // red_min / red_max are free again
-}
-
-// The big buckets k_bucket_step listed in this sub-step (kBucketCap < n <=
-// capg sheets): each is cut by key into chunks that fit in shared memory --
-// a histogram of its keys over BIGBINS bins, chunks along the bins -- and
-// every chunk is gathered from the layout and processed like a bucket, the
-// chunks in key order with the mass and rank prefix carried from one to the
-// next.  A bucket whose keys crowd into one bin beyond CAP - CHUNK cannot be
-// cut this way: the simulation is flagged (ocount[2]) and its host side
-// re-sorts the layout this sub-step read, which the sub-step leaves intact.
-template <bool LAST, bool EXPR>
-__global__ void __launch_bounds__(BT, CTAS) k_bucket_big(const StepLaunch L) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  StepSmem& S = *reinterpret_cast<StepSmem*>(smem_raw);
-  const int tid = threadIdx.x;
-  const int sub = L.sub;
-  const unsigned ep = L.epochs[sub];
-  const unsigned total = *L.big_count;  // final: k_bucket_step ran before
-  const unsigned ntask = total < L.big_cap ? total : L.big_cap;
-  for (;;) {
+  // ---- the big buckets this CTA claimed
+  for (int b = S.big_head; b >= 0;) {
+    const TaskMeta bt = L.big_list[b];
+    b = L.big_next[b];
+    process_big<LAST, EXPR>(L, S, bt, sub, ep);
     __syncthreads();
-    if (tid == 0) S.next_ticket = atomicAdd(L.big_ticket, 1u);
-    __syncthreads();
-    const unsigned t = S.next_ticket;
-    if (t >= ntask) break;
-    const BigTask bt = L.big_list[t];
-    const SimDev& D = L.sims[bt.sim];
-    const int n = bt.n;
-    const int64_t base = (int64_t)bt.bucket * D.capg;
-    const double* gx = D.bx[bt.lay] + base;
-    const double* gv = D.bv[bt.lay] + base;
-    const double* gm = D.bm[bt.lay] + base;
-    const int32_t* gi = D.bi[bt.lay] + base;
-    const double pre = sub == 0 ? D.pre_dt : 0.0;
-    // the splitter window of the next layout around the bucket
-    {
-      const int qs = (D.qsel0 + sub) & 1;
-      for (int j = tid; j <= bt.whi - bt.wlo; j += BT) {
-        S.wkey[0][j] = D.qk[qs][bt.wlo + j];
-        S.widx[0][j] = D.qi[qs][bt.wlo + j];
-      }
-    }
-    if (tid == 0) {
-      S.win_lo = bt.wlo;
-      S.win_hi = bt.whi;
-      S.cur_wbuf = 0;
-      S.maxv = 0;
-      S.maxc = 0;
-      S.nsamp = 0;
-      S.prefix_mass = (((u128)bt.pm_hi) << 64) | bt.pm_lo;
-      S.prefix_cnt = bt.pcnt;
-      S.amp = bt.amp;
-      S.inv_h = bt.inv_h;
-      S.nchunks = 0;
-      S.splittable = 1u;
-      for (int c = 0; c <= kMaxChunks; ++c) S.chunk_lo[c] = BIGBINS;
-    }
-    // ---- the bucket's key range and the histogram of its keys
-    uint64_t kmin = ~0ull, kmax = 0;
-    for (int j = tid; j < n; j += BT) {
-      const uint64_t k = key_of(big_pos(gx, gv, j, pre));
-      kmin = k < kmin ? k : kmin;
-      kmax = k > kmax ? k : kmax;
-    }
-    // BIGBINS 32-bit counters where the chunks' positions go later
-    uint32_t* hist = reinterpret_cast<uint32_t*>(S.x);
-    for (int j = tid; j < BIGBINS; j += BT) hist[j] = 0u;
-    block_range(S, kmin, kmax);
-    const uint64_t span = kmax - kmin;
-    uint64_t scale = 0;
-    if (span >= (uint64_t)BIGBINS)
-      scale = (uint64_t)((float)BIGBINS / ((float)span + 1.0f) * 18446744073709551616.0f *
-                         (1.0f - 9.5367431640625e-07f));
-    for (int j = tid; j < n; j += BT) {
-      const int bin = big_bin(key_of(big_pos(gx, gv, j, pre)), kmin, span, scale);
-      atomicAdd(&hist[bin], 1u);
-    }
-    __syncthreads();
-    // ---- chunks: thread tid owns bins [16 tid, 16 tid + 16)
-    {
-      constexpr int BPT = BIGBINS / BT;
-      uint32_t c[BPT], sum = 0, mx = 0;
-#pragma unroll
-      for (int k = 0; k < BPT; ++k) {
-        c[k] = hist[tid * BPT + k];
-        sum += c[k];
-        mx = c[k] > mx ? c[k] : mx;
-      }
-      uint32_t tot;
-      uint32_t ex = block_excl_scan(S, sum, tot);
-      if (mx > (uint32_t)(CAP - CHUNK)) atomicAnd(&S.splittable, 0u);
-      // non-empty bin i belongs to chunk floor(ex_i / CHUNK), ex_i the
-      // sheets in earlier bins; a chunk starts at its first bin.  With no
-      // bin above CHUNK, consecutive non-empty bins differ by at most one
-      // chunk, and a chunk holds fewer than 2 CHUNK = CAP sheets.
-#pragma unroll
-      for (int k = 0; k < BPT; ++k) {
-        if (c[k]) {
-          const uint32_t chunk = ex / CHUNK;
-          if (chunk < (uint32_t)kMaxChunks) atomicMin(&S.chunk_lo[chunk], tid * BPT + k);
-          atomicMax(&S.nchunks, (int)chunk + 1);
-        }
-        ex += c[k];
-      }
-    }
-    __syncthreads();
-    const int nchunks = S.nchunks;
-    if (!S.splittable || nchunks > kMaxChunks) {
-      // keys crowded into one bin: the host re-sorts the layout read here
-      if (tid == 0) {
-        atomicCAS(D.ocount + 2, 0u, (unsigned)(sub + 1));
-        atomicCAS(D.ocount + 1, 0u, (unsigned)(sub + 1));
-      }
-      continue;
-    }
-    if (tid == 0) {
-      S.chunk_lo[0] = 0;  // bins below the first non-empty one are empty
-      S.chunk_lo[nchunks] = BIGBINS;
-    }
-    __syncthreads();
-    // ---- the chunks in key order
-    for (int ch = 0; ch < nchunks; ++ch) {
-      const int blo = S.chunk_lo[ch], bhi = S.chunk_lo[ch + 1];
-      clear_bins(S, step_sort_bits(D));
-      for (int j = tid; j <= S.win_hi - S.win_lo; j += BT) S.dcount[j] = 0;
-      if (tid == 0) {
-        S.load_cnt = 0;
-        S.nsamp = 0;  // splitter samples of this chunk
-      }
-      __syncthreads();
-      for (int j = tid; j < n; j += BT) {
-        const double x = big_pos(gx, gv, j, pre);
-        const uint64_t k = key_of(x);
-        const int bin = big_bin(k, kmin, span, scale);
-        if (bin >= blo && bin < bhi) {
-          const unsigned slot = atomicAdd(&S.load_cnt, 1u);
-          if (slot < (unsigned)CAP) {
-            S.x[slot] = x;
-            S.v[slot] = gv[j];
-            S.m[slot] = gm[j];
-            S.idx[slot] = gi[j];
-          }
-        }
-      }
-      __syncthreads();
-      const int nc = (int)S.load_cnt;
-      if (nc > CAP) {  // cannot happen with the chunk rule; never write past the arrays
-        if (tid == 0) atomicOr(L.err, DEV_ERR_BAD_STATE);
-        break;
-      }
-      if (nc == 0) continue;
-      const int rcell = route_cell(S, S.wkey[0], bt.wlo, bt.whi, D.nb);
-      process_bucket<LAST, EXPR, false>(L, S, D, bt.bucket, bt.lay, nc, sub, ep, true, 0.0, rcell,
-                                        0u);
-    }
   }
 }
 
@@ -1628,14 +1589,6 @@ void bucket_attr_init() {
                        (int)sizeof(StepSmem));
   cudaFuncSetAttribute(k_bucket_step<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)sizeof(StepSmem));
-  cudaFuncSetAttribute(k_bucket_big<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)sizeof(StepSmem));
-  cudaFuncSetAttribute(k_bucket_big<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)sizeof(StepSmem));
-  cudaFuncSetAttribute(k_bucket_big<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)sizeof(StepSmem));
-  cudaFuncSetAttribute(k_bucket_big<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)sizeof(StepSmem));
 }
 
 void bucket_step_prepare() {
@@ -1651,6 +1604,7 @@ __global__ void __launch_bounds__(256) k_split_out(const OutRec* __restrict__ re
                                                    double* __restrict__ x_out,
                                                    double* __restrict__ v_out,
                                                    double* __restrict__ a_out) {
+  chain_begin();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
     const double2* r2 = reinterpret_cast<const double2*>(rec + i);
@@ -1666,7 +1620,7 @@ void launch_split_out(const OutRec* rec, int64_t n, double* x_out, double* v_out
   int64_t g = (n + 255) / 256;
   if (g > 152 * 8) g = 152 * 8;
   if (g < 1) g = 1;
-  k_split_out<<<(unsigned)g, 256, 0, s>>>(rec, n, x_out, v_out, a_out);
+  launch_chained(k_split_out, (unsigned)g, 256, 0, s, rec, n, x_out, v_out, a_out);
 }
 
 void launch_bucket_step(const StepLaunch& a, int grid, cudaStream_t s) {
@@ -1674,16 +1628,9 @@ void launch_bucket_step(const StepLaunch& a, int grid, cudaStream_t s) {
   if (grid > a.ntasks) grid = a.ntasks;
   if (grid < 1) grid = 1;
   const bool last = a.sub == a.nleap - 1;
-  if (a.any_expr) {
-    if (last)
-      k_bucket_step<true, true><<<grid, BT, sizeof(StepSmem), s>>>(a);
-    else
-      k_bucket_step<false, true><<<grid, BT, sizeof(StepSmem), s>>>(a);
-  } else if (last) {
-    k_bucket_step<true, false><<<grid, BT, sizeof(StepSmem), s>>>(a);
-  } else {
-    k_bucket_step<false, false><<<grid, BT, sizeof(StepSmem), s>>>(a);
-  }
+  auto* const k = a.any_expr ? (last ? k_bucket_step<true, true> : k_bucket_step<false, true>)
+                             : (last ? k_bucket_step<true, false> : k_bucket_step<false, false>);
+  launch_chained(k, (unsigned)grid, BT, sizeof(StepSmem), s, a);
 }
 
 __global__ void __launch_bounds__(256) k_member_splitters(const SimDev* devs, const int* list,
@@ -1760,6 +1707,7 @@ __global__ void __launch_bounds__(kRankThreads) k_rank_samples(const StateTable*
                                                                uint64_t* qk, int32_t* qi) {
   const int lane = threadIdx.x & 31;
   const int j = blockIdx.x * (kRankThreads / 32) + (threadIdx.x >> 5);
+  chain_begin();
   if (j >= m) return;
   const StateRef c = table->cur;
   const uint64_t kj = key_of(c.x[j]);
@@ -1787,7 +1735,8 @@ __global__ void __launch_bounds__(kRankThreads) k_rank_samples(const StateTable*
 void launch_rank_samples(const StateTable* table, int m, uint64_t* qk, int32_t* qi,
                          cudaStream_t s) {
   const int per = kRankThreads / 32;
-  k_rank_samples<<<(unsigned)((m + per - 1) / per), kRankThreads, 0, s>>>(table, m, qk, qi);
+  launch_chained(k_rank_samples, (unsigned)((m + per - 1) / per), kRankThreads, 0, s, table, m, qk,
+                 qi);
 }
 
 // Exclusive scan of each batch member's clamped bucket counts (one block per
@@ -1931,22 +1880,6 @@ void launch_samples_to_splitters(const StateTable* table, int64_t m, uint64_t* q
   int64_t g = (m + 255) / 256;
   if (g > 1216) g = 1216;
   k_samples_to_splitters<<<(unsigned)(g < 1 ? 1 : g), 256, 0, s>>>(table, m, qk, qi);
-}
-
-void launch_bucket_big(const StepLaunch& a, int grid, cudaStream_t s) {
-  bucket_step_prepare();
-  if (grid < 1) grid = 1;
-  const bool last = a.sub == a.nleap - 1;
-  if (a.any_expr) {
-    if (last)
-      k_bucket_big<true, true><<<grid, BT, sizeof(StepSmem), s>>>(a);
-    else
-      k_bucket_big<false, true><<<grid, BT, sizeof(StepSmem), s>>>(a);
-  } else if (last) {
-    k_bucket_big<true, false><<<grid, BT, sizeof(StepSmem), s>>>(a);
-  } else {
-    k_bucket_big<false, false><<<grid, BT, sizeof(StepSmem), s>>>(a);
-  }
 }
 
 void launch_bucketize(const StateTable* table, int64_t n, int target, int64_t nb, int capg, int E,

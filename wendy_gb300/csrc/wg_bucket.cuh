@@ -132,20 +132,26 @@ struct BucketTask {
   int bucket;
 };
 
-// A bucket with more sheets than shared memory holds (kBucketCap < n <=
-// capg), listed by k_bucket_step for k_bucket_big with what its preparation
-// found: its exclusive (mass, count) prefix, splitter window and force
-// factors.
-struct BigTask {
+// What the processing of one task needs, prepared by warp 0 one task ahead
+// (while the other warps write out the current bucket), so that a bucket's
+// load waits only for its bulk copies and not for a chain of dependent global
+// reads, and its mass prefix is known before it starts.
+struct TaskMeta {
+  const double* x;  // the bucket's sheets
+  const double* v;
+  const double* m;
+  const int32_t* idx;
+  int64_t bucket;
+  unsigned task;  // ticket; ntasks or more ends the launch
   int sim;
-  int bucket;
-  int n;
-  int lay;
-  int wlo, whi;
-  uint32_t pcnt;
-  uint32_t pad;
-  uint64_t pm_lo, pm_hi;
-  double amp, inv_h;
+  int n;          // sheets in the bucket; -1: the simulation has aborted this call
+  int lay;        // layout read by this sub-step
+  uint32_t pcnt;  // sheets in the simulation's earlier buckets
+  int wlo, whi;   // splitter window [wlo, whi] of the next layout ...
+  int wbuf;       // ... in wkey[wbuf], widx[wbuf]
+  double amp;     // time factor of a pulsed external force at this sub-step
+  double inv_h;   // 1 / h of a pulsed external force
+  uint64_t pm_lo, pm_hi;  // their fixed-point mass
 };
 
 struct StepLaunch {
@@ -159,17 +165,14 @@ struct StepLaunch {
   unsigned* err;
   int profile;           // 1: dt = 0 and no outputs (timing harness)
   int any_expr;          // some simulation of the launch has an expression force
-  // big buckets of this sub-step (simulations with capg > kBucketCap only):
-  // the list k_bucket_step fills and k_bucket_big takes in ticket order
-  BigTask* big_list;
-  unsigned* big_count;   // zero before the launch
-  unsigned* big_ticket;  // zero before the launch
-  unsigned big_cap;      // entries of big_list
+  // big buckets (simulations with capg > kBucketCap): by bucket, the task and
+  // the next bucket of the CTA that claimed it; how many there were
+  TaskMeta* big_list;
+  int* big_next;
+  unsigned* big_count;
 };
 
 void launch_bucket_step(const StepLaunch& a, int grid, cudaStream_t s);
-// The big buckets k_bucket_step listed (launch right after it, same arguments).
-void launch_bucket_big(const StepLaunch& a, int grid, cudaStream_t s);
 // Pool members with predicted splitters (SimDev::ptab set): block k sorts the
 // nb - 1 samples member list[k] (k itself without a list) wrote in sub-step
 // `sub` in shared memory and writes them as the splitters that sub-step

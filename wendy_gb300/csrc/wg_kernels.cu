@@ -101,6 +101,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_force_kick_drift(const ForceArgs
   __shared__ unsigned s_epoch;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  chain_begin();
   if (tid == 0) {
     s_tile = atomicAdd(a.ticket, 1u);
     s_unsorted = 0;
@@ -331,12 +332,9 @@ void launch_force(const ForceArgs& a, int64_t n_tiles, cudaStream_t s) {
   ForceArgs b = a;
   b.spin_limit = g_spin_limit;
   b.withhold_tile = g_withhold_tile;
-  if (b.ext.kind == EXT_EXPR)
-    k_force_kick_drift<kForceThreads, kForceItems, true>
-        <<<(unsigned)n_tiles, kForceThreads, 0, s>>>(b);
-  else
-    k_force_kick_drift<kForceThreads, kForceItems, false>
-        <<<(unsigned)n_tiles, kForceThreads, 0, s>>>(b);
+  auto* const k = b.ext.kind == EXT_EXPR ? k_force_kick_drift<kForceThreads, kForceItems, true>
+                                         : k_force_kick_drift<kForceThreads, kForceItems, false>;
+  launch_chained(k, (unsigned)n_tiles, kForceThreads, 0, s, b);
 }
 
 void launch_drift(const StateTable* table, int64_t n, double dt, StepFlags* flag,

@@ -907,10 +907,9 @@ static int pool_step_begin(wg_pool* p, int count, const int* ids, const double* 
       L.err = p->err;
       L.profile = 0;
       L.any_expr = launch_expr;
-      L.big_list = nullptr;
+      L.big_list = nullptr;  // members have no big buckets
+      L.big_next = nullptr;
       L.big_count = nullptr;
-      L.big_ticket = nullptr;
-      L.big_cap = 0;
       launch_bucket_step(L, grid, p->stream);
       // members with predicted splitters: their samples, sorted, become the
       // splitters this sub-step published (one CTA per member; the others
@@ -1166,10 +1165,9 @@ static int pool_step_end(wg_pool* p, double* time_elapsed) {
       L.err = p->err;
       L.profile = 0;
       L.any_expr = any_expr;
-      L.big_list = nullptr;
+      L.big_list = nullptr;  // members have no big buckets
+      L.big_next = nullptr;
       L.big_count = nullptr;
-      L.big_ticket = nullptr;
-      L.big_cap = 0;
       launch_bucket_step(L, bucket_step_grid(p->sms, cps), p->stream);
       launch_member_splitters(p->d_dev, p->rlist, (int)m, i, p->stream);
       p->launches += 2;

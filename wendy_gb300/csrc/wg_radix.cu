@@ -92,6 +92,7 @@ constexpr int kHistThreads = 256;
 __global__ void __launch_bounds__(kHistThreads) k_radix_hist(
     const StateTable* table, int64_t n, int first, uint32_t* hist, uint32_t* plan,
     uint32_t* counters, const StepFlags* flag) {
+  chain_begin();
   if (!flag->unsorted) return;
   __shared__ uint32_t sh[8 * R];
   __shared__ int s_last;
@@ -214,6 +215,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_radix_pass(const PassArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   Smem& S = *reinterpret_cast<Smem*>(smem_raw);
 
+  chain_begin();
   if (!a.flag->unsorted) return;
   // an earlier pass gave up on a wait: its output is incomplete
   if (*a.err & DEV_ERR_RADIX_TIMEOUT) return;
@@ -459,6 +461,7 @@ __global__ void __launch_bounds__(kGatherThreads) k_radix_gather(
     StateTable* table, int64_t n, const uint32_t* pos0, const uint32_t* pos1,
     const uint32_t* plan, uint32_t* counters, const StepFlags* flag, const unsigned* err) {
   constexpr int GU = kGatherUnroll;
+  chain_begin();
   // nothing after a pass that gave up on a wait: its slots are incomplete
   if (!flag->unsorted || (*err & DEV_ERR_RADIX_TIMEOUT)) return;
   const int fb = (int)plan[kPlanFinal];
@@ -527,6 +530,7 @@ constexpr int64_t kShortRun = 32;
 __global__ void k_radix_ties(StateTable* table, int64_t n, int low_bits, uint32_t* counters,
                              uint32_t* list_start, uint32_t* list_len, const StepFlags* flag,
                              const unsigned* err) {
+  chain_begin();
   if (!flag->unsorted || !counters[kCntTie] || (*err & DEV_ERR_RADIX_TIMEOUT)) return;
   const StateRef oth = table->other;
   auto lead = [&](int64_t p) { return key_of(ld_relaxed_f64(oth.x + p)) >> low_bits; };
@@ -592,6 +596,7 @@ __global__ void __launch_bounds__(kLongTieThreads) k_radix_long_ties(
     StateTable* table, int64_t n, int low_bits, uint64_t* bufa, uint64_t* bufb,
     uint32_t* counters, const uint32_t* list_start, const uint32_t* list_len,
     const StepFlags* flag, const unsigned* err) {
+  chain_begin();
   // after an expired wait the current set stays as it was (unsorted, intact)
   if (!flag->unsorted || (*err & DEV_ERR_RADIX_TIMEOUT)) return;
   constexpr int T = kLongTieThreads;
@@ -709,8 +714,8 @@ void pass_launch(const PassArgs& a, int per_sm, int sms, cudaStream_t s) {
   int64_t pg = (int64_t)per_sm * sms;
   if (pg > a.n_tiles) pg = a.n_tiles;
   if (pg < 1) pg = 1;
-  k_radix_pass<kRadixThreads, ITEMS, FIRST, WIDE>
-      <<<(unsigned)pg, kRadixThreads, pass_smem<ITEMS, FIRST, WIDE>(), s>>>(a);
+  launch_chained(k_radix_pass<kRadixThreads, ITEMS, FIRST, WIDE>, (unsigned)pg, kRadixThreads,
+                 pass_smem<ITEMS, FIRST, WIDE>(), s, a);
 }
 
 void radix_cfg_init(RadixDevCfg& c, int dev) {
@@ -787,8 +792,8 @@ void radix_sort_state(StateTable* table, int64_t n, RadixWork* w, const StepFlag
   int64_t hist_grid = (n + 16 * kHistThreads - 1) / (16 * kHistThreads);
   if (hist_grid < 8) hist_grid = n < 8 * kHistThreads ? (n + kHistThreads - 1) / kHistThreads : 8;
   if (hist_grid > sms * 4) hist_grid = sms * 4;
-  k_radix_hist<<<(unsigned)hist_grid, kHistThreads, 0, s>>>(table, n, first, w->hist, w->plan,
-                                                            w->counters, flag);
+  launch_chained(k_radix_hist, (unsigned)hist_grid, kHistThreads, 0, s, table, n, first, w->hist,
+                 w->plan, w->counters, flag);
   PassArgs a;
   a.table = table;
   a.n = n;
@@ -823,17 +828,17 @@ void radix_sort_state(StateTable* table, int64_t n, RadixWork* w, const StepFlag
   int64_t gg = (n + kGatherThreads * kGatherUnroll - 1) / (kGatherThreads * kGatherUnroll);
   if (gg > (int64_t)sms * 8) gg = (int64_t)sms * 8;
   if (gg < 1) gg = 1;
-  k_radix_gather<<<(unsigned)gg, kGatherThreads, 0, s>>>(table, n, w->pos[0], w->pos[1], w->plan,
-                                                          w->counters, flag, err);
+  launch_chained(k_radix_gather, (unsigned)gg, kGatherThreads, 0, s, table, n, w->pos[0], w->pos[1],
+                 w->plan, w->counters, flag, err);
   int64_t g = (n + 255) / 256;
   if (g > (int64_t)sms * 16) g = (int64_t)sms * 16;
   if (g < 1) g = 1;
   // pos[] is free once gathered: it holds the list of long runs
-  k_radix_ties<<<(unsigned)g, 256, 0, s>>>(table, n, 8 * first, w->counters, w->pos[0], w->pos[1],
-                                           flag, err);
+  launch_chained(k_radix_ties, (unsigned)g, 256, 0, s, table, n, 8 * first, w->counters, w->pos[0],
+                 w->pos[1], flag, err);
   // and the key buffers are scratch for long ones
-  k_radix_long_ties<<<sms, kLongTieThreads, 0, s>>>(table, n, 8 * first, w->keys[0], w->keys[1],
-                                                    w->counters, w->pos[0], w->pos[1], flag, err);
+  launch_chained(k_radix_long_ties, (unsigned)sms, kLongTieThreads, 0, s, table, n, 8 * first,
+                 w->keys[0], w->keys[1], w->counters, w->pos[0], w->pos[1], flag, err);
 }
 
 }  // namespace wg
