@@ -157,7 +157,7 @@ struct wg_sim {
   unsigned* h_ep = nullptr;
   StepFlags* h_flags = nullptr;
   unsigned* h_big = nullptr;
-  unsigned* h_ab = nullptr;      // page-locked: overflow words [0..3], error word [4], drop-in [8]
+  unsigned* h_ab = nullptr;      // page-locked: overflow words [0..3], error word [4], drop-in [8, 9]
   // a call enqueued by wg_step_begin and not yet completed by wg_step_end
   bool pend_active = false;
   bool pend_compact = false;     // ... and it runs on the compact path
@@ -235,6 +235,8 @@ struct wg_sim {
   // physics
   uint64_t T_lo = 0, T_hi = 0;
   int E = 0;
+  int eq = kEqNo;        // equal masses (kEqWord: d_diff[1] says, zero if they are) ...
+  double meq = 0;        // ... of this mass
   double totmass = 0, omega2 = -1;
   ExtForce ext{};        // the force as the kernels see it
   ExtSpec ext_spec{};    // ... with an expression force's program on the host
@@ -567,8 +569,9 @@ int make_sim(int64_t n, double totmass, double omega2, const ExtSpec& ext, wg_si
   return WG_OK;
 }
 
+// equal (optional): whether all masses have the same bits.
 int validate_sheets(int64_t n, const double* x, const double* v, const double* m,
-                    double totmass) {
+                    double totmass, bool* equal = nullptr) {
   if (n < 1 || n >= (1ll << 30)) {
     set_error("number of sheets %lld outside [1, 2^30)", (long long)n);
     return WG_ERR_ARG;
@@ -597,6 +600,7 @@ int validate_sheets(int64_t n, const double* x, const double* v, const double* m
     set_error("a single mass exceeds twice totmass; totmass must be the sum of the masses");
     return WG_ERR_ARG;
   }
+  if (equal) *equal = std::memcmp(m, m + 1, sizeof(double) * (size_t)(n - 1)) == 0;
   return WG_OK;
 }
 
@@ -607,6 +611,8 @@ int copy_back(wg_sim* s, int nleap) {
   WG_CUDA(cudaMemcpyAsync(s->h_ab + 4, s->err, 4, cudaMemcpyDeviceToHost, s->stream));
   WG_CUDA(cudaMemcpyAsync(s->h_flags, s->flags, sizeof(StepFlags) * (nleap + 1),
                           cudaMemcpyDeviceToHost, s->stream));
+  if (s->eq == kEqWord)
+    WG_CUDA(cudaMemcpyAsync(s->h_ab + 9, s->d_diff + 1, 4, cudaMemcpyDeviceToHost, s->stream));
   if (s->capg > kBucketCap && nleap > 0)
     WG_CUDA(cudaMemcpyAsync(s->h_big, s->big_counts, 4 * (size_t)nleap, cudaMemcpyDeviceToHost,
                             s->stream));
@@ -617,6 +623,7 @@ int copy_back(wg_sim* s, int nleap) {
 // device error word.
 int finish_copied(wg_sim* s, int nleap, bool count_sorts) {
   const unsigned err = s->h_ab[4];
+  if (s->eq == kEqWord) s->eq = s->h_ab[9] == 0 ? kEqYes : kEqNo;
   for (int i = 0; i < nleap && count_sorts; ++i) {
     if (s->h_flags[i].unsorted)
       s->st.sorts_full++;
@@ -758,6 +765,12 @@ void fill_dev(wg_sim* s, double dt, double pre) {
   d.T_lo = s->T_lo;
   d.T_hi = s->T_hi;
   d.E = s->E;
+  d.eq = s->eq;
+  d.eq_word = s->d_diff ? s->d_diff + 1 : nullptr;
+  d.meq = s->meq;
+  const u128 M = s->eq != kEqNo ? host_mass_to_fixed(s->meq, s->E) : (u128)0;
+  d.meq_lo = (uint64_t)M;
+  d.meq_hi = (uint64_t)(M >> 64);
   d.has_omega = s->omega2 >= 0;
   d.omega2 = s->omega2;
   d.ext = s->ext;
@@ -780,6 +793,7 @@ StepLaunch step_launch(wg_sim* s, int i, int nleap, int profile) {
   L.ticket = s->tickets + i;
   L.err = s->err;
   L.profile = profile;
+  L.mass = s->eq == kEqNo ? kMassAny : s->eq == kEqYes ? kMassEqual : kMassMixed;
   L.any_expr = s->ext.kind == EXT_EXPR;
   L.big_list = s->big_list;
   L.big_next = s->big_next;
@@ -845,9 +859,12 @@ __global__ void k_inputs_differ(int64_t n, const wg_sheet* xi, const wg_sheet* x
   if (__syncthreads_or(d) && threadIdx.x == 0) atomicOr(diff, 1u);
 }
 
+// differ: set when the masses are not all the same.
 __global__ void k_load_sheets(StateTable* table, int64_t n, const wg_sheet* xi, const double* v,
-                              const double* m) {
+                              const double* m, unsigned* differ) {
   const StateRef st = table->cur;
+  const long long m0 = __double_as_longlong(m[0]);
+  bool d = false;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
     const int32_t j = xi[i].idx;
@@ -855,7 +872,9 @@ __global__ void k_load_sheets(StateTable* table, int64_t n, const wg_sheet* xi, 
     st.x[i] = xi[i].val;
     st.v[i] = v[j];
     st.m[i] = m[j];
+    d |= __double_as_longlong(m[j]) != m0;
   }
+  if (__syncthreads_or(d) && threadIdx.x == 0) atomicOr(differ, 1u);
 }
 
 __global__ void k_store_sheets(const StateTable* table, int64_t n, wg_sheet* xi) {
@@ -934,7 +953,8 @@ int wg_create(int64_t n, const double* x, const double* v, const double* m, doub
     return WG_ERR_ARG;
   }
   *out = nullptr;
-  int rc = validate_sheets(n, x, v, m, totmass);
+  bool equal = false;
+  int rc = validate_sheets(n, x, v, m, totmass, &equal);
   if (rc) return rc;
   if (!std::isfinite(omega2)) {
     set_error("omega2 must be finite");
@@ -946,6 +966,8 @@ int wg_create(int64_t n, const double* x, const double* v, const double* m, doub
   wg_sim* s = nullptr;
   rc = make_sim(n, totmass, omega2, ext, &s);
   if (rc) return rc;
+  s->eq = equal ? kEqYes : kEqNo;
+  s->meq = m[0];
   const StateRef c = s->set[0];
   auto up = [&](void* d, const void* h, size_t b) {
     return cudaMemcpyAsync(d, h, b, cudaMemcpyHostToDevice, s->stream);
@@ -1887,7 +1909,11 @@ int wg_nbody_approx_onestep(int n, wg_sheet* xi, double* x, double* v, const dou
     t0tab.cur = s->set[0];
     t0tab.other = s->set[1];
     WG_CUDA(cudaMemcpyAsync(s->table, &t0tab, sizeof(t0tab), cudaMemcpyHostToDevice, s->stream));
-    k_load_sheets<<<152 * 8, 256, 0, s->stream>>>(s->table, n, s->in_xi, s->in_v, s->in_m);
+    WG_CUDA(cudaMemsetAsync(s->d_diff + 1, 0, 4, s->stream));
+    k_load_sheets<<<152 * 8, 256, 0, s->stream>>>(s->table, n, s->in_xi, s->in_v, s->in_m,
+                                                  s->d_diff + 1);
+    s->eq = kEqWord;
+    s->meq = m[0];
     // the sheets are compact with the opening half drift pending: the call
     // sorts them and runs on the bucket path
     s->mode = 0;

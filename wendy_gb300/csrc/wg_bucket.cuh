@@ -111,6 +111,14 @@ struct SimDev {
   int capg;              // slots per bucket in the layouts (kBucketCap .. kBucketCapBig)
   uint64_t T_lo, T_hi;   // totmass in fixed point
   int E;
+  // Simulations whose masses are all the same (kEqYes, or kEqWord where a
+  // device word says so, zero meaning yes): the mass of a set of sheets is
+  // then their number times meq, and the kernel neither reads masses nor sums
+  // them.
+  int eq;
+  const unsigned* eq_word;
+  double meq;            // the mass, and in fixed point
+  uint64_t meq_lo, meq_hi;
   int has_omega;
   double omega2;
   ExtForce ext;
@@ -126,6 +134,10 @@ struct SimDev {
   // sub-step and takes it as the splitters of the layout after next
   StateTable* ptab;
 };
+
+enum : int { kEqNo = 0, kEqYes = 1, kEqWord = 2 };
+// The masses of a launch's simulations: any, all equal, or decided per task.
+enum : int { kMassAny = 0, kMassEqual = 1, kMassMixed = 2 };
 
 struct BucketTask {
   int sim;
@@ -149,6 +161,7 @@ struct TaskMeta {
   uint32_t pcnt;  // sheets in the simulation's earlier buckets
   int wlo, whi;   // splitter window [wlo, whi] of the next layout ...
   int wbuf;       // ... in wkey[wbuf], widx[wbuf]
+  int eq;         // equal masses
   double amp;     // time factor of a pulsed external force at this sub-step
   double inv_h;   // 1 / h of a pulsed external force
   uint64_t pm_lo, pm_hi;  // their fixed-point mass
@@ -164,6 +177,7 @@ struct StepLaunch {
   unsigned* ticket;      // zero before the launch
   unsigned* err;
   int profile;           // 1: dt = 0 and no outputs (timing harness)
+  int mass;              // kMass...: equal masses in none, all or some of the simulations
   int any_expr;          // some simulation of the launch has an expression force
   // big buckets (simulations with capg > kBucketCap): by bucket, the task and
   // the next bucket of the CTA that claimed it; how many there were
@@ -172,6 +186,9 @@ struct StepLaunch {
   unsigned* big_count;
 };
 
+typedef void (*StepKernel)(StepLaunch);
+// The sub-step kernel for launches with expression forces (wg_bucket_expr.cu).
+StepKernel step_kernel_expr(bool last, int mass);
 void launch_bucket_step(const StepLaunch& a, int grid, cudaStream_t s);
 // Pool members with predicted splitters (SimDev::ptab set): block k sorts the
 // nb - 1 samples member list[k] (k itself without a list) wrote in sub-step

@@ -91,6 +91,8 @@ struct PoolSim {
   double *done_x = nullptr, *done_v = nullptr;  // during a step: the output before it
   uint64_t T_lo = 0, T_hi = 0;
   int E = 0;
+  bool eq = false;  // all masses the same ...
+  double meq = 0;   // ... as this one
   double totmass = 0, omega2 = -1;
   ExtForce ext{};
   ExtSpec ext_spec{};         // the force with an expression's program on the host
@@ -269,6 +271,7 @@ struct wg_pool {
   cudaStream_t dl_stream = nullptr;  // downloads while a step runs
   int64_t g_ntasks = -1;
   void* g_small = nullptr;
+  int g_mass = -1;       // ... and the instantiation for these masses
   bool g_expr = false;   // the graph launches the expression-force instantiation
   int64_t graph_builds = 0;
   wg_pool_stats stats{};  // counters (launches and graph_builds are filled on read)
@@ -496,6 +499,13 @@ __global__ void k_read_back(const unsigned* src, unsigned* dst, int n) {
   for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
 }
 
+// The masses of a launch over these members (kMass...).
+int masses_of(const std::vector<PoolSim*>& act) {
+  size_t eq = 0;
+  for (const PoolSim* s : act) eq += s->eq ? 1 : 0;
+  return eq == 0 ? kMassAny : eq == act.size() ? kMassEqual : kMassMixed;
+}
+
 int grid_1d(int64_t n) {
   int64_t g = (n + 255) / 256;
   if (g > 152 * 8) g = 152 * 8;
@@ -668,6 +678,8 @@ int wg_pool_add(wg_pool* p, int64_t n, const double* x, const double* v, const d
                      cudaGetErrorString(e));
   }
   carve(s);
+  s->eq = std::memcmp(m, m + 1, sizeof(double) * (size_t)(n - 1)) == 0;
+  s->meq = m[0];
   s->totmass = totmass;
   s->omega2 = omega2;
   s->ext_spec = ext;
@@ -856,6 +868,12 @@ static int pool_step_begin(wg_pool* p, int count, const int* ids, const double* 
     d.T_lo = s->T_lo;
     d.T_hi = s->T_hi;
     d.E = s->E;
+    d.eq = s->eq ? kEqYes : kEqNo;
+    d.eq_word = nullptr;
+    d.meq = s->meq;
+    const u128 M = s->eq ? fixed_of(s->meq, s->E) : (u128)0;
+    d.meq_lo = (uint64_t)M;
+    d.meq_hi = (uint64_t)(M >> 64);
     d.has_omega = s->omega2 >= 0;
     d.omega2 = s->omega2;
     d.ext = s->ext;
@@ -870,9 +888,10 @@ static int pool_step_begin(wg_pool* p, int count, const int* ids, const double* 
   // the number of simulations, buckets and sub-steps stays the same
   bool launch_expr = false;  // the graph's kernels carry the expression interpreter
   for (PoolSim* a : act) launch_expr |= a->ext.kind == EXT_EXPR;
+  const int launch_mass = masses_of(act);
   const bool rebuild = !p->gexec || p->g_count != count || p->g_nleap != nleap ||
                        p->g_ntasks != ntasks || p->g_small != p->small ||
-                       p->g_expr != launch_expr;
+                       p->g_expr != launch_expr || p->g_mass != launch_mass;
   if (rebuild) {
     if (p->gexec) cudaGraphExecDestroy(p->gexec);
     p->gexec = nullptr;
@@ -906,6 +925,7 @@ static int pool_step_begin(wg_pool* p, int count, const int* ids, const double* 
       L.ticket = p->tickets + i;
       L.err = p->err;
       L.profile = 0;
+      L.mass = launch_mass;
       L.any_expr = launch_expr;
       L.big_list = nullptr;  // members have no big buckets
       L.big_next = nullptr;
@@ -932,6 +952,7 @@ static int pool_step_begin(wg_pool* p, int count, const int* ids, const double* 
     p->g_ntasks = ntasks;
     p->g_small = p->small;
     p->g_expr = launch_expr;
+    p->g_mass = launch_mass;
     p->graph_builds++;
   }
   PC(cudaGraphLaunch(p->gexec, p->stream));
@@ -1164,6 +1185,7 @@ static int pool_step_end(wg_pool* p, double* time_elapsed) {
       L.ticket = p->tickets + i;
       L.err = p->err;
       L.profile = 0;
+      L.mass = masses_of(act);
       L.any_expr = any_expr;
       L.big_list = nullptr;  // members have no big buckets
       L.big_next = nullptr;
