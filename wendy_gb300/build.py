@@ -16,7 +16,7 @@ CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "_wendy_gb300.so")
 BUILD_DIR = os.path.join(HERE, "_build")
 SOURCES = ["wg_kernels.cu", "wg_radix.cu", "wg_bucket.cu", "wg_bucket_expr.cu", "wg_api.cu", "wg_pool.cu",
-           "wg_exact.cu", "wg_noalloc.cu", "wg_small.cu"]
+           "wg_exact.cu", "wg_noalloc.cu", "wg_small.cu", "wg_blocks.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2"]
 # the exact solver follows the reference's operation order without FMA contraction

@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "../../include/wendy_gb300.h"
+#include "wg_blocks.cuh"
 #include "wg_bucket.cuh"
 #include "wg_ext.cuh"
 #include "wg_internal.cuh"
@@ -153,7 +154,8 @@ struct wg_sim {
   int spec_set = 0, spec_nleap = 0;
   double spec_dt = 0, spec_t0_in = 0, spec_t0_out = 0, spec_totmass = 0, spec_omega2 = 0;
   ExtSpec spec_ext{};
-  double* h_t = nullptr;         // pinned host mirrors
+  void* h_small = nullptr;       // pinned host mirrors, one block:
+  double* h_t = nullptr;
   unsigned* h_ep = nullptr;
   StepFlags* h_flags = nullptr;
   unsigned* h_big = nullptr;
@@ -278,20 +280,15 @@ int alloc_call_arrays(wg_sim* s, int nleap) {
     WG_CUDA(cudaStreamSynchronize(s->stream));
     WG_CUDA(cudaMemcpy(&t, s->table, sizeof(t), cudaMemcpyDeviceToHost));
   }
-  if (s->small) cudaFree(s->small);
-  if (s->h_t) cudaFreeHost(s->h_t);
-  if (s->h_ep) cudaFreeHost(s->h_ep);
-  if (s->h_flags) cudaFreeHost(s->h_flags);
-  if (s->h_big) cudaFreeHost(s->h_big);
+  block_free(s->small);
+  host_block_free(s->h_small);
   s->small = nullptr;
-  s->h_t = nullptr;
-  s->h_ep = nullptr;
-  s->h_flags = nullptr;
-  s->h_big = nullptr;
+  s->h_small = nullptr;
+  s->cap = 0;
   const size_t b = al(sizeof(StateTable)) + al(64) + al(sizeof(StepFlags) * (cap + 1)) +
                    al(4 * (size_t)cap) + al(8 * (size_t)cap) + al(4 * (size_t)cap) +
                    al(8 * (size_t)cap);
-  WG_CUDA(cudaMalloc(&s->small, b));
+  WG_CUDA(block_alloc(&s->small, b));
   char* p = static_cast<char*>(s->small);
   s->table = reinterpret_cast<StateTable*>(p); p += al(sizeof(StateTable));
   s->err = reinterpret_cast<unsigned*>(p); p += al(64);
@@ -302,11 +299,14 @@ int alloc_call_arrays(wg_sim* s, int nleap) {
   s->big_counts = reinterpret_cast<unsigned*>(p); p += al(4 * (size_t)cap);
   WG_CUDA(cudaMemsetAsync(s->small, 0, b, s->stream));
   WG_CUDA(cudaMemcpyAsync(s->table, &t, sizeof(t), cudaMemcpyHostToDevice, s->stream));
-  WG_CUDA(cudaMallocHost(&s->h_t, 8 * (size_t)cap));
-  WG_CUDA(cudaMallocHost(&s->h_ep, 4 * (size_t)cap));
-  WG_CUDA(cudaMallocHost(&s->h_flags, sizeof(StepFlags) * (cap + 1)));
-  WG_CUDA(cudaMallocHost(&s->h_big, 4 * (size_t)cap));
-  if (!s->h_ab) WG_CUDA(cudaMallocHost(&s->h_ab, 64));
+  // page-locked mirrors, one block
+  WG_CUDA(host_block_alloc(&s->h_small, 64 + 16 * (size_t)cap + sizeof(StepFlags) * (cap + 1)));
+  char* h = static_cast<char*>(s->h_small);
+  s->h_ab = reinterpret_cast<unsigned*>(h); h += 64;
+  s->h_t = reinterpret_cast<double*>(h); h += 8 * (size_t)cap;
+  s->h_flags = reinterpret_cast<StepFlags*>(h); h += sizeof(StepFlags) * (cap + 1);
+  s->h_ep = reinterpret_cast<unsigned*>(h); h += 4 * (size_t)cap;
+  s->h_big = reinterpret_cast<unsigned*>(h);
   WG_CUDA(cudaStreamSynchronize(s->stream));
   s->cap = cap;
   return WG_OK;
@@ -314,30 +314,27 @@ int alloc_call_arrays(wg_sim* s, int nleap) {
 
 void free_sim(wg_sim* s) {
   if (!s) return;
-  if (s->stream) cudaStreamSynchronize(s->stream);
-  if (s->big) cudaFree(s->big);
-  if (s->bk) cudaFree(s->bk);
-  if (s->pmem) cudaFree(s->pmem);
-  if (s->small) cudaFree(s->small);
-  if (s->stage) cudaFree(s->stage);
-  if (s->h_t) cudaFreeHost(s->h_t);
-  if (s->h_ep) cudaFreeHost(s->h_ep);
-  if (s->h_flags) cudaFreeHost(s->h_flags);
-  if (s->h_big) cudaFreeHost(s->h_big);
-  if (s->h_ab) cudaFreeHost(s->h_ab);
-  if (s->up_stream) cudaStreamSynchronize(s->up_stream);
-  if (s->down_stream) cudaStreamSynchronize(s->down_stream);
-  if (s->dl_stream) cudaStreamSynchronize(s->dl_stream);
-  if (s->out2) cudaFree(s->out2);
+  // nothing may be in flight on what is handed back
+  for (cudaStream_t t : {s->stream, s->up_stream, s->down_stream, s->dl_stream})
+    if (t) cudaStreamSynchronize(t);
+  block_free(s->big);
+  block_free(s->bk);
+  block_free(s->pmem);
+  block_free(s->small);
+  block_free(s->stage);
+  block_free(s->out2);
+  host_block_free(s->h_small);
   if (s->d_prog) cudaFree(s->d_prog);
   if (s->ev_done) cudaEventDestroy(s->ev_done);
-  if (s->dl_stream) cudaStreamDestroy(s->dl_stream);
-  if (s->ev0) cudaEventDestroy(s->ev0);
-  if (s->ev1) cudaEventDestroy(s->ev1);
   if (s->ev_up) cudaEventDestroy(s->ev_up);
-  if (s->stream) cudaStreamDestroy(s->stream);
+  if (s->dl_stream) cudaStreamDestroy(s->dl_stream);
   if (s->up_stream) cudaStreamDestroy(s->up_stream);
   if (s->down_stream) cudaStreamDestroy(s->down_stream);
+  StreamSet set;
+  set.stream = s->stream;
+  set.ev0 = s->ev0;
+  set.ev1 = s->ev1;
+  stream_set_give(set);
   delete s;
 }
 
@@ -363,9 +360,10 @@ int balanced_target(int64_t n, int target, int grid) {
 }
 
 // Allocate a simulation for n sheets with the given physics; sheet data is
-// uploaded by the caller.
+// uploaded by the caller.  accel_only: for force evaluations, without the
+// bucket layouts.
 int make_sim(int64_t n, double totmass, double omega2, const ExtSpec& ext, wg_sim** out,
-             bool big_buckets = true) {
+             bool accel_only = false) {
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev < 1) {
     cudaGetLastError();
@@ -394,10 +392,17 @@ int make_sim(int64_t n, double totmass, double omega2, const ExtSpec& ext, wg_si
     free_sim(s);
     return code;
   };
-  if (cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaEventCreate(&s->ev0) != cudaSuccess || cudaEventCreate(&s->ev1) != cudaSuccess) {
-    set_error("stream/event creation failed: %s", cudaGetErrorString(cudaGetLastError()));
-    return fail(WG_ERR_CUDA);
+  {
+    StreamSet set;
+    const cudaError_t es = stream_set_take(&set);
+    s->stream = set.stream;
+    s->ev0 = set.ev0;
+    s->ev1 = set.ev1;
+    if (es != cudaSuccess) {
+      cudaGetLastError();
+      set_error("stream/event creation failed: %s", cudaGetErrorString(es));
+      return fail(WG_ERR_CUDA);
+    }
   }
   const size_t nd = al((size_t)n * 8), ni = al((size_t)n * 4);
   const size_t set_b = 3 * nd + ni;
@@ -405,7 +410,7 @@ int make_sim(int64_t n, double totmass, double omega2, const ExtSpec& ext, wg_si
   const size_t radix_b = radix_bytes(n);
   const size_t out_b = 3 * nd;  // x_out, v_out, a_sorted
   const size_t total = 2 * set_b + recs_b + radix_b + out_b;
-  cudaError_t e = cudaMalloc(&s->big, total);
+  cudaError_t e = block_alloc(&s->big, total);
   if (e != cudaSuccess) {
     cudaGetLastError();
     set_error("cudaMalloc of %zu bytes for %lld sheets failed: %s", total, (long long)n,
@@ -441,7 +446,8 @@ int make_sim(int64_t n, double totmass, double omega2, const ExtSpec& ext, wg_si
     s->grid_bucket = bucket_step_grid(sms, s->tune.ctas_per_sm);
   }
   s->tune.target = balanced_target(n, s->tune.target, s->grid_bucket);
-  s->nb = (n + s->tune.target - 1) / s->tune.target;
+  // (a force evaluation alone runs on the compact sets)
+  s->nb = accel_only ? 1 : (n + s->tune.target - 1) / s->tune.target;
   const int64_t nb = s->nb;
   // layouts with room for big buckets where asked for and where the memory
   // allows, else kBucketCap slots per bucket
@@ -458,14 +464,14 @@ int make_sim(int64_t n, double totmass, double omega2, const ExtSpec& ext, wg_si
   };
   // (a bucket of up to kBucketCap / 4 sheets has room for four times its
   // target already: such layouts need no big buckets)
-  s->capg = big_buckets && 4 * s->tune.target > kBucketCap ? kBucketCapBig : kBucketCap;
+  s->capg = !accel_only && 4 * s->tune.target > kBucketCap ? kBucketCapBig : kBucketCap;
   bucket_bytes(s->capg);
-  e = cudaMalloc(&s->bk, bk_b);
+  e = block_alloc(&s->bk, bk_b);
   if (e != cudaSuccess && s->capg > kBucketCap) {
     cudaGetLastError();
     s->capg = kBucketCap;
     bucket_bytes(s->capg);
-    e = cudaMalloc(&s->bk, bk_b);
+    e = block_alloc(&s->bk, bk_b);
   }
   if (e != cudaSuccess) {
     cudaGetLastError();
@@ -513,14 +519,14 @@ int make_sim(int64_t n, double totmass, double omega2, const ExtSpec& ext, wg_si
       return fail(WG_ERR_CUDA);
     }
   }
-  if (big_buckets && nb >= 3) {
+  if (!accel_only && nb >= 3) {
     // predicted splitters: two sample sets of nb - 1 entries (SoA as the
     // radix sort wants them), their table, the sort's workspace and flags
     const int64_t m = nb - 1;
     const size_t nd = al(8 * (size_t)m), ni = al(4 * (size_t)m);
     const size_t pb = 2 * (3 * nd + ni) + al(sizeof(StateTable)) + al(sizeof(StepFlags)) +
                       radix_bytes(m);
-    if (cudaMalloc(&s->pmem, pb) == cudaSuccess) {
+    if (block_alloc(&s->pmem, pb) == cudaSuccess) {
       char* q = static_cast<char*>(s->pmem);
       StateRef set[2];
       for (int k = 0; k < 2; ++k) {
@@ -569,14 +575,14 @@ int make_sim(int64_t n, double totmass, double omega2, const ExtSpec& ext, wg_si
   return WG_OK;
 }
 
-// equal (optional): whether all masses have the same bits.
+// v may be null (no velocities to look at).  equal (optional): whether all masses have the same bits.
 int validate_sheets(int64_t n, const double* x, const double* v, const double* m,
                     double totmass, bool* equal = nullptr) {
   if (n < 1 || n >= (1ll << 30)) {
     set_error("number of sheets %lld outside [1, 2^30)", (long long)n);
     return WG_ERR_ARG;
   }
-  if (!x || !v || !m) {
+  if (!x || !m) {
     set_error("null array");
     return WG_ERR_ARG;
   }
@@ -584,17 +590,30 @@ int validate_sheets(int64_t n, const double* x, const double* v, const double* m
     set_error("totmass must be finite and >= 0");
     return WG_ERR_ARG;
   }
+  // one pass over the bits (it vectorises); the offender is looked for only
+  // when there is one.  Non-finite: all exponent bits set.  A negative mass has
+  // the sign bit, and so has -0.0, which is let through below.
+  uint64_t any_x = 0, any_m = 0;
   double mmax = 0;
+  constexpr uint64_t kExp = 0x7FF0000000000000ull;
   for (int64_t i = 0; i < n; ++i) {
+    uint64_t bx, bv, bm;
+    std::memcpy(&bx, &x[i], 8);
+    std::memcpy(&bv, v ? &v[i] : &x[i], 8);
+    std::memcpy(&bm, &m[i], 8);
+    any_x |= (uint64_t)((bx & kExp) == kExp) | (uint64_t)((bv & kExp) == kExp);
+    any_m |= (uint64_t)((bm & kExp) == kExp) | (bm >> 63);
+    mmax = m[i] > mmax ? m[i] : mmax;
+  }
+  for (int64_t i = 0; i < n && (any_x | any_m); ++i) {
     if (!(m[i] >= 0) || !std::isfinite(m[i])) {
       set_error("mass %lld is negative or not finite", (long long)i);
       return WG_ERR_ARG;
     }
-    if (!std::isfinite(x[i]) || !std::isfinite(v[i])) {
+    if (!std::isfinite(x[i]) || (v && !std::isfinite(v[i]))) {
       set_error("position or velocity %lld is not finite", (long long)i);
       return WG_ERR_ARG;
     }
-    if (m[i] > mmax) mmax = m[i];
   }
   if (mmax > 2 * totmass) {
     set_error("a single mass exceeds twice totmass; totmass must be the sum of the masses");
@@ -938,6 +957,7 @@ int wg_device_info(int* sm_count, int64_t* free_bytes, int64_t* total_bytes) {
   int dev = 0;
   WG_CUDA(cudaGetDevice(&dev));
   if (sm_count) WG_CUDA(cudaDeviceGetAttribute(sm_count, cudaDevAttrMultiProcessorCount, dev));
+  blocks_trim();  // what is kept idle counts as free
   size_t fr = 0, tot = 0;
   WG_CUDA(cudaMemGetInfo(&fr, &tot));
   if (free_bytes) *free_bytes = (int64_t)fr;
@@ -954,6 +974,10 @@ int wg_create(int64_t n, const double* x, const double* v, const double* m, doub
   }
   *out = nullptr;
   bool equal = false;
+  if (!v) {
+    set_error("null array");
+    return WG_ERR_ARG;
+  }
   int rc = validate_sheets(n, x, v, m, totmass, &equal);
   if (rc) return rc;
   if (!std::isfinite(omega2)) {
@@ -1359,7 +1383,7 @@ int wg_step_begin(wg_sim* s, double dt, int nleap, double* t0) {
   s->call_xi = nullptr;
   s->call_a = nullptr;
   if (!s->out2) {
-    WG_CUDA(cudaMalloc(&s->out2, 16 * (size_t)s->n));
+    WG_CUDA(block_alloc(&s->out2, 16 * (size_t)s->n));
     WG_CUDA(cudaStreamCreateWithFlags(&s->dl_stream, cudaStreamNonBlocking));
     WG_CUDA(cudaEventCreateWithFlags(&s->ev_done, cudaEventDisableTiming));
     s->st.device_bytes += 16 * s->n;
@@ -1604,13 +1628,13 @@ int wg_host_alloc(int64_t bytes, void** ptr) {
     return WG_ERR_ARG;
   }
   *ptr = nullptr;
-  WG_CUDA(cudaHostAlloc(ptr, (size_t)bytes, cudaHostAllocDefault));
+  WG_CUDA(host_block_alloc(ptr, (size_t)bytes));
   return WG_OK;
 }
 
 int wg_host_free(void* ptr) {
   if (!ptr) return WG_OK;
-  WG_CUDA(cudaFreeHost(ptr));
+  if (!host_block_free(ptr)) WG_CUDA(cudaFreeHost(ptr));
   return WG_OK;
 }
 
@@ -1690,14 +1714,13 @@ int wg_ext_force_eval(int64_t n, const double* x, double t, int ext_kind,
 int wg_accel(int64_t n, const double* x, const double* m, double totmass, double omega2,
              int ext_kind, const double* ext_params, int n_ext_params, double t, double* a,
              int32_t* perm) {
-  std::vector<double> zero((size_t)(n > 0 ? n : 1), 0.0);
-  int rc = validate_sheets(n, x, zero.data(), m, totmass);
+  int rc = validate_sheets(n, x, nullptr, m, totmass);
   if (rc) return rc;
   ExtSpec ext;
   rc = check_ext(ext_kind, ext_params, n_ext_params, &ext);
   if (rc) return rc;
   wg_sim* s = nullptr;
-  rc = make_sim(n, totmass, omega2, ext, &s, false);
+  rc = make_sim(n, totmass, omega2, ext, &s, true);
   if (rc) return rc;
   const StateRef c = s->set[0];
   cudaMemcpyAsync(c.x, x, 8 * n, cudaMemcpyHostToDevice, s->stream);
@@ -1710,16 +1733,21 @@ int wg_accel(int64_t n, const double* x, const double* m, double totmass, double
   // dt_kick = dt_drift = 0.
   rc = enqueue_step(s, 0.0, 1, true, 0.0);
   if (rc == WG_OK) {
-    StateTable tab;
-    launch_scatter_accel(s->table, n, s->a_sorted, s->x_out, s->stream);
-    cudaMemcpyAsync(&tab, s->table, sizeof(tab), cudaMemcpyDeviceToHost, s->stream);
-    if (cudaStreamSynchronize(s->stream) != cudaSuccess) {
-      set_error("accel failed: %s", cudaGetErrorString(cudaGetLastError()));
+    // accelerations in original order, the order itself beside them
+    int32_t* const order = reinterpret_cast<int32_t*>(s->v_out);
+    launch_scatter_accel(s->table, n, s->a_sorted, s->x_out, s->stream, perm ? order : nullptr);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) rc = copy_back(s, 1);
+    if (e == cudaSuccess && a)
+      e = cudaMemcpyAsync(a, s->x_out, 8 * n, cudaMemcpyDeviceToHost, s->stream);
+    if (e == cudaSuccess && perm)
+      e = cudaMemcpyAsync(perm, order, 4 * n, cudaMemcpyDeviceToHost, s->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
+    if (e != cudaSuccess) {
+      set_error("accel failed: %s", cudaGetErrorString(e));
       rc = WG_ERR_CUDA;
-    } else {
-      if (a) cudaMemcpy(a, s->x_out, 8 * n, cudaMemcpyDeviceToHost);
-      if (perm) cudaMemcpy(perm, tab.cur.idx, 4 * n, cudaMemcpyDeviceToHost);
-      rc = finish_call(s, 1);
+    } else if (rc == WG_OK) {
+      rc = finish_copied(s, 1, true);
     }
   }
   free_sim(s);
@@ -1821,7 +1849,7 @@ int wg_nbody_approx_onestep(int n, wg_sheet* xi, double* x, double* v, const dou
   if (!s->stage) {
     const size_t bx = al(sizeof(wg_sheet) * (size_t)n), bd = al(8 * (size_t)n);
     const size_t b = 3 * bx + 9 * bd + al(16);
-    WG_CUDA(cudaMalloc(&s->stage, b));
+    WG_CUDA(block_alloc(&s->stage, b));
     char* q = static_cast<char*>(s->stage);
     for (int k = 0; k < 2; ++k) {
       s->outs[k].xi = reinterpret_cast<wg_sheet*>(q); q += bx;

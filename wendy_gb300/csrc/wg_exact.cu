@@ -45,6 +45,7 @@
 #include <vector>
 
 #include "../../include/wendy_gb300.h"
+#include "wg_blocks.cuh"
 #include "wg_internal.cuh"
 
 using namespace wg;
@@ -549,11 +550,13 @@ namespace {
 void free_exact(wg_exact* e) {
   if (!e) return;
   if (e->stream) cudaStreamSynchronize(e->stream);
-  if (e->mem) cudaFree(e->mem);
-  if (e->h_ret) cudaFreeHost(e->h_ret);
-  if (e->ev0) cudaEventDestroy(e->ev0);
-  if (e->ev1) cudaEventDestroy(e->ev1);
-  if (e->stream) cudaStreamDestroy(e->stream);
+  block_free(e->mem);
+  host_block_free(e->h_ret);
+  StreamSet set;
+  set.stream = e->stream;
+  set.ev0 = e->ev0;
+  set.ev1 = e->ev1;
+  stream_set_give(set);
   delete e;
 }
 
@@ -615,14 +618,17 @@ int wg_exact_create(int64_t n, const double* x, const double* v, const double* a
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   A.use_smem = smem + kExactStatic <= (size_t)optin;
   const size_t total = 6 * nd + ni + tree_b + al(64) + (A.use_smem ? 0 : 4 * nd + ni);
-  if (cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaEventCreate(&e->ev0) != cudaSuccess || cudaEventCreate(&e->ev1) != cudaSuccess ||
-      cudaMallocHost(&e->h_ret, 64) != cudaSuccess) {
+  StreamSet set;
+  const cudaError_t es = stream_set_take(&set);
+  e->stream = set.stream;
+  e->ev0 = set.ev0;
+  e->ev1 = set.ev1;
+  if (es != cudaSuccess || host_block_alloc(&e->h_ret, 64) != cudaSuccess) {
     cudaGetLastError();
     free_exact(e);
     return fail(WG_ERR_CUDA, "exact solver: stream set-up failed");
   }
-  if (cudaMalloc(&e->mem, total) != cudaSuccess) {
+  if (block_alloc(&e->mem, total) != cudaSuccess) {
     cudaGetLastError();
     free_exact(e);
     return fail(WG_ERR_NOMEM, "exact solver: cudaMalloc of %zu bytes failed", total);

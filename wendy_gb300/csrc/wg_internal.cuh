@@ -144,8 +144,9 @@ void set_wait_debug(unsigned spin_limit, int64_t withhold_tile);
 void launch_drift(const StateTable* table, int64_t n, double dt, StepFlags* flag, cudaStream_t s);
 void launch_desort(const StateTable* table, int64_t n, double* x_out, double* v_out,
                    cudaStream_t s);
+// order (optional): original index of the sheet at each sorted place.
 void launch_scatter_accel(const StateTable* table, int64_t n, const double* a_sorted,
-                          double* a_orig, cudaStream_t s);
+                          double* a_orig, cudaStream_t s, int32_t* order = nullptr);
 void launch_init_state(StateTable* table, int64_t n, cudaStream_t s);
 // Energy / momentum sums of the sorted state (deterministic): scratch[0..3]
 // receives sum m v^2/2, sum m x^2/2, -sum m x a, sum m v; scratch holds

@@ -295,11 +295,15 @@ __global__ void k_desort(const StateTable* table, int64_t n, double* x_out, doub
 }
 
 __global__ void k_scatter_accel(const StateTable* table, int64_t n, const double* a_sorted,
-                                double* a_orig) {
+                                double* a_orig, int32_t* order) {
   const StateRef st = table->cur;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride)
-    a_orig[st.idx[i]] = a_sorted[i];
+  {
+    const int32_t j = st.idx[i];
+    a_orig[j] = a_sorted[i];
+    if (order) order[i] = j;
+  }
 }
 
 __global__ void k_iota(const StateTable* table, int64_t n) {
@@ -348,8 +352,8 @@ void launch_desort(const StateTable* table, int64_t n, double* x_out, double* v_
 }
 
 void launch_scatter_accel(const StateTable* table, int64_t n, const double* a_sorted,
-                          double* a_orig, cudaStream_t s) {
-  k_scatter_accel<<<grid_for(n, 256), 256, 0, s>>>(table, n, a_sorted, a_orig);
+                          double* a_orig, cudaStream_t s, int32_t* order) {
+  k_scatter_accel<<<grid_for(n, 256), 256, 0, s>>>(table, n, a_sorted, a_orig, order);
 }
 
 // F(x_i, t) of a registered external force, with the force kernels' code:

@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "../../include/wendy_gb300.h"
+#include "wg_blocks.cuh"
 #include "wg_bucket.cuh"
 #include "wg_ext.cuh"
 #include "wg_internal.cuh"
@@ -671,6 +672,11 @@ int wg_pool_add(wg_pool* p, int64_t n, const double* x, const double* v, const d
   s->nb = (n + s->tune.target - 1) / s->tune.target;
   s->bytes = bytes;
   cudaError_t e = cudaMallocAsync(&s->mem, bytes, p->stream);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    blocks_trim();  // idle memory kept from other simulations
+    e = cudaMallocAsync(&s->mem, bytes, p->stream);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     delete s;
