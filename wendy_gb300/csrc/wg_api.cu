@@ -349,7 +349,6 @@ void free_sim(wg_sim* s) {
 // 36.7 (one round) / 40.4 (two) / 50.7 at 3e5; at 1e6, 1280 (two rounds) 70.1 against
 // 1536 (two rounds, the second half empty) 77.5 and 1024 (three) 81.4.
 constexpr int kBalanceRounds = 4;
-constexpr int kMinTarget = 384;
 int balanced_target(int64_t n, int target, int grid) {
   const int64_t rounds = (n + (int64_t)grid * target - 1) / ((int64_t)grid * target);
   if (rounds > kBalanceRounds) return target;

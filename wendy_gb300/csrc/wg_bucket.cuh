@@ -21,6 +21,7 @@ constexpr int kMemberSampleCap = 4096; // most splitter samples a pool member so
 constexpr int kSortBitsMin = 9;       // smallest counting-sort offset (bits)
 constexpr int kSortBitsMax = 13;      // largest counting-sort offset (bits)
 constexpr int kMaxTarget = kBucketCap * 3 / 4;  // largest bucket target
+constexpr int kMinTarget = 384;  // smallest target that launches with few buckets are cut to
 
 // Tunables of the fused sub-step, chosen per simulation size by the
 // autotuner (wendy_gb300/autotune.py) or left at their defaults.

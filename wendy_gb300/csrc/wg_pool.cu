@@ -73,7 +73,12 @@ u128 fixed_of(double m, int E) {
 
 // Persistent device memory of one simulation, in one allocation.
 struct PoolSim {
-  int64_t n = 0, nb = 0;
+  int64_t n = 0;
+  int64_t nb_tuned = 0;  // buckets at the tuned target; the layouts' slots are for these
+  int64_t nb_room = 0;   // buckets the per-bucket arrays have room for
+  int64_t nb = 0;        // buckets of the present layouts ...
+  int target = 0;        // ... of this many sheets each at a re-sort ...
+  int capg = kBucketCap; // ... with this many slots each
   void* mem = nullptr;
   size_t bytes = 0;
   double* bx[2];
@@ -115,10 +120,19 @@ struct PoolSim {
 // A member's samples are sorted by one CTA in shared memory.
 constexpr int kPredMemberCalls = 16;
 
+// Buckets a member's per-bucket arrays have room for: the tuned number, or for
+// smaller members what smaller buckets (member_target) would make of them.
+int64_t bucket_room(int64_t n, int64_t nb_tuned) {
+  int64_t r = (n + kMinTarget - 1) / kMinTarget;
+  if (r > 1024) r = 1024;
+  return r > nb_tuned ? r : nb_tuned;
+}
+
 size_t sim_bytes(int64_t n) {
   const BucketTuning t = tuning_for(n);
-  const int64_t nb = (n + t.target - 1) / t.target;
-  const size_t slots = (size_t)nb * kBucketCap;
+  const int64_t nb_tuned = (n + t.target - 1) / t.target;
+  const int64_t nb = bucket_room(n, nb_tuned);
+  const size_t slots = (size_t)nb_tuned * kBucketCap;
   const size_t pred = (nb >= 3 && nb - 1 <= kMemberSampleCap)
                           ? al(sizeof(StateTable)) + al(8 * (size_t)nb) + al(4 * (size_t)nb)
                           : 0;
@@ -130,7 +144,7 @@ size_t sim_bytes(int64_t n) {
 }
 
 void carve(PoolSim* s) {
-  const size_t slots = (size_t)s->nb * kBucketCap;
+  const size_t slots = (size_t)s->nb_tuned * kBucketCap;
   char* p = static_cast<char*>(s->mem);
   for (int k = 0; k < 2; ++k) {
     s->bx[k] = reinterpret_cast<double*>(p); p += al(slots * 8);
@@ -139,14 +153,14 @@ void carve(PoolSim* s) {
     s->bi[k] = reinterpret_cast<int32_t*>(p); p += al(slots * 4);
   }
   for (int k = 0; k < kAggSlots; ++k) {
-    s->bcnt[k] = reinterpret_cast<unsigned*>(p); p += al(4 * (size_t)s->nb);
-    s->bmass[k] = reinterpret_cast<unsigned long long*>(p); p += al(32 * (size_t)s->nb);
+    s->bcnt[k] = reinterpret_cast<unsigned*>(p); p += al(4 * (size_t)s->nb_room);
+    s->bmass[k] = reinterpret_cast<unsigned long long*>(p); p += al(32 * (size_t)s->nb_room);
   }
   for (int k = 0; k < 2; ++k) {
-    s->qk[k] = reinterpret_cast<uint64_t*>(p); p += al(8 * (size_t)(s->nb + 1));
-    s->qi[k] = reinterpret_cast<int32_t*>(p); p += al(4 * (size_t)(s->nb + 1));
+    s->qk[k] = reinterpret_cast<uint64_t*>(p); p += al(8 * (size_t)(s->nb_room + 1));
+    s->qi[k] = reinterpret_cast<int32_t*>(p); p += al(4 * (size_t)(s->nb_room + 1));
   }
-  s->recs = reinterpret_cast<BucketRec*>(p); p += al(sizeof(BucketRec) * (size_t)s->nb);
+  s->recs = reinterpret_cast<BucketRec*>(p); p += al(sizeof(BucketRec) * (size_t)s->nb_room);
   s->ox = reinterpret_cast<double*>(p); p += al(8 * (size_t)s->n);
   s->ov = reinterpret_cast<double*>(p); p += al(8 * (size_t)s->n);
   s->om = reinterpret_cast<double*>(p); p += al(8 * (size_t)s->n);
@@ -156,7 +170,7 @@ void carve(PoolSim* s) {
   s->x_out2 = reinterpret_cast<double*>(p); p += al(8 * (size_t)s->n);
   s->v_out2 = reinterpret_cast<double*>(p); p += al(8 * (size_t)s->n);
   s->ptab = nullptr;
-  if (s->nb >= 3 && s->nb - 1 <= kMemberSampleCap) {
+  if (s->nb_room >= 3 && s->nb_room - 1 <= kMemberSampleCap) {
     s->ptab = reinterpret_cast<StateTable*>(p); p += al(sizeof(StateTable));
   }
 }
@@ -167,7 +181,7 @@ StateTable member_sample_table(const PoolSim* s) {
   char* p = reinterpret_cast<char*>(s->ptab) + al(sizeof(StateTable));
   StateTable t{};
   t.cur.x = reinterpret_cast<double*>(p);
-  t.cur.idx = reinterpret_cast<int32_t*>(p + al(8 * (size_t)s->nb));
+  t.cur.idx = reinterpret_cast<int32_t*>(p + al(8 * (size_t)s->nb_room));
   t.other = t.cur;
   return t;
 }
@@ -513,6 +527,41 @@ int grid_1d(int64_t n) {
   return (int)(g < 1 ? 1 : g);
 }
 
+// Buckets of `target` sheets for a member that is to be laid out anew: as many
+// slots each as the layouts hold.
+void set_target(PoolSim* s, int target) {
+  s->target = target;
+  s->nb = (s->n + target - 1) / target;
+  const int64_t slots = s->nb_tuned * kBucketCap / s->nb & ~(int64_t)3;
+  s->capg = slots < kBucketCap ? (int)slots : kBucketCap;
+}
+
+// Targets of the members of a step that are about to be laid out (their sheets
+// are compact): the tuned ones, unless the step's buckets would leave resident
+// CTAs idle, as for single simulations (balanced_target).  Then all members
+// take buckets of the size that fills the launch, down to kMinTarget sheets
+// (a bucket keeps the share of spare slots of the tuned ones, a third).
+// Measured per output of 20 sub-steps (5): 4 members of 500 .. 20000 sheets 418 us
+// (175) against 733 (254) with tuned buckets in the kernel before it, 64 of
+// 1000 .. 20000 1240 (580) against 1420 (625).
+void balance_targets(wg_pool* p, const std::vector<PoolSim*>& act) {
+  int64_t sheets = 0, buckets = 0;
+  for (const PoolSim* s : act) {
+    sheets += s->n;
+    buckets += s->nb_tuned;
+  }
+  const int grid = bucket_step_grid(p->sms, 2);
+  int64_t t = (sheets + grid - 1) / grid;
+  t = (t + 31) / 32 * 32;
+  if (t < kMinTarget) t = kMinTarget;
+  for (PoolSim* s : act) {
+    if (s->mode != 0) continue;
+    int target = s->tune.target;
+    if (buckets < grid && t < target && (s->n + t - 1) / t <= s->nb_room) target = (int)t;
+    if (target != s->target) set_target(s, target);
+  }
+}
+
 // Bring a mode-0 simulation to its bucket layout: half drift of dt/2 on the
 // compact store, full radix sort, bucketize.  Uses the shared workspace.
 int to_buckets(wg_pool* p, PoolSim* s, double dt) {
@@ -522,7 +571,7 @@ int to_buckets(wg_pool* p, PoolSim* s, double dt) {
   k_set_table<<<1, 1, 0, p->stream>>>(p->table, own, p->set[1]);
   launch_drift(p->table, s->n, dt / 2., &p->wflags[0], p->stream);  // also marks "unsorted"
   radix_sort_state(p->table, s->n, &p->radix, &p->wflags[0], p->err, p->stream);
-  launch_bucketize(p->table, s->n, s->tune.target, s->nb, kBucketCap, s->E, s->bx[0], s->bv[0],
+  launch_bucketize(p->table, s->n, s->target, s->nb, s->capg, s->E, s->bx[0], s->bv[0],
                    s->bm[0],
                    s->bi[0], s->bcnt, s->bmass, s->qk[0], s->qi[0], p->stream);
   p->launches += 3 + kRadixLaunches;
@@ -538,7 +587,7 @@ int to_buckets(wg_pool* p, PoolSim* s, double dt) {
 // overflow entries counted in oc) -> the workspace's first set, unsorted.
 void buckets_to_workspace(wg_pool* p, PoolSim* s, int lay, int cslot, const unsigned* oc) {
   k_set_table<<<1, 1, 0, p->stream>>>(p->table, p->set[0], p->set[1]);
-  launch_compact(p->table, s->nb, kBucketCap, s->bx[lay], s->bv[lay], s->bm[lay], s->bi[lay],
+  launch_compact(p->table, s->nb, s->capg, s->bx[lay], s->bv[lay], s->bm[lay], s->bi[lay],
                  s->bcnt[cslot],
                  p->offs, s->ox, s->ov, s->om, s->oi, oc, s->n, p->stream);
   p->launches += 3;
@@ -669,7 +718,9 @@ int wg_pool_add(wg_pool* p, int64_t n, const double* x, const double* v, const d
   PoolSim* s = new PoolSim();
   s->n = n;
   s->tune = tuning_for(n);
-  s->nb = (n + s->tune.target - 1) / s->tune.target;
+  s->nb_tuned = (n + s->tune.target - 1) / s->tune.target;
+  s->nb_room = bucket_room(n, s->nb_tuned);
+  set_target(s, s->tune.target);
   s->bytes = bytes;
   cudaError_t e = cudaMallocAsync(&s->mem, bytes, p->stream);
   if (e != cudaSuccess) {
@@ -706,7 +757,7 @@ int wg_pool_add(wg_pool* p, int64_t n, const double* x, const double* v, const d
   const u128 T = fixed_of(totmass, s->E);
   s->T_lo = (uint64_t)T;
   s->T_hi = (uint64_t)(T >> 64);
-  PC(cudaMemsetAsync(s->recs, 0, sizeof(BucketRec) * (size_t)s->nb, p->stream));
+  PC(cudaMemsetAsync(s->recs, 0, sizeof(BucketRec) * (size_t)s->nb_room, p->stream));
   if (s->ptab) {
     const StateTable t = member_sample_table(s);
     PC(cudaMemcpyAsync(s->ptab, &t, sizeof(t), cudaMemcpyHostToDevice, p->stream));
@@ -765,8 +816,9 @@ static int pool_step_begin(wg_pool* p, int count, const int* ids, const double* 
     for (int j = 0; j < k; ++j)
       if (ids[j] == ids[k]) return pool_fail(WG_ERR_ARG, "simulation %d listed twice", ids[k]);
     act[(size_t)k] = p->sims[(size_t)ids[k]];
-    ntasks += act[(size_t)k]->nb;
   }
+  balance_targets(p, act);
+  for (const PoolSim* s : act) ntasks += s->nb;
   if (ntasks >= (1ll << 31)) return pool_fail(WG_ERR_ARG, "too many buckets in one step");
   int rc = ensure_small(p, count, nleap, ntasks);
   if (rc) return rc;
@@ -783,7 +835,7 @@ static int pool_step_begin(wg_pool* p, int count, const int* ids, const double* 
   if (p->epoch + (unsigned)nleap > kEpochLimit) {
     // restart epochs: forget every look-back record
     for (PoolSim* s : p->sims)
-      if (s) PC(cudaMemsetAsync(s->recs, 0, sizeof(BucketRec) * (size_t)s->nb, p->stream));
+      if (s) PC(cudaMemsetAsync(s->recs, 0, sizeof(BucketRec) * (size_t)s->nb_room, p->stream));
     if (p->ws)
       PC(cudaMemsetAsync(p->trecs, 0,
                          sizeof(TileRec) * (size_t)((p->ws_n + kForceTile - 1) / kForceTile),
@@ -866,10 +918,10 @@ static int pool_step_begin(wg_pool* p, int count, const int* ids, const double* 
     d.t_seq = p->t_seq + (size_t)k * L1;
     d.n = s->n;
     d.nb = s->nb;
-    d.target = s->tune.target;
+    d.target = s->target;
     d.window = s->tune.window;
     d.sort_bits = s->tune.sort_bits;
-    d.capg = kBucketCap;  // members have no big buckets
+    d.capg = s->capg;  // at most kBucketCap: members have no big buckets
     d.ptab = s->pred_calls > 0 ? s->ptab : nullptr;
     d.T_lo = s->T_lo;
     d.T_hi = s->T_hi;
