@@ -160,8 +160,7 @@ struct TaskMeta {
   int n;          // sheets in the bucket; -1: the simulation has aborted this call
   int lay;        // layout read by this sub-step
   uint32_t pcnt;  // sheets in the simulation's earlier buckets
-  int wlo, whi;   // splitter window [wlo, whi] of the next layout ...
-  int wbuf;       // ... in wkey[wbuf], widx[wbuf]
+  int wlo, whi;   // splitter window [wlo, whi] of the next layout
   int eq;         // equal masses
   double amp;     // time factor of a pulsed external force at this sub-step
   double inv_h;   // 1 / h of a pulsed external force

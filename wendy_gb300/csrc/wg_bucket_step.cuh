@@ -100,10 +100,9 @@ struct __align__(16) StepSmem {
     // entry is the window length for a bucket outside the window
     uint32_t dest[CAP];
   } u;
-  // splitter windows of the next layout, double-buffered: the one of the
-  // next task is read while the current task runs
-  uint64_t wkey[2][2 * RWIN + 2];
-  int32_t widx[2][2 * RWIN + 2];
+  // splitter window of the next layout
+  uint64_t wkey[2 * RWIN + 2];
+  int32_t widx[2 * RWIN + 2];
   uint32_t dcount[2 * RWIN + 2];  // sheets bound for each window entry (+ outside the window)
   uint32_t dstart[2 * RWIN + 3];  // their exclusive prefix: segments of the grouped order
   uint32_t dbase[2 * RWIN + 2];   // first slot of each window bucket taken by this bucket
@@ -119,7 +118,9 @@ struct __align__(16) StepSmem {
   uint32_t prefix_cnt;
   uint64_t red_min[WARPS], red_max[WARPS];
   TaskMeta next;
-  int win_lo, win_hi, cur_wbuf;
+  int win_lo, win_hi;
+  int amp_sim;            // simulation whose time factor warp 0 has at hand (-1: none) ...
+  double amp_kept, inv_h_kept;  // ... and the factor
   double amp, inv_h;
   unsigned long long maxv;
   unsigned maxc;  // largest destination count this task saw after its reservations
@@ -143,6 +144,7 @@ struct __align__(16) StepSmem {
 // bound by latency and issue, and the third CTA hides more of it than the
 // recomputed conversions cost.
 static_assert(CTAS * (sizeof(StepSmem) + 1024) <= 228 * 1024, "StepSmem too large");
+static_assert(2 * RWIN + 2 <= BT, "one window entry per thread");
 static_assert(LUTN == BT, "one routing-table cell per thread");
 // process_big keeps its histogram where its chunks' positions go later
 static_assert(sizeof(double) * CAP >= 4 * BIGBINS, "big-bucket histogram");
@@ -300,13 +302,15 @@ __device__ __forceinline__ int lut_cell(float x, float x0, float scale) {
 // zero).  Here the cell of this thread's splitter (threads 1 .. wlen - 1;
 // -1 for the others); the sort counts the splitters per cell and sums the
 // counts along with its own bins.
-__device__ __forceinline__ int route_cell(StepSmem& S, const uint64_t* wk, int lo, int hi,
-                                          int64_t nb) {
-  const int j = threadIdx.x, wlen = hi - lo;
+// wk: the window's keys; first, last: it begins or ends with the layout (and
+// with an infinite splitter).
+__device__ __forceinline__ int route_cell(StepSmem& S, const uint64_t* wk, int wlen, bool first,
+                                          bool last) {
+  const int j = threadIdx.x;
   if (j < LUTN / 4) S.cell_cnt[j] = 0u;
   if (j >= wlen) return -1;
   // the first and last finite splitters of the window
-  const int j0 = lo == 0 ? 1 : 0, j1 = hi == (int)nb ? wlen - 1 : wlen;
+  const int j0 = first ? 1 : 0, j1 = last ? wlen - 1 : wlen;
   float x0 = 0.f, scale = 0.f;
   if (j1 > j0) {
     x0 = (float)pos_of_key(wk[j0]);
@@ -638,12 +642,9 @@ __device__ __forceinline__ PredLoad load_pred(const unsigned* cnt, const unsigne
 // loads of the first look-back group are issued together with all the others.
 template <int MASS>
 __device__ __forceinline__ void prepare_task(const StepLaunch& L, int sub, unsigned ep, int lane,
-                                             unsigned t, BucketTask tk, StepSmem& S, int wbuf) {
+                                             unsigned t, BucketTask tk, StepSmem& S) {
   TaskMeta& out = S.next;
-  if (lane == 0) {
-    out.task = t;
-    out.wbuf = wbuf;
-  }
+  if (lane == 0) out.task = t;
   if (t >= (unsigned)L.ntasks) return;
   const SimDev& D = L.sims[tk.sim];
   const int64_t b = tk.bucket;
@@ -655,9 +656,6 @@ __device__ __forceinline__ void prepare_task(const StepLaunch& L, int sub, unsig
   const int64_t nbk = D.nb;
   const int wlo = (int)(b > rw ? b - rw : 0);
   const int whi = (int)((b + rw + 1) < nbk ? (b + rw + 1) : nbk);
-  const int qs = (D.qsel0 + sub) & 1;
-  const uint64_t* qdk = D.qk[qs];
-  const int32_t* qdi = D.qi[qs];
   // ---- one round of loads
   const unsigned ab = __ldcg(D.ocount + 1);
   const bool eq = MASS == kMassEqual ||
@@ -665,23 +663,19 @@ __device__ __forceinline__ void prepare_task(const StepLaunch& L, int sub, unsig
                    (D.eq == kEqYes || (D.eq == kEqWord && __ldcg(D.eq_word) == 0u)));
   const unsigned own_c = cnt[b];
   const u128 own_m = eq ? (u128)0 : mass_of_limbs(mass + 4 * b);
-  constexpr int WQ = (2 * RWIN + 2 + 31) / 32;
-  uint64_t wkr[WQ];
-  int32_t wir[WQ];
-#pragma unroll
-  for (int q = 0; q < WQ; ++q) {
-    const int j = lane + 32 * q;
-    if (j <= whi - wlo) {
-      wkr[q] = qdk[wlo + j];
-      wir[q] = qdi[wlo + j];
-    }
-  }
   int64_t j = b - 1;
   PredLoad pl = load_pred(cnt, mass, recs, j - lane, eq);
   double amp = 0.0, inv_h = 0.0;
   if (lane == 0 && D.ext.kind == EXT_PULSE_TANH) {
-    amp = pulse_amplitude(D.ext, D.t_seq[sub]);
-    inv_h = 1.0 / D.ext.p[3];
+    // (an exponential and three divisions in FP64, 64 cycles an instruction:
+    // once per simulation, not per bucket)
+    if (S.amp_sim != tk.sim) {
+      S.amp_sim = tk.sim;
+      S.amp_kept = pulse_amplitude(D.ext, D.t_seq[sub]);
+      S.inv_h_kept = 1.0 / D.ext.p[3];
+    }
+    amp = S.amp_kept;
+    inv_h = S.inv_h_kept;
   }
   // an earlier sub-step of this call overflowed the simulation: its host
   // side finishes the call on the compact path
@@ -700,14 +694,6 @@ __device__ __forceinline__ void prepare_task(const StepLaunch& L, int sub, unsig
     bulk_prefetch_l2(D.bv[lay] + base, n4 * 8u);
     if (!eq) bulk_prefetch_l2(D.bm[lay] + base, n4 * 8u);
     bulk_prefetch_l2(D.bi[lay] + base, n4 * 4u);
-  }
-#pragma unroll
-  for (int q = 0; q < WQ; ++q) {
-    const int jw = lane + 32 * q;
-    if (jw <= whi - wlo) {
-      S.wkey[wbuf][jw] = wkr[q];
-      S.widx[wbuf][jw] = wir[q];
-    }
   }
   {
     const int cz = (cs + 2) % kAggSlots;
@@ -732,10 +718,7 @@ __device__ __forceinline__ void prepare_task(const StepLaunch& L, int sub, unsig
     const int stop = pmask ? (__ffs(pmask) - 1) : 31;
     const bool take = lane <= stop;
     if (!eq) pm += warp_sum_u128(take ? vm : (u128)0);
-    uint32_t c = take ? vcl : 0u;
-#pragma unroll
-    for (int d = 16; d >= 1; d >>= 1) c += __shfl_xor_sync(0xffffffffu, c, d);
-    pc += c;
+    pc += __reduce_add_sync(0xffffffffu, take ? vcl : 0u);
     if (pmask) break;
     j -= 32;
     if (j >= 0) pl = load_pred(cnt, mass, recs, j - lane, eq);
@@ -769,13 +752,13 @@ __device__ __forceinline__ void prepare_task(const StepLaunch& L, int sub, unsig
 // Claims a ticket and prepares its task; all lanes of one warp.
 template <int MASS>
 __device__ __forceinline__ void claim_task(const StepLaunch& L, int sub, unsigned ep, int lane,
-                                           StepSmem& S, int wbuf) {
+                                           StepSmem& S) {
   unsigned t = 0;
   if (lane == 0) t = atomicAdd(L.ticket, 1u);
   t = __shfl_sync(0xffffffffu, t, 0);
   BucketTask tk{0, 0};
   if (t < (unsigned)L.ntasks) tk = L.tasks[t];
-  prepare_task<MASS>(L, sub, ep, lane, t, tk, S, wbuf);
+  prepare_task<MASS>(L, sub, ep, lane, t, tk, S);
 }
 
 // Counting-sort bits of a simulation as the kernel uses them: at least four
@@ -793,7 +776,7 @@ __device__ __forceinline__ void clear_bins(StepSmem& S, int qb) {
 // a bucket (or of one chunk of a big bucket) that sit in shared memory, with
 // their bins cleared; S.prefix_mass / S.prefix_cnt hold the exclusive (mass,
 // count) prefix of the first of them, the splitter window of the next layout
-// is in S.wkey[S.cur_wbuf] and its routing table in S.lut.  arrived: this
+// is in S.wkey and its routing table in S.lut.  arrived: this
 // thread saw the sheets' copies complete; returns false, having done nothing,
 // if some thread did not.  rcell: from route_cell.  pre: the opening half drift still to be applied.
 // PREP: warp 0 prepares the next task (ticket nt of thread 0) during the
@@ -812,8 +795,8 @@ __device__ __forceinline__ bool process_bucket(const StepLaunch& L, StepSmem& S,
   if (!bucket_sort(S, n, ipt, step_sort_bits(D), arrived, pre, rcell)) return false;
   BucketTask ntk{0, 0};
   if (PREP && tid == 0 && nt < (unsigned)L.ntasks) ntk = L.tasks[nt];
-  const uint64_t* const wk = S.wkey[S.cur_wbuf];
-  const int32_t* const wi = S.widx[S.cur_wbuf];
+  const uint64_t* const wk = S.wkey;
+  const int32_t* const wi = S.widx;
 
   // ---- exact prefix of the masses in sorted order: thread tid holds the
   // sorted positions [tid * ipt, tid * ipt + ipt)
@@ -1028,70 +1011,80 @@ __device__ __forceinline__ bool process_bucket(const StepLaunch& L, StepSmem& S,
     c.x[q - 1] = fma(2.0 * dt, (double)(vs / (float)n), S.samp_x[tid]);
     c.idx[q - 1] = S.samp_idx[tid];
   }
-  // ---- the sheets grouped by destination bucket of the next layout: every
-  // thread takes its positions' destinations into registers, one warp forms
-  // the segments, and the same array then holds the grouped order
-  const int cw = (D.cs0 + sub + 1) % kAggSlots;
-  unsigned* const cnt_out = D.bcnt[cw];
-  unsigned long long* const mass_out = D.bmass[cw];
-  const uint64_t* const qfar = D.qk[(D.qsel0 + sub) & 1];
-  const int32_t* const ifar = D.qi[(D.qsel0 + sub) & 1];
-  // slots: one atomic per window bucket, its round trip overlapping the
-  // grouping (warps 2 on; warp 1 forms the segments)
-  uint32_t db = 0, dcn = 0;
-  const int wt = tid - 64;
-  if (wt >= 0 && wt < wlen) {
-    dcn = S.dcount[wt];
-    if (dcn) db = atomicAdd(&cnt_out[S.win_lo + wt], dcn);
-  }
-  uint32_t mydest[MAXI];
-#pragma unroll
-  for (int i = 0; i < MAXI; ++i)
-    if (i < nmine) mydest[i] = S.u.dest[j0 + i];
-  if (warp == 1) {
-    // segments: exclusive prefix of the counts of the wlen + 1 entries
-    constexpr int E5 = (2 * RWIN + 2 + 31) / 32;
-    uint32_t cv[E5];
-    uint32_t sum = 0;
-#pragma unroll
-    for (int k = 0; k < E5; ++k) {
-      const int j = lane * E5 + k;
-      cv[k] = j <= wlen ? S.dcount[j] : 0u;
-      sum += cv[k];
-    }
-    uint32_t incl2 = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, incl2, o);
-      if (lane >= o) incl2 += y;
-    }
-    uint32_t ex = incl2 - sum;
-#pragma unroll
-    for (int k = 0; k < E5; ++k) {
-      const int j = lane * E5 + k;
-      if (j <= wlen) S.dstart[j] = ex;
-      ex += cv[k];
-    }
-    if (lane == 31) S.dstart[wlen + 1] = incl2;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < MAXI; ++i)
-    if (i < nmine) {
-      const uint32_t w = mydest[i] >> 16;
-      S.u.dest[S.dstart[w] + (mydest[i] & 0xffffu)] = (w << 16) | S.perm[j0 + i];
-    }
-  if (dcn) {
-    S.dbase[wt] = db;
-    atomicMax(&S.maxc, db + dcn);
-  }
-  __syncthreads();
+  // ---- warp 0 prepares the next task, which takes it about as long as the
+  // others take for the rest of this one: they group the sheets by destination
+  // bucket of the next layout and write them out, synchronising among
+  // themselves (named barrier 1)
   bool overflow = false;
   if (PREP && warp == 0) {
-    // warp 0 prepares the next task while the others write out
-    prepare_task<MASS>(L, sub, ep, lane, S.next_ticket, S.next_tk, S, S.cur_wbuf ^ 1);
+    prepare_task<MASS>(L, sub, ep, lane, S.next_ticket, S.next_tk, S);
   } else {
-    const int nw = PREP ? BT - 32 : BT, t0 = PREP ? tid - 32 : tid;
+    constexpr int nw = PREP ? BT - 32 : BT;
+    constexpr int MAXD = (CAP + nw - 1) / nw;
+    const int t0 = PREP ? tid - 32 : tid, w0 = t0 >> 5;
+    auto sync_out = [] {
+      if constexpr (PREP)
+        asm volatile("bar.sync 1, %0;" ::"n"(BT - 32) : "memory");
+      else
+        __syncthreads();
+    };
+    const int cw = (D.cs0 + sub + 1) % kAggSlots;
+    unsigned* const cnt_out = D.bcnt[cw];
+    unsigned long long* const mass_out = D.bmass[cw];
+    const uint64_t* const qfar = D.qk[(D.qsel0 + sub) & 1];
+    const int32_t* const ifar = D.qi[(D.qsel0 + sub) & 1];
+    // slots: one atomic per window bucket, its round trip overlapping the
+    // grouping (the second of these warps on; the first forms the segments)
+    uint32_t db = 0, dcn = 0;
+    const int wt = t0 - 32;
+    if (wt >= 0 && wt < wlen) {
+      dcn = S.dcount[wt];
+      if (dcn) db = atomicAdd(&cnt_out[S.win_lo + wt], dcn);
+    }
+    // the destinations go through registers: the same array then holds the
+    // grouped order
+    uint32_t dest[MAXD];
+#pragma unroll
+    for (int i = 0; i < MAXD; ++i)
+      if (t0 + i * nw < n) dest[i] = S.u.dest[t0 + i * nw];
+    if (w0 == 0) {
+      // segments: exclusive prefix of the counts of the wlen + 1 entries
+      constexpr int E5 = (2 * RWIN + 2 + 31) / 32;
+      uint32_t cv[E5];
+      uint32_t sum = 0;
+#pragma unroll
+      for (int k = 0; k < E5; ++k) {
+        const int j = lane * E5 + k;
+        cv[k] = j <= wlen ? S.dcount[j] : 0u;
+        sum += cv[k];
+      }
+      uint32_t incl2 = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl2, o);
+        if (lane >= o) incl2 += y;
+      }
+      uint32_t ex = incl2 - sum;
+#pragma unroll
+      for (int k = 0; k < E5; ++k) {
+        const int j = lane * E5 + k;
+        if (j <= wlen) S.dstart[j] = ex;
+        ex += cv[k];
+      }
+      if (lane == 31) S.dstart[wlen + 1] = incl2;
+    }
+    sync_out();
+#pragma unroll
+    for (int i = 0; i < MAXD; ++i)
+      if (t0 + i * nw < n) {
+        const uint32_t w = dest[i] >> 16;
+        S.u.dest[S.dstart[w] + (dest[i] & 0xffffu)] = (w << 16) | S.perm[t0 + i * nw];
+      }
+    if (dcn) {
+      S.dbase[wt] = db;
+      atomicMax(&S.maxc, db + dcn);
+    }
+    sync_out();
     // write-out grouped by destination: consecutive positions of a segment
     // take consecutive slots, so a warp's stores coalesce
     double* const xout = D.bx[1 - lay];
@@ -1142,7 +1135,7 @@ __device__ __forceinline__ bool process_bucket(const StepLaunch& L, StepSmem& S,
     }
     // ---- masses of the next layout: a warp sums the fixed-point masses of
     // a window bucket's segment and adds them to that bucket's accumulators
-    for (int w = eq ? wlen : PREP ? warp - 1 : warp; w < wlen; w += PREP ? WARPS - 1 : WARPS) {
+    for (int w = eq ? wlen : w0; w < wlen; w += nw / 32) {
       const int q0 = (int)S.dstart[w], q1 = (int)S.dstart[w + 1];
       if (q0 == q1) continue;
       u128 P = 0;
@@ -1245,14 +1238,13 @@ __device__ __forceinline__ void process_big(const StepLaunch& L, StepSmem& S, co
   {
     const int qs = (D.qsel0 + sub) & 1;
     for (int j = tid; j <= bt.whi - bt.wlo; j += BT) {
-      S.wkey[0][j] = D.qk[qs][bt.wlo + j];
-      S.widx[0][j] = D.qi[qs][bt.wlo + j];
+      S.wkey[j] = D.qk[qs][bt.wlo + j];
+      S.widx[j] = D.qi[qs][bt.wlo + j];
     }
   }
   if (tid == 0) {
     S.win_lo = bt.wlo;
     S.win_hi = bt.whi;
-    S.cur_wbuf = 0;
     S.maxv = 0;
     S.maxc = 0;
     S.nsamp = 0;
@@ -1359,7 +1351,7 @@ __device__ __forceinline__ void process_big(const StepLaunch& L, StepSmem& S, co
       break;
     }
     if (nc == 0) continue;
-    const int rcell = route_cell(S, S.wkey[0], bt.wlo, bt.whi, D.nb);
+    const int rcell = route_cell(S, S.wkey, bt.whi - bt.wlo, bt.wlo == 0, bt.whi == (int)D.nb);
     process_bucket<LAST, EXPR, MASS, false>(L, S, D, bt.bucket, bt.lay, nc, sub, ep, true, 0.0, rcell,
                                       0u);
   }
@@ -1378,12 +1370,13 @@ __global__ void __launch_bounds__(BT, CTAS) k_bucket_step(const __grid_constant_
   const int sub = L.sub;
   if (tid == 0) {
     S.big_head = -1;
+    S.amp_sim = -1;
     mbar_init(&S.mbar, 1);
     fence_proxy_async_smem();
   }
   chain_begin();
   const unsigned ep = L.epochs[sub];
-  if (warp == 0) claim_task<MASS>(L, sub, ep, lane, S, 0);
+  if (warp == 0) claim_task<MASS>(L, sub, ep, lane, S);
   unsigned parity = 0;
   for (;;) {
     __syncthreads();
@@ -1395,7 +1388,7 @@ __global__ void __launch_bounds__(BT, CTAS) k_bucket_step(const __grid_constant_
       // them), taken in chunks after the others
       if (tm.n > CAP && tid == 0) list_big(S, L.big_list, L.big_next, L.big_count);
       __syncthreads();  // every thread has read S.next
-      if (warp == 0) claim_task<MASS>(L, sub, ep, lane, S, tm.wbuf);
+      if (warp == 0) claim_task<MASS>(L, sub, ep, lane, S);
       continue;
     }
     const SimDev& D = L.sims[tm.sim];
@@ -1420,13 +1413,19 @@ __global__ void __launch_bounds__(BT, CTAS) k_bucket_step(const __grid_constant_
     unsigned nt = 0;
     if (tid == 0) nt = atomicAdd(L.ticket, 1u);
     const double pre = sub == 0 ? D.pre_dt : 0.0;
-    // the splitter window of the next layout around this bucket arrived with
-    // the task; the per-destination counters are cleared here
-    for (int j = tid; j <= tm.whi - tm.wlo; j += BT) S.dcount[j] = 0;  // wlen + 1 entries
+    // the splitter window of the next layout around this bucket (wlen + 1
+    // entries, at most one per thread); the per-destination counters are cleared
+    const int wlen = tm.whi - tm.wlo;
+    const int qs = (D.qsel0 + sub) & 1;
+    const uint64_t* const qk = D.qk[qs] + tm.wlo;
+    if (tid <= wlen) {
+      S.wkey[tid] = qk[tid];
+      S.widx[tid] = D.qi[qs][tm.wlo + tid];
+      S.dcount[tid] = 0;
+    }
     if (tid == 0) {
       S.win_lo = tm.wlo;
       S.win_hi = tm.whi;
-      S.cur_wbuf = tm.wbuf;
       S.maxv = 0;
       S.maxc = 0;
       S.nsamp = 0;
@@ -1439,7 +1438,7 @@ __global__ void __launch_bounds__(BT, CTAS) k_bucket_step(const __grid_constant_
     // while the copies are in flight: the counting-sort bins are cleared and
     // the window's splitters take their cells of the routing table
     clear_bins(S, step_sort_bits(D));
-    const int rcell = route_cell(S, S.wkey[tm.wbuf], tm.wlo, tm.whi, D.nb);
+    const int rcell = route_cell(S, qk, wlen, tm.wlo == 0, tm.whi == (int)D.nb);
     // the copies' completion: a thread that did not see it within the bounded
     // wait leaves the data alone, and the first barrier of the sort (which
     // every thread reaches) decides for the whole CTA
