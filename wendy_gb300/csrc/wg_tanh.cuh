@@ -194,10 +194,10 @@ __device__ __forceinline__ double tanh_fixed(double y) {
 // 0 <= D < 2^-10 the remainder is below 2^-64 (the Taylor coefficients of
 // tanh are below 1), s is formed in fixed point and the higher coefficients
 // in double (their rounding enters multiplied by D^2 <= 2^-20), and each
-// Horner step is one signed high product with D 2^64, so the absolute error
+// Horner step is a signed product with D (below), so the absolute error
 // stays within that of tanh_q62 plus 2^-61.  The cell and D come from the
 // argument's bits (D is exact up to one truncation of 2^-64).  Per argument
-// this is some 35 integer instructions and three 16-byte loads, which hit
+// this is some 60 integer instructions and three 16-byte loads, which hit
 // in L1 for the sorted positions of a bucket or tile, against about 150
 // instructions and two conversions on the FP64 pipe for tanh_fixed.  The
 // table (20480 cells, 960 KB) is computed once per device by
@@ -223,8 +223,8 @@ __device__ __forceinline__ void tanh_table_row(int i, long long* row) {
   row[5] = __double2ll_rn(sd * (2.0 - 15.0 * t2 + 15.0 * t2 * t2) / 15.0 * 0x1p62);
 }
 
-// tanh(y) with the table (16-byte aligned, kTanhCells rows).
-__device__ __forceinline__ double tanh_tab(const long long* __restrict__ tab, double y) {
+// Small and large arguments and those below the second cell.
+static __device__ __noinline__ double tanh_tab_ends(const long long* __restrict__ tab, double y) {
   const uint64_t bits = (uint64_t)__double_as_longlong(y);
   const uint64_t sign = bits & 0x8000000000000000ull;
   const uint64_t abits = bits ^ sign;
@@ -233,30 +233,63 @@ __device__ __forceinline__ double tanh_tab(const long long* __restrict__ tab, do
     if (abits > 0x7ff0000000000000ull) return y;
     return __longlong_as_double((long long)(sign | 0x3ff0000000000000ull));
   }
-  const int e = (int)(abits >> 52) - 1023;  // -27 .. 4
+  // |y| < 2^-10: the first cell, |y| = D 2^-64
+  const int e = (int)(abits >> 52) - 1023;  // -27 .. -11
   const uint64_t m = (abits & 0x000fffffffffffffull) | 0x0010000000000000ull;
-  // |y| = m 2^(e - 52) = cell 2^-10 + D 2^-64
-  int cell;
-  uint64_t D;
-  if (e >= -10) {
-    const int sh = 42 - e;  // 38 .. 52
-    cell = (int)(m >> sh);
-    D = (m & ((1ull << sh) - 1)) << (e + 12);
-  } else {
-    cell = 0;
-    D = e >= -12 ? m << (e + 12) : m >> (-12 - e);
-  }
-  const longlong2* r = reinterpret_cast<const longlong2*>(tab + kTanhRow * cell);
+  const long long d = (long long)(e >= -12 ? m << (e + 12) : m >> (-12 - e));
+  const longlong2* r = reinterpret_cast<const longlong2*>(tab);
   const longlong2 r0 = __ldg(r), r1 = __ldg(r + 1), r2 = __ldg(r + 2);
-  const long long d = (long long)D;  // < 2^54
   long long p = r2.y;
   p = r2.x + __mul64hi(p, d);
   p = r1.y + __mul64hi(p, d);
   p = r1.x + __mul64hi(p, d);
   p = r0.y + __mul64hi(p, d);
-  const long long T = r0.x + __mul64hi(p, d);  // tanh(|y|) 2^62, in (2^35, 2^62)
+  return q62_to_double((uint64_t)(r0.x + __mul64hi(p, d)), sign);
+}
+
+// (s d) >> 32 of a signed 64-bit s and a non-negative 31-bit d.
+__device__ __forceinline__ long long mul_64_31(long long s, int d) {
+  return (long long)(int)(s >> 32) * d + (long long)__umulhi((uint32_t)s, (uint32_t)d);
+}
+
+// tanh(y) with the table (16-byte aligned, kTanhCells rows).  The offset D in
+// the cell has 54 bits; a Horner step needs as many of them as the powers of D
+// still to come leave significant: the first two work on 32-bit words, the
+// third on the upper 31 bits of D (rounded), and only the last two on all of
+// it, as 31 + 23 bits.  Their truncations are made up for by one unit, which
+// leaves the largest absolute error over the range at 2^-61.3 and the mean at
+// 0.48 units of 2^-62 (2^-61.2 and 0.52 with full products throughout), for
+// half of their instructions.
+__device__ __forceinline__ double tanh_tab(const long long* __restrict__ tab, double y) {
+  const uint32_t yh = (uint32_t)__double2hiint(y), yl = (uint32_t)__double2loint(y);
+  const uint32_t ah = yh & 0x7fffffffu;
+  if (ah - 0x3f500000u >= 0x40340000u - 0x3f500000u) return tanh_tab_ends(tab, y);
+  // |y| in [2^-10, 20): |y| = cell 2^-10 + D 2^-64, in 32-bit words
+  const int e = (int)(ah >> 20) - 1023;  // -10 .. 4
+  const uint32_t mh = (ah & 0xfffffu) | 0x100000u;
+  const uint32_t cell = mh >> (10 - e);
+  const uint32_t fh = mh & ((1u << (10 - e)) - 1u);
+  const uint32_t dh = __funnelshift_l(yl, fh, e + 12), dw = yl << (e + 12);
+  const int dt = (int)__funnelshift_l(dw, dh, 9);  // D >> 23
+  const int dl = (int)(dw & 0x7fffffu);
+  const int d = min((uint32_t)dt + (uint32_t)(dl >> 22), 0x7fffffffu);  // rounded
+  const longlong2* r = reinterpret_cast<const longlong2*>(tab + kTanhRow * cell);
+  const longlong2 r0 = __ldg(r), r1 = __ldg(r + 1), r2 = __ldg(r + 2);
+  const int s4 = (int)(r2.x >> 32) + (__mulhi((int)(r2.y >> 32), d) >> 9);
+  const long long s3 = r1.y + (((long long)s4 * d) >> 9);
+  const long long s2 = r1.x + (mul_64_31(s3, d) >> 9);
+  const long long s1 = r0.y + (mul_64_31(s2, dt) >> 9) + __mulhi((int)(s2 >> 32), dl);
+  const long long T = r0.x + (mul_64_31(s1, dt) >> 9) + __mulhi((int)(s1 >> 32), dl) + 1;
+  // T 2^-62 in [2^-10, 1] to double, rounded half up; the carry of the
+  // rounding may run into the exponent
   const uint64_t Tq = T >= (1ll << 62) ? (1ull << 62) - 1 : (uint64_t)T;
-  return q62_to_double(Tq, sign);
+  const uint32_t th = (uint32_t)(Tq >> 32), tl = (uint32_t)Tq;
+  const int lz = __clz((int)th);  // 2 .. 11
+  const uint32_t nh = __funnelshift_l(tl, th, lz), nl = tl << lz;
+  const uint64_t mant = (((uint64_t)(nh >> 11) << 32) | __funnelshift_r(nl, nh, 11)) +
+                        ((nl >> 10) & 1u);
+  const uint64_t bits = mant + ((uint64_t)(1023 - lz) << 52);
+  return __longlong_as_double((long long)(bits | ((uint64_t)(yh & 0x80000000u) << 32)));
 }
 
 }  // namespace wg
