@@ -15,7 +15,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "_wendy_gb300.so")
 BUILD_DIR = os.path.join(HERE, "_build")
-SOURCES = ["wg_kernels.cu", "wg_radix.cu", "wg_bucket.cu", "wg_bucket_expr.cu", "wg_api.cu", "wg_pool.cu",
+SOURCES = ["wg_bucket.cu", "wg_bucket_closed.cu", "wg_bucket_expr.cu", "wg_kernels.cu",
+           "wg_radix.cu", "wg_api.cu", "wg_pool.cu",
            "wg_exact.cu", "wg_noalloc.cu", "wg_small.cu", "wg_blocks.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2"]

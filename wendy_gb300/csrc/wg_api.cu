@@ -812,7 +812,7 @@ StepLaunch step_launch(wg_sim* s, int i, int nleap, int profile) {
   L.err = s->err;
   L.profile = profile;
   L.mass = s->eq == kEqNo ? kMassAny : s->eq == kEqYes ? kMassEqual : kMassMixed;
-  L.any_expr = s->ext.kind == EXT_EXPR;
+  L.force = force_class(s->ext);
   L.big_list = s->big_list;
   L.big_next = s->big_next;
   L.big_count = s->big_counts + i;

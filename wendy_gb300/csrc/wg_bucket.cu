@@ -147,20 +147,23 @@ void set_tuning(const std::vector<std::pair<int64_t, BucketTuning>>& rows) {
   g_tune = rows;
 }
 
+StepKernel step_kernel_none(bool last, int mass) {
+  if (mass == kMassAny)
+    return last ? k_bucket_step<true, kForceNone, kMassAny> : k_bucket_step<false, kForceNone, kMassAny>;
+  if (mass == kMassEqual)
+    return last ? k_bucket_step<true, kForceNone, kMassEqual> : k_bucket_step<false, kForceNone, kMassEqual>;
+  return last ? k_bucket_step<true, kForceNone, kMassMixed> : k_bucket_step<false, kForceNone, kMassMixed>;
+}
+
 // The sub-step kernel's dynamic shared-memory limit, raised once per device
 // (function attributes belong to the device they were set on).
 void bucket_attr_init() {
-  auto set = [](StepKernel k) {
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(StepSmem));
-  };
-  set(k_bucket_step<false, false, kMassAny>);
-  set(k_bucket_step<true, false, kMassAny>);
-  set(k_bucket_step<false, false, kMassEqual>);
-  set(k_bucket_step<true, false, kMassEqual>);
-  set(k_bucket_step<false, false, kMassMixed>);
-  set(k_bucket_step<true, false, kMassMixed>);
   for (int mass : {kMassAny, kMassEqual, kMassMixed})
-    for (bool last : {false, true}) set(step_kernel_expr(last, mass));
+    for (bool last : {false, true})
+      for (StepKernel k : {step_kernel_none(last, mass), step_kernel_closed(last, mass),
+                           step_kernel_expr(last, mass)})
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(StepSmem));
 }
 
 void bucket_step_prepare() {
@@ -200,17 +203,9 @@ void launch_bucket_step(const StepLaunch& a, int grid, cudaStream_t s) {
   if (grid > a.ntasks) grid = a.ntasks;
   if (grid < 1) grid = 1;
   const bool last = a.sub == a.nleap - 1;
-  StepKernel k;
-  if (a.any_expr) {
-    k = step_kernel_expr(last, a.mass);
-  } else {
-    k = a.mass == kMassEqual
-            ? (last ? k_bucket_step<true, false, kMassEqual> : k_bucket_step<false, false, kMassEqual>)
-        : a.mass == kMassAny
-            ? (last ? k_bucket_step<true, false, kMassAny> : k_bucket_step<false, false, kMassAny>)
-            : (last ? k_bucket_step<true, false, kMassMixed>
-                    : k_bucket_step<false, false, kMassMixed>);
-  }
+  const StepKernel k = a.force == kForceNone     ? step_kernel_none(last, a.mass)
+                       : a.force == kForceClosed ? step_kernel_closed(last, a.mass)
+                                                 : step_kernel_expr(last, a.mass);
   launch_chained(k, (unsigned)grid, BT, sizeof(StepSmem), s, a);
 }
 

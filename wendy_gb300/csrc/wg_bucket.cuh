@@ -137,6 +137,12 @@ struct SimDev {
 };
 
 enum : int { kEqNo = 0, kEqYes = 1, kEqWord = 2 };
+// The external forces of a launch's simulations: none, closed forms, or
+// expressions among them.
+enum : int { kForceNone = 0, kForceClosed = 1, kForceExpr = 2 };
+inline int force_class(const ExtForce& f) {
+  return f.kind == EXT_NONE ? kForceNone : f.kind == EXT_EXPR ? kForceExpr : kForceClosed;
+}
 // The masses of a launch's simulations: any, all equal, or decided per task.
 enum : int { kMassAny = 0, kMassEqual = 1, kMassMixed = 2 };
 
@@ -178,7 +184,7 @@ struct StepLaunch {
   unsigned* err;
   int profile;           // 1: dt = 0 and no outputs (timing harness)
   int mass;              // kMass...: equal masses in none, all or some of the simulations
-  int any_expr;          // some simulation of the launch has an expression force
+  int force;             // kForce...: the external forces among the simulations
   // big buckets (simulations with capg > kBucketCap): by bucket, the task and
   // the next bucket of the CTA that claimed it; how many there were
   TaskMeta* big_list;
@@ -187,7 +193,10 @@ struct StepLaunch {
 };
 
 typedef void (*StepKernel)(StepLaunch);
-// The sub-step kernel for launches with expression forces (wg_bucket_expr.cu).
+// The sub-step kernel of one kind of launch, by external force (wg_bucket.cu,
+// wg_bucket_closed.cu, wg_bucket_expr.cu).
+StepKernel step_kernel_none(bool last, int mass);
+StepKernel step_kernel_closed(bool last, int mass);
 StepKernel step_kernel_expr(bool last, int mass);
 void launch_bucket_step(const StepLaunch& a, int grid, cudaStream_t s);
 // Pool members with predicted splitters (SimDev::ptab set): block k sorts the

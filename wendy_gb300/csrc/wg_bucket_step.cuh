@@ -1,6 +1,6 @@
 // wg_bucket_step.cuh -- the fused sub-step kernel on bucketed state, a template
-// over the kinds of launch, instantiated by wg_bucket.cu and, with expression
-// forces, by wg_bucket_expr.cu.
+// over the kinds of launch, instantiated by wg_bucket.cu (no external force),
+// wg_bucket_closed.cu and wg_bucket_expr.cu, which compile side by side.
 //
 // Between sub-steps the sheets of a simulation live in B buckets of fixed
 // capacity; bucket b holds exactly the sheets whose (position key, index)
@@ -640,7 +640,7 @@ __device__ __forceinline__ PredLoad load_pred(const unsigned* cnt, const unsigne
 // aggregate.  Aggregates were completed by the previous launch, so the walk
 // never waits; the bucket then publishes its own inclusive prefix.  The
 // loads of the first look-back group are issued together with all the others.
-template <int MASS>
+template <int FORCE, int MASS>
 __device__ __forceinline__ void prepare_task(const StepLaunch& L, int sub, unsigned ep, int lane,
                                              unsigned t, BucketTask tk, StepSmem& S) {
   TaskMeta& out = S.next;
@@ -666,7 +666,7 @@ __device__ __forceinline__ void prepare_task(const StepLaunch& L, int sub, unsig
   int64_t j = b - 1;
   PredLoad pl = load_pred(cnt, mass, recs, j - lane, eq);
   double amp = 0.0, inv_h = 0.0;
-  if (lane == 0 && D.ext.kind == EXT_PULSE_TANH) {
+  if (FORCE != kForceNone && lane == 0 && D.ext.kind == EXT_PULSE_TANH) {
     // (an exponential and three divisions in FP64, 64 cycles an instruction:
     // once per simulation, not per bucket)
     if (S.amp_sim != tk.sim) {
@@ -750,7 +750,7 @@ __device__ __forceinline__ void prepare_task(const StepLaunch& L, int sub, unsig
 }
 
 // Claims a ticket and prepares its task; all lanes of one warp.
-template <int MASS>
+template <int FORCE, int MASS>
 __device__ __forceinline__ void claim_task(const StepLaunch& L, int sub, unsigned ep, int lane,
                                            StepSmem& S) {
   unsigned t = 0;
@@ -758,7 +758,7 @@ __device__ __forceinline__ void claim_task(const StepLaunch& L, int sub, unsigne
   t = __shfl_sync(0xffffffffu, t, 0);
   BucketTask tk{0, 0};
   if (t < (unsigned)L.ntasks) tk = L.tasks[t];
-  prepare_task<MASS>(L, sub, ep, lane, t, tk, S);
+  prepare_task<FORCE, MASS>(L, sub, ep, lane, t, tk, S);
 }
 
 // Counting-sort bits of a simulation as the kernel uses them: at least four
@@ -782,7 +782,7 @@ __device__ __forceinline__ void clear_bins(StepSmem& S, int qb) {
 // PREP: warp 0 prepares the next task (ticket nt of thread 0) during the
 // grouping, as the main kernel's pipeline does; otherwise (chunks of a big
 // bucket) the prefix base is advanced past these sheets at the end.
-template <bool LAST, bool EXPR, int MASS, bool PREP>
+template <bool LAST, int FORCE, int MASS, bool PREP>
 __device__ __forceinline__ bool process_bucket(const StepLaunch& L, StepSmem& S, const SimDev& D,
                                                const int64_t b, const int lay, const int n,
                                                const int sub, const unsigned ep,
@@ -843,9 +843,9 @@ __device__ __forceinline__ bool process_bucket(const StepLaunch& L, StepSmem& S,
   const double omega2 = D.omega2;
   const ExtForce ext = D.ext;
   // an expression force: its time phase, once per task and thread
-  double xr[EXPR ? kExprRegs : 1];
+  double xr[FORCE == kForceExpr ? kExprRegs : 1];
   double t_ev = 0.0;
-  if constexpr (EXPR) {
+  if constexpr (FORCE == kForceExpr) {
     if (ext.kind == EXT_EXPR) {
       t_ev = D.t_seq[sub];
       expr_time(ext, t_ev, xr);
@@ -911,12 +911,12 @@ __device__ __forceinline__ bool process_bucket(const StepLaunch& L, StepSmem& S,
       double acc = fixed_to_double(A, E);
       A -= (i128)M;
       if (has_omega) acc = fma(-omega2, x, acc);
-      if constexpr (EXPR) {
+      if constexpr (FORCE == kForceExpr) {
         if (ext.kind == EXT_EXPR)
           acc = expr_space(ext, xr, x, t_ev) + acc;
         else if (ext.kind != EXT_NONE)
           acc = ext_force_at(ext, S.amp, S.inv_h, x) + acc;
-      } else if (ext.kind != EXT_NONE) {
+      } else if (FORCE == kForceClosed && ext.kind != EXT_NONE) {
         acc = ext_force_at(ext, S.amp, S.inv_h, x) + acc;
       }
       const double vn = fma(dt, acc, v);
@@ -1017,7 +1017,7 @@ __device__ __forceinline__ bool process_bucket(const StepLaunch& L, StepSmem& S,
   // themselves (named barrier 1)
   bool overflow = false;
   if (PREP && warp == 0) {
-    prepare_task<MASS>(L, sub, ep, lane, S.next_ticket, S.next_tk, S);
+    prepare_task<FORCE, MASS>(L, sub, ep, lane, S.next_ticket, S.next_tk, S);
   } else {
     constexpr int nw = PREP ? BT - 32 : BT;
     constexpr int MAXD = (CAP + nw - 1) / nw;
@@ -1223,7 +1223,7 @@ static __device__ __noinline__ void list_big(StepSmem& S, TaskMeta* big_list, in
 // intact.  A CTA keeps the big buckets it has claimed for when it has no other
 // task left; a second launch per sub-step for buckets that are rarely there
 // cost 3.3 us and the gap before it, empty.
-template <bool LAST, bool EXPR, int MASS>
+template <bool LAST, int FORCE, int MASS>
 __device__ __forceinline__ void process_big(const StepLaunch& L, StepSmem& S, const TaskMeta& bt,
                                             int sub, unsigned ep) {
   const int tid = threadIdx.x;
@@ -1352,17 +1352,17 @@ __device__ __forceinline__ void process_big(const StepLaunch& L, StepSmem& S, co
     }
     if (nc == 0) continue;
     const int rcell = route_cell(S, S.wkey, bt.whi - bt.wlo, bt.wlo == 0, bt.whi == (int)D.nb);
-    process_bucket<LAST, EXPR, MASS, false>(L, S, D, bt.bucket, bt.lay, nc, sub, ep, true, 0.0, rcell,
+    process_bucket<LAST, FORCE, MASS, false>(L, S, D, bt.bucket, bt.lay, nc, sub, ep, true, 0.0, rcell,
                                       0u);
   }
 }
 
 // The fused sub-step.  LAST: the call's last sub-step (half drift, outputs).
-// EXPR: the launch has simulations with expression forces (the interpreter
-// is compiled only into this instantiation).  MASS: the launch's simulations
-// have any masses, equal ones, or there are some of each (kMass...): the choice
-// per task costs the general path 4 % in registers.
-template <bool LAST, bool EXPR, int MASS>
+// FORCE: the external forces of the launch's simulations -- none, closed forms
+// (and none), or expressions among them (the interpreter).  MASS: their masses
+// -- any, all equal, or decided per task.  What a launch does not need costs it
+// registers: the choice of masses per task 4 %, the unused force 1.6 %.
+template <bool LAST, int FORCE, int MASS>
 __global__ void __launch_bounds__(BT, CTAS) k_bucket_step(const __grid_constant__ StepLaunch L) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   StepSmem& S = *reinterpret_cast<StepSmem*>(smem_raw);
@@ -1376,7 +1376,7 @@ __global__ void __launch_bounds__(BT, CTAS) k_bucket_step(const __grid_constant_
   }
   chain_begin();
   const unsigned ep = L.epochs[sub];
-  if (warp == 0) claim_task<MASS>(L, sub, ep, lane, S);
+  if (warp == 0) claim_task<FORCE, MASS>(L, sub, ep, lane, S);
   unsigned parity = 0;
   for (;;) {
     __syncthreads();
@@ -1388,7 +1388,7 @@ __global__ void __launch_bounds__(BT, CTAS) k_bucket_step(const __grid_constant_
       // them), taken in chunks after the others
       if (tm.n > CAP && tid == 0) list_big(S, L.big_list, L.big_next, L.big_count);
       __syncthreads();  // every thread has read S.next
-      if (warp == 0) claim_task<MASS>(L, sub, ep, lane, S);
+      if (warp == 0) claim_task<FORCE, MASS>(L, sub, ep, lane, S);
       continue;
     }
     const SimDev& D = L.sims[tm.sim];
@@ -1443,7 +1443,7 @@ __global__ void __launch_bounds__(BT, CTAS) k_bucket_step(const __grid_constant_
     // wait leaves the data alone, and the first barrier of the sort (which
     // every thread reaches) decides for the whole CTA
     const bool arrived = n4 > 0 ? mbar_wait(&S.mbar, parity) : true;
-    if (!process_bucket<LAST, EXPR, MASS, true>(L, S, D, b, lay, n, sub, ep, arrived, pre, rcell,
+    if (!process_bucket<LAST, FORCE, MASS, true>(L, S, D, b, lay, n, sub, ep, arrived, pre, rcell,
                                           nt)) {
       // the bucket's copies did not complete within the bounded wait: its
       // contents are unknown, so this CTA writes nothing more.  It gives the
@@ -1459,7 +1459,7 @@ __global__ void __launch_bounds__(BT, CTAS) k_bucket_step(const __grid_constant_
   for (int b = S.big_head; b >= 0;) {
     const TaskMeta bt = L.big_list[b];
     b = L.big_next[b];
-    process_big<LAST, EXPR, MASS>(L, S, bt, sub, ep);
+    process_big<LAST, FORCE, MASS>(L, S, bt, sub, ep);
     __syncthreads();
   }
 }

@@ -287,7 +287,7 @@ struct wg_pool {
   int64_t g_ntasks = -1;
   void* g_small = nullptr;
   int g_mass = -1;       // ... and the instantiation for these masses
-  bool g_expr = false;   // the graph launches the expression-force instantiation
+  int g_force = -1;      // the graph launches the instantiation for these forces
   int64_t graph_builds = 0;
   wg_pool_stats stats{};  // counters (launches and graph_builds are filled on read)
 };
@@ -514,6 +514,12 @@ __global__ void k_read_back(const unsigned* src, unsigned* dst, int n) {
   for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
 }
 
+// The external forces of a launch over these members (kForce...).
+int forces_of(const std::vector<PoolSim*>& act) {
+  int f = kForceNone;
+  for (const PoolSim* s : act) f = std::max(f, force_class(s->ext));
+  return f;
+}
 // The masses of a launch over these members (kMass...).
 int masses_of(const std::vector<PoolSim*>& act) {
   size_t eq = 0;
@@ -944,12 +950,11 @@ static int pool_step_begin(wg_pool* p, int count, const int* ids, const double* 
   }
   // device sequence of the call, captured in a CUDA graph and replayed while
   // the number of simulations, buckets and sub-steps stays the same
-  bool launch_expr = false;  // the graph's kernels carry the expression interpreter
-  for (PoolSim* a : act) launch_expr |= a->ext.kind == EXT_EXPR;
+  const int launch_force = forces_of(act);
   const int launch_mass = masses_of(act);
   const bool rebuild = !p->gexec || p->g_count != count || p->g_nleap != nleap ||
                        p->g_ntasks != ntasks || p->g_small != p->small ||
-                       p->g_expr != launch_expr || p->g_mass != launch_mass;
+                       p->g_force != launch_force || p->g_mass != launch_mass;
   if (rebuild) {
     if (p->gexec) cudaGraphExecDestroy(p->gexec);
     p->gexec = nullptr;
@@ -984,7 +989,7 @@ static int pool_step_begin(wg_pool* p, int count, const int* ids, const double* 
       L.err = p->err;
       L.profile = 0;
       L.mass = launch_mass;
-      L.any_expr = launch_expr;
+      L.force = launch_force;
       L.big_list = nullptr;  // members have no big buckets
       L.big_next = nullptr;
       L.big_count = nullptr;
@@ -1009,7 +1014,7 @@ static int pool_step_begin(wg_pool* p, int count, const int* ids, const double* 
     p->g_nleap = nleap;
     p->g_ntasks = ntasks;
     p->g_small = p->small;
-    p->g_expr = launch_expr;
+    p->g_force = launch_force;
     p->g_mass = launch_mass;
     p->graph_builds++;
   }
@@ -1212,7 +1217,6 @@ static int pool_step_end(wg_pool* p, double* time_elapsed) {
     int64_t nt = 0;
     std::vector<int64_t> upto(batch.size());
     int cps = 1;
-    bool any_expr = false;
     for (size_t j = 0; j < batch.size(); ++j) {
       const int k = batch[j].second;
       PoolSim* s = act[(size_t)k];
@@ -1220,7 +1224,6 @@ static int pool_step_end(wg_pool* p, double* time_elapsed) {
       upto[j] = nt;
       p->h_rlist[j] = k;
       cps = s->tune.ctas_per_sm > cps ? s->tune.ctas_per_sm : cps;
-      any_expr |= s->ext.kind == EXT_EXPR;
     }
     PC(cudaMemcpyAsync(p->rtasks, p->h_rtasks, sizeof(BucketTask) * (size_t)nt,
                        cudaMemcpyHostToDevice, p->stream));
@@ -1244,7 +1247,7 @@ static int pool_step_end(wg_pool* p, double* time_elapsed) {
       L.err = p->err;
       L.profile = 0;
       L.mass = masses_of(act);
-      L.any_expr = any_expr;
+      L.force = forces_of(act);
       L.big_list = nullptr;  // members have no big buckets
       L.big_next = nullptr;
       L.big_count = nullptr;

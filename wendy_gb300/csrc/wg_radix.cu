@@ -694,8 +694,6 @@ struct RadixDevCfg {
   int per_sm[2][4] = {};  // [small tiles][kind]
 };
 
-// The four kinds of pass: whole keys or their upper halves, first or not.
-constexpr int kKinds = 4;
 template <int ITEMS, bool FIRST, bool WIDE>
 constexpr size_t pass_smem() {
   return sizeof(PassSmem<kRadixThreads, ITEMS, typename KeyWord<FIRST || WIDE>::type>);
