@@ -1644,11 +1644,13 @@ int wg_energy(wg_sim* s, double twopiG, double omega2, double* energy, double* m
     set_error("wg_energy needs a simulation, a positive finite twopiG and a finite omega2");
     return WG_ERR_ARG;
   }
-  // the current state in sorted order: the bucket layout (if any) goes back
-  // to the compact sets, which the next wg_step re-sorts and re-buckets
+  // the current state in sorted order: a bucket layout (routed for the next
+  // half drift, so not in the order of the present positions) is copied to the
+  // compact sets, which are free while the sheets live in buckets, and stays
+  // what the next wg_step continues from
   if (s->mode == 1) {
+    WG_CUDA(cudaMemsetAsync(s->ocount, 0, 16, s->stream));
     bucket_to_compact(s, s->lay, s->cslot);
-    s->mode = 0;
   }
   int rc = alloc_call_arrays(s, 1);
   if (rc) return rc;

@@ -79,7 +79,7 @@ class Simulation:
         Same quantities as wendy.energy(x, v, m, twopiG, omega=omega) and
         wendy.momentum(v, m) (wendy/wendy.py:439-491) for the masses m this
         simulation was created with divided by twopiG; returns (energy,
-        momentum).  Leaves the sheets compact: the next step re-sorts once.
+        momentum).
         """
         e, p = ctypes.c_double(0.), ctypes.c_double(0.)
         omega2 = -1. if omega is None else float(omega) ** 2.
