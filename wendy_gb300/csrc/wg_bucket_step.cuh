@@ -285,6 +285,18 @@ __device__ __forceinline__ uint64_t warp_max_u64(uint64_t k) {
   return ((uint64_t)h << 32) | l;
 }
 
+// A position in single precision, truncated, on the integer pipe (a conversion
+// would be one of the four to six FP64 instructions a sheet costs, on the pipe
+// that is nearest to its limit).  Non-decreasing in x; magnitudes below the
+// normal single-precision range become zero, above it its end.
+__device__ __forceinline__ float float_of_pos(double x) {
+  const uint32_t h = (uint32_t)__double2hiint(x), l = (uint32_t)__double2loint(x);
+  const uint32_t a = h & 0x7fffffffu;
+  const uint32_t c = min(a, 0x47efffffu);
+  const uint32_t f = __funnelshift_l(c == a ? l : 0xffffffffu, c, 3) + 0x40000000u;
+  return a < 0x38100000u ? 0.f : __uint_as_float(f | (h & 0x80000000u));
+}
+
 // Cell of a position in the routing table.  Every step (rounding to single
 // precision, subtraction, product with a non-negative scale, truncation,
 // clamping) is non-decreasing, so a splitter in a lower cell than a position
@@ -313,8 +325,8 @@ __device__ __forceinline__ int route_cell(StepSmem& S, const uint64_t* wk, int w
   const int j0 = first ? 1 : 0, j1 = last ? wlen - 1 : wlen;
   float x0 = 0.f, scale = 0.f;
   if (j1 > j0) {
-    x0 = (float)pos_of_key(wk[j0]);
-    const float w = (float)pos_of_key(wk[j1]) - x0;
+    x0 = float_of_pos(pos_of_key(wk[j0]));
+    const float w = float_of_pos(pos_of_key(wk[j1])) - x0;
     if (w > 1e-30f && w < 1e30f) scale = (float)LUTN / w;
   }
   if (j == 0) {
@@ -322,7 +334,7 @@ __device__ __forceinline__ int route_cell(StepSmem& S, const uint64_t* wk, int w
     S.lut_scale = scale;
     return -1;
   }
-  return lut_cell((float)pos_of_key(wk[j]), x0, scale);
+  return lut_cell(float_of_pos(pos_of_key(wk[j])), x0, scale);
 }
 
 // The splitters in this thread's cell (at most 128 in all: a byte holds them).
@@ -950,7 +962,7 @@ __device__ __forceinline__ bool process_bucket(const StepLaunch& L, StepSmem& S,
       }
       const double xd = LAST && dest_dt != 0.0 ? fma(dest_dt, vn, xn) : xn;
       kd[u] = key_of(xd);
-      xf[u] = (float)xd;
+      xf[u] = float_of_pos(xd);
     }
     // routing: the window entry among the table's candidates
 #pragma unroll
