@@ -371,7 +371,7 @@ int make_sim(int64_t n, double totmass, double omega2, const ExtSpec& ext, wg_si
   }
   wg_sim* s = new wg_sim();
   s->n = n;
-  s->n_tiles = (n + kForceTile - 1) / kForceTile;
+  s->n_tiles = force_tiles(n);
   s->totmass = totmass;
   s->omega2 = omega2;
   s->ext_spec = ext;
@@ -729,7 +729,7 @@ int enqueue_step(wg_sim* s, double dt, int nleap, bool want_accel, double dt_las
     a.a_out = (want_accel && i == nleap - 1) ? s->a_sorted : nullptr;
     a.ticket = s->tickets + i;
     a.flag_out = &s->flags[i + 1];
-    launch_force(a, s->n_tiles, s->stream);
+    launch_force(a, s->stream);
   }
   WG_CUDA(cudaGetLastError());
   return WG_OK;
@@ -1040,7 +1040,7 @@ static int compact_continue(wg_sim* s, double dt, int nleap, int from) {
     f.ticket = s->tickets + i;
     f.flag_out = &s->flags[i + 1];
     f.a_out = (i == nleap - 1 && s->call_a) ? s->a_sorted : nullptr;
-    launch_force(f, s->n_tiles, s->stream);
+    launch_force(f, s->stream);
   }
   if (s->call_a) launch_scatter_accel(s->table, s->n, s->a_sorted, s->call_a, s->stream);
   if (s->call_xi) store_sheets(s->table, s->n, reinterpret_cast<wg_sheet*>(s->call_xi), s->stream);
@@ -1528,7 +1528,7 @@ int wg_profile(wg_sim* s, int what, int reps, double* avg_seconds) {
     } else if (what == WG_PROF_FORCE) {
       a.sub = i;
       a.ticket = s->tickets + i;
-      launch_force(a, s->n_tiles, s->stream);
+      launch_force(a, s->stream);
     } else {
       radix_sort_state(s->table, s->n, &s->radix, &s->flags[i], s->err, s->stream);
     }

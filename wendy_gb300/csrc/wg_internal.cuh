@@ -121,21 +121,40 @@ inline void launch_chained(void (*kernel)(P...), unsigned grid, unsigned block, 
   cudaLaunchKernelEx(&c, kernel, P(args)...);
 }
 
+// Sheets per thread of the force kernel: eight where their tiles fill the
+// device, two up to 2^16 sheets, whose launch is a chain of the look-back and
+// one thread's FP64 instructions (20011 sheets 11.6 -> 7.3 us, 65536 sheets
+// 11.3 -> 9.8 us; at 150001 sheets both take 12.7 us, above that two lose).
 constexpr int kForceThreads = 256;
-constexpr int kForceItems = 8;
-constexpr int kForceTile = kForceThreads * kForceItems;
+constexpr int kForceItems = 8, kForceItemsSmall = 2;
+constexpr int64_t kForceSmallSheets = 1 << 16;
+// Tile of a force launch over n sheets, its tiles, and the tile records that
+// launches over up to n sheets need.
+inline int64_t force_tile(int64_t n) {
+  return kForceThreads * (n <= kForceSmallSheets ? kForceItemsSmall : kForceItems);
+}
+inline int64_t force_tiles(int64_t n) { return (n + force_tile(n) - 1) / force_tile(n); }
+inline int64_t force_tiles_room(int64_t n) {
+  const int64_t small = force_tiles(n < kForceSmallSheets ? n : kForceSmallSheets);
+  return force_tiles(n) > small ? force_tiles(n) : small;
+}
 
-constexpr int kRadixThreads = 256;
-// Keys per thread of a pass: tiles of 4096 keys where they fill the device;
-// smaller sorts take tiles of 1024, whose latency (a tile is ranked, staged and
-// written by one CTA) is a third of it.
-constexpr int kRadixItems = 16, kRadixItemsSmall = 4;
+// Tile of a radix pass (it is ranked, staged and written by one CTA): 4096 keys
+// where they fill the device, 256 threads with 16 each (two CTAs per SM); up
+// to one tile per SM 512 threads with eight each, which halves a tile's chain
+// of ranks (a sort of 262145 sheets 75 -> 67 us, of 500000 90 -> 75 us; 700000
+// sheets are more tiles than SMs and take 98 us with either, 1e6 103 us against
+// 111); and up to 2^18 sheets tiles of 1024, whose latency is a third
+// (20011 sheets 48 -> 38 us, 150001 sheets 62 -> 54 us).
+constexpr int kRadixThreads = 256, kRadixThreadsMid = 512;
+constexpr int kRadixItems = 16, kRadixItemsMid = 8, kRadixItemsSmall = 4;
 constexpr int kRadixTile = kRadixThreads * kRadixItems;
+static_assert(kRadixTile == kRadixThreadsMid * kRadixItemsMid, "tiles of one size");
 constexpr int kRadixTileSmall = kRadixThreads * kRadixItemsSmall;
 constexpr int64_t kRadixSmallSheets = 1 << 18;
 
 // --- launchers (wg_kernels.cu) ---
-void launch_force(const ForceArgs& a, int64_t n_tiles, cudaStream_t s);
+void launch_force(const ForceArgs& a, cudaStream_t s);
 // Wait settings of the force kernel's look-back (a test hook behind
 // wg_set_debug_wait): the iteration limit of its waits, and a tile whose
 // look-back record is never published (-1: none), so that the waits on it

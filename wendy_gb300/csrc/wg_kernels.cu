@@ -332,13 +332,15 @@ void set_wait_debug(unsigned spin_limit, int64_t withhold_tile) {
   g_withhold_tile = withhold_tile;
 }
 
-void launch_force(const ForceArgs& a, int64_t n_tiles, cudaStream_t s) {
+void launch_force(const ForceArgs& a, cudaStream_t s) {
   ForceArgs b = a;
   b.spin_limit = g_spin_limit;
   b.withhold_tile = g_withhold_tile;
-  auto* const k = b.ext.kind == EXT_EXPR ? k_force_kick_drift<kForceThreads, kForceItems, true>
-                                         : k_force_kick_drift<kForceThreads, kForceItems, false>;
-  launch_chained(k, (unsigned)n_tiles, kForceThreads, 0, s, b);
+  constexpr int T = kForceThreads, W = kForceItems, N = kForceItemsSmall;
+  const bool expr = b.ext.kind == EXT_EXPR, small = b.n <= kForceSmallSheets;
+  auto* const k = small ? (expr ? k_force_kick_drift<T, N, true> : k_force_kick_drift<T, N, false>)
+                        : (expr ? k_force_kick_drift<T, W, true> : k_force_kick_drift<T, W, false>);
+  launch_chained(k, (unsigned)force_tiles(b.n), T, 0, s, b);
 }
 
 void launch_drift(const StateTable* table, int64_t n, double dt, StepFlags* flag,

@@ -77,7 +77,7 @@ Layout carve(unsigned char* base, int64_t n) {
     L.set[k].idx = reinterpret_cast<int32_t*>(p); p += ni;
   }
   L.a_sorted = reinterpret_cast<double*>(p); p += nd;
-  const int64_t max_tiles = (kMaxSheets + kForceTile - 1) / kForceTile;
+  const int64_t max_tiles = force_tiles_room(kMaxSheets);
   L.recs = reinterpret_cast<TileRec*>(p); p += al(sizeof(TileRec) * (size_t)max_tiles);
   radix_bind(&L.radix, p, n);
   p += radix_bytes(kMaxSheets);
@@ -218,7 +218,7 @@ extern "C" int wg_accel_noalloc(int64_t n, const double* x, const double* m, dou
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (epoch >= (1u << 29)) {
     // keep (epoch << 2) in 32 bits: forget old tile records and restart
-    const int64_t max_tiles = (kMaxSheets + kForceTile - 1) / kForceTile;
+    const int64_t max_tiles = force_tiles_room(kMaxSheets);
     cudaMemsetAsync(L.recs, 0, sizeof(TileRec) * (size_t)max_tiles, s);
     std::lock_guard<std::mutex> lock(g_mu);
     g_epoch[dev] = 2;
@@ -254,7 +254,7 @@ extern "C" int wg_accel_noalloc(int64_t n, const double* x, const double* m, dou
   f.err = L.err;
   f.dt_kick = 0.0;
   f.dt_drift = 0.0;
-  launch_force(f, (n + kForceTile - 1) / kForceTile, s);
+  launch_force(f, s);
   k_noalloc_store<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(L, n, a, perm);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(WG_ERR_CUDA, "wg_accel_noalloc: launch failed: %s",

@@ -372,7 +372,7 @@ int ensure_workspace(wg_pool* p, int64_t n) {
   if (p->ws) cudaFree(p->ws);
   p->ws = nullptr;
   const size_t nd = al((size_t)n * 8), ni = al((size_t)n * 4);
-  const int64_t tiles = (n + kForceTile - 1) / kForceTile;
+  const int64_t tiles = force_tiles_room(n);
   const int64_t nb = n;  // compaction offsets: at most one bucket per sheet
   const size_t b = 2 * (3 * nd + ni) + al(sizeof(TileRec) * (size_t)tiles) + radix_bytes(n) +
                    al(4 * (size_t)nb);
@@ -635,7 +635,7 @@ int finish_compact(wg_pool* p, PoolSim* s, int k, int kk, int lay, int cslot, do
   f.recs = p->trecs;
   f.err = p->err;
   f.a_out = nullptr;
-  const int64_t tiles = (s->n + kForceTile - 1) / kForceTile;
+  const int64_t tiles = force_tiles(s->n);
   PC(cudaMemsetAsync(p->tickets, 0, 4 * (size_t)nleap, p->stream));
   // the tile records are shared by every member finished this way: cleared,
   // so that no tile takes another member's prefix
@@ -648,7 +648,7 @@ int finish_compact(wg_pool* p, PoolSim* s, int k, int kk, int lay, int cslot, do
     f.dt_drift = (i == nleap - 1) ? dt / 2. : dt;
     f.ticket = p->tickets + i;
     f.flag_out = &p->wflags[i + 1];
-    launch_force(f, tiles, p->stream);
+    launch_force(f, p->stream);
   }
   launch_desort(p->table, s->n, s->x_out, s->v_out, p->stream);
   store_compact(p, s);
@@ -844,7 +844,7 @@ static int pool_step_begin(wg_pool* p, int count, const int* ids, const double* 
       if (s) PC(cudaMemsetAsync(s->recs, 0, sizeof(BucketRec) * (size_t)s->nb_room, p->stream));
     if (p->ws)
       PC(cudaMemsetAsync(p->trecs, 0,
-                         sizeof(TileRec) * (size_t)((p->ws_n + kForceTile - 1) / kForceTile),
+                         sizeof(TileRec) * (size_t)force_tiles_room(p->ws_n),
                          p->stream));
     p->epoch = 1;
   }

@@ -88,7 +88,10 @@ struct PassArgs {
 // Digit histograms of bytes first .. 7; the last block to finish turns them
 // into the plan.  The top byte (sign and seven exponent bits) takes a few
 // values only, so its counts are formed per warp, one atomic per value.
-constexpr int kHistThreads = 256;
+// Four positions per thread, their loads in flight together, and as many blocks
+// as that takes: a chain of 16 or more dependent rounds in a few blocks took
+// 16 us at 20011 sheets and 22 us at 150001, of a sort of 48 and 62 us.
+constexpr int kHistThreads = 256, kHistUnroll = 4;
 __global__ void __launch_bounds__(kHistThreads) k_radix_hist(
     const StateTable* table, int64_t n, int first, uint32_t* hist, uint32_t* plan,
     uint32_t* counters, const StepFlags* flag) {
@@ -101,19 +104,29 @@ __global__ void __launch_bounds__(kHistThreads) k_radix_hist(
   __syncthreads();
   const double* x = table->cur.x;
   const int64_t stride = (int64_t)gridDim.x * kHistThreads;
-  for (int64_t i0 = (int64_t)blockIdx.x * kHistThreads + (tid & ~31); i0 < n; i0 += stride) {
-    const bool ok = i0 + lane < n;
-    const uint64_t k = ok ? key_of(x[i0 + lane]) : 0ull;
-    if (ok)
-      for (int p = first; p < 7; ++p) atomicAdd(&sh[p * R + ((k >> (8 * p)) & 255u)], 1u);
-    unsigned todo = __ballot_sync(0xffffffffu, ok);
-    const unsigned top = (unsigned)(k >> 56);
-    while (todo) {
-      const int leader = __ffs(todo) - 1;
-      const unsigned t = __shfl_sync(0xffffffffu, top, leader);
-      const unsigned same = __ballot_sync(0xffffffffu, ok && top == t);
-      if (lane == leader) atomicAdd(&sh[7 * R + t], (uint32_t)__popc(same));
-      todo &= ~same;
+  for (int64_t b0 = (int64_t)blockIdx.x * kHistThreads + (tid & ~31); b0 < n;
+       b0 += kHistUnroll * stride) {
+    double xs[kHistUnroll];
+#pragma unroll
+    for (int u = 0; u < kHistUnroll; ++u)
+      xs[u] = b0 + u * stride + lane < n ? x[b0 + u * stride + lane] : 0.0;
+#pragma unroll
+    for (int u = 0; u < kHistUnroll; ++u) {
+      const int64_t i0 = b0 + u * stride;
+      if (i0 >= n) break;  // (the same for the whole warp)
+      const bool ok = i0 + lane < n;
+      const uint64_t k = key_of(xs[u]);
+      if (ok)
+        for (int p = first; p < 7; ++p) atomicAdd(&sh[p * R + ((k >> (8 * p)) & 255u)], 1u);
+      unsigned todo = __ballot_sync(0xffffffffu, ok);
+      const unsigned top = (unsigned)(k >> 56);
+      while (todo) {
+        const int leader = __ffs(todo) - 1;
+        const unsigned t = __shfl_sync(0xffffffffu, top, leader);
+        const unsigned same = __ballot_sync(0xffffffffu, ok && top == t);
+        if (lane == leader) atomicAdd(&sh[7 * R + t], (uint32_t)__popc(same));
+        todo &= ~same;
+      }
     }
   }
   __syncthreads();
@@ -187,7 +200,7 @@ struct PassSmem {
   uint32_t whist[WARPS][R];
   uint32_t tile_excl[R];
   uint32_t gbase[R];
-  uint32_t tmp[WARPS];
+  uint32_t tmp[R / 32];
   uint64_t mbar[2];
   int64_t tile[2];
   int64_t bad;  // 1 + the tile whose offsets are unknown (a bounded wait expired)
@@ -203,7 +216,7 @@ struct PassSmem {
 // hold a tile and the look-back always progresses: the smallest tile in work
 // has every predecessor finished.
 template <int THREADS, int ITEMS, bool FIRST, bool WIDE>
-__global__ void __launch_bounds__(THREADS, 2) k_radix_pass(const PassArgs a) {
+__global__ void __launch_bounds__(THREADS, 512 / THREADS) k_radix_pass(const PassArgs a) {
   // what a tile is read and staged as (the first pass reads positions and
   // needs the whole key for its digit), and what is written
   using KEY = typename KeyWord<FIRST || WIDE>::type;
@@ -211,7 +224,8 @@ __global__ void __launch_bounds__(THREADS, 2) k_radix_pass(const PassArgs a) {
   using Smem = PassSmem<THREADS, ITEMS, KEY>;
   constexpr int TILE = Smem::TILE;
   constexpr int WARPS = Smem::WARPS;
-  static_assert(THREADS == R, "one thread per digit");
+  constexpr int DW = R / 32;  // warps with a digit per thread
+  static_assert(THREADS % R == 0, "a thread per digit");
   extern __shared__ __align__(128) unsigned char smem_raw[];
   Smem& S = *reinterpret_cast<Smem*>(smem_raw);
 
@@ -328,33 +342,37 @@ __global__ void __launch_bounds__(THREADS, 2) k_radix_pass(const PassArgs a) {
     // Column of digit `tid`: exclusive offsets of the warps, tile count;
     // the count is published at once for the tiles behind this one.
     const int d = tid;
-    uint32_t count = 0;
+    uint32_t count = 0, incl = 0, tex = 0;
+    if (warp < DW) {
 #pragma unroll
-    for (int w = 0; w < WARPS; ++w) {
-      const uint32_t c = S.whist[w][d];
-      S.whist[w][d] = count;
-      count += c;
-    }
-    if (S.bad == tile + 1)
-      st_relaxed_u32(&stat[tile * R + d], kStatX);
-    else if (tile == 0)
-      st_relaxed_u32(&stat[d], kStatP | count);
-    else
-      st_relaxed_u32(&stat[tile * R + d], kStatA | count);
-    // Exclusive scan of the tile's counts over digits.
-    uint32_t incl = count;
+      for (int w = 0; w < WARPS; ++w) {
+        const uint32_t c = S.whist[w][d];
+        S.whist[w][d] = count;
+        count += c;
+      }
+      if (S.bad == tile + 1)
+        st_relaxed_u32(&stat[tile * R + d], kStatX);
+      else if (tile == 0)
+        st_relaxed_u32(&stat[d], kStatP | count);
+      else
+        st_relaxed_u32(&stat[tile * R + d], kStatA | count);
+      // Exclusive scan of the tile's counts over digits.
+      incl = count;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += y;
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      if (lane == 31) S.tmp[warp] = incl;
     }
-    if (lane == 31) S.tmp[warp] = incl;
     __syncthreads();
-    uint32_t wpre = 0;
+    if (warp < DW) {
+      uint32_t wpre = 0;
 #pragma unroll
-    for (int w = 0; w < WARPS; ++w) wpre += (w < warp) ? S.tmp[w] : 0u;
-    const uint32_t tex = wpre + incl - count;
-    S.tile_excl[d] = tex;
+      for (int w = 0; w < DW; ++w) wpre += (w < warp) ? S.tmp[w] : 0u;
+      tex = wpre + incl - count;
+      S.tile_excl[d] = tex;
+    }
     __syncthreads();
     // Stage the tile in digit order (over the buffer it arrived in); this
     // needs only the tile's own offsets, and gives the tiles ahead time to
@@ -374,7 +392,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_radix_pass(const PassArgs a) {
     // predecessors are read per round, their loads in flight together, and
     // summed in order up to the nearest inclusive one.
     uint32_t excl = 0;
-    if (tile != 0 && S.bad != tile + 1) {
+    if (warp < DW && tile != 0 && S.bad != tile + 1) {
       constexpr int LB = 8;
       int64_t j = tile - 1;
       unsigned spins = 0;
@@ -423,7 +441,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_radix_pass(const PassArgs a) {
         st_relaxed_u32(&stat[tile * R + d], kStatP | (excl + count));
       }
     }
-    S.gbase[d] = a.plan[kPlanStarts + pass * R + d] + excl - tex;
+    if (warp < DW) S.gbase[d] = a.plan[kPlanStarts + pass * R + d] + excl - tex;
     // claim the next tile once this one's offsets are known (claim order
     // then follows processing order) and start its copy into the other buffer
     if (tid == 0) {
@@ -689,45 +707,56 @@ size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 // Launch configuration of the radix passes on one device: its SM count and
 // the resident pass CTAs per SM, after raising the pass kernels' dynamic
 // shared-memory limits on that device.  Set up once per device (thread-safe).
+enum { kTilesSmall = 0, kTilesMid = 1, kTilesLarge = 2 };
 struct RadixDevCfg {
   int sms = 1;
-  int per_sm[2][4] = {};  // [small tiles][kind]
+  int per_sm[3][4] = {};  // [tiles][whole keys: 2 | not the first pass: 1]
 };
 
-template <int ITEMS, bool FIRST, bool WIDE>
+template <int THREADS, int ITEMS, bool FIRST, bool WIDE>
 constexpr size_t pass_smem() {
-  return sizeof(PassSmem<kRadixThreads, ITEMS, typename KeyWord<FIRST || WIDE>::type>);
+  return sizeof(PassSmem<THREADS, ITEMS, typename KeyWord<FIRST || WIDE>::type>);
 }
-template <int ITEMS, bool FIRST, bool WIDE>
+template <int THREADS, int ITEMS, bool FIRST, bool WIDE>
 void pass_init(int& per_sm) {
-  constexpr size_t dyn = pass_smem<ITEMS, FIRST, WIDE>();
-  auto* k = k_radix_pass<kRadixThreads, ITEMS, FIRST, WIDE>;
+  constexpr size_t dyn = pass_smem<THREADS, ITEMS, FIRST, WIDE>();
+  auto* k = k_radix_pass<THREADS, ITEMS, FIRST, WIDE>;
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
   int c = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, k, kRadixThreads, dyn);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, k, THREADS, dyn);
   per_sm = c < 1 ? 1 : c;
 }
-template <int ITEMS, bool FIRST, bool WIDE>
+template <int THREADS, int ITEMS, bool FIRST, bool WIDE>
 void pass_launch(const PassArgs& a, int per_sm, int sms, cudaStream_t s) {
   int64_t pg = (int64_t)per_sm * sms;
   if (pg > a.n_tiles) pg = a.n_tiles;
   if (pg < 1) pg = 1;
-  launch_chained(k_radix_pass<kRadixThreads, ITEMS, FIRST, WIDE>, (unsigned)pg, kRadixThreads,
-                 pass_smem<ITEMS, FIRST, WIDE>(), s, a);
+  launch_chained(k_radix_pass<THREADS, ITEMS, FIRST, WIDE>, (unsigned)pg, THREADS,
+                 pass_smem<THREADS, ITEMS, FIRST, WIDE>(), s, a);
+}
+
+template <int THREADS, int ITEMS>
+void pass_init_all(int* per_sm) {
+  pass_init<THREADS, ITEMS, true, false>(per_sm[0]);
+  pass_init<THREADS, ITEMS, false, false>(per_sm[1]);
+  pass_init<THREADS, ITEMS, true, true>(per_sm[2]);
+  pass_init<THREADS, ITEMS, false, true>(per_sm[3]);
+}
+template <int THREADS, int ITEMS>
+void pass_launch_kind(const PassArgs& a, int kind, const int* per_sm, int sms, cudaStream_t s) {
+  if (kind == 0) pass_launch<THREADS, ITEMS, true, false>(a, per_sm[0], sms, s);
+  if (kind == 1) pass_launch<THREADS, ITEMS, false, false>(a, per_sm[1], sms, s);
+  if (kind == 2) pass_launch<THREADS, ITEMS, true, true>(a, per_sm[2], sms, s);
+  if (kind == 3) pass_launch<THREADS, ITEMS, false, true>(a, per_sm[3], sms, s);
 }
 
 void radix_cfg_init(RadixDevCfg& c, int dev) {
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   c.sms = sms < 1 ? 1 : sms;
-  pass_init<kRadixItems, true, false>(c.per_sm[0][0]);
-  pass_init<kRadixItems, false, false>(c.per_sm[0][1]);
-  pass_init<kRadixItems, true, true>(c.per_sm[0][2]);
-  pass_init<kRadixItems, false, true>(c.per_sm[0][3]);
-  pass_init<kRadixItemsSmall, true, false>(c.per_sm[1][0]);
-  pass_init<kRadixItemsSmall, false, false>(c.per_sm[1][1]);
-  pass_init<kRadixItemsSmall, true, true>(c.per_sm[1][2]);
-  pass_init<kRadixItemsSmall, false, true>(c.per_sm[1][3]);
+  pass_init_all<kRadixThreadsMid, kRadixItemsMid>(c.per_sm[kTilesMid]);
+  pass_init_all<kRadixThreads, kRadixItems>(c.per_sm[kTilesLarge]);
+  pass_init_all<kRadixThreads, kRadixItemsSmall>(c.per_sm[kTilesSmall]);
 }
 
 RadixDevCfg radix_cfg() {
@@ -787,8 +816,8 @@ void radix_sort_state(StateTable* table, int64_t n, RadixWork* w, const StepFlag
   // look-back words and launches follow n
   const int64_t tiles = tiles_of(n);
   cudaMemsetAsync(w->hist, 0, (8 * R + kCounters + (size_t)(8 - first) * tiles * R) * 4, s);
-  int64_t hist_grid = (n + 16 * kHistThreads - 1) / (16 * kHistThreads);
-  if (hist_grid < 8) hist_grid = n < 8 * kHistThreads ? (n + kHistThreads - 1) / kHistThreads : 8;
+  constexpr int64_t kHistKeys = kHistUnroll * kHistThreads;
+  int64_t hist_grid = (n + kHistKeys - 1) / kHistKeys;
   if (hist_grid > sms * 4) hist_grid = sms * 4;
   launch_chained(k_radix_hist, (unsigned)hist_grid, kHistThreads, 0, s, table, n, first, w->hist,
                  w->plan, w->counters, flag);
@@ -806,22 +835,17 @@ void radix_sort_state(StateTable* table, int64_t n, RadixWork* w, const StepFlag
   a.counters = w->counters;
   a.flag = flag;
   a.err = err;
-  const bool small = n <= kRadixSmallSheets;
-  const int* per_sm = cfg.per_sm[small ? 1 : 0];
+  const int kt = n <= kRadixSmallSheets ? kTilesSmall : tiles <= sms ? kTilesMid : kTilesLarge;
+  const int* per_sm = cfg.per_sm[kt];
   for (int p = first; p < 8; ++p) {
     a.pass = p;
     const int kind = (whole_keys ? 2 : 0) + (p == first ? 0 : 1);
-    if (small) {
-      if (kind == 0) pass_launch<kRadixItemsSmall, true, false>(a, per_sm[0], sms, s);
-      if (kind == 1) pass_launch<kRadixItemsSmall, false, false>(a, per_sm[1], sms, s);
-      if (kind == 2) pass_launch<kRadixItemsSmall, true, true>(a, per_sm[2], sms, s);
-      if (kind == 3) pass_launch<kRadixItemsSmall, false, true>(a, per_sm[3], sms, s);
-    } else {
-      if (kind == 0) pass_launch<kRadixItems, true, false>(a, per_sm[0], sms, s);
-      if (kind == 1) pass_launch<kRadixItems, false, false>(a, per_sm[1], sms, s);
-      if (kind == 2) pass_launch<kRadixItems, true, true>(a, per_sm[2], sms, s);
-      if (kind == 3) pass_launch<kRadixItems, false, true>(a, per_sm[3], sms, s);
-    }
+    if (kt == kTilesSmall)
+      pass_launch_kind<kRadixThreads, kRadixItemsSmall>(a, kind, per_sm, sms, s);
+    else if (kt == kTilesMid)
+      pass_launch_kind<kRadixThreadsMid, kRadixItemsMid>(a, kind, per_sm, sms, s);
+    else
+      pass_launch_kind<kRadixThreads, kRadixItems>(a, kind, per_sm, sms, s);
   }
   int64_t gg = (n + kGatherThreads * kGatherUnroll - 1) / (kGatherThreads * kGatherUnroll);
   if (gg > (int64_t)sms * 8) gg = (int64_t)sms * 8;
