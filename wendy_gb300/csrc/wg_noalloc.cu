@@ -131,6 +131,7 @@ __global__ void k_noalloc_setup(Layout L, double t, unsigned epoch) {
 
 // Copy the caller's positions and masses into the first set, checking them.
 __global__ void k_noalloc_load(Layout L, int64_t n, const double* x, const double* m) {
+  chain_begin();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   bool bad = false;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -149,6 +150,7 @@ __global__ void k_noalloc_load(Layout L, int64_t n, const double* x, const doubl
 }
 
 __global__ void k_noalloc_store(Layout L, int64_t n, double* a, int32_t* perm) {
+  chain_begin();
   const StateRef cur = L.table->cur;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -233,7 +235,7 @@ extern "C" int wg_accel_noalloc(int64_t n, const double* x, const double* m, dou
   const u128 T = fixed_of(totmass, E);
 
   k_noalloc_setup<<<1, 32, 0, s>>>(L, t, epoch);
-  k_noalloc_load<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(L, n, x, m);
+  launch_chained(k_noalloc_load, (unsigned)((n + 255) / 256), 256, 0, s, L, n, x, m);
   radix_sort_state(L.table, n, &L.radix, &L.flags[0], L.err, s);
   ForceArgs f;
   f.table = L.table;
@@ -255,7 +257,7 @@ extern "C" int wg_accel_noalloc(int64_t n, const double* x, const double* m, dou
   f.dt_kick = 0.0;
   f.dt_drift = 0.0;
   launch_force(f, s);
-  k_noalloc_store<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(L, n, a, perm);
+  launch_chained(k_noalloc_store, (unsigned)((n + 255) / 256), 256, 0, s, L, n, a, perm);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(WG_ERR_CUDA, "wg_accel_noalloc: launch failed: %s",
                                     cudaGetErrorString(e));
