@@ -13,7 +13,7 @@ Tolerances, fixed beforehand:
     1e-13 a sub-step, dt and the number of sub-steps keep its growth below 10);
   * accelerations 1e-12 of the acceleration scale, orders exact;
   * powers by products: half an ulp and a few 2^-53 of it, against a library
-    power within one ulp: 2 x 2^-52 relative.
+    power within one ulp: 2 x 2^-52 relative; quotients: the same bits.
 """
 import ctypes
 import threading
@@ -181,7 +181,7 @@ def test_force_evaluation_at_the_limits_of_its_tiles(n):
     assert numpy.max(numpy.abs(got - ref)) <= 1e-12 * scale
 
 
-@pytest.mark.parametrize("k", ["2", "3", "4", "7", "8", "9", "-3", "2.5"])
+@pytest.mark.parametrize("k", ["2", "3", "4", "7", "8", "9", "-3", "2.5", "3.5", "16"])
 def test_powers_of_an_expression(k):
     rng = numpy.random.default_rng(5)
     x = numpy.concatenate([rng.normal(0., 3., 1001), 10. ** rng.uniform(-300., 300., 1000),
@@ -199,6 +199,26 @@ def test_powers_of_an_expression(k):
         assert numpy.array_equal(numpy.signbit(got[fin | low]), numpy.signbit(ref[fin | low]))
         rest = ~(fin | low)
         assert numpy.array_equal(got[rest], ref[rest], equal_nan=True)
+
+
+@pytest.mark.parametrize("t", [1., -3., 0.1, 1e-150, 2. ** -501, 2. ** -500, 1.9999 * 2. ** 499,
+                               2. ** 500, 1e-300, 5e-324, 1e308, 0., -0.])
+def test_quotients_of_an_expression(t):
+    # the same bits as the division: dividends and divisors over the whole
+    # range, at the limits of the shorter form, and mantissas of few and many ones
+    rng = numpy.random.default_rng(6)
+    e = numpy.concatenate([rng.integers(-1074, 1024, 4000), rng.integers(-30, 30, 4000),
+                           rng.integers(-503, -497, 500), rng.integers(497, 503, 500)])
+    f = rng.choice([1., 1.5, 2. - 2. ** -52, 1. + 2. ** -52, 1. + 2. ** -23], len(e))
+    f[::2] = rng.uniform(1., 2., len(f[::2]))
+    x = numpy.concatenate([numpy.ldexp(f * rng.choice([-1., 1.], len(e)), e),
+                           [0., -0., numpy.inf, -numpy.inf, numpy.nan, t]])
+    with numpy.errstate(all="ignore"):
+        for prog, ref in (("x/t", x / t), ("t/x", t / x)):
+            got = evaluate_on_device(Expression(prog), x, t)
+            assert numpy.array_equal(got, ref, equal_nan=True)
+            num = ~numpy.isnan(ref)
+            assert numpy.array_equal(numpy.signbit(got[num]), numpy.signbit(ref[num]))
 
 
 def test_simulations_of_several_threads_share_no_memory():
