@@ -154,10 +154,11 @@ def test_ensemble_launch_variants(force, masses):
 
 # one sheet on either side of the force tiles (512 sheets, up to 2^16; 2048
 # above), of the sort's tiles (1024 keys up to 2^18 sheets; 4096 above, with 512
-# threads up to one tile per SM of 152) and of its leading bytes (four up to 2^17)
+# threads up to one tile per SM of 152) and of its leading bytes (four up to 2^17,
+# five up to 2^22, six above)
 @pytest.mark.parametrize("n", [511, 512, 513, 1024, 1025, 65535, 65536, 65537, 1 << 17,
                                (1 << 17) + 1, 1 << 18, (1 << 18) + 1, 152 * 4096,
-                               152 * 4096 + 1])
+                               152 * 4096 + 1, 1 << 22, (1 << 22) + 1])
 def test_force_evaluation_at_the_limits_of_its_tiles(n):
     # a third of the positions shares its leading bytes: runs of pairs, of equal
     # positions and of positions a few units in the last place apart
@@ -179,6 +180,17 @@ def test_force_evaluation_at_the_limits_of_its_tiles(n):
     ref[order] = (tot - 2. * cum + ms).astype(numpy.float64) - 1.21 * x[order]
     scale = max(tot, float(numpy.max(numpy.abs(ref))))
     assert numpy.max(numpy.abs(got - ref)) <= 1e-12 * scale
+
+
+@pytest.mark.parametrize("n", [70001, 300001, (1 << 22) + 3])
+@pytest.mark.parametrize("step", [0.25, 0.25 + 2. ** -16, 0.25 + 2. ** -29])
+def test_sort_of_positions_whose_bytes_are_partly_constant(n, step):
+    # digits that are the same for every key are skipped, but not the pass that
+    # halves the keys
+    rng = numpy.random.default_rng(n)
+    x = 4. + step * rng.integers(0, 8, n)
+    got, perm = wendy_gb300.accel(x, numpy.full(n, 1. / n), 1.)
+    assert numpy.array_equal(perm, numpy.argsort(x, kind="stable"))
 
 
 @pytest.mark.parametrize("k", ["2", "3", "4", "7", "8", "9", "-3", "2.5", "3.5", "16"])

@@ -152,6 +152,13 @@ constexpr int kRadixTile = kRadixThreads * kRadixItems;
 static_assert(kRadixTile == kRadixThreadsMid * kRadixItemsMid, "tiles of one size");
 constexpr int kRadixTileSmall = kRadixThreads * kRadixItemsSmall;
 constexpr int64_t kRadixSmallSheets = 1 << 18;
+// Leading bytes a sort goes by: four up to 2^17 sheets, five up to 2^22, six
+// above.  Fewer passes against more ties, each ordered by one thread: sheets
+// spread evenly take 437 us by five bytes and 476 by six at 2^22, 2.2 and
+// 2.3 ms at 2^24; with half of them in a core of width 2e-3 523 against 478 us
+// and 2.8 against 2.3 ms; with all of them in two cores, the narrower of width 1e-4,
+// 1.26 against 0.50 ms and 34.5 against 2.6 ms.
+constexpr int64_t kRadixFourSheets = 1 << 17, kRadixFiveSheets = 1 << 22;
 
 // --- launchers (wg_kernels.cu) ---
 void launch_force(const ForceArgs& a, cudaStream_t s);

@@ -9,9 +9,10 @@
 // Positions of N sheets are told apart by about log2 N bits, not by 64: the
 // leading five bytes of a key (sign, exponent, 28 bits of the mantissa) leave
 // one pair in a hundred together at 1e6 sheets, four bytes one in thirty at
-// 65536.  A pass costs a launch and about 10 us at least, and what the
-// following passes need fits in 32 bits once the first one is done, so five
-// passes move 80 bytes per sheet where eight of 64-bit keys moved 190.
+// 65536; above 2^22 sheets, whose crowded states would leave runs of many, six
+// bytes are sorted by.  A pass costs a launch and about 10 us at least, and what
+// the passes after byte 3 need fits in 32 bits, so five passes move 80 bytes
+// per sheet, six 104, where eight of 64-bit keys moved 190.
 // A sort of 20011 sheets with its force evaluation 205 -> 126 us, of 2^21 in a
 // diagnostics call 560 -> 350 us.
 //
@@ -23,9 +24,9 @@
 //          (bit-plane ballots + per-warp shared-memory counters, stable),
 //          publish the tile's digit counts, stage in digit order, look back
 //          for the tile's global digit offsets, write out
-//   gather permute x, v, m, idx into the other state set; notes whether any
-//          sheet precedes its predecessor in (key, index)
-//   ties   (only then) runs of equal leading bytes are ordered by key and
+//   gather permute x, v, m, idx into the other state set; notes in small sorts
+//          whether any sheet precedes its predecessor in (key, index)
+//   ties   (unless none does) runs of equal leading bytes are ordered by key and
 //          original index: short runs in place, long runs by one CTA each,
 //          whose last block makes the other set the current one
 //
@@ -38,6 +39,7 @@
 #include <cstdint>
 #include <functional>
 #include <mutex>
+#include <type_traits>
 
 #include "wg_internal.cuh"
 
@@ -62,7 +64,7 @@ constexpr int kPlanWords = kPlanStarts + 8 * R;
 
 // counters (uint32 words, cleared before each sort)
 constexpr int kCntClaim = 0;   // [8] next tile of each pass
-constexpr int kCntTie = 8;     // some sheet out of (key, index) order after the gather
+constexpr int kCntTie = 8;     // some sheet may be out of (key, index) order
 constexpr int kCntRuns = 9;    // long runs listed
 constexpr int kCntHist = 10;   // histogram blocks done
 constexpr int kCntLong = 11;   // k_radix_long_ties blocks done
@@ -86,14 +88,13 @@ struct PassArgs {
 };
 
 // Digit histograms of bytes first .. 7; the last block to finish turns them
-// into the plan.  The top byte (sign and seven exponent bits) takes a few
-// values only, so its counts are formed per warp, one atomic per value.
+// into the plan.  halve: the pass that halves the keys, which is never skipped.
 // Four positions per thread, their loads in flight together, and as many blocks
 // as that takes: a chain of 16 or more dependent rounds in a few blocks took
 // 16 us at 20011 sheets and 22 us at 150001, of a sort of 48 and 62 us.
 constexpr int kHistThreads = 256, kHistUnroll = 4;
 __global__ void __launch_bounds__(kHistThreads) k_radix_hist(
-    const StateTable* table, int64_t n, int first, uint32_t* hist, uint32_t* plan,
+    const StateTable* table, int64_t n, int first, int halve, uint32_t* hist, uint32_t* plan,
     uint32_t* counters, const StepFlags* flag) {
   chain_begin();
   if (!flag->unsorted) return;
@@ -116,16 +117,10 @@ __global__ void __launch_bounds__(kHistThreads) k_radix_hist(
       if (i0 >= n) break;  // (the same for the whole warp)
       const bool ok = i0 + lane < n;
       const uint64_t k = key_of(xs[u]);
-      if (ok)
-        for (int p = first; p < 7; ++p) atomicAdd(&sh[p * R + ((k >> (8 * p)) & 255u)], 1u);
-      unsigned todo = __ballot_sync(0xffffffffu, ok);
-      const unsigned top = (unsigned)(k >> 56);
-      while (todo) {
-        const int leader = __ffs(todo) - 1;
-        const unsigned t = __shfl_sync(0xffffffffu, top, leader);
-        const unsigned same = __ballot_sync(0xffffffffu, ok && top == t);
-        if (lane == leader) atomicAdd(&sh[7 * R + t], (uint32_t)__popc(same));
-        todo &= ~same;
+      if (ok) {
+#pragma unroll
+        for (int p = 0; p < 8; ++p)
+          if (p >= first) atomicAdd(&sh[p * R + ((k >> (8 * p)) & 255u)], 1u);
       }
     }
   }
@@ -170,7 +165,7 @@ __global__ void __launch_bounds__(kHistThreads) k_radix_hist(
     plan[kPlanSrc + first] = 0;
     plan[kPlanDst + first] = 0;
     for (int p = first + 1; p < 8; ++p) {
-      const int act = !sh[p];
+      const int act = !sh[p] || p == halve;
       plan[kPlanActive + p] = act;
       plan[kPlanSrc + p] = cur;
       plan[kPlanDst + p] = act ? 1 - cur : cur;
@@ -182,12 +177,14 @@ __global__ void __launch_bounds__(kHistThreads) k_radix_hist(
 constexpr int kHistWarps = kHistThreads / 32;
 static_assert(kHistWarps == 8, "one warp per byte, one thread per digit");
 
-template <bool WIDE>
+// What a pass reads and writes: the first one reads positions (double); whole
+// keys or their upper halves after that.
+template <typename IN>
 struct KeyWord {
-  typedef uint32_t type;  // the upper half of the key
+  typedef IN type;
 };
 template <>
-struct KeyWord<true> {
+struct KeyWord<double> {
   typedef uint64_t type;
 };
 
@@ -215,12 +212,12 @@ struct PassSmem {
 // staging time to finish.  Claims are dynamic, so only running CTAs ever
 // hold a tile and the look-back always progresses: the smallest tile in work
 // has every predecessor finished.
-template <int THREADS, int ITEMS, bool FIRST, bool WIDE>
+template <int THREADS, int ITEMS, typename IN, typename OUT>
 __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_radix_pass(const PassArgs a) {
-  // what a tile is read and staged as (the first pass reads positions and
-  // needs the whole key for its digit), and what is written
-  using KEY = typename KeyWord<FIRST || WIDE>::type;
-  using OUT = typename KeyWord<WIDE>::type;
+  // what a tile is read and staged as
+  using KEY = typename KeyWord<IN>::type;
+  constexpr bool FIRST = std::is_same<IN, double>::value;
+  constexpr bool HALVE = sizeof(KEY) > sizeof(OUT);
   using Smem = PassSmem<THREADS, ITEMS, KEY>;
   constexpr int TILE = Smem::TILE;
   constexpr int WARPS = Smem::WARPS;
@@ -236,9 +233,9 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_radix_pass(const Pas
   const int pass = a.pass;
   if (!a.plan[kPlanActive + pass]) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int shift = 8 * (FIRST || WIDE ? pass : pass - 4);
+  const int shift = 8 * (sizeof(KEY) == 8 ? pass : pass - 4);
   const int srcb = (int)a.plan[kPlanSrc + pass], dstb = (int)a.plan[kPlanDst + pass];
-  const OUT* ksrc = static_cast<const OUT*>(srcb ? a.keys1 : a.keys0);
+  const KEY* ksrc = static_cast<const KEY*>(srcb ? a.keys1 : a.keys0);
   const uint32_t* psrc = srcb ? a.pos1 : a.pos0;
   OUT* kdst = static_cast<OUT*>(dstb ? a.keys1 : a.keys0);
   uint32_t* pdst = dstb ? a.pos1 : a.pos0;
@@ -464,7 +461,7 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_radix_pass(const Pas
         const KEY kk = S.keys[b][p];
         const unsigned dd = (unsigned)((kk >> shift) & 255u);
         const int64_t o = (int64_t)S.gbase[dd] + p;
-        kdst[o] = FIRST && !WIDE ? (OUT)((uint64_t)kk >> 32) : (OUT)kk;
+        kdst[o] = HALVE ? (OUT)((uint64_t)kk >> 32) : (OUT)kk;
         pdst[o] = S.vals[b][p];
       }
     }
@@ -473,12 +470,19 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_radix_pass(const Pas
 }
 
 // Permute x, v, m, idx into the other set; GU sheets per thread with their
-// loads in flight together (the reads are random when the input was).
-constexpr int kGatherThreads = 256, kGatherUnroll = 4;
+// loads in flight together.  The reads are random when the input was (a slab
+// whose streams interpenetrate), and bound by the sectors in flight: beyond L2
+// sixteen sheets per thread (at 2^26 four take 3.2 ms, eight 2.8, sixteen 2.7); up
+// to 2^22 sheets four, which leave enough blocks.  NOTE: notes whether any sheet precedes its
+// predecessor in (key, index), which spares small sorts the next kernel's work;
+// in large ones some sheet nearly always does, and the looking costs a fifth
+// (2^26: 3.75 ms with it, 3.2 without).
+constexpr int kGatherThreads = 256;
+constexpr int64_t kGatherWideSheets = 1 << 22;
+template <int GU, bool NOTE>
 __global__ void __launch_bounds__(kGatherThreads) k_radix_gather(
     StateTable* table, int64_t n, const uint32_t* pos0, const uint32_t* pos1,
     const uint32_t* plan, uint32_t* counters, const StepFlags* flag, const unsigned* err) {
-  constexpr int GU = kGatherUnroll;
   chain_begin();
   // nothing after a pass that gave up on a wait: its slots are incomplete
   if (!flag->unsorted || (*err & DEV_ERR_RADIX_TIMEOUT)) return;
@@ -487,47 +491,58 @@ __global__ void __launch_bounds__(kGatherThreads) k_radix_gather(
   const StateRef cur = table->cur, oth = table->other;
   const int lane = threadIdx.x & 31;
   const int64_t chunk = (int64_t)gridDim.x * kGatherThreads * GU;
-  bool tie = false;
+  bool tie = !NOTE && blockIdx.x == 0;
   for (int64_t b0 = (int64_t)blockIdx.x * kGatherThreads * GU; b0 < n; b0 += chunk) {
     const int64_t p0 = b0 + threadIdx.x;
-    uint32_t q[GU], qn[GU];
+    uint32_t q[GU], qn[NOTE ? GU : 1];
 #pragma unroll
     for (int u = 0; u < GU; ++u) {
       const int64_t p = p0 + (int64_t)u * kGatherThreads;
       q[u] = p < n ? __ldcs(pos + p) : 0u;
-      qn[u] = lane == 31 && p + 1 < n ? __ldg(pos + p + 1) : 0u;
+      if (NOTE) qn[u] = lane == 31 && p + 1 < n ? __ldg(pos + p + 1) : 0u;
     }
-    double xs[GU], vs[GU], ms[GU], xn[GU];
-    int32_t is[GU], in[GU];
+    double xs[GU], vs[GU], ms[GU], xn[NOTE ? GU : 1];
+    int32_t is[GU], in[NOTE ? GU : 1];
 #pragma unroll
     for (int u = 0; u < GU; ++u) {
       const int64_t p = p0 + (int64_t)u * kGatherThreads;
-      xs[u] = xn[u] = 0.0;
-      is[u] = in[u] = 0;
+      if (NOTE) xs[u] = 0.0, is[u] = 0;
       if (p < n) {
         xs[u] = __ldg(cur.x + q[u]);
         vs[u] = __ldg(cur.v + q[u]);
         ms[u] = __ldg(cur.m + q[u]);
         is[u] = __ldg(cur.idx + q[u]);
       }
-      if (lane == 31 && p + 1 < n) {  // the first sheet of the next warp
-        xn[u] = __ldg(cur.x + qn[u]);
-        in[u] = __ldg(cur.idx + qn[u]);
+      if (NOTE) {
+        xn[u] = 0.0;
+        in[u] = 0;
+        if (lane == 31 && p + 1 < n) {  // the first sheet of the next warp
+          xn[u] = __ldg(cur.x + qn[u]);
+          in[u] = __ldg(cur.idx + qn[u]);
+        }
       }
     }
 #pragma unroll
     for (int u = 0; u < GU; ++u) {
       const int64_t p = p0 + (int64_t)u * kGatherThreads;
-      const double xd = __shfl_down_sync(0xffffffffu, xs[u], 1);
-      const int32_t id = __shfl_down_sync(0xffffffffu, is[u], 1);
+      double xd = 0.0;
+      int32_t id = 0;
+      if (NOTE) {
+        xd = __shfl_down_sync(0xffffffffu, xs[u], 1);
+        id = __shfl_down_sync(0xffffffffu, is[u], 1);
+        if (lane == 31) {
+          xd = xn[u];
+          id = in[u];
+        }
+      }
       if (p < n) {
         oth.x[p] = xs[u];
         oth.v[p] = vs[u];
         oth.m[p] = ms[u];
         oth.idx[p] = is[u];
-        if (p + 1 < n) {
-          const uint64_t k = key_of(xs[u]), kn = key_of(lane < 31 ? xd : xn[u]);
-          tie |= kn < k || (kn == k && (lane < 31 ? id : in[u]) < is[u]);
+        if (NOTE && p + 1 < n) {
+          const uint64_t k = key_of(xs[u]), kn = key_of(xd);
+          tie |= kn < k || (kn == k && id < is[u]);
         }
       }
     }
@@ -540,32 +555,35 @@ __global__ void __launch_bounds__(kGatherThreads) k_radix_gather(
 // search over the sorted leading bytes; runs of up to kShortRun sheets are
 // insertion-sorted in place, longer ones are listed (start in list_start,
 // length in list_len, count in counters[kCntRuns]) for k_radix_long_ties, so
-// no thread ever does work quadratic in a run.  Threads read the leading bytes
-// of sheets that the run's first thread may be moving: moves stay inside a
-// run, whose leading bytes are all the same, and both sides use relaxed
+// no thread ever does work quadratic in a run.  A warp reads four groups of 32
+// keys at a time, and a pair in order is passed over on these, before anything
+// of its run has moved: one group at a time, each pair's sheets loaded again, took
+// 0.44 ms at 2^26 and more than twice that at 2^27; so 0.25 ms.  Threads read the
+// leading bytes of sheets that a run's first thread may be moving: moves stay
+// inside a run, whose leading bytes are all the same, and both sides use relaxed
 // accesses.
 constexpr int64_t kShortRun = 32;
+constexpr int kTieUnroll = 4;
 __global__ void k_radix_ties(StateTable* table, int64_t n, int low_bits, uint32_t* counters,
                              uint32_t* list_start, uint32_t* list_len, const StepFlags* flag,
                              const unsigned* err) {
   chain_begin();
   if (!flag->unsorted || !counters[kCntTie] || (*err & DEV_ERR_RADIX_TIMEOUT)) return;
   const StateRef oth = table->other;
-  auto lead = [&](int64_t p) { return key_of(ld_relaxed_f64(oth.x + p)) >> low_bits; };
+  auto whole = [&](int64_t p) { return key_of(ld_relaxed_f64(oth.x + p)); };
+  auto lead = [&](int64_t p) { return whole(p) >> low_bits; };
   const int lane = threadIdx.x & 31;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t w0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); w0 < n;
-       w0 += stride) {
-    const int64_t p = w0 + lane;
-    const uint64_t kp = p < n ? lead(p) : 0ull;
-    uint64_t kn = __shfl_down_sync(0xffffffffu, kp, 1);
-    uint64_t kb = __shfl_up_sync(0xffffffffu, kp, 1);
-    if (lane == 31 && p + 1 < n) kn = lead(p + 1);
-    if (lane == 0 && p > 0) kb = lead(p - 1);
-    if (p + 1 >= n || kp != kn || (p > 0 && kb == kp)) continue;
+  // the run that starts at sheet p, whose first keys are k0, k1 (and k2, except
+  // in the last two lanes)
+  auto order_run = [&](int64_t p, uint64_t k0, uint64_t k1, uint64_t k2) {
+    const uint64_t kp = k0 >> low_bits;
+    // nearly every run is a pair, and most of those are in order already
+    if (lane >= 30 && p + 2 < n) k2 = whole(p + 2);
+    const bool pair = p + 2 >= n || k2 >> low_bits != kp;
+    if (pair && k0 < k1) return;
     // last index e with the same leading bytes
-    int64_t lo = p + 1, hi = n - 1;
-    if (hi > p + 1 && lead(p + 2) != kp) hi = p + 1;  // nearly every run is a pair
+    int64_t lo = p + 1, hi = pair ? p + 1 : n - 1;
     while (lo < hi) {
       const int64_t mid = lo + (hi - lo + 1) / 2;
       if (lead(mid) == kp) lo = mid; else hi = mid - 1;
@@ -575,7 +593,7 @@ __global__ void k_radix_ties(StateTable* table, int64_t n, int low_bits, uint32_
       const unsigned slot = atomicAdd(&counters[kCntRuns], 1u);
       list_start[slot] = (uint32_t)p;
       list_len[slot] = (uint32_t)(e - p + 1);
-      continue;
+      return;
     }
     for (int64_t i = p + 1; i <= e; ++i) {
       const double xi = ld_relaxed_f64(oth.x + i), vi = oth.v[i], mi = oth.m[i];
@@ -598,6 +616,31 @@ __global__ void k_radix_ties(StateTable* table, int64_t n, int low_bits, uint32_
         oth.m[j + 1] = mi;
         oth.idx[j + 1] = ii;
       }
+    }
+  };
+  for (int64_t w0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31); w0 < n;
+       w0 += kTieUnroll * stride) {
+    // keys of kTieUnroll groups of 32 sheets and of their neighbours
+    uint64_t ks[kTieUnroll], ke[kTieUnroll];
+#pragma unroll
+    for (int u = 0; u < kTieUnroll; ++u) {
+      const int64_t p = w0 + u * stride + lane;
+      const int64_t pe = lane == 31 ? p + 1 : p - 1;
+      ks[u] = p < n ? whole(p) : 0ull;
+      ke[u] = (lane == 31 || lane == 0) && pe >= 0 && pe < n ? whole(pe) : 0ull;
+    }
+#pragma unroll
+    for (int u = 0; u < kTieUnroll; ++u) {
+      const int64_t p = w0 + u * stride + lane;
+      const uint64_t k0 = ks[u], kp = k0 >> low_bits;
+      uint64_t k1 = __shfl_down_sync(0xffffffffu, k0, 1);
+      const uint64_t k2 = __shfl_down_sync(0xffffffffu, k0, 2);
+      uint64_t kb = __shfl_up_sync(0xffffffffu, k0, 1);
+      if (lane == 31) k1 = ke[u];
+      if (lane == 0) kb = ke[u];
+      if (p + 1 < n && kp == k1 >> low_bits && (p == 0 || kb >> low_bits != kp))
+        order_run(p, k0, k1, k2);
+      __syncwarp();
     }
   }
 }
@@ -708,46 +751,50 @@ size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 // the resident pass CTAs per SM, after raising the pass kernels' dynamic
 // shared-memory limits on that device.  Set up once per device (thread-safe).
 enum { kTilesSmall = 0, kTilesMid = 1, kTilesLarge = 2 };
+enum { kPosHalf = 0, kPosWhole = 1, kWhole = 2, kWholeHalf = 3, kHalf = 4 };
 struct RadixDevCfg {
   int sms = 1;
-  int per_sm[3][4] = {};  // [tiles][whole keys: 2 | not the first pass: 1]
+  int per_sm[3][5] = {};  // [tiles][what the pass reads and writes]
 };
 
-template <int THREADS, int ITEMS, bool FIRST, bool WIDE>
+template <int THREADS, int ITEMS, typename IN, typename OUT>
 constexpr size_t pass_smem() {
-  return sizeof(PassSmem<THREADS, ITEMS, typename KeyWord<FIRST || WIDE>::type>);
+  return sizeof(PassSmem<THREADS, ITEMS, typename KeyWord<IN>::type>);
 }
-template <int THREADS, int ITEMS, bool FIRST, bool WIDE>
+template <int THREADS, int ITEMS, typename IN, typename OUT>
 void pass_init(int& per_sm) {
-  constexpr size_t dyn = pass_smem<THREADS, ITEMS, FIRST, WIDE>();
-  auto* k = k_radix_pass<THREADS, ITEMS, FIRST, WIDE>;
+  constexpr size_t dyn = pass_smem<THREADS, ITEMS, IN, OUT>();
+  auto* k = k_radix_pass<THREADS, ITEMS, IN, OUT>;
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
   int c = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, k, THREADS, dyn);
   per_sm = c < 1 ? 1 : c;
 }
-template <int THREADS, int ITEMS, bool FIRST, bool WIDE>
+template <int THREADS, int ITEMS, typename IN, typename OUT>
 void pass_launch(const PassArgs& a, int per_sm, int sms, cudaStream_t s) {
   int64_t pg = (int64_t)per_sm * sms;
   if (pg > a.n_tiles) pg = a.n_tiles;
   if (pg < 1) pg = 1;
-  launch_chained(k_radix_pass<THREADS, ITEMS, FIRST, WIDE>, (unsigned)pg, THREADS,
-                 pass_smem<THREADS, ITEMS, FIRST, WIDE>(), s, a);
+  launch_chained(k_radix_pass<THREADS, ITEMS, IN, OUT>, (unsigned)pg, THREADS,
+                 pass_smem<THREADS, ITEMS, IN, OUT>(), s, a);
 }
 
 template <int THREADS, int ITEMS>
 void pass_init_all(int* per_sm) {
-  pass_init<THREADS, ITEMS, true, false>(per_sm[0]);
-  pass_init<THREADS, ITEMS, false, false>(per_sm[1]);
-  pass_init<THREADS, ITEMS, true, true>(per_sm[2]);
-  pass_init<THREADS, ITEMS, false, true>(per_sm[3]);
+  pass_init<THREADS, ITEMS, double, uint32_t>(per_sm[kPosHalf]);
+  pass_init<THREADS, ITEMS, double, uint64_t>(per_sm[kPosWhole]);
+  pass_init<THREADS, ITEMS, uint64_t, uint64_t>(per_sm[kWhole]);
+  pass_init<THREADS, ITEMS, uint64_t, uint32_t>(per_sm[kWholeHalf]);
+  pass_init<THREADS, ITEMS, uint32_t, uint32_t>(per_sm[kHalf]);
 }
 template <int THREADS, int ITEMS>
 void pass_launch_kind(const PassArgs& a, int kind, const int* per_sm, int sms, cudaStream_t s) {
-  if (kind == 0) pass_launch<THREADS, ITEMS, true, false>(a, per_sm[0], sms, s);
-  if (kind == 1) pass_launch<THREADS, ITEMS, false, false>(a, per_sm[1], sms, s);
-  if (kind == 2) pass_launch<THREADS, ITEMS, true, true>(a, per_sm[2], sms, s);
-  if (kind == 3) pass_launch<THREADS, ITEMS, false, true>(a, per_sm[3], sms, s);
+  const int c = per_sm[kind];
+  if (kind == kPosHalf) pass_launch<THREADS, ITEMS, double, uint32_t>(a, c, sms, s);
+  if (kind == kPosWhole) pass_launch<THREADS, ITEMS, double, uint64_t>(a, c, sms, s);
+  if (kind == kWhole) pass_launch<THREADS, ITEMS, uint64_t, uint64_t>(a, c, sms, s);
+  if (kind == kWholeHalf) pass_launch<THREADS, ITEMS, uint64_t, uint32_t>(a, c, sms, s);
+  if (kind == kHalf) pass_launch<THREADS, ITEMS, uint32_t, uint32_t>(a, c, sms, s);
 }
 
 void radix_cfg_init(RadixDevCfg& c, int dev) {
@@ -809,9 +856,8 @@ void radix_sort_state(StateTable* table, int64_t n, RadixWork* w, const StepFlag
                       unsigned* err, cudaStream_t s, bool whole_keys) {
   const RadixDevCfg cfg = radix_cfg();
   const int sms = cfg.sms;
-  // bytes sorted by: five tell the positions of any number of sheets apart
-  // well enough, four those of up to 2^17 (see the top of this file)
-  const int first = whole_keys ? 0 : n <= (1 << 17) ? 4 : 3;
+  // the least significant byte sorted by (kRadixFourSheets, kRadixFiveSheets)
+  const int first = whole_keys ? 0 : n <= kRadixFourSheets ? 4 : n <= kRadixFiveSheets ? 3 : 2;
   // the workspace may be bound for more sheets than this sort has: tiles,
   // look-back words and launches follow n
   const int64_t tiles = tiles_of(n);
@@ -819,7 +865,8 @@ void radix_sort_state(StateTable* table, int64_t n, RadixWork* w, const StepFlag
   constexpr int64_t kHistKeys = kHistUnroll * kHistThreads;
   int64_t hist_grid = (n + kHistKeys - 1) / kHistKeys;
   if (hist_grid > sms * 4) hist_grid = sms * 4;
-  launch_chained(k_radix_hist, (unsigned)hist_grid, kHistThreads, 0, s, table, n, first, w->hist,
+  launch_chained(k_radix_hist, (unsigned)hist_grid, kHistThreads, 0, s, table, n, first,
+                 !whole_keys && first < 3 ? 3 : first, w->hist,
                  w->plan, w->counters, flag);
   PassArgs a;
   a.table = table;
@@ -839,7 +886,11 @@ void radix_sort_state(StateTable* table, int64_t n, RadixWork* w, const StepFlag
   const int* per_sm = cfg.per_sm[kt];
   for (int p = first; p < 8; ++p) {
     a.pass = p;
-    const int kind = (whole_keys ? 2 : 0) + (p == first ? 0 : 1);
+    // the upper halves of the keys are enough once the bytes left lie in them
+    const bool half = !whole_keys && p >= 3;
+    const int kind = p == first               ? (half ? kPosHalf : kPosWhole)
+                     : whole_keys || p <= 3 ? (half ? kWholeHalf : kWhole)
+                                              : kHalf;
     if (kt == kTilesSmall)
       pass_launch_kind<kRadixThreads, kRadixItemsSmall>(a, kind, per_sm, sms, s);
     else if (kt == kTilesMid)
@@ -847,10 +898,12 @@ void radix_sort_state(StateTable* table, int64_t n, RadixWork* w, const StepFlag
     else
       pass_launch_kind<kRadixThreads, kRadixItems>(a, kind, per_sm, sms, s);
   }
-  int64_t gg = (n + kGatherThreads * kGatherUnroll - 1) / (kGatherThreads * kGatherUnroll);
+  const bool wide = n > kGatherWideSheets;
+  const int64_t per = kGatherThreads * (wide ? 16 : 4);
+  int64_t gg = (n + per - 1) / per;
   if (gg > (int64_t)sms * 8) gg = (int64_t)sms * 8;
   if (gg < 1) gg = 1;
-  launch_chained(k_radix_gather, (unsigned)gg, kGatherThreads, 0, s, table, n, w->pos[0], w->pos[1],
+  launch_chained(wide ? k_radix_gather<16, false> : k_radix_gather<4, true>, (unsigned)gg, kGatherThreads, 0, s, table, n, w->pos[0], w->pos[1],
                  w->plan, w->counters, flag, err);
   int64_t g = (n + 255) / 256;
   if (g > (int64_t)sms * 16) g = (int64_t)sms * 16;
