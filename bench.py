@@ -241,9 +241,9 @@ HBM_FALLBACK_GBS = 6800.0
 # dram__bytes_read.sum + dram__bytes_write.sum of one k_bucket_step launch
 # from an ncu capture of a smaller case of the same family, per sheet
 TRAFFIC_PER_SHEET = {
-    "sech2": ((237.496576e6 + 185.93152e6) / (1 << 23),
+    "sech2": (434.158e6 / (1 << 23),
               "ncu capture of one sub-step of the sech2 disk at N = 2^23"),
-    "tophat": ((237.603328e6 + 187.855872e6) / (1 << 23),
+    "tophat": (363.018e6 / (1 << 23),
                "ncu capture of one sub-step of the cold top-hat with the pulsed force at "
                "N = 2^23"),
 }
@@ -586,12 +586,15 @@ def main():
         return out.value
     f_s = prof(0, 10)   # fused force kernel on compact sets (initial call, fallback)
     s_s = prof(1, 3)    # full radix re-sort (initial sort, fallback)
+    # histogram 8 B, passes (16 B each by halves of keys, 40 B for the two of six
+    # that go by whole ones), gather 60 B
+    sort_b = 8 + (64 if n <= 1 << 17 else 80 if n <= 1 << 22 else 104) + 60
     comps = {"k_bucket_step": {"ms": sub_s * 1e3, "algorithmic_bytes_per_sheet": 56,
                                "achieved_gbs": bucket_gbs, "share_of_timed_region": 1.0},
              "k_force_kick_drift": {"ms": f_s * 1e3, "algorithmic_bytes_per_sheet": 40,
                                     "achieved_gbs": 40.0 * n / f_s / 1e9},
-             "radix_resort": {"ms": s_s * 1e3, "algorithmic_bytes_per_sheet": 250,
-                              "achieved_gbs": 250.0 * n / s_s / 1e9}}
+             "radix_resort": {"ms": s_s * 1e3, "algorithmic_bytes_per_sheet": sort_b,
+                              "achieved_gbs": sort_b * n / s_s / 1e9}}
     traffic_per_sheet, traffic_src = TRAFFIC_PER_SHEET.get(
         w["family"], TRAFFIC_PER_SHEET["sech2"])
     traffic = traffic_per_sheet * n

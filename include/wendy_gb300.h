@@ -153,9 +153,10 @@ int wg_profile(wg_sim *s, int what, int reps, double *avg_seconds);
 
 /* Tuning of the fused bucket sub-step by simulation size.  Row i applies to
    simulations of n >= n_min[i] sheets (rows ascending in n_min) created after
-   the call: sheets per bucket after a re-sort (64..1024), splitter window
-   (1..64 buckets each side), counting-sort bits (8..12), persistent CTAs per
-   SM (1..2).  Written by the autotuner (wendy_gb300/autotune.py); no
+   the call: sheets per bucket after a re-sort (64..1536; a simulation with
+   few buckets takes smaller ones), splitter window (1..64 buckets each side),
+   counting-sort bits (9..13, of which the kernel uses 11 or 12), persistent
+   CTAs per SM (1, or 2 for as many as fit).  Written by the autotuner (wendy_gb300/autotune.py); no
    reference counterpart. */
 typedef struct wg_tuning {
   int64_t n_min;

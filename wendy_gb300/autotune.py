@@ -5,10 +5,11 @@ number of sheets of a simulation (how many buckets there are to keep the SMs
 busy, how far sheets travel in bucket units, how clustered the keys inside a
 bucket are):
 
-  target       sheets per bucket right after a re-sort (capacity 2048, at most 1536)
+  target       sheets per bucket right after a re-sort (capacity 2048, at most 1536;
+               launches with few buckets take smaller ones)
   window       splitters searched in shared memory on each side of a bucket
   sort_bits    2^sort_bits bins of the in-bucket counting sort
-  ctas_per_sm  persistent CTAs per SM
+  ctas_per_sm  persistent CTAs per SM: 1, or 2 for as many as fit
 
 :func:`tune` times candidate settings by coordinate descent from the
 defaults, for a few simulation sizes n.  Each timing advances a pool of
