@@ -114,6 +114,28 @@ def test_equal_masses_give_the_bits_of_the_general_form(n):
     assert numpy.array_equal(got[0], gen[0][:n]) and numpy.array_equal(got[1], gen[1][:n])
 
 
+def test_equal_masses_through_overflowing_buckets():
+    # a slab falling through its centre in a few sub-steps: layouts overflow, are
+    # compacted and laid out again
+    n = 1 << 18
+    rng = numpy.random.default_rng(9)
+    x = rng.uniform(-1., 1., n)
+    v = -60. * x + 0.3 * rng.normal(size=n)
+    m = numpy.full(n, 1. / n)
+    got = _alone(x, v, m, None, None, 0.002, 8, nout=3, totmass=1.)
+    tracer = (numpy.append(x, 1e3), numpy.append(v, 0.), numpy.append(m, 0.))
+    gen = _alone(*tracer, None, None, 0.002, 8, nout=3, totmass=1.)
+    assert numpy.array_equal(got[0], gen[0][:n]) and numpy.array_equal(got[1], gen[1][:n])
+    other = ics.sech2_disk(3000, seed=1, masses="lognormal")
+    for mem in ([(x, v, m, None, None)], [(x, v, m, None, None), (*other, None, None)]):
+        assert _same(got, _members(mem, 0.002, 8, nout=3)[0])
+    sim = wendy_gb300.Simulation(x, v, m, 1., -1.)
+    sim.step(0.002, 8, ctypes.c_double(4.))
+    st = sim.stats()
+    sim.close()
+    assert st["sorts_full"] > 1  # it did overflow
+
+
 @pytest.mark.parametrize("n", [900, 40001])
 def test_stateless_calls_whose_masses_change(n):
     # equal masses for two calls, unequal ones in the third, equal in the fourth

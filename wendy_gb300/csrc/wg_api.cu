@@ -740,7 +740,8 @@ int enqueue_step(wg_sim* s, double dt, int nleap, bool want_accel, double dt_las
 void bucket_to_compact(wg_sim* s, int lay, int cslot) {
   launch_compact(s->table, s->nb, s->capg, s->bx[lay], s->bv[lay], s->bm[lay], s->bi[lay],
                  s->bcnt[cslot],
-                 s->offs, s->ox, s->ov, s->om, s->oi, s->ocount, s->n, s->stream);
+                 s->offs, s->ox, s->ov, s->om, s->oi, s->ocount, s->n,
+                 EqMass{s->eq, s->d_diff ? s->d_diff + 1 : nullptr, s->meq}, s->stream);
   s->st.launches += 2;
 }
 

@@ -72,8 +72,9 @@ __global__ void k_compact(StateTable* table, int64_t nb, int capg, const double*
                           const double* m, const int32_t* idx, const unsigned* cnt,
                           const unsigned* offs, const double* ox, const double* ov,
                           const double* om, const int32_t* oi, const unsigned* ocount,
-                          int64_t n) {
+                          int64_t n, EqMass em) {
   const StateRef st = table->cur;
+  const bool eq = em.all_equal();
   for (int64_t b = blockIdx.x; b < nb; b += gridDim.x) {
     const unsigned c = cnt[b] < (unsigned)capg ? cnt[b] : (unsigned)capg;
     const int64_t o = offs[b];
@@ -81,7 +82,7 @@ __global__ void k_compact(StateTable* table, int64_t nb, int capg, const double*
       const int64_t s = b * capg + j;
       st.x[o + j] = x[s];
       st.v[o + j] = v[s];
-      st.m[o + j] = m[s];
+      st.m[o + j] = eq ? em.m : m[s];
       st.idx[o + j] = idx[s];
     }
   }
@@ -369,7 +370,7 @@ __global__ void k_batch_compact(const SimDev* devs, const BatchSeg* segs, const 
          j += blockDim.x) {
       dst.x[o + j] = x[base + j];
       dst.v[o + j] = v[base + j];
-      dst.m[o + j] = m[base + j];
+      dst.m[o + j] = d.eq == kEqYes ? d.meq : m[base + j];
       dst.idx[o + j] = idx[base + j];
     }
   } else {
@@ -471,12 +472,12 @@ void launch_bucketize(const StateTable* table, int64_t n, int target, int64_t nb
 void launch_compact(StateTable* table, int64_t nb, int capg, const double* x, const double* v,
                     const double* m, const int32_t* idx, const unsigned* cnt, unsigned* offs,
                     const double* ox, const double* ov, const double* om, const int32_t* oi,
-                    const unsigned* ocount, int64_t n, cudaStream_t s) {
+                    const unsigned* ocount, int64_t n, EqMass em, cudaStream_t s) {
   k_count_offsets<<<1, 1024, 0, s>>>(cnt, nb, capg, offs);
   int64_t g = nb < 152 * 8 ? nb : 152 * 8;
   if (g < 1) g = 1;
   k_compact<<<(unsigned)g, 256, 0, s>>>(table, nb, capg, x, v, m, idx, cnt, offs, ox, ov, om,
-                                         oi, ocount, n);
+                                         oi, ocount, n, em);
 }
 
 }  // namespace wg

@@ -115,7 +115,7 @@ struct SimDev {
   // Simulations whose masses are all the same (kEqYes, or kEqWord where a
   // device word says so, zero meaning yes): the mass of a set of sheets is
   // then their number times meq, and the kernel neither reads masses nor sums
-  // them.
+  // them, nor writes them to the next layout.
   int eq;
   const unsigned* eq_word;
   double meq;            // the mass, and in fixed point
@@ -137,6 +137,14 @@ struct SimDev {
 };
 
 enum : int { kEqNo = 0, kEqYes = 1, kEqWord = 2 };
+// The masses of a layout's sheets, as SimDev has them: where they are equal the
+// layout's mass slots are not written.
+struct EqMass {
+  int eq;
+  const unsigned* eq_word;
+  double m;
+  __device__ bool all_equal() const { return eq == kEqYes || (eq == kEqWord && *eq_word == 0u); }
+};
 // The external forces of a launch's simulations: none, closed forms, or
 // expressions among them.
 enum : int { kForceNone = 0, kForceClosed = 1, kForceExpr = 2 };
@@ -256,6 +264,6 @@ void launch_bucketize(const StateTable* table, int64_t n, int target, int64_t nb
 void launch_compact(StateTable* table, int64_t nb, int capg, const double* x, const double* v,
                     const double* m, const int32_t* idx, const unsigned* cnt, unsigned* offs,
                     const double* ox, const double* ov, const double* om, const int32_t* oi,
-                    const unsigned* ocount, int64_t n, cudaStream_t s);
+                    const unsigned* ocount, int64_t n, EqMass em, cudaStream_t s);
 
 }  // namespace wg

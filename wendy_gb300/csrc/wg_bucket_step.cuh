@@ -1134,7 +1134,7 @@ __device__ __forceinline__ bool process_bucket(const StepLaunch& L, StepSmem& S,
         const int64_t o = (int64_t)d * capg + slot;
         xout[o] = xn;
         vout[o] = vn;
-        mout[o] = mn;
+        if (!eq) mout[o] = mn;  // (equal masses are read from D.meq everywhere)
         iout[o] = in;
       } else {
         const uint32_t o = atomicAdd(D.ocount, 1u);

@@ -595,7 +595,8 @@ void buckets_to_workspace(wg_pool* p, PoolSim* s, int lay, int cslot, const unsi
   k_set_table<<<1, 1, 0, p->stream>>>(p->table, p->set[0], p->set[1]);
   launch_compact(p->table, s->nb, s->capg, s->bx[lay], s->bv[lay], s->bm[lay], s->bi[lay],
                  s->bcnt[cslot],
-                 p->offs, s->ox, s->ov, s->om, s->oi, oc, s->n, p->stream);
+                 p->offs, s->ox, s->ov, s->om, s->oi, oc, s->n,
+                 EqMass{s->eq ? kEqYes : kEqNo, nullptr, s->meq}, p->stream);
   p->launches += 3;
 }
 
