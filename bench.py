@@ -243,7 +243,7 @@ HBM_FALLBACK_GBS = 6800.0
 TRAFFIC_PER_SHEET = {
     "sech2": (434.158e6 / (1 << 23),
               "ncu capture of one sub-step of the sech2 disk at N = 2^23"),
-    "tophat": (363.018e6 / (1 << 23),
+    "tophat": (299.887e6 / (1 << 23),
                "ncu capture of one sub-step of the cold top-hat with the pulsed force at "
                "N = 2^23"),
 }
