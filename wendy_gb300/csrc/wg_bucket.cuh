@@ -9,19 +9,17 @@
 #include <cstdint>
 
 #include "wg_internal.cuh"
+#include "wg_layout.h"
 
 namespace wg {
 
 constexpr int kBucketThreads = 256;
-constexpr int kBucketCap = 2048;      // sheets a bucket's shared-memory pass can hold
 constexpr int kBucketCapBig = 3 * kBucketCap;  // sheets a bucket of a single simulation
                                                // can hold (taken in chunks above kBucketCap)
 constexpr int kSplitterWindow = 64;   // largest splitter window (buckets on each side)
 constexpr int kMemberSampleCap = 4096; // most splitter samples a pool member sorts in one CTA
 constexpr int kSortBitsMin = 9;       // smallest counting-sort offset (bits)
 constexpr int kSortBitsMax = 13;      // largest counting-sort offset (bits)
-constexpr int kMaxTarget = kBucketCap * 3 / 4;  // largest bucket target
-constexpr int kMinTarget = 384;  // smallest target that launches with few buckets are cut to
 
 // Tunables of the fused sub-step, chosen per simulation size by the
 // autotuner (wendy_gb300/autotune.py) or left at their defaults.

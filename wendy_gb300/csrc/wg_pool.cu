@@ -121,7 +121,7 @@ struct PoolSim {
 constexpr int kPredMemberCalls = 16;
 
 // Buckets a member's per-bucket arrays have room for: the tuned number, or for
-// smaller members what smaller buckets (member_target) would make of them.
+// smaller members what smaller buckets (member_layout) would make of them.
 int64_t bucket_room(int64_t n, int64_t nb_tuned) {
   int64_t r = (n + kMinTarget - 1) / kMinTarget;
   if (r > 1024) r = 1024;
@@ -533,20 +533,17 @@ int grid_1d(int64_t n) {
   return (int)(g < 1 ? 1 : g);
 }
 
-// Buckets of `target` sheets for a member that is to be laid out anew: as many
-// slots each as the layouts hold.
-void set_target(PoolSim* s, int target) {
-  s->target = target;
-  s->nb = (s->n + target - 1) / target;
-  const int64_t slots = s->nb_tuned * kBucketCap / s->nb & ~(int64_t)3;
-  s->capg = slots < kBucketCap ? (int)slots : kBucketCap;
+void set_layout(PoolSim* s, const MemberLayout& l) {
+  s->target = l.target;
+  s->nb = l.nb;
+  s->capg = l.capg;
 }
 
 // Targets of the members of a step that are about to be laid out (their sheets
 // are compact): the tuned ones, unless the step's buckets would leave resident
 // CTAs idle, as for single simulations (balanced_target).  Then all members
-// take buckets of the size that fills the launch, down to kMinTarget sheets
-// (a bucket keeps the share of spare slots of the tuned ones, a third).
+// take buckets of about the size that fills the launch, down to kMinTarget sheets,
+// as far as their slots allow (member_layout).
 // Measured per output of 20 sub-steps (5): 4 members of 500 .. 20000 sheets 418 us
 // (175) against 733 (254) with tuned buckets in the kernel before it, 64 of
 // 1000 .. 20000 1240 (580) against 1420 (625).
@@ -562,9 +559,8 @@ void balance_targets(wg_pool* p, const std::vector<PoolSim*>& act) {
   if (t < kMinTarget) t = kMinTarget;
   for (PoolSim* s : act) {
     if (s->mode != 0) continue;
-    int target = s->tune.target;
-    if (buckets < grid && t < target && (s->n + t - 1) / t <= s->nb_room) target = (int)t;
-    if (target != s->target) set_target(s, target);
+    set_layout(s, member_layout(s->n, s->tune.target, s->nb_tuned, s->nb_room,
+                                buckets < grid ? t : s->tune.target));
   }
 }
 
@@ -727,7 +723,7 @@ int wg_pool_add(wg_pool* p, int64_t n, const double* x, const double* v, const d
   s->tune = tuning_for(n);
   s->nb_tuned = (n + s->tune.target - 1) / s->tune.target;
   s->nb_room = bucket_room(n, s->nb_tuned);
-  set_target(s, s->tune.target);
+  set_layout(s, layout_for(n, s->nb_tuned, s->tune.target));
   s->bytes = bytes;
   cudaError_t e = cudaMallocAsync(&s->mem, bytes, p->stream);
   if (e != cudaSuccess) {
