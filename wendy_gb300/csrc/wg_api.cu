@@ -108,6 +108,7 @@ struct wg_sim {
   int64_t n_tiles = 0;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  int stream_dev = -1;       // their device
   void* big = nullptr;       // per-sheet arrays
   void* small = nullptr;     // tables, flags, per-call parameters
   size_t bytes = 0;
@@ -334,6 +335,7 @@ void free_sim(wg_sim* s) {
   set.stream = s->stream;
   set.ev0 = s->ev0;
   set.ev1 = s->ev1;
+  set.dev = s->stream_dev;
   stream_set_give(set);
   delete s;
 }
@@ -397,6 +399,7 @@ int make_sim(int64_t n, double totmass, double omega2, const ExtSpec& ext, wg_si
     s->stream = set.stream;
     s->ev0 = set.ev0;
     s->ev1 = set.ev1;
+    s->stream_dev = set.dev;
     if (es != cudaSuccess) {
       cudaGetLastError();
       set_error("stream/event creation failed: %s", cudaGetErrorString(es));

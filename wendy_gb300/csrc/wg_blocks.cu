@@ -1,11 +1,11 @@
-// wg_blocks.cu -- see wg_blocks.cuh.
+// wg_blocks.cu -- see wg_blocks.cuh.  Host code only: it compiles without the rest
+// of the library, against any implementation of the runtime calls it makes.
 #include <list>
 #include <mutex>
 #include <unordered_map>
 #include <vector>
 
 #include "wg_blocks.cuh"
-#include "wg_internal.cuh"
 
 namespace wg {
 
@@ -22,12 +22,21 @@ struct Kept {
   std::unordered_map<void*, Block> out;  // handed out
   std::list<Block> idle;                 // kept, oldest first
   size_t idle_device = 0, idle_host = 0;
-  std::vector<std::pair<int, StreamSet>> sets;  // (device, set)
+  std::vector<StreamSet> sets;
 };
 
 Kept& kept() {
   static Kept* k = new Kept();  // outlives every user of the library
   return *k;
+}
+
+int device_now() {
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return -1;
+  }
+  return dev;
 }
 
 void release(const Block& b) {
@@ -112,7 +121,7 @@ bool give(void* p) {
 }  // namespace
 
 cudaError_t block_alloc(void** p, size_t bytes) {
-  const int dev = current_device();
+  const int dev = device_now();
   if (dev < 0) return cudaErrorNoDevice;
   return alloc(dev, p, bytes);
 }
@@ -123,16 +132,17 @@ bool host_block_free(void* p) { return give(p); }
 
 cudaError_t stream_set_take(StreamSet* s) {
   Kept& k = kept();
-  const int dev = current_device();
+  const int dev = device_now();
   {
     std::lock_guard<std::mutex> lock(k.mu);
-    for (size_t i = 0; i < k.sets.size(); ++i)
-      if (k.sets[i].first == dev) {
-        *s = k.sets[i].second;
-        k.sets.erase(k.sets.begin() + (long)i);
+    for (auto it = k.sets.begin(); it != k.sets.end(); ++it)
+      if (it->dev == dev) {
+        *s = *it;
+        k.sets.erase(it);
         return cudaSuccess;
       }
   }
+  s->dev = dev;
   cudaError_t e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreate(&s->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&s->ev1);
@@ -140,11 +150,11 @@ cudaError_t stream_set_take(StreamSet* s) {
 }
 
 void stream_set_give(const StreamSet& s) {
-  if (s.stream && s.ev0 && s.ev1) {
+  if (s.stream && s.ev0 && s.ev1 && s.dev >= 0) {
     Kept& k = kept();
     std::lock_guard<std::mutex> lock(k.mu);
     if (k.sets.size() < (size_t)kKeepSets) {
-      k.sets.emplace_back(current_device(), s);
+      k.sets.push_back(s);
       return;
     }
   }
@@ -156,7 +166,7 @@ void stream_set_give(const StreamSet& s) {
 void blocks_trim() {
   Kept& k = kept();
   std::list<Block> idle;
-  std::vector<std::pair<int, StreamSet>> sets;
+  std::vector<StreamSet> sets;
   {
     std::lock_guard<std::mutex> lock(k.mu);
     idle.swap(k.idle);
@@ -164,10 +174,10 @@ void blocks_trim() {
     k.idle_device = k.idle_host = 0;
   }
   for (const Block& b : idle) release(b);
-  for (const auto& p : sets) {
-    cudaEventDestroy(p.second.ev0);
-    cudaEventDestroy(p.second.ev1);
-    cudaStreamDestroy(p.second.stream);
+  for (const StreamSet& s : sets) {
+    cudaEventDestroy(s.ev0);
+    cudaEventDestroy(s.ev1);
+    cudaStreamDestroy(s.stream);
   }
 }
 

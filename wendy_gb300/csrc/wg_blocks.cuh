@@ -39,10 +39,12 @@ cudaError_t host_block_alloc(T** p, size_t bytes) {
   return host_block_alloc(reinterpret_cast<void**>(p), bytes);
 }
 
-// A non-blocking stream and two timing events of the current device.
+// A non-blocking stream and two timing events, of the device that is current
+// when they are taken (they may be given back from any other).
 struct StreamSet {
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  int dev = -1;
 };
 cudaError_t stream_set_take(StreamSet* s);
 void stream_set_give(const StreamSet& s);

@@ -541,6 +541,7 @@ struct wg_exact {
   ExactArgs args{};
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  int stream_dev = -1;  // their device
   size_t smem = 0;
   int* h_ret = nullptr;  // page-locked: cindx, err, ncoll (as two ints), next (as two ints)
 };
@@ -556,6 +557,7 @@ void free_exact(wg_exact* e) {
   set.stream = e->stream;
   set.ev0 = e->ev0;
   set.ev1 = e->ev1;
+  set.dev = e->stream_dev;
   stream_set_give(set);
   delete e;
 }
@@ -623,6 +625,7 @@ int wg_exact_create(int64_t n, const double* x, const double* v, const double* a
   e->stream = set.stream;
   e->ev0 = set.ev0;
   e->ev1 = set.ev1;
+  e->stream_dev = set.dev;
   if (es != cudaSuccess || host_block_alloc(&e->h_ret, 64) != cudaSuccess) {
     cudaGetLastError();
     free_exact(e);
