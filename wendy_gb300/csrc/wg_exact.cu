@@ -38,10 +38,12 @@
 // reference's C is), so trajectories agree to rounding; pair times that are NaN
 // (pairs that never meet in the harmonic case) never come first, and among
 // equal pair times the lowest pair index comes first.
+#include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "../../include/wendy_gb300.h"
@@ -564,6 +566,41 @@ void free_exact(wg_exact* e) {
 
 size_t al(size_t b) { return (b + 255) & ~(size_t)255; }
 
+// Dynamic shared memory an event loop may ask for on the current device (0: the
+// limit could not be raised).  The limit belongs to the kernel, not to a handle:
+// raised once to all that a block can have, so that simulations of different sizes
+// can be alive at once.
+size_t raise_smem_limit() {
+  int dev = 0, optin = 0;
+  cudaFuncAttributes fa[2];
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) !=
+          cudaSuccess ||
+      cudaFuncGetAttributes(&fa[0], k_exact_step<true>) != cudaSuccess ||
+      cudaFuncGetAttributes(&fa[1], k_exact_step<false>) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  const size_t fixed = std::max(fa[0].sharedSizeBytes, fa[1].sharedSizeBytes);
+  const size_t most = (size_t)optin > fixed ? (size_t)optin - fixed : 0;
+  if (cudaFuncSetAttribute(k_exact_step<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)most) != cudaSuccess ||
+      cudaFuncSetAttribute(k_exact_step<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)most) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return most;
+}
+size_t smem_limit() {
+  static std::once_flag once[kMaxDevices];
+  static size_t limit[kMaxDevices];
+  const int dev = current_device();
+  if (dev < 0 || dev >= kMaxDevices) return raise_smem_limit();
+  std::call_once(once[dev], [&] { limit[dev] = raise_smem_limit(); });
+  return limit[dev];
+}
+
 }  // namespace
 
 extern "C" {
@@ -668,11 +705,7 @@ int wg_exact_create(int64_t n, const double* x, const double* v, const double* a
   // the lowest level's indices (the last part of the tree) stay outside
   A.idx0_global = fits && e->smem + kExactStatic > (size_t)optin;
   if (A.idx0_global) e->smem -= 4 * (size_t)A.level_n[1];
-  if (!fits ||
-      cudaFuncSetAttribute(A.omega > 0 ? k_exact_step<true> : k_exact_step<false>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)e->smem) != cudaSuccess) {
-    cudaGetLastError();
+  if (!fits || e->smem > smem_limit()) {
     free_exact(e);
     return fail(WG_ERR_ARG, "exact solver: %lld sheets need more shared memory for the pair-time "
                             "tree than a block has", (long long)n);
@@ -734,8 +767,12 @@ int wg_exact_step(wg_exact* e, double dt, int64_t maxcoll, int64_t* ncoll,
     k_exact_step<false><<<1, 64, e->smem, s>>>(A);
   if (!A.use_smem) k_exact_scatter<<<blocks, 256, 0, s>>>(A);
   cudaEventRecord(e->ev1, s);
-  cudaMemcpyAsync(e->h_ret, A.cindx, 24, cudaMemcpyDeviceToHost, s);
-  const cudaError_t ce = cudaStreamSynchronize(s);
+  // (a launch that was refused leaves the state, and what is read back, as it was)
+  cudaError_t ce = cudaGetLastError();
+  if (ce == cudaSuccess)
+    ce = cudaMemcpyAsync(e->h_ret, A.cindx, 24, cudaMemcpyDeviceToHost, s);
+  const cudaError_t cw = cudaStreamSynchronize(s);
+  if (ce == cudaSuccess) ce = cw;
   if (ce != cudaSuccess) return fail(WG_ERR_CUDA, "exact solver: %s", cudaGetErrorString(ce));
   long long nc = 0;
   std::memcpy(&nc, e->h_ret + 2, 8);
