@@ -208,7 +208,10 @@ __device__ __forceinline__ bool bin_sort(SmallSmem& S, Own<K>& o, int n) {
       q[k] = (uint32_t)fminf(fmaxf((float)(o.x[k] - x0) * scale, 0.f), (float)(BINS - 1));
       const int sh = (int)(q[k] & 1u) << 4;
       rk[k] = (atomicAdd(&bins[q[k] >> 1], 1u << sh) >> sh) & 0xffffu;
-      full |= rk[k] >= MAXBIN;
+      // (a NaN falls into bin 0, where its key belongs if its sign is set, as
+      // arithmetic here leaves it; the order does not rest on that: above
+      // infinity's key it is left to the sort by whole keys)
+      full |= rk[k] >= MAXBIN || o.key[k] > 0xFFF0000000000000ull;
     }
   if (__syncthreads_or(full)) return false;
   // exclusive scan: thread t owns the words [t wpt, t wpt + wpt)
