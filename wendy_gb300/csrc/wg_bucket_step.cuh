@@ -72,6 +72,9 @@ constexpr int NWORD = NBIN / 2;
 __device__ __forceinline__ uint32_t bin_get(const uint32_t* bins, int b) {
   return (bins[b >> 1] >> ((b & 1) << 4)) & 0xffffu;
 }
+// Most splitters that one pass over CAP sheets can publish: a bucket may have
+// grown to CAP whatever its target.
+constexpr int SAMPLES = CAP / kSmallestTarget + 1;
 // Cells of the routing table over a splitter window (see route_table).
 constexpr int LUTN = 256;
 // Sheets a thread takes at once through the force loop.
@@ -125,10 +128,10 @@ struct __align__(16) StepSmem {
   unsigned long long maxv;
   unsigned maxc;  // largest destination count this task saw after its reservations
   float vsum[WARPS];      // per warp: sum of the new velocities (predicted splitters)
-  unsigned nsamp;         // splitter samples of this task (at most 3: n <= CAP < 3 target)
-  double samp_x[4];
-  int32_t samp_idx[4];
-  uint32_t samp_q[4];
+  unsigned nsamp;         // splitter samples of this task
+  double samp_x[SAMPLES];
+  int32_t samp_idx[SAMPLES];
+  uint32_t samp_q[SAMPLES];
   uint64_t mbar;  // completion of the bucket's bulk copies
   int big_head;   // first of the big buckets this CTA has claimed (-1: none)
   // a big bucket (process_big): its chunks as ranges of key bins
@@ -911,7 +914,7 @@ __device__ __forceinline__ bool process_bucket(const StepLaunch& L, StepSmem& S,
         qni[qnext] = idv[u];
         if (ptab) {
           const unsigned k = atomicAdd(&S.nsamp, 1u);
-          if (k < 4u) {
+          if (k < (unsigned)SAMPLES) {
             S.samp_x[k] = x;
             S.samp_idx[k] = idv[u];
             S.samp_q[k] = qnext;
@@ -1008,7 +1011,7 @@ __device__ __forceinline__ bool process_bucket(const StepLaunch& L, StepSmem& S,
   maxv = warp_max_u64(maxv);
   if (lane == 0 && maxv) atomicMax(&S.maxv, maxv);
   __syncthreads();
-  if (ptab && tid < (int)min(S.nsamp, 4u)) {
+  if (ptab && tid < (int)min(S.nsamp, (unsigned)SAMPLES)) {
     // the sample's position moved on by two drifts at the bucket's mean
     // velocity: where the bucket is heading.  The mean, not the sample's
     // own velocity: in a warm region single velocities would scatter the

@@ -7,6 +7,7 @@ namespace wg {
 
 constexpr int kBucketCap = 2048;      // sheets a bucket's shared-memory pass can hold
 constexpr int kMaxTarget = kBucketCap * 3 / 4;  // largest bucket target
+constexpr int kSmallestTarget = 64;  // smallest target a tuning row may ask for
 constexpr int kMinTarget = 384;  // smallest target that launches with few buckets are cut to
 
 // Buckets of `target` sheets at a re-sort, `capg` slots each.
