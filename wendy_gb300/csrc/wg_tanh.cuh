@@ -252,14 +252,27 @@ __device__ __forceinline__ long long mul_64_31(long long s, int d) {
   return (long long)(int)(s >> 32) * d + (long long)__umulhi((uint32_t)s, (uint32_t)d);
 }
 
-// tanh(y) with the table (16-byte aligned, kTanhCells rows).  The offset D in
-// the cell has 54 bits; a Horner step needs as many of them as the powers of D
-// still to come leave significant: the first two work on 32-bit words, the
-// third on the upper 31 bits of D (rounded), and only the last two on all of
-// it, as 31 + 23 bits.  Their truncations are made up for by one unit, which
-// leaves the largest absolute error over the range at 2^-61.3 and the mean at
-// 0.48 units of 2^-62 (2^-61.2 and 0.52 with full products throughout), for
-// half of their instructions.
+// tanh 2^62 in a cell: the row's polynomial at D 2^64 = dh 2^32 + dw (54 bits).  A
+// Horner step needs as many of these bits as the powers of D still to come leave
+// significant: the first two work on 32-bit words, the third on the upper 31 bits
+// of D (rounded), the last two on all of it, as 31 + 23 bits, and the very last is
+// rounded, not truncated.  Against 113-bit tanh over all cells the largest error is
+// 1.42 units of 2^-62 and the mean 0.33 (full products, truncated: 1.54 and 0.52; with
+// the last step truncated too, and a unit added: 1.84 and 0.50), for half of the
+// instructions of full products.
+__device__ __forceinline__ long long tanh_poly(const longlong2 r0, const longlong2 r1,
+                                               const longlong2 r2, uint32_t dh, uint32_t dw) {
+  const int dt = (int)__funnelshift_l(dw, dh, 9);  // D >> 23
+  const int dl = (int)(dw & 0x7fffffu);
+  const int d = (int)min((uint32_t)dt + (uint32_t)(dl >> 22), 0x7fffffffu);  // rounded
+  const int s4 = (int)(r2.x >> 32) + (__mulhi((int)(r2.y >> 32), d) >> 9);
+  const long long s3 = r1.y + (((long long)s4 * d) >> 9);
+  const long long s2 = r1.x + (mul_64_31(s3, d) >> 9);
+  const long long s1 = r0.y + (mul_64_31(s2, dt) >> 9) + __mulhi((int)(s2 >> 32), dl);
+  return r0.x + ((mul_64_31(s1, dt) + (((long long)(int)(s1 >> 32) * dl) >> 23) + 256) >> 9);
+}
+
+// tanh(y) with the table (16-byte aligned, kTanhCells rows).
 __device__ __forceinline__ double tanh_tab(const long long* __restrict__ tab, double y) {
   const uint32_t yh = (uint32_t)__double2hiint(y), yl = (uint32_t)__double2loint(y);
   const uint32_t ah = yh & 0x7fffffffu;
@@ -270,16 +283,8 @@ __device__ __forceinline__ double tanh_tab(const long long* __restrict__ tab, do
   const uint32_t cell = mh >> (10 - e);
   const uint32_t fh = mh & ((1u << (10 - e)) - 1u);
   const uint32_t dh = __funnelshift_l(yl, fh, e + 12), dw = yl << (e + 12);
-  const int dt = (int)__funnelshift_l(dw, dh, 9);  // D >> 23
-  const int dl = (int)(dw & 0x7fffffu);
-  const int d = min((uint32_t)dt + (uint32_t)(dl >> 22), 0x7fffffffu);  // rounded
   const longlong2* r = reinterpret_cast<const longlong2*>(tab + kTanhRow * cell);
-  const longlong2 r0 = __ldg(r), r1 = __ldg(r + 1), r2 = __ldg(r + 2);
-  const int s4 = (int)(r2.x >> 32) + (__mulhi((int)(r2.y >> 32), d) >> 9);
-  const long long s3 = r1.y + (((long long)s4 * d) >> 9);
-  const long long s2 = r1.x + (mul_64_31(s3, d) >> 9);
-  const long long s1 = r0.y + (mul_64_31(s2, dt) >> 9) + __mulhi((int)(s2 >> 32), dl);
-  const long long T = r0.x + (mul_64_31(s1, dt) >> 9) + __mulhi((int)(s1 >> 32), dl) + 1;
+  const long long T = tanh_poly(__ldg(r), __ldg(r + 1), __ldg(r + 2), dh, dw);
   // T 2^-62 in [2^-10, 1] to double, rounded half up; the carry of the
   // rounding may run into the exponent
   const uint64_t Tq = T >= (1ll << 62) ? (1ull << 62) - 1 : (uint64_t)T;
