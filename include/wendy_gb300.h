@@ -87,6 +87,10 @@ int wg_version(void);
 const char *wg_status_string(int status);
 const char *wg_last_error(void); /* detail of the last failure on this thread */
 int wg_device_info(int *sm_count, int64_t *free_bytes, int64_t *total_bytes);
+/* Up to 512 MiB of device memory, 64 MiB of page-locked memory and 8 streams of
+   closed simulations are kept for the next ones.  They are given back when an
+   allocation of the library fails, by wg_device_info, and by this call. */
+int wg_trim(void);
 
 /* ---- the stateful path behind nbody(..., approx=True, sort='cuda') ------
    Replaces the per-output ctypes call to _wendy_nbody_approx_onestep

@@ -1,7 +1,9 @@
 """What the library keeps from one simulation for the next (wendy_gb300/csrc/
 wg_blocks.cu, host code): compiled here against a stand-in for the CUDA runtime
 with two devices and an allocator that can be made to fail."""
+import ctypes.util
 import os
+import re
 import shutil
 import subprocess
 
@@ -74,6 +76,29 @@ int main() {
 }
 """
 
+ROOM = r"""
+int main() {
+  // a closed simulation's memory is all the device has: every kind of allocation
+  // takes it back before it fails
+  const size_t most = (size_t)400 << 20;
+  room = most;
+  void* p = nullptr;
+  for (int k = 0; k < 4; ++k) {
+    CHECK(block_alloc(&p, most - 1000) == cudaSuccess);
+    block_free(p);
+    CHECK(room == 1000 && live.size() == 1);  // kept
+    if (k == 0) CHECK(device_alloc(&p, 2000) == cudaSuccess && cudaFree(p) == cudaSuccess);
+    if (k == 1) CHECK(page_locked_alloc(&p, 2000) == cudaSuccess && cudaFreeHost(p) == cudaSuccess);
+    if (k == 2) CHECK(host_block_alloc(&p, 2000) == cudaSuccess && host_block_free(p));
+    if (k == 3) blocks_trim();
+    blocks_trim();
+    CHECK(room == most && live.empty());
+  }
+  CHECK(device_alloc(&p, most + 1) == cudaErrorMemoryAllocation);
+  return 0;
+}
+"""
+
 
 def _run(tmp_path, main):
     cuda = os.path.dirname(os.path.dirname(shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"))
@@ -90,3 +115,38 @@ def _run(tmp_path, main):
 
 def test_streams_stay_with_their_device(tmp_path):
     _run(tmp_path, STREAMS)
+
+
+def test_kept_memory_is_given_back_before_an_allocation_fails(tmp_path):
+    _run(tmp_path, ROOM)
+
+
+def test_no_source_allocates_past_what_is_kept():
+    # wg_blocks.cu alone calls the allocators that fail while memory is kept idle
+    for f in sorted(os.listdir(CSRC)):
+        if f != "wg_blocks.cu" and f.endswith((".cu", ".cuh")):
+            with open(os.path.join(CSRC, f)) as src:
+                code = [line.split("//")[0] for line in src]
+            assert not [c for c in code
+                        if re.search(r"\bcuda(Malloc|MallocHost|HostAlloc)\(", c)], f
+
+
+@pytest.mark.gpu
+def test_trim_gives_the_memory_of_closed_simulations_back():
+    import ctypes
+
+    import wendy_gb300
+    from wendy_gb300 import ics
+    rt = ctypes.CDLL(ctypes.util.find_library("cudart") or "libcudart.so")
+    rt.cudaMemGetInfo.argtypes = [ctypes.POINTER(ctypes.c_size_t)] * 2
+
+    def free_bytes():
+        f, t = ctypes.c_size_t(), ctypes.c_size_t()
+        assert rt.cudaMemGetInfo(ctypes.byref(f), ctypes.byref(t)) == 0
+        return f.value
+
+    x, v, m = ics.sech2_disk(1 << 20, seed=1)
+    wendy_gb300.Simulation(x, v, m, 1., -1.).close()
+    kept = free_bytes()
+    wendy_gb300.trim()
+    assert free_bytes() >= kept + (100 << 20)

@@ -6,6 +6,6 @@ shared library (include/wendy_gb300.h) loaded through ctypes.
 """
 from .diagnostics import energy, momentum, potential  # noqa: F401
 from .extforce import Harmonic, PulseTanh  # noqa: F401
-from .wendy import Simulation, accel, approx_onestep, nbody  # noqa: F401
+from .wendy import Simulation, accel, approx_onestep, nbody, trim  # noqa: F401
 
-__all__ = ["nbody", "accel", "approx_onestep", "energy", "momentum", "potential", "Simulation", "Harmonic", "PulseTanh"]
+__all__ = ["nbody", "accel", "approx_onestep", "energy", "momentum", "potential", "Simulation", "Harmonic", "PulseTanh", "trim"]

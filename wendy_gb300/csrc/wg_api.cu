@@ -968,6 +968,11 @@ int wg_device_info(int* sm_count, int64_t* free_bytes, int64_t* total_bytes) {
   return WG_OK;
 }
 
+int wg_trim(void) {
+  blocks_trim();
+  return WG_OK;
+}
+
 int wg_create(int64_t n, const double* x, const double* v, const double* m, double totmass,
               double omega2, int ext_kind, const double* ext_params, int n_ext_params,
               wg_sim** out) {
@@ -1692,7 +1697,7 @@ int wg_ext_force_eval(int64_t n, const double* x, double t, int ext_kind,
   if (rc) return rc;
   double* d = nullptr;
   ExprOp* d_prog = nullptr;
-  cudaError_t e = cudaMalloc(&d, 16 * (size_t)n);
+  cudaError_t e = device_alloc(&d, 16 * (size_t)n);
   if (e == cudaSuccess) e = attach_ext_program(&ext, &d_prog, 0);
   if (e != cudaSuccess) {
     cudaGetLastError();

@@ -63,15 +63,10 @@ bool take(Kept& k, int dev, size_t bytes, Block* out) {
   return true;
 }
 
-cudaError_t alloc(int dev, void** p, size_t bytes) {
-  Kept& k = kept();
-  Block b;
-  if (take(k, dev, bytes, &b)) {
-    *p = b.p;
-    return cudaSuccess;
-  }
+// From the system; what is kept idle is given back to it if there is no room.
+cudaError_t fresh(bool host, void** p, size_t bytes) {
   auto raw = [&] {
-    return dev < 0 ? cudaHostAlloc(p, bytes, cudaHostAllocDefault) : cudaMalloc(p, bytes);
+    return host ? cudaHostAlloc(p, bytes, cudaHostAllocDefault) : cudaMalloc(p, bytes);
   };
   cudaError_t e = raw();
   if (e != cudaSuccess) {
@@ -79,6 +74,17 @@ cudaError_t alloc(int dev, void** p, size_t bytes) {
     blocks_trim();
     e = raw();
   }
+  return e;
+}
+
+cudaError_t alloc(int dev, void** p, size_t bytes) {
+  Kept& k = kept();
+  Block b;
+  if (take(k, dev, bytes, &b)) {
+    *p = b.p;
+    return cudaSuccess;
+  }
+  const cudaError_t e = fresh(dev < 0, p, bytes);
   if (e == cudaSuccess) {
     std::lock_guard<std::mutex> lock(k.mu);
     k.out[*p] = Block{*p, bytes, dev};
@@ -129,6 +135,9 @@ void block_free(void* p) { give(p); }
 
 cudaError_t host_block_alloc(void** p, size_t bytes) { return alloc(-1, p, bytes); }
 bool host_block_free(void* p) { return give(p); }
+
+cudaError_t device_alloc(void** p, size_t bytes) { return fresh(false, p, bytes); }
+cudaError_t page_locked_alloc(void** p, size_t bytes) { return fresh(true, p, bytes); }
 
 cudaError_t stream_set_take(StreamSet* s) {
   Kept& k = kept();

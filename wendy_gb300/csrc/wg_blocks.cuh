@@ -8,7 +8,8 @@
 // releases is kept here, up to kKeepDevice and kKeepHost bytes and kKeepSets
 // streams per process, oldest dropped first, and handed to the next one that
 // asks for it.  It is given back to the system when an allocation of the
-// library fails, when the free memory is asked for, and by blocks_trim().
+// library fails, when the free memory is asked for, and by blocks_trim() (wg_trim
+// for other users of the device's memory in the process).
 // Callers hand back only memory and streams with no work in flight, so that
 // nothing depends on the stream that used them last.  All functions may be
 // called from several threads.
@@ -37,6 +38,19 @@ bool host_block_free(void* p);
 template <typename T>
 cudaError_t host_block_alloc(T** p, size_t bytes) {
   return host_block_alloc(reinterpret_cast<void**>(p), bytes);
+}
+
+// cudaMalloc and cudaMallocHost for memory that is not handed on (released with
+// cudaFree and cudaFreeHost): what is kept idle is given back before they fail.
+cudaError_t device_alloc(void** p, size_t bytes);
+cudaError_t page_locked_alloc(void** p, size_t bytes);
+template <typename T>
+cudaError_t device_alloc(T** p, size_t bytes) {
+  return device_alloc(reinterpret_cast<void**>(p), bytes);
+}
+template <typename T>
+cudaError_t page_locked_alloc(T** p, size_t bytes) {
+  return page_locked_alloc(reinterpret_cast<void**>(p), bytes);
 }
 
 // A non-blocking stream and two timing events, of the device that is current

@@ -18,6 +18,7 @@
 #include <cstring>
 
 #include "../../include/wendy_gb300.h"
+#include "wg_blocks.cuh"
 #include "wg_common.cuh"
 
 namespace wg {
@@ -126,7 +127,7 @@ inline cudaError_t attach_ext_program(ExtSpec* spec, ExprOp** d_prog, cudaStream
     return cudaSuccess;
   }
   if (!*d_prog) {
-    const cudaError_t e = cudaMalloc(d_prog, sizeof(ExprOp) * kExprMaxOps);
+    const cudaError_t e = device_alloc(d_prog, sizeof(ExprOp) * kExprMaxOps);
     if (e != cudaSuccess) return e;
   }
   const cudaError_t e = cudaMemcpyAsync(*d_prog, spec->ops, sizeof(ExprOp) * spec->f.n_ops,

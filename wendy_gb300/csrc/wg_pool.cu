@@ -329,7 +329,7 @@ int ensure_small(wg_pool* p, int nsims, int nleap, int64_t ntasks) {
                    al(sizeof(StepFlags) * (size_t)cs * (cl + 1)) + al(8 * (size_t)cs * cl) +
                    al(8 * (size_t)cs) + al(sizeof(BucketTask) * (size_t)ct) +
                    al(sizeof(BucketTask) * (size_t)ct) + al(4 * (size_t)cs);
-  PC(cudaMalloc(&p->small, b));
+  PC(device_alloc(&p->small, b));
   char* q = static_cast<char*>(p->small);
   p->table = reinterpret_cast<StateTable*>(q); q += al(sizeof(StateTable));
   p->err = reinterpret_cast<unsigned*>(q); q += al(64);
@@ -344,14 +344,14 @@ int ensure_small(wg_pool* p, int nsims, int nleap, int64_t ntasks) {
   p->rtasks = reinterpret_cast<BucketTask*>(q); q += al(sizeof(BucketTask) * (size_t)ct);
   p->rlist = reinterpret_cast<int*>(q); q += al(4 * (size_t)cs);
   PC(cudaMemsetAsync(p->small, 0, b, p->stream));
-  PC(cudaMallocHost(&p->h_dev, sizeof(SimDev) * (size_t)cs));
-  PC(cudaMallocHost(&p->h_t, 8 * (size_t)cs * cl));
-  PC(cudaMallocHost(&p->h_ep, 4 * (size_t)cl));
-  PC(cudaMallocHost(&p->h_oc, 8 * (size_t)cs));
+  PC(page_locked_alloc(&p->h_dev, sizeof(SimDev) * (size_t)cs));
+  PC(page_locked_alloc(&p->h_t, 8 * (size_t)cs * cl));
+  PC(page_locked_alloc(&p->h_ep, 4 * (size_t)cl));
+  PC(page_locked_alloc(&p->h_oc, 8 * (size_t)cs));
   PC(cudaHostGetDevicePointer(reinterpret_cast<void**>(&p->d_oc), p->h_oc, 0));
-  PC(cudaMallocHost(&p->h_tasks, sizeof(BucketTask) * (size_t)ct));
-  PC(cudaMallocHost(&p->h_rtasks, sizeof(BucketTask) * (size_t)ct));
-  PC(cudaMallocHost(&p->h_rlist, 4 * (size_t)cs));
+  PC(page_locked_alloc(&p->h_tasks, sizeof(BucketTask) * (size_t)ct));
+  PC(page_locked_alloc(&p->h_rtasks, sizeof(BucketTask) * (size_t)ct));
+  PC(page_locked_alloc(&p->h_rlist, 4 * (size_t)cs));
   p->cap_sims = cs;
   p->cap_leap = cl;
   p->cap_tasks = ct;
@@ -376,7 +376,7 @@ int ensure_workspace(wg_pool* p, int64_t n) {
   const int64_t nb = n;  // compaction offsets: at most one bucket per sheet
   const size_t b = 2 * (3 * nd + ni) + al(sizeof(TileRec) * (size_t)tiles) + radix_bytes(n) +
                    al(4 * (size_t)nb);
-  PC(cudaMalloc(&p->ws, b));
+  PC(device_alloc(&p->ws, b));
   char* q = static_cast<char*>(p->ws);
   for (int k = 0; k < 2; ++k) {
     p->set[k].x = reinterpret_cast<double*>(q); q += nd;
@@ -414,7 +414,7 @@ int ensure_batch(wg_pool* p, int64_t n, int64_t ntasks, int nsegs) {
   const size_t b = 6 * set + radix_bytes(n) + 2 * al(sizeof(StateTable)) + al(sizeof(StepFlags)) +
                    al(4 * (size_t)ntasks) + al(sizeof(BatchSeg) * (size_t)nsegs) +
                    al(8 * (size_t)(nsegs + 1)) + al(sizeof(BucketTask) * (size_t)ntasks);
-  PC(cudaMalloc(&p->bws, b));
+  PC(device_alloc(&p->bws, b));
   char* q = static_cast<char*>(p->bws);
   StateRef* sets[6] = {&p->bW, &p->bA[0], &p->bA[1], &p->bB[0], &p->bB[1], &p->bO};
   for (StateRef* r : sets) {

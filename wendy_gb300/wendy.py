@@ -277,6 +277,13 @@ def _nbody_approx(x, v, m, dt, nleap, t0=0., omega=None, ext_force=None, sort="c
             pass
 
 
+def trim():
+    """Gives back the device and page-locked memory that the library keeps from closed
+    simulations for the next ones (wg_trim; at most 512 and 64 MiB), for programs
+    whose other libraries need it.  No reference counterpart."""
+    _lib.check(_lib.lib().wg_trim(), "wg_trim")
+
+
 def accel(x, m, totmass, omega2=-1., ext_force=None, t=0.):
     """One force evaluation at positions x (original order).
 
