@@ -70,7 +70,7 @@ struct RadixWork {
   uint64_t* keys[2];
   uint32_t* pos[2];
   uint32_t* plan;       // per-pass: active, src, dst; final buffer; digit starts
-  uint32_t* hist;       // 8 x 256 digit counts ...
+  uint32_t* hist;       // 12 x 256 digit counts ...
   uint32_t* counters;   // ... tile tickets, tie flag ...
   uint32_t* status;     // ... passes x tiles x 256 look-back words: cleared together
 };

@@ -27,8 +27,11 @@
 //   gather permute x, v, m, idx into the other state set; notes in small sorts
 //          whether any sheet precedes its predecessor in (key, index)
 //   ties   (unless none does) runs of equal leading bytes are ordered by key and
-//          original index: short runs in place, long runs by one CTA each,
-//          whose last block makes the other set the current one
+//          original index: short runs in place, longer ones by one warp or one
+//          CTA each, whose last block makes the other set the current one; where
+//          longer runs hold too much -- positions far from the origin against their spread, or
+//          crowded about a few places -- all sheets are sorted by their whole keys
+//          instead, by the same launch
 //
 // Keys that differ in their low bytes only (ranks packed into the bits of a
 // double) are sorted whole: first_byte = 0, eight passes of 64-bit keys.
@@ -65,10 +68,18 @@ constexpr int kPlanWords = kPlanStarts + 8 * R;
 // counters (uint32 words, cleared before each sort)
 constexpr int kCntClaim = 0;   // [8] next tile of each pass
 constexpr int kCntTie = 8;     // some sheet may be out of (key, index) order
-constexpr int kCntRuns = 9;    // long runs listed
 constexpr int kCntHist = 10;   // histogram blocks done
 constexpr int kCntLong = 11;   // k_radix_long_ties blocks done
-constexpr int kCounters = 16;
+constexpr int kCntRuns = 12;   // longer runs listed and, in the upper half of 64 bits,
+constexpr int kCntSheets = 13;  // ... the sheets in those of more than a warp's lanes
+constexpr int kCntMaxRun = 9;   // the longest of these
+constexpr int kCntInv = 14;     // neighbours of one run whose keys were out of order
+constexpr int kCntMixed = 15;   // the current set is not in the order of the indices
+constexpr int kCntStage = 16;   // [2 x 16] whole sort: tiles claimed and done of each stage
+constexpr int kCounters = 48;
+// rows of the digit histogram: the eight bytes of the keys, then the four of the
+// indices (whole sort)
+constexpr int kHistRows = 12;
 
 struct PassArgs {
   const StateTable* table;
@@ -554,15 +565,14 @@ __global__ void __launch_bounds__(kGatherThreads) k_radix_gather(
 // original index.  The thread at a run's first sheet finds its end by binary
 // search over the sorted leading bytes; runs of up to kShortRun sheets are
 // insertion-sorted in place, longer ones are listed (start in list_start,
-// length in list_len, count in counters[kCntRuns]) for k_radix_long_ties, so
-// no thread ever does work quadratic in a run.  A warp reads four groups of 32
-// keys at a time, and a pair in order is passed over on these, before anything
+// length in list_len) for k_radix_long_ties, so no thread ever does work quadratic
+// in a run.  A warp reads four groups of 32 keys at a time, and a pair in order is passed over on these, before anything
 // of its run has moved: one group at a time, each pair's sheets loaded again, took
 // 0.44 ms at 2^26 and more than twice that at 2^27; so 0.25 ms.  Threads read the
 // leading bytes of sheets that a run's first thread may be moving: moves stay
 // inside a run, whose leading bytes are all the same, and both sides use relaxed
 // accesses.
-constexpr int64_t kShortRun = 32;
+constexpr int64_t kShortRun = 8, kWarpRun = 32;
 constexpr int kTieUnroll = 4;
 __global__ void k_radix_ties(StateTable* table, int64_t n, int low_bits, uint32_t* counters,
                              uint32_t* list_start, uint32_t* list_len, const StepFlags* flag,
@@ -574,6 +584,10 @@ __global__ void k_radix_ties(StateTable* table, int64_t n, int low_bits, uint32_
   auto lead = [&](int64_t p) { return whole(p) >> low_bits; };
   const int lane = threadIdx.x & 31;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  __shared__ unsigned s_inv;
+  if (threadIdx.x == 0) s_inv = 0u;
+  __syncthreads();
+  unsigned inv = 0;  // neighbours of one run out of order
   // the run that starts at sheet p, whose first keys are k0, k1 (and k2, except
   // in the last two lanes)
   auto order_run = [&](int64_t p, uint64_t k0, uint64_t k1, uint64_t k2) {
@@ -590,9 +604,13 @@ __global__ void k_radix_ties(StateTable* table, int64_t n, int low_bits, uint32_
     }
     const int64_t e = lo;
     if (e - p + 1 > kShortRun) {
-      const unsigned slot = atomicAdd(&counters[kCntRuns], 1u);
+      const uint32_t len = (uint32_t)(e - p + 1);
+      const uint32_t slot =
+          (uint32_t)atomicAdd(reinterpret_cast<unsigned long long*>(&counters[kCntRuns]),
+                              ((unsigned long long)(len > kWarpRun ? len : 0u) << 32) | 1ull);
       list_start[slot] = (uint32_t)p;
-      list_len[slot] = (uint32_t)(e - p + 1);
+      list_len[slot] = len;
+      if (len > kWarpRun) atomicMax(&counters[kCntMaxRun], len);
       return;
     }
     for (int64_t i = p + 1; i <= e; ++i) {
@@ -638,47 +656,389 @@ __global__ void k_radix_ties(StateTable* table, int64_t n, int low_bits, uint32_
       uint64_t kb = __shfl_up_sync(0xffffffffu, k0, 1);
       if (lane == 31) k1 = ke[u];
       if (lane == 0) kb = ke[u];
+      inv += p + 1 < n && kp == k1 >> low_bits && k1 < k0;
       if (p + 1 < n && kp == k1 >> low_bits && (p == 0 || kb >> low_bits != kp))
         order_run(p, k0, k1, k2);
       __syncwarp();
     }
   }
+  inv = __reduce_add_sync(0xffffffffu, inv);
+  if (lane == 0 && inv) atomicAdd(&s_inv, inv);
+  __syncthreads();
+  if (threadIdx.x == 0 && s_inv) atomicAdd(&counters[kCntInv], s_inv);
 }
 
-// Long runs of equal leading bytes, one CTA per run: a stable LSD radix sort
+constexpr int kLongTieThreads = 256;
+
+// ---- the sort by whole keys --------------------------------------------------
+// Positions that share their leading bytes by the thousand (a system of unit width
+// at 1e6 has three values of its leading four bytes) leave runs of which one CTA
+// takes 3 ms for 1e5 sheets.  Whether that is so is known only after the ties have
+// been looked at; the sort by whole keys then runs in the launch that would have
+// ordered the runs, so that it costs nothing where it is not needed: a stable radix
+// sort of (word, place) pairs by the bytes of the indices and then of the keys, bytes
+// that are the same for all sheets left out.  One launch, several passes: tiles of
+// all stages are claimed in order, a stage begins when all tiles of the one before
+// are done, and those have been claimed by running CTAs, so that every (bounded) wait
+// ends however many CTAs are resident.
+// Force evaluations on host arrays, a unit-width system about 0 / at 1e6 / at 1e9:
+// 307 / 346 / 333 us at 1e5 sheets (309 / 1226 / 3492 with the runs one by one), 2.0 /
+// 1.7 / 1.7 ms at 1e6 (2.0 / 2.5 / 19.5), 6.6 / 7.0 / 6.3 ms at 4e6 (6.7 / 8.6 / 134).
+// Tiles of 1024 sheets up to 2^17, of 2048 above (20011 sheets 173 -> 153 us a force
+// evaluation on device arrays; 1e6 sheets 1.91 -> 1.78 ms on host arrays).
+constexpr int kWholeItems = 8, kWholeItemsSmall = 4;
+constexpr int64_t kWholeSmallSheets = 1 << 17;
+// (the look-back words, two sets used alternately, fit where the passes' were: two
+// for every tile against eight for every tile of theirs)
+static_assert(2 * kRadixTile <= 8 * kLongTieThreads * kWholeItemsSmall &&
+                  2 * kRadixTileSmall <= 8 * kLongTieThreads * kWholeItemsSmall,
+              "look-back words");
+
+struct WholeSmem {
+  uint64_t word[kLongTieThreads * kWholeItems];
+  uint32_t pos[kLongTieThreads * kWholeItems];
+  uint32_t whist[kLongTieThreads / 32][R];
+  uint32_t tile_excl[R];
+  uint32_t gbase[R];
+  uint32_t starts[R];
+  uint32_t tmp[R / 32];
+  int64_t tile;
+  int stop;
+};
+
+struct WholeArgs {
+  StateTable* table;
+  int64_t n;
+  int first;  // bytes of the keys below this one have not been counted yet
+  uint64_t* word[2];
+  uint32_t* pos[2];
+  uint32_t* hist;
+  uint32_t* status;
+  uint32_t* counters;
+  unsigned* err;
+};
+
+// Whether runs of more than a warp's lanes hold more sheets than should be left to
+// one CTA per run: more than 2048 (and a 256th of all, at most 30720, more), and not
+// just equal positions that are in order already.
+__device__ __forceinline__ bool crowded(const uint32_t* counters, int64_t n) {
+  const int64_t part = n >> 8;
+  const uint32_t most = 2048u + (uint32_t)(part < 30720 ? part : 30720);
+  const uint32_t inv = counters[kCntInv];
+  return counters[kCntSheets] > most &&
+         (inv > most / 8 || (inv && counters[kCntMaxRun] > most));
+}
+
+// Exclusive scan of one value per thread over the R threads.
+__device__ __forceinline__ uint32_t digit_scan(WholeSmem& S, uint32_t v) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t incl = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) S.tmp[warp] = incl;
+  __syncthreads();
+  uint32_t pre = 0;
+#pragma unroll
+  for (int w = 0; w < R / 32; ++w) pre += w < warp ? S.tmp[w] : 0u;
+  __syncthreads();
+  return pre + incl - v;
+}
+
+// Returns whether the sheets are in the other set (else in the current one).
+template <int ITEMS>
+__device__ __noinline__ bool sort_whole(const WholeArgs& a, WholeSmem& S) {
+  constexpr int T = kLongTieThreads, WARPS = T / 32, TILE = T * ITEMS;
+  static_assert(T == R, "a thread per digit");
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t n = a.n, tiles = (n + TILE - 1) / TILE;
+  const StateRef oth = a.table->other, cur = a.table->cur;
+  auto claim = [&](int stage) {
+    __syncthreads();
+    if (tid == 0) S.tile = atomicAdd(&a.counters[kCntStage + 2 * stage], 1u);
+    __syncthreads();
+    return S.tile;
+  };
+  // `count` tiles of a stage are complete, and what was written for them visible
+  auto done = [&](int stage, unsigned count) {
+    __threadfence();
+    __syncthreads();
+    if (tid == 0 && count) atomicAdd(&a.counters[kCntStage + 2 * stage + 1], count);
+  };
+  auto all_done = [&](int stage) {
+    if (tid == 0) {
+      unsigned spins = 0;
+      S.stop = 0;
+      while (ld_relaxed_u32(&a.counters[kCntStage + 2 * stage + 1]) < (unsigned)tiles) {
+        if (++spins > kSpinLimit) {
+          atomicOr(a.err, DEV_ERR_RADIX_TIMEOUT);
+          S.stop = 1;
+          break;
+        }
+        __nanosleep(64);
+      }
+      __threadfence();
+    }
+    __syncthreads();
+    return S.stop == 0;
+  };
+  // ---- stage 0: the bytes not counted yet, and clean look-back words
+  uint32_t* const sh = &S.whist[0][0];  // rows 0 .. 3: indices; 4 ..: bytes 0 .. first - 1
+  static_assert(WARPS >= 8, "rows");
+  for (int i = tid; i < 8 * R; i += T) sh[i] = 0u;
+  unsigned mine = 0;
+  bool mixed = false;
+  for (int64_t tile; (tile = claim(0)) < tiles; ++mine) {
+    a.status[tile * R + tid] = 0u;
+    a.status[(tiles + tile) * R + tid] = 0u;
+    for (int i = 0; i < ITEMS; ++i) {
+      const int64_t p = tile * TILE + i * T + tid;
+      if (p >= n) break;
+      const uint32_t id = (uint32_t)oth.idx[p];
+      mixed |= p + 1 < n && cur.idx[p + 1] < cur.idx[p];
+      const uint64_t k = key_of(oth.x[p]);
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        atomicAdd(&sh[b * R + ((id >> (8 * b)) & 255u)], 1u);
+        if (b < a.first) atomicAdd(&sh[(4 + b) * R + ((k >> (8 * b)) & 255u)], 1u);
+      }
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < (4 + a.first) * R; i += T)
+    if (sh[i]) atomicAdd(&a.hist[i < 4 * R ? 8 * R + i : i - 4 * R], sh[i]);
+  if (__syncthreads_or(mixed) && tid == 0) atomicOr(&a.counters[kCntMixed], 1u);
+  done(0, mine);
+  if (!all_done(0)) return false;
+  // from the current set where that is in the order of the indices already (force
+  // evaluations, first sorts), which spares the passes by index
+  const bool mix = __ldcg(&a.counters[kCntMixed]) != 0u;
+  const StateRef from = mix ? oth : cur, to = mix ? cur : oth;
+  // ---- the passes: indices (0 .. 3), then keys (4 .. 11)
+  int src = -1;        // the buffers that hold the words and places (-1: none yet)
+  bool keyed = false;  // ... and whether the words are keys
+  int par = 0;         // the look-back words of this pass
+  for (int q = mix ? 0 : 4; q < 12; ++q) {
+    const int stage = 1 + q, row = q < 4 ? 8 + q : q - 4;
+    const int shift = 8 * (q < 4 ? q : q - 4);
+    const uint32_t h = __ldcg(&a.hist[row * R + tid]);
+    if (__syncthreads_or(h == (uint32_t)n)) continue;
+    S.starts[tid] = digit_scan(S, h);
+    uint32_t* const stat = a.status + (int64_t)par * tiles * R;
+    uint32_t* const next_stat = a.status + (int64_t)(par ^ 1) * tiles * R;
+    const int dst = src < 0 ? 0 : src ^ 1;
+    for (int64_t tile; (tile = claim(stage)) < tiles;) {
+      const int64_t base = tile * TILE;
+      const int tile_n = (int)(n - base < TILE ? n - base : TILE);
+      uint64_t word[ITEMS];
+      uint32_t pos[ITEMS], rank[ITEMS];
+#pragma unroll
+      for (int i = 0; i < ITEMS; ++i) {
+        const int local = warp * (32 * ITEMS) + i * 32 + lane;
+        word[i] = 0;
+        pos[i] = 0;
+        if (local < tile_n) {
+          const int64_t e = base + local;
+          pos[i] = src < 0 ? (uint32_t)e : __ldcg(a.pos[src] + e);
+          if (q >= 4 && !keyed)
+            word[i] = key_of(from.x[pos[i]]);
+          else
+            word[i] = src < 0 ? (uint64_t)(uint32_t)from.idx[e]
+                              : ld_cg_u64(a.word[src] + e);
+        }
+      }
+      for (int i = tid; i < WARPS * R; i += T) sh[i] = 0u;
+      __syncthreads();
+      // stable ranks inside the warp: items in order, lanes in order
+#pragma unroll
+      for (int i = 0; i < ITEMS; ++i) {
+        const bool ok = warp * (32 * ITEMS) + i * 32 + lane < tile_n;
+        const unsigned d = ok ? (unsigned)(word[i] >> shift) & 255u : 256u + lane;
+        const unsigned peers = __match_any_sync(0xffffffffu, d);
+        uint32_t old = 0;
+        if (ok) {
+          old = S.whist[warp][d];
+          rank[i] = old + __popc(peers & lanemask_lt());
+        }
+        __syncwarp();
+        if (ok && lane == __ffs(peers) - 1) S.whist[warp][d] = old + __popc(peers);
+        __syncwarp();
+      }
+      __syncthreads();
+      uint32_t count = 0;
+#pragma unroll
+      for (int w = 0; w < WARPS; ++w) {
+        const uint32_t c = S.whist[w][tid];
+        S.whist[w][tid] = count;
+        count += c;
+      }
+      st_relaxed_u32(&stat[tile * R + tid], (tile == 0 ? kStatP : kStatA) | count);
+      next_stat[tile * R + tid] = 0u;
+      const uint32_t tex = digit_scan(S, count);
+      S.tile_excl[tid] = tex;
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < ITEMS; ++i)
+        if (warp * (32 * ITEMS) + i * 32 + lane < tile_n) {
+          const unsigned d = (unsigned)(word[i] >> shift) & 255u;
+          const uint32_t p = S.tile_excl[d] + S.whist[warp][d] + rank[i];
+          S.word[p] = word[i];
+          S.pos[p] = pos[i];
+        }
+      // look-back over the same digit of earlier tiles, LB loads in flight
+      constexpr int LB = 4;
+      uint32_t excl = 0;
+      bool lost = false, found = tile == 0;
+      unsigned spins = 0;
+      for (int64_t j = tile - 1; !found && !lost;) {
+        uint32_t sv[LB];
+#pragma unroll
+        for (int w = 0; w < LB; ++w)
+          sv[w] = j - w >= 0 ? ld_relaxed_u32(&stat[(j - w) * R + tid]) : kStatP;
+        int w = 0;
+        for (; w < LB && !found; ++w) {
+          const uint32_t st = sv[w] >> 30;
+          if (st == 0u) break;  // not published yet: resume here
+          lost |= st == 3u;
+          excl += sv[w] & kCountMask;
+          found = st >= 2u;
+        }
+        if (w < LB && !found) {
+          lost |= ++spins > kSpinLimit;
+          __nanosleep(16);
+        }
+        j -= w;
+      }
+      if (tile > 0)
+        st_relaxed_u32(&stat[tile * R + tid], lost ? kStatX : kStatP | (excl + count));
+      S.gbase[tid] = S.starts[tid] + excl - tex;
+      if (__syncthreads_or(lost)) {
+        // offsets unknown: nothing leaves the tile, and the sort is given up
+        if (tid == 0) atomicOr(a.err, DEV_ERR_RADIX_TIMEOUT);
+        return false;
+      }
+#pragma unroll
+      for (int i = 0; i < ITEMS; ++i) {
+        const int p = i * T + tid;
+        if (p < tile_n) {
+          const uint64_t w = S.word[p];
+          const int64_t o = (int64_t)S.gbase[(unsigned)(w >> shift) & 255u] + p;
+          a.word[dst][o] = w;
+          a.pos[dst][o] = S.pos[p];
+        }
+      }
+      done(stage, 1u);
+    }
+    if (!all_done(stage)) return false;
+    src = dst;
+    keyed = q >= 4;
+    par ^= 1;
+  }
+  // ---- the sheets, in order
+  for (int64_t p = blockIdx.x * (int64_t)T + tid; p < n; p += (int64_t)gridDim.x * T) {
+    const int64_t o = src < 0 ? p : (int64_t)__ldcg(a.pos[src] + p);
+    to.x[p] = from.x[o];
+    to.v[p] = from.v[o];
+    to.m[p] = from.m[o];
+    to.idx[p] = from.idx[o];
+  }
+  return !mix;
+}
+
+// Longer runs of equal leading bytes: up to kWarpRun sheets by one warp, ranked by
+// comparing all pairs; above that by one CTA, a stable LSD radix sort
 // (4-bit digits, each thread a contiguous chunk) of (index, place in run)
 // pairs in the key buffers' slots of the run, by index and then by the low
 // bits of the key, then the run's sheets are permuted through the current set
 // (free until the flip) and copied back.  Runs already in order are left
-// alone.  O(run length) work per digit.  The last block to finish makes the
-// other set the current one.
-constexpr int kLongTieThreads = 256;
+// alone.  O(run length) work per digit.  Crowded states are sorted whole (sort_whole).
 __global__ void __launch_bounds__(kLongTieThreads) k_radix_long_ties(
-    StateTable* table, int64_t n, int low_bits, uint64_t* bufa, uint64_t* bufb,
-    uint32_t* counters, const uint32_t* list_start, const uint32_t* list_len,
-    const StepFlags* flag, const unsigned* err) {
+    const __grid_constant__ WholeArgs a, const StepFlags* flag) {
   chain_begin();
   // after an expired wait the current set stays as it was (unsorted, intact)
-  if (!flag->unsorted || (*err & DEV_ERR_RADIX_TIMEOUT)) return;
+  if (!flag->unsorted || (*a.err & DEV_ERR_RADIX_TIMEOUT)) return;
   constexpr int T = kLongTieThreads;
-  __shared__ uint32_t cnt[16][T + 1];
-  __shared__ uint32_t tot[16];
+  struct RunSmem {
+    uint32_t cnt[16][T + 1];
+    uint32_t tot[16];
+  };
+  __shared__ __align__(16) union {
+    RunSmem run;
+    WholeSmem whole;
+  } sm;
+  StateTable* const table = a.table;
+  const int64_t n = a.n;
+  uint32_t* const counters = a.counters;
   const int tid = threadIdx.x;
   const StateRef oth = table->other, cur = table->cur;
+  // the last block to finish makes the other set the current one
+  auto flip = [&] {
+    __syncthreads();
+    if (tid == 0) {
+      __threadfence();
+      if (atomicAdd(&counters[kCntLong], 1u) == gridDim.x - 1) {
+        table->cur = oth;
+        table->other = cur;
+      }
+    }
+  };
+  if (crowded(counters, n)) {
+    if (n <= kWholeSmallSheets ? sort_whole<kWholeItemsSmall>(a, sm.whole)
+                               : sort_whole<kWholeItems>(a, sm.whole))
+      flip();
+    return;
+  }
+  auto& cnt = sm.run.cnt;
+  auto& tot = sm.run.tot;
+  const uint32_t* const list_start = a.pos[0];
+  const uint32_t* const list_len = a.pos[1];
+  const int low_bits = 8 * a.first;
   int bits = 1;
   while (bits < 31 && ((int64_t)1 << bits) < n) ++bits;
   const int ipass = (bits + 3) / 4, npass = ipass + (low_bits + 3) / 4;
   const unsigned nruns = counters[kCntRuns];
+  // runs of up to a warp's lanes: each sheet's rank among the others
+  const int lane = tid & 31, nw = T / 32;
+  for (unsigned r = blockIdx.x * nw + (tid >> 5); r < nruns; r += gridDim.x * nw) {
+    const int64_t s = list_start[r];
+    const int L = (int)list_len[r];
+    if (L > (int)kWarpRun) continue;
+    uint64_t k = ~0ull;
+    int32_t id = 0x7fffffff;
+    double x = 0., v = 0., m = 0.;
+    if (lane < L) {
+      x = oth.x[s + lane];
+      v = oth.v[s + lane];
+      m = oth.m[s + lane];
+      id = oth.idx[s + lane];
+      k = key_of(x);
+    }
+    int rank = 0;
+    for (int j = 0; j < L; ++j) {
+      const uint64_t kj = __shfl_sync(0xffffffffu, k, j);
+      const int32_t ij = __shfl_sync(0xffffffffu, id, j);
+      rank += kj < k || (kj == k && (ij < id || (ij == id && j < lane)));
+    }
+    if (lane < L && rank != lane) {
+      oth.x[s + rank] = x;
+      oth.v[s + rank] = v;
+      oth.m[s + rank] = m;
+      oth.idx[s + rank] = id;
+    }
+  }
   for (unsigned r = blockIdx.x; r < nruns; r += gridDim.x) {
     const int64_t s = list_start[r], L = list_len[r];
+    if (L <= kWarpRun) continue;
     bool unordered = false;
     for (int64_t j = tid; j + 1 < L; j += T) {
       const uint64_t k = key_of(oth.x[s + j]), kn = key_of(oth.x[s + j + 1]);
       unordered |= kn < k || (kn == k && oth.idx[s + j + 1] < oth.idx[s + j]);
     }
     if (!__syncthreads_or(unordered)) continue;
-    uint64_t* src = bufa + s;
-    uint64_t* dst = bufb + s;
+    uint64_t* src = a.word[0] + s;
+    uint64_t* dst = a.word[1] + s;
     for (int64_t j = tid; j < L; j += T)
       src[j] = ((uint64_t)(uint32_t)oth.idx[s + j] << 32) | (uint64_t)j;
     const int64_t chunk = (L + T - 1) / T;
@@ -735,14 +1095,7 @@ __global__ void __launch_bounds__(kLongTieThreads) k_radix_long_ties(
     }
     __syncthreads();
   }
-  __syncthreads();
-  if (tid == 0) {
-    __threadfence();
-    if (atomicAdd(&counters[kCntLong], 1u) == gridDim.x - 1) {
-      table->cur = oth;
-      table->other = cur;
-    }
-  }
+  flip();
 }
 
 size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
@@ -835,7 +1188,7 @@ size_t radix_bytes(int64_t n) {
   b += 2 * align256((size_t)n * 8);
   b += 2 * align256((size_t)n * 4);
   b += align256(kPlanWords * 4);
-  b += 8 * R * 4 + kCounters * 4;
+  b += kHistRows * R * 4 + kCounters * 4;
   b += align256((size_t)8 * tiles * R * 4);
   return b;
 }
@@ -848,7 +1201,7 @@ void radix_bind(RadixWork* w, void* base, int64_t n) {
   w->pos[1] = reinterpret_cast<uint32_t*>(p); p += align256((size_t)n * 4);
   w->plan = reinterpret_cast<uint32_t*>(p); p += align256(kPlanWords * 4);
   w->hist = reinterpret_cast<uint32_t*>(p);
-  w->counters = w->hist + 8 * R;
+  w->counters = w->hist + kHistRows * R;
   w->status = w->counters + kCounters;
 }
 
@@ -861,7 +1214,7 @@ void radix_sort_state(StateTable* table, int64_t n, RadixWork* w, const StepFlag
   // the workspace may be bound for more sheets than this sort has: tiles,
   // look-back words and launches follow n
   const int64_t tiles = tiles_of(n);
-  cudaMemsetAsync(w->hist, 0, (8 * R + kCounters + (size_t)(8 - first) * tiles * R) * 4, s);
+  cudaMemsetAsync(w->hist, 0, (kHistRows * R + kCounters + (size_t)(8 - first) * tiles * R) * 4, s);
   constexpr int64_t kHistKeys = kHistUnroll * kHistThreads;
   int64_t hist_grid = (n + kHistKeys - 1) / kHistKeys;
   if (hist_grid > sms * 4) hist_grid = sms * 4;
@@ -911,9 +1264,20 @@ void radix_sort_state(StateTable* table, int64_t n, RadixWork* w, const StepFlag
   // pos[] is free once gathered: it holds the list of long runs
   launch_chained(k_radix_ties, (unsigned)g, 256, 0, s, table, n, 8 * first, w->counters, w->pos[0],
                  w->pos[1], flag, err);
-  // and the key buffers are scratch for long ones
-  launch_chained(k_radix_long_ties, (unsigned)sms, kLongTieThreads, 0, s, table, n, 8 * first,
-                 w->keys[0], w->keys[1], w->counters, w->pos[0], w->pos[1], flag, err);
+  // and the key buffers are scratch for long ones and for the sort by whole keys
+  WholeArgs wa;
+  wa.table = table;
+  wa.n = n;
+  wa.first = first;
+  for (int k = 0; k < 2; ++k) {
+    wa.word[k] = w->keys[k];
+    wa.pos[k] = w->pos[k];
+  }
+  wa.hist = w->hist;
+  wa.status = w->status;
+  wa.counters = w->counters;
+  wa.err = err;
+  launch_chained(k_radix_long_ties, (unsigned)sms, kLongTieThreads, 0, s, wa, flag);
 }
 
 }  // namespace wg
