@@ -710,7 +710,7 @@ int enqueue_step(wg_sim* s, double dt, int nleap, bool want_accel, double dt_las
   WG_CUDA(cudaMemsetAsync(s->flags, 0, sizeof(StepFlags) * (nleap + 1), s->stream));
   WG_CUDA(cudaMemsetAsync(s->tickets, 0, 4 * (size_t)nleap, s->stream));
   launch_drift(s->table, s->n, dt / 2., &s->flags[0], s->stream);
-  s->st.launches += 1 + (int64_t)nleap * (1 + kRadixLaunches);
+  s->st.launches += 1 + (int64_t)nleap * (1 + radix_launches(s->n));
   ForceArgs a;
   a.table = s->table;
   a.n = s->n;
@@ -837,7 +837,7 @@ void launch_substep(wg_sim* s, int i, int nleap, int profile) {
     } else {
       radix_sort_state(s->ptab, s->nb - 1, &s->pradix, s->pflag, s->err, s->stream);
       launch_samples_to_splitters(s->ptab, s->nb - 1, s->qk[q], s->qi[q], s->stream);
-      s->st.launches += kRadixLaunches + 1;
+      s->st.launches += radix_launches(s->nb - 1) + 1;
     }
     if (!profile) s->st.substeps_predicted += 1;
   }
@@ -1053,7 +1053,7 @@ static int compact_continue(wg_sim* s, double dt, int nleap, int from) {
   }
   if (s->call_a) launch_scatter_accel(s->table, s->n, s->a_sorted, s->call_a, s->stream);
   if (s->call_xi) store_sheets(s->table, s->n, reinterpret_cast<wg_sheet*>(s->call_xi), s->stream);
-  s->st.launches += (int64_t)(nleap - from) * (1 + kRadixLaunches);
+  s->st.launches += (int64_t)(nleap - from) * (1 + radix_launches(s->n));
   s->st.substeps_compact += nleap - from;
   WG_CUDA(cudaStreamSynchronize(s->stream));
   return WG_OK;
@@ -1157,7 +1157,7 @@ static int run_call_begin(wg_sim* s, double dt, int nleap, double* t0, bool reco
     launch_bucketize(s->table, s->n, s->tune.target, s->nb, s->capg, s->E, s->bx[0], s->bv[0],
                      s->bm[0],
                      s->bi[0], s->bcnt, s->bmass, s->qk[0], s->qi[0], s->stream);
-    s->st.launches += 2 + kRadixLaunches;
+    s->st.launches += 2 + radix_launches(s->n);
     s->st.sorts_full += 1;
   } else {
     pre = dt / 2.;
@@ -1317,7 +1317,7 @@ static int run_call_end(wg_sim* s, double* time_elapsed) {
     s->lay = (lay0 + nleap) & 1;
     s->qsel = (qs0 + nleap) & 1;
     s->cslot = (cs0 + nleap) % kAggSlots;
-    s->st.launches += 4 + kRadixLaunches + (nleap - from);
+    s->st.launches += 4 + radix_launches(s->n) + (nleap - from);
     WG_CUDA(cudaGetLastError());
     rc = copy_back(s, nleap);
     if (rc) return rc;
@@ -1548,7 +1548,7 @@ int wg_profile(wg_sim* s, int what, int reps, double* avg_seconds) {
   float ms = 0;
   WG_CUDA(cudaEventElapsedTime(&ms, s->ev0, s->ev1));
   *avg_seconds = ms * 1e-3 / reps;
-  s->st.launches += what == WG_PROF_SORT ? (int64_t)reps * kRadixLaunches : reps;
+  s->st.launches += what == WG_PROF_SORT ? (int64_t)reps * radix_launches(s->n) : reps;
   if (what == WG_PROF_BUCKET) {
     // dt = 0 kept every sheet in place, but the layout is now routed by the
     // stored positions rather than by the pending half drift: hand the
@@ -1674,7 +1674,7 @@ int wg_energy(wg_sim* s, double twopiG, double omega2, double* energy, double* m
   s->ext = ext;
   if (rc) return rc;
   launch_energy(s->table, s->n, s->a_sorted, s->diag, s->stream);
-  s->st.launches += 3 + kRadixLaunches;
+  s->st.launches += 2;
   double sums[4];
   WG_CUDA(cudaMemcpyAsync(sums, s->diag, sizeof(sums), cudaMemcpyDeviceToHost, s->stream));
   rc = finish_call(s, 0, false);  // synchronises and checks the device error word

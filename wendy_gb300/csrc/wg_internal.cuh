@@ -194,8 +194,14 @@ void record_last_error(const char* msg);
 void host_pages_dirty(void* p, size_t bytes);
 
 // --- launchers (wg_radix.cu) ---
-constexpr int kRadixLaunches = 9;  // kernels radix_sort_state enqueues (hist, five passes,
-                                   // gather, ties, long ties)
+// Leading byte of a key that its sort begins with (whole keys: 0).
+inline int radix_first_byte(int64_t n, bool whole_keys) {
+  return whole_keys ? 0 : n <= kRadixFourSheets ? 4 : n <= kRadixFiveSheets ? 3 : 2;
+}
+// Kernels radix_sort_state enqueues (hist, a pass per byte, gather, ties, long ties).
+inline int radix_launches(int64_t n, bool whole_keys = false) {
+  return 4 + 8 - radix_first_byte(n, whole_keys);
+}
 size_t radix_bytes(int64_t n);
 void radix_bind(RadixWork* w, void* base, int64_t n);
 // Sort table->cur by (position key, original index) unless flags->unsorted

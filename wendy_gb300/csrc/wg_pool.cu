@@ -576,7 +576,7 @@ int to_buckets(wg_pool* p, PoolSim* s, double dt) {
   launch_bucketize(p->table, s->n, s->target, s->nb, s->capg, s->E, s->bx[0], s->bv[0],
                    s->bm[0],
                    s->bi[0], s->bcnt, s->bmass, s->qk[0], s->qi[0], p->stream);
-  p->launches += 3 + kRadixLaunches;
+  p->launches += 3 + radix_launches(s->n);
   s->lay = 0;
   s->qsel = 0;
   s->cslot = 0;
@@ -649,7 +649,7 @@ int finish_compact(wg_pool* p, PoolSim* s, int k, int kk, int lay, int cslot, do
   }
   launch_desort(p->table, s->n, s->x_out, s->v_out, p->stream);
   store_compact(p, s);
-  p->launches += (int64_t)(nleap - kk - 1) * (1 + kRadixLaunches) + 1;
+  p->launches += (int64_t)(nleap - kk - 1) * (1 + radix_launches(s->n)) + 1;
   s->mode = 0;
   return WG_OK;
 }
@@ -1178,12 +1178,12 @@ static int pool_step_end(wg_pool* p, double* time_elapsed) {
         k_seg_prep_b<<<grid_1d(sheets), 256, 0, p->stream>>>(p->btA, p->bseg_out, nseg,
                                                              p->bB[0], sheets, rank_bits);
         radix_sort_state(p->btB, sheets, &p->bradix, p->bflag, p->err, p->stream, true);
-        p->launches += 1 + kRadixLaunches;
+        p->launches += 1 + radix_launches(sheets, true);
       }
       k_seg_final<<<grid_1d(sheets), 256, 0, p->stream>>>(p->btA, nseg > 1 ? p->btB : nullptr,
                                                           p->bW, p->bO, sheets);
       launch_batch_bucketize(p->d_dev, p->bsegs, p->btasks, nbk, p->bO, sheets, p->stream);
-      p->launches += 7 + kRadixLaunches;
+      p->launches += 7 + radix_launches(sheets);
       j0 = j1;
     }
     // their sub-steps from the restart on: `from` reads layout 0, aggregate

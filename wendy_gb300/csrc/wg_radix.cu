@@ -1210,7 +1210,7 @@ void radix_sort_state(StateTable* table, int64_t n, RadixWork* w, const StepFlag
   const RadixDevCfg cfg = radix_cfg();
   const int sms = cfg.sms;
   // the least significant byte sorted by (kRadixFourSheets, kRadixFiveSheets)
-  const int first = whole_keys ? 0 : n <= kRadixFourSheets ? 4 : n <= kRadixFiveSheets ? 3 : 2;
+  const int first = radix_first_byte(n, whole_keys);
   // the workspace may be bound for more sheets than this sort has: tiles,
   // look-back words and launches follow n
   const int64_t tiles = tiles_of(n);
