@@ -281,15 +281,22 @@ int alloc_call_arrays(wg_sim* s, int nleap) {
     WG_CUDA(cudaStreamSynchronize(s->stream));
     WG_CUDA(cudaMemcpy(&t, s->table, sizeof(t), cudaMemcpyDeviceToHost));
   }
-  block_free(s->small);
-  host_block_free(s->h_small);
-  s->small = nullptr;
-  s->h_small = nullptr;
-  s->cap = 0;
   const size_t b = al(sizeof(StateTable)) + al(64) + al(sizeof(StepFlags) * (cap + 1)) +
                    al(4 * (size_t)cap) + al(8 * (size_t)cap) + al(4 * (size_t)cap) +
                    al(8 * (size_t)cap);
-  WG_CUDA(block_alloc(&s->small, b));
+  // (the old arrays go when there are new ones: where there is no room the
+  // simulation stays as it is)
+  void *dev = nullptr, *host = nullptr;
+  WG_CUDA(block_alloc(&dev, b));
+  const cudaError_t eh =
+      host_block_alloc(&host, 64 + 16 * (size_t)cap + sizeof(StepFlags) * (cap + 1));
+  if (eh != cudaSuccess) block_free(dev);
+  WG_CUDA(eh);
+  block_free(s->small);
+  host_block_free(s->h_small);
+  s->small = dev;
+  s->h_small = host;
+  s->cap = 0;
   char* p = static_cast<char*>(s->small);
   s->table = reinterpret_cast<StateTable*>(p); p += al(sizeof(StateTable));
   s->err = reinterpret_cast<unsigned*>(p); p += al(64);
@@ -301,7 +308,6 @@ int alloc_call_arrays(wg_sim* s, int nleap) {
   WG_CUDA(cudaMemsetAsync(s->small, 0, b, s->stream));
   WG_CUDA(cudaMemcpyAsync(s->table, &t, sizeof(t), cudaMemcpyHostToDevice, s->stream));
   // page-locked mirrors, one block
-  WG_CUDA(host_block_alloc(&s->h_small, 64 + 16 * (size_t)cap + sizeof(StepFlags) * (cap + 1)));
   char* h = static_cast<char*>(s->h_small);
   s->h_ab = reinterpret_cast<unsigned*>(h); h += 64;
   s->h_t = reinterpret_cast<double*>(h); h += 8 * (size_t)cap;
