@@ -89,12 +89,28 @@ int main() {
     CHECK(room == 1000 && live.size() == 1);  // kept
     if (k == 0) CHECK(device_alloc(&p, 2000) == cudaSuccess && cudaFree(p) == cudaSuccess);
     if (k == 1) CHECK(page_locked_alloc(&p, 2000) == cudaSuccess && cudaFreeHost(p) == cudaSuccess);
-    if (k == 2) CHECK(host_block_alloc(&p, 2000) == cudaSuccess && host_block_free(p));
+    if (k == 2) CHECK(host_block_alloc(&p, 2000) == cudaSuccess && host_block_free(p) == cudaSuccess);
     if (k == 3) blocks_trim();
     blocks_trim();
     CHECK(room == most && live.empty());
   }
   CHECK(device_alloc(&p, most + 1) == cudaErrorMemoryAllocation);
+  return 0;
+}
+"""
+
+TWICE = r"""
+int main() {
+  // a second release is refused, and what is kept stays intact
+  void *p = nullptr, *q = nullptr;
+  CHECK(host_block_alloc(&p, 5000) == cudaSuccess);
+  CHECK(host_block_free(p) == cudaSuccess);
+  CHECK(host_block_free(p) != cudaSuccess && live.count(p) == 1);
+  CHECK(host_block_alloc(&q, 5000) == cudaSuccess && q == p);
+  void* other = nullptr;
+  CHECK(cudaHostAlloc(&other, 5000, 0) == cudaSuccess);
+  CHECK(host_block_free(other) == cudaSuccess && live.count(other) == 0);
+  CHECK(host_block_free(q) == cudaSuccess && host_block_free(nullptr) == cudaSuccess);
   return 0;
 }
 """
@@ -119,6 +135,10 @@ def test_streams_stay_with_their_device(tmp_path):
 
 def test_kept_memory_is_given_back_before_an_allocation_fails(tmp_path):
     _run(tmp_path, ROOM)
+
+
+def test_a_second_release_is_refused(tmp_path):
+    _run(tmp_path, TWICE)
 
 
 def test_no_source_allocates_past_what_is_kept():

@@ -1648,7 +1648,7 @@ int wg_host_alloc(int64_t bytes, void** ptr) {
 
 int wg_host_free(void* ptr) {
   if (!ptr) return WG_OK;
-  if (!host_block_free(ptr)) WG_CUDA(cudaFreeHost(ptr));
+  WG_CUDA(host_block_free(ptr));
   return WG_OK;
 }
 

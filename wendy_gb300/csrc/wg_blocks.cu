@@ -134,7 +134,16 @@ cudaError_t block_alloc(void** p, size_t bytes) {
 void block_free(void* p) { give(p); }
 
 cudaError_t host_block_alloc(void** p, size_t bytes) { return alloc(-1, p, bytes); }
-bool host_block_free(void* p) { return give(p); }
+cudaError_t host_block_free(void* p) {
+  if (give(p)) return cudaSuccess;
+  Kept& k = kept();
+  {
+    std::lock_guard<std::mutex> lock(k.mu);
+    for (const Block& b : k.idle)
+      if (b.p == p) return cudaErrorInvalidValue;
+  }
+  return cudaFreeHost(p);
+}
 
 cudaError_t device_alloc(void** p, size_t bytes) { return fresh(false, p, bytes); }
 cudaError_t page_locked_alloc(void** p, size_t bytes) { return fresh(true, p, bytes); }

@@ -33,8 +33,9 @@ cudaError_t block_alloc(T** p, size_t bytes) {
 
 // Page-locked host memory.
 cudaError_t host_block_alloc(void** p, size_t bytes);
-// false: p is not from host_block_alloc.
-bool host_block_free(void* p);
+// An error if p was released already; memory page-locked by others is released as
+// cudaFreeHost does.
+cudaError_t host_block_free(void* p);
 template <typename T>
 cudaError_t host_block_alloc(T** p, size_t bytes) {
   return host_block_alloc(reinterpret_cast<void**>(p), bytes);
