@@ -77,8 +77,6 @@ __device__ __forceinline__ uint32_t bin_get(const uint32_t* bins, int b) {
 constexpr int SAMPLES = CAP / kSmallestTarget + 1;
 // Cells of the routing table over a splitter window (see route_table).
 constexpr int LUTN = 256;
-// Sheets a thread takes at once through the force loop.
-constexpr int FU = 1;
 
 struct LsdSmem {
   uint16_t p[CAP];           // the other slot permutation (S.perm is the first)
@@ -887,117 +885,94 @@ __device__ __forceinline__ bool process_bucket(const StepLaunch& L, StepSmem& S,
   // C_j the mass before it; from one sheet to the next A falls by M_j + M_j+1
   i128 A = (i128)(((((u128)D.T_hi) << 64) | D.T_lo) - 2 * C);
 #pragma unroll 1
-  for (int i0 = 0; i0 < nmine; i0 += FU) {
-    int sl[FU];
-    uint64_t kd[FU];
-    float xf[FU];
-    int32_t idv[FU];
-    bool live[FU];
-#pragma unroll
-    for (int u = 0; u < FU; ++u) {
-      live[u] = u == 0 || i0 + u < nmine;
-      sl[u] = S.perm[j0 + (live[u] ? i0 + u : i0)];
-      idv[u] = S.idx[sl[u]];
-    }
-#pragma unroll
-    for (int u = 0; u < FU; ++u) {
-      if (!live[u]) {
-        kd[u] = 0;
-        xf[u] = 0.f;
-        continue;
-      }
-      const int sidx = sl[u];
-      const uint32_t r = rank0 + (uint32_t)(i0 + u);
-      const double x = S.x[sidx], v = S.v[sidx];
-      if (r == rnext) {
-        qnk[qnext] = key_of(x);
-        qni[qnext] = idv[u];
-        if (ptab) {
-          const unsigned k = atomicAdd(&S.nsamp, 1u);
-          if (k < (unsigned)SAMPLES) {
-            S.samp_x[k] = x;
-            S.samp_idx[k] = idv[u];
-            S.samp_q[k] = qnext;
-          }
+  for (int i = 0; i < nmine; ++i) {
+    const int sidx = S.perm[j0 + i];
+    const int32_t idv = S.idx[sidx];
+    const uint32_t r = rank0 + (uint32_t)i;
+    const double x = S.x[sidx], v = S.v[sidx];
+    if (r == rnext) {
+      qnk[qnext] = key_of(x);
+      qni[qnext] = idv;
+      if (ptab) {
+        const unsigned k = atomicAdd(&S.nsamp, 1u);
+        if (k < (unsigned)SAMPLES) {
+          S.samp_x[k] = x;
+          S.samp_idx[k] = idv;
+          S.samp_q[k] = qnext;
         }
       }
-      const u128 M = eq ? Meq : mass_to_fixed(S.m[sidx], E);
-      A -= (i128)M;
-      double acc = fixed_to_double(A, E);
-      A -= (i128)M;
-      if (has_omega) acc = fma(-omega2, x, acc);
-      if constexpr (FORCE == kForceExpr) {
-        if (ext.kind == EXT_EXPR)
-          acc = expr_space(ext, xr, x, t_ev) + acc;
-        else if (ext.kind != EXT_NONE)
-          acc = ext_force_at(ext, S.amp, S.inv_h, x) + acc;
-      } else if (FORCE == kForceClosed && ext.kind != EXT_NONE) {
+    }
+    const u128 M = eq ? Meq : mass_to_fixed(S.m[sidx], E);
+    A -= (i128)M;
+    double acc = fixed_to_double(A, E);
+    A -= (i128)M;
+    if (has_omega) acc = fma(-omega2, x, acc);
+    if constexpr (FORCE == kForceExpr) {
+      if (ext.kind == EXT_EXPR)
+        acc = expr_space(ext, xr, x, t_ev) + acc;
+      else if (ext.kind != EXT_NONE)
         acc = ext_force_at(ext, S.amp, S.inv_h, x) + acc;
-      }
-      const double vn = fma(dt, acc, v);
-      const double xn = fma(dt_drift, vn, x);
-      S.x[sidx] = xn;
-      S.v[sidx] = vn;
+    } else if (FORCE == kForceClosed && ext.kind != EXT_NONE) {
+      acc = ext_force_at(ext, S.amp, S.inv_h, x) + acc;
+    }
+    const double vn = fma(dt, acc, v);
+    const double xn = fma(dt_drift, vn, x);
+    S.x[sidx] = xn;
+    S.v[sidx] = vn;
 
-      const unsigned long long av =
-          (unsigned long long)__double_as_longlong(vn) & 0x7FFFFFFFFFFFFFFFull;
-      maxv = av > maxv ? av : maxv;
-      if (LAST && !L.profile) {
-        OutRec* const ro = D.rec_out;
-        if (ro) {
-          double2* const r2 = reinterpret_cast<double2*>(ro + idv[u]);
-          r2[0] = make_double2(xn, vn);
-          r2[1] = make_double2(acc, 0.0);
-        } else {
-          D.x_out[idv[u]] = xn;
-          D.v_out[idv[u]] = vn;
-          double* const a_out = D.a_out;
-          if (a_out) a_out[idv[u]] = acc;
-        }
-        SheetRec* const xi_out = D.xi_out;
-        if (xi_out) {
-          SheetRec rec;
-          rec.idx = idv[u];
-          rec.pad = 0;
-          rec.val = xn;
-          xi_out[r] = rec;
-        }
+    const unsigned long long av =
+        (unsigned long long)__double_as_longlong(vn) & 0x7FFFFFFFFFFFFFFFull;
+    maxv = av > maxv ? av : maxv;
+    if (LAST && !L.profile) {
+      OutRec* const ro = D.rec_out;
+      if (ro) {
+        double2* const r2 = reinterpret_cast<double2*>(ro + idv);
+        r2[0] = make_double2(xn, vn);
+        r2[1] = make_double2(acc, 0.0);
+      } else {
+        D.x_out[idv] = xn;
+        D.v_out[idv] = vn;
+        double* const a_out = D.a_out;
+        if (a_out) a_out[idv] = acc;
       }
-      const double xd = LAST && dest_dt != 0.0 ? fma(dest_dt, vn, xn) : xn;
-      kd[u] = key_of(xd);
-      xf[u] = float_of_pos(xd);
+      SheetRec* const xi_out = D.xi_out;
+      if (xi_out) {
+        SheetRec rec;
+        rec.idx = idv;
+        rec.pad = 0;
+        rec.val = xn;
+        xi_out[r] = rec;
+      }
     }
+    const double xd = LAST && dest_dt != 0.0 ? fma(dest_dt, vn, xn) : xn;
     // routing: the window entry among the table's candidates
-#pragma unroll
-    for (int u = 0; u < FU; ++u) {
-      if (!live[u]) continue;
-      const int c = lut_cell(xf[u], lut_x0, lut_scale);
-      int a = S.lut[c], z = S.lut[c + 1];
-      // a position in an end cell may lie outside the window (or on its end):
-      // unless it is strictly inside, its bucket is found by the search over
-      // all splitters where it is needed.  The cells between lie inside.
-      bool inw = true;
-      if (c == 0 || c == LUTN - 1) inw = kd[u] > wk[0] && kd[u] < wk[wlen];
-      // the largest entry with key Q <= key (entry a of the table lies below
-      // the position's cell); then splitters with an equal key and a larger
-      // index step back (pair order)
-      bool eq = false;
-      while (a < z) {
-        const int mid = (a + z + 1) >> 1;
-        const uint64_t K = wk[mid];
-        if (K <= kd[u]) {
-          a = mid;
-          eq = K == kd[u];
-        } else {
-          z = mid - 1;
-        }
+    const uint64_t kd = key_of(xd);
+    const int c = lut_cell(float_of_pos(xd), lut_x0, lut_scale);
+    int a = S.lut[c], z = S.lut[c + 1];
+    // a position in an end cell may lie outside the window (or on its end):
+    // unless it is strictly inside, its bucket is found by the search over
+    // all splitters where it is needed.  The cells between lie inside.
+    bool inw = true;
+    if (c == 0 || c == LUTN - 1) inw = kd > wk[0] && kd < wk[wlen];
+    // the largest entry with key Q <= key (entry a of the table lies below
+    // the position's cell); then splitters with an equal key and a larger
+    // index step back (pair order)
+    bool tie = false;
+    while (a < z) {
+      const int mid = (a + z + 1) >> 1;
+      const uint64_t K = wk[mid];
+      if (K <= kd) {
+        a = mid;
+        tie = K == kd;
+      } else {
+        z = mid - 1;
       }
-      if (eq)
-        while (a > 0 && wk[a] == kd[u] && wi[a] > idv[u]) --a;
-      // destination: window entry a, or wlen for a bucket outside the window
-      const int w = inw ? a : wlen;
-      S.u.dest[j0 + i0 + u] = ((uint32_t)w << 16) | atomicAdd(&S.dcount[w], 1u);
     }
+    if (tie)
+      while (a > 0 && wk[a] == kd && wi[a] > idv) --a;
+    // destination: window entry a, or wlen for a bucket outside the window
+    const int w = inw ? a : wlen;
+    S.u.dest[j0 + i] = ((uint32_t)w << 16) | atomicAdd(&S.dcount[w], 1u);
   }
   if (ptab) {
     // the new velocities of this thread's sheets (back from shared memory:
@@ -1249,6 +1224,7 @@ __device__ __forceinline__ void process_big(const StepLaunch& L, StepSmem& S, co
   const double* gm = bt.m;
   const int32_t* gi = bt.idx;
   const double pre = sub == 0 ? D.pre_dt : 0.0;
+  const bool eq = MASS == kMassMixed ? bt.eq != 0 : MASS == kMassEqual;
   // the splitter window of the next layout around the bucket
   {
     const int qs = (D.qsel0 + sub) & 1;
@@ -1354,7 +1330,7 @@ __device__ __forceinline__ void process_big(const StepLaunch& L, StepSmem& S, co
         if (slot < (unsigned)CAP) {
           S.x[slot] = x;
           S.v[slot] = gv[j];
-          S.m[slot] = gm[j];
+          if (!eq) S.m[slot] = gm[j];
           S.idx[slot] = gi[j];
         }
       }
