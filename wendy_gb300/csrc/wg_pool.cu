@@ -544,9 +544,9 @@ void set_layout(PoolSim* s, const MemberLayout& l) {
 // CTAs idle, as for single simulations (balanced_target).  Then all members
 // take buckets of about the size that fills the launch, down to kMinTarget sheets,
 // as far as their slots allow (member_layout).
-// Measured per output of 20 sub-steps (5): 4 members of 500 .. 20000 sheets 418 us
-// (175) against 733 (254) with tuned buckets in the kernel before it, 64 of
-// 1000 .. 20000 1240 (580) against 1420 (625).
+// Measured per step of 20 sub-steps (5): 4 members of 500 .. 20000 sheets 301 us
+// (121) against 545 (185) with tuned buckets, 64 of 1000 .. 20000 699 (228) against 760
+// (243), 400 of 1200 734 (272) against 744 (276).
 void balance_targets(wg_pool* p, const std::vector<PoolSim*>& act) {
   int64_t sheets = 0, buckets = 0;
   for (const PoolSim* s : act) {
